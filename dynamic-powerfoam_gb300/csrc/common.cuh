@@ -36,6 +36,19 @@ __device__ __forceinline__ d3 cross(d3 a, d3 b) {
     return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
 }
 __device__ __forceinline__ double norm(d3 a) { return sqrt(dot(a, a)); }
+// acc + a x b and acc - a x b in six fused multiply-adds (the sum of a product
+// and a vector written out costs nine operations).
+__device__ __forceinline__ d3 cross_add(d3 acc, d3 a, d3 b) {
+    return {fma(a.y, b.z, fma(-a.z, b.y, acc.x)), fma(a.z, b.x, fma(-a.x, b.z, acc.y)),
+            fma(a.x, b.y, fma(-a.y, b.x, acc.z))};
+}
+__device__ __forceinline__ d3 cross_sub(d3 acc, d3 a, d3 b) { return cross_add(acc, b, a); }
+__device__ __forceinline__ double dot_add(double acc, d3 a, d3 b) {
+    return fma(a.x, b.x, fma(a.y, b.y, fma(a.z, b.z, acc)));
+}
+__device__ __forceinline__ d3 axpy(double s, d3 a, d3 b) {
+    return {fma(s, a.x, b.x), fma(s, a.y, b.y), fma(s, a.z, b.z)};
+}
 
 __device__ __forceinline__ d3 ld3(const double *p) { return {p[0], p[1], p[2]}; }
 __device__ __forceinline__ d3 ld3(const double *p, int64_t i) { return ld3(p + 3 * i); }
@@ -76,6 +89,135 @@ __device__ __forceinline__ d3 apply(const Transport &t, d3 v) {
     return t.c * out + t.s * cross(t.n1, out) + ((1.0 - t.c) * dot(t.n1, out)) * t.n1;
 }
 
+// ---- the same transport for unit normals, with few float64 operations --------
+//
+// The float64 bond passes are bound by the float64 pipe (two lanes per SM and
+// clock: about 3.1 us per operation and bond at 2M bonds, against 2.3 us to
+// read eight bytes per bond), so what they gain is operations left out.  With
+// |n0| = |n1| = 1 the shortest-arc rotation is the unit quaternion
+// r (1 + c, n0 x n1), r = 1/sqrt(2 + 2 c), c = n0 . n1; followed by the spin
+// about n1 by the angle r spin.(n0 + n1) it is
+//   w = r cos(h) (1 + c),  v = r (cos(h) n0 x n1 + sin(h) (n0 + n1)),
+// h half that angle, because n1 x (n0 x n1) = n0 - c n1.  One reciprocal root
+// and two short series instead of a root, two divisions and a sincos, and 15
+// operations a rotated vector instead of 37.
+
+struct Turn {
+    double w;
+    d3 v, v2;        // vector part and twice it
+    d3 sum;          // n0 + n1
+    double r, half, sh, ch;
+};
+
+// sin h and cos h: Maclaurin series for |h| < 0.25 (relative truncation below
+// 1e-17 and 2e-17 there; the rotation guard keeps a step's |h| below 0.125).
+__device__ __forceinline__ void sincos_small(double h, double &s, double &c) {
+    if (fabs(h) < 0.25) {
+        const double q = h * h;
+        double a = -1.0 / 39916800.0;               // 1/11!
+        a = fma(a, q, 1.0 / 362880.0);              // 1/9!
+        a = fma(a, q, -1.0 / 5040.0);               // 1/7!
+        a = fma(a, q, 1.0 / 120.0);                 // 1/5!
+        a = fma(a, q, -1.0 / 6.0);                  // 1/3!
+        s = fma(a * q, h, h);
+        double b = 1.0 / 479001600.0;               // 1/12!
+        b = fma(b, q, -1.0 / 3628800.0);            // 1/10!
+        b = fma(b, q, 1.0 / 40320.0);               // 1/8!
+        b = fma(b, q, -1.0 / 720.0);                // 1/6!
+        b = fma(b, q, 1.0 / 24.0);                  // 1/4!
+        b = fma(b, q, -0.5);
+        c = fma(b, q, 1.0);
+    } else {
+        sincos(h, &s, &c);
+    }
+}
+
+// A normal that geometry() formed has |n|^2 = 1 within a few 1e-16.
+__device__ __forceinline__ bool is_unit(d3 n) { return fabs(dot(n, n) - 1.0) < 1e-12; }
+
+// All three numbers are +0 or -0 (integer tests: the float64 pipe is the scarce one).
+__device__ __forceinline__ bool is_zero(d3 a) {
+    return ((__double_as_longlong(a.x) | __double_as_longlong(a.y) | __double_as_longlong(a.z)) << 1) == 0;
+}
+
+__device__ __forceinline__ Turn make_turn(d3 n0, d3 n1, d3 spin, int &flags) {
+    Turn t;
+    const double c = dot(n0, n1);
+    if (!(c >= kCosQuarter)) flags |= DPF_ERR_NORMAL_TURN;
+    t.sum = n0 + n1;
+    t.r = rsqrt(2.0 + 2.0 * c);
+    t.half = 0.5 * t.r * dot(spin, t.sum);
+    sincos_small(t.half, t.sh, t.ch);
+    const double rc = t.r * t.ch, rs = t.r * t.sh;
+    t.w = rc + rc * c;
+    t.v = axpy(rs, t.sum, rc * cross(n0, n1));
+    t.v2 = t.v + t.v;
+    return t;
+}
+
+__device__ __forceinline__ d3 apply(const Turn &t, d3 a) {
+    const d3 x = cross(t.v2, a);
+    return cross_add(axpy(t.w, x, a), t.v, x);
+}
+
+// Angular velocity of the transport when its normal moves by dn and its spin
+// by dspin: d(R a) = omega x (R a) for every vector a.  The shortest-arc
+// rotation is a half turn about the committed normal followed by one about
+// the middle of the two normals, so it turns with (n0 + n) x dn / (1 + c);
+// the spin by the angle th about n adds th' n + sin(th) dn +
+// (1 - cos(th)) n x dn and rotates the former.
+__device__ __forceinline__ d3 turn_rate(const Turn &t, d3 n, d3 dn, d3 spin, d3 dspin) {
+    const double sine = 2.0 * t.sh * t.ch, versine = 2.0 * t.sh * t.sh;
+    const d3 arc = (2.0 * t.r * t.r) * cross(t.sum, dn);
+    const double dth = t.r * dot_add(dot_add(-(2.0 * t.half * t.r) * dot(t.sum, dn), spin, dn), dspin, t.sum);
+    const d3 side = axpy(sine, arc, versine * cross_add(dn, n, arc));
+    return cross_add(axpy(dth, n, axpy(sine, dn, arc)), n, side);
+}
+
+// Normal turns more than 0.25 rad (or is not a number) from unit n to the
+// direction of d: n . d >= cos(0.25) |d| without forming |d|.
+__device__ __forceinline__ bool turned(d3 n, d3 d, double d2) {
+    const double c = dot(n, d);
+    return !(c > 0.0 && c * c >= (kCosQuarter * kCosQuarter) * d2);
+}
+
+// Wrench [F_i, T_i, T_j] of the frozen tangent on one bond (F_j = -F_i):
+// du = u_j - u_i + w_j x r_j - w_i x r_i, dw = w_j - w_i,
+// f = ks du + (kn - ks)(du.n) n, m likewise of dw; F_i = -f,
+// T_i = -(r_i x f) - m, T_j = r_j x f + m.  52 float64 operations.
+struct Wrench {
+    d3 f, ti, tj;
+};
+
+__device__ __forceinline__ Wrench stiffness_wrench(d3 n, d3 ri, d3 rj, double kn, double ks, double kb, double kt,
+                                                   const double *qi, const double *qj) {
+    const d3 wi = ld3(qi + 3), wj = ld3(qj + 3);
+    const d3 du = cross_sub(cross_add(ld3(qj) - ld3(qi), wj, rj), wi, ri);
+    const d3 dw = wj - wi;
+    const d3 f = axpy((kn - ks) * dot(du, n), n, ks * du);
+    const d3 m = axpy((kt - kb) * dot(dw, n), n, kb * dw);
+    return {-f, cross_add(-m, f, ri), cross_add(m, rj, f)};
+}
+
+// A warp's 32 consecutive wrenches (bonds first, first + 1, ..; `count` of
+// them exist) to memory through the warp's 288 doubles of shared memory, in
+// consecutive addresses: stored by the lanes one number at a time, at a stride
+// of 72 bytes, every store instruction touched 32 sectors of L2.
+__device__ __forceinline__ void store_wrenches(double *wrench, int64_t first, int count, const Wrench &w,
+                                               double *stage) {
+    const int lane = threadIdx.x & 31;
+    double *p = stage + 9 * lane;
+    st3(p, w.f);
+    st3(p + 3, w.ti);
+    st3(p + 6, w.tj);
+    __syncwarp();
+    double *out = wrench + 9 * first;
+#pragma unroll
+    for (int k = 0; k < 9; ++k)
+        if (32 * k + lane < 9 * count) out[32 * k + lane] = stage[32 * k + lane];
+    __syncwarp();
+}
+
 // Sum over the incidences of site s of the bond wrenches [F, T_i, T_j]
 // (nine doubles per bond; the j end receives (-F, T_j)), in incidence order.
 __device__ __forceinline__ void gather_wrench(const int32_t *__restrict__ ptr, const int32_t *__restrict__ inc,
@@ -101,9 +243,67 @@ __device__ __forceinline__ void gather_wrench(const int32_t *__restrict__ ptr, c
     }
 }
 
+// Half of gather_wrench: the force (part 0) or the torque (part 1) of site s,
+// for site passes that give a site two neighbouring lanes.  The same sums in
+// the same order; the sign and the place of the end's three numbers are
+// chosen without a branch so that the loads of several incidences are in
+// flight together, and the site's other work is split by rows of its 6x6
+// block.  Reads `w` with plain loads when the caller's launch writes it too.
+template <bool kConst = true>
+__device__ __forceinline__ d3 gather_half(const int32_t *__restrict__ ptr, const int32_t *__restrict__ inc,
+                                          const double *w, int64_t s, int part) {
+    d3 acc = mk(0.0, 0.0, 0.0);
+    const int e1 = ptr[s + 1];
+#pragma unroll 4
+    for (int e = ptr[s]; e < e1; ++e) {
+        const int v = inc[e];
+        const int j = v >> 31;               // 0: i end, -1: j end
+        const double *p = w + 9 * (int64_t)(v ^ j) + (part ? 3 - 3 * j : 0);
+        const unsigned long long flip = part ? 0ull : (unsigned long long)((unsigned)j & 0x80000000u) << 32;
+        const double x = kConst ? __ldg(p) : p[0], y = kConst ? __ldg(p + 1) : p[1], z = kConst ? __ldg(p + 2) : p[2];
+        acc.x += __longlong_as_double(__double_as_longlong(x) ^ (long long)flip);
+        acc.y += __longlong_as_double(__double_as_longlong(y) ^ (long long)flip);
+        acc.z += __longlong_as_double(__double_as_longlong(z) ^ (long long)flip);
+    }
+    return acc;
+}
+
+// The other lane's half of a site vector (lanes 2k and 2k + 1 share a site;
+// both call it), and this lane's three rows of a 6x6 block times the vector
+// whose halves are `own` and `other`.
+__device__ __forceinline__ d3 other_half(d3 a) {
+    return mk(__shfl_xor_sync(0xffffffffu, a.x, 1), __shfl_xor_sync(0xffffffffu, a.y, 1),
+              __shfl_xor_sync(0xffffffffu, a.z, 1));
+}
+
+__device__ __forceinline__ d3 half_rows(const double *__restrict__ P, int part, d3 own, d3 other) {
+    const d3 lo = part ? other : own, hi = part ? own : other;
+    double r[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const double *row = P + 18 * part + 6 * c;
+        double v = row[0] * lo.x;
+        v += row[1] * lo.y;
+        v += row[2] * lo.z;
+        v += row[3] * hi.x;
+        v += row[4] * hi.y;
+        v += row[5] * hi.z;
+        r[c] = v;
+    }
+    return mk(r[0], r[1], r[2]);
+}
+
+// a / u for one half of a site's units: [r, r, r] or [1, 1, 1] in every solver
+// of this library, so one division instead of three, or none.
+__device__ __forceinline__ d3 over_units(d3 a, d3 u) {
+    if (u.x == u.y && u.x == u.z) return u.x == 1.0 ? a : (1.0 / u.x) * a;
+    return mk(a.x / u.x, a.y / u.y, a.z / u.z);
+}
+
 // Inverse of a symmetric positive definite 6x6 matrix via Cholesky
 // (A = L L^T, A^-1 = L^-T L^-1), fully unrolled into registers: every loop
-// has a constant trip count so all indices fold.
+// has a constant trip count so all indices fold.  L's diagonal is kept as
+// its reciprocal.
 __device__ __forceinline__ void spd_inverse6(const double A[36], double P[36]) {
     double L[36];
 #pragma unroll
@@ -114,9 +314,10 @@ __device__ __forceinline__ void spd_inverse6(const double A[36], double P[36]) {
 #pragma unroll
         for (int kk = 0; kk < 6; ++kk)
             if (kk < jj) s -= L[6 * jj + kk] * L[6 * jj + kk];
-        const double ljj = sqrt(s);
-        L[6 * jj + jj] = ljj;
-        const double inv = 1.0 / ljj;
+        // only the reciprocal of the diagonal is used: one reciprocal root
+        // instead of a root and two divisions
+        const double inv = rsqrt(s);
+        L[6 * jj + jj] = inv;
 #pragma unroll
         for (int ii = 0; ii < 6; ++ii) {
             if (ii > jj) {
@@ -133,7 +334,7 @@ __device__ __forceinline__ void spd_inverse6(const double A[36], double P[36]) {
     for (int c = 0; c < 36; ++c) W[c] = 0.0;
 #pragma unroll
     for (int ii = 0; ii < 6; ++ii) {
-        W[6 * ii + ii] = 1.0 / L[6 * ii + ii];
+        W[6 * ii + ii] = L[6 * ii + ii];
 #pragma unroll
         for (int jj = 0; jj < 6; ++jj) {
             if (jj < ii) {
