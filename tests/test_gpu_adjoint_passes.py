@@ -1,0 +1,94 @@
+"""The adjoint's bond passes against torch.autograd of the same trial written in
+torch (float64, CPU): input adjoints for given output adjoints, and the local
+Jacobians through <lam, J d> = <J^T lam, d>, on graphs whose bond counts
+straddle warps and blocks, with classical and given contacts, committed normals
+that are unit vectors and not.  The derivatives are sums of a few hundred
+products of order one: 1e-10 relative."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from tests.helpers import host
+from tests.test_gpu_float64_passes import DT, _pair
+
+pytestmark = pytest.mark.gpu
+
+
+def _carry(torch, n0, n1, spin, v):
+    cross = lambda a, b: torch.linalg.cross(a, b, dim=1)
+    dot = lambda a, b: (a*b).sum(1, keepdim=True)
+    k, c = cross(n0, n1), dot(n0, n1).clamp(-1, 1)
+    b = n0 + n1
+    angle = dot(spin, b/torch.linalg.vector_norm(b, dim=1, keepdim=True).clamp_min(1e-12))
+    v = v + cross(k, v) + cross(k, cross(k, v))/(1 + c)
+    return torch.cos(angle)*v + torch.sin(angle)*cross(n1, v) + (1 - torch.cos(angle))*dot(n1, v)*n1
+
+
+def _trial(torch, cpu, y, x, normal, offset, fn, fs, mt, mb, k):
+    """Wrenches [F, T_i, T_j] and end history [normal, offset, fn, fs, mt, mb] of every bond."""
+    cross = lambda a, b: torch.linalg.cross(a, b, dim=1)
+    dot = lambda a, b: (a*b).sum(1, keepdim=True)
+    i, j = torch.as_tensor(cpu.i), torch.as_tensor(cpu.j)
+    rad = torch.as_tensor(.5*(cpu.radii[cpu.i] - cpu.radii[cpu.j]))[:, None]
+    unit = lambda d: d/torch.linalg.vector_norm(d, dim=1, keepdim=True)
+    u, w = y[:, :3], y[:, 3:]
+    mid, end = x + .5*u, x + u
+    n, ne = unit(mid[j] - mid[i]), unit(end[j] - end[i])
+    spin = .25*(w[i] + w[j])
+    off, fs0, mb0 = (_carry(torch, normal, n, spin, a) for a in (offset, fs, mb))
+    contact = .5*(mid[i] + mid[j]) + rad*n + off
+    ri, rj = contact - mid[i], contact - mid[j]
+    du, dw = u[j] - u[i] + cross(w[j], rj) - cross(w[i], ri), w[j] - w[i]
+    dn, tw = dot(du, n), dot(dw, n)
+    fn1, mt1 = fn[:, None] + k[:, :1]*dn, mt[:, None] + k[:, 3:]*tw
+    fs1, mb1 = fs0 + k[:, 1:2]*(du - dn*n), mb0 + k[:, 2:3]*(dw - tw*n)
+    f, c = .5*(fn[:, None] + fn1)*n + .5*(fs0 + fs1), .5*(mt[:, None] + mt1)*n + .5*(mb0 + mb1)
+    wrench = torch.cat((f, cross(ri, f) + c, -cross(rj, f) - c), 1)
+    return wrench, torch.cat((ne, _carry(torch, n, ne, spin, off), fn1, _carry(torch, n, ne, spin, fs1), mt1,
+                              _carry(torch, n, ne, spin, mb1)), 1)
+
+
+@pytest.mark.parametrize('n,m', [(2, 1), (17, 33), (65, 255)])
+@pytest.mark.parametrize('contacts,unit', [(False, True), (True, True), (True, False)])
+@pytest.mark.parametrize('end', [False, True])
+def test_input_adjoints_and_transposed_product(n, m, contacts, unit, end):
+    import torch
+    from dpf_gb300 import _lib
+    gpu, cpu, rng = _pair(n, m, contacts, unit, seed=n)
+    t = lambda a: torch.as_tensor(np.array(a, dtype=np.float64))
+    y = rng.normal(0, .02, (n, 6))
+    inputs = [t(a).requires_grad_(True) for a in (
+        y, cpu.x, cpu.normal, cpu.offset, cpu.fn, cpu.fs, cpu.mt, cpu.mb,
+        np.stack((cpu.kn, cpu.ks, cpu.kb, cpu.kt), 1))]
+    lam, end_bar, coef = rng.normal(size=(n, 6)), rng.normal(size=(m, 14)), .7
+    wrench, history = _trial(torch, cpu, *inputs)
+    i, j = cpu.i, cpu.j
+    wrench_bar = coef*np.concatenate((lam[i, :3] - lam[j, :3], lam[i, 3:], lam[j, 3:]), 1)
+    total = (wrench*t(wrench_bar)).sum() + ((history*t(end_bar)).sum() if end else 0.)
+    want = torch.autograd.grad(total, inputs, allow_unused=True)
+
+    lib, g = _lib.load(), gpu.tensor
+    hist, stiff, y_bar, x_bar = (torch.zeros(s, dtype=torch.float64, device=gpu.device)
+                                 for s in ((m, 14), (m, 4), (n, 6), (n, 3)))
+    slots = torch.empty(lib.dpf_adjoint_slot_doubles(m), dtype=torch.float64, device=gpu.device)
+    y_d, lam_d, end_d = g(y), g(lam), g(end_bar)
+    args = (ctypes.byref(gpu._graph), ctypes.byref(gpu._stiffness_struct()), ctypes.byref(gpu._history_struct()))
+    _lib.call('dpf_adjoint_bond_vjp', *args, y_d.data_ptr(), lam_d.data_ptr(), coef,
+              end_d.data_ptr() if end else None, 1, hist.data_ptr(), stiff.data_ptr(), y_bar.data_ptr(),
+              x_bar.data_ptr(), slots.data_ptr(), gpu._stream())
+    got = [y_bar, x_bar, hist[:, 0:3], hist[:, 3:6], hist[:, 6], hist[:, 7:10], hist[:, 10], hist[:, 11:14], stiff]
+    for name, a, b in zip(('y', 'x', 'normal', 'offset', 'fn', 'fs', 'mt', 'mb', 'k'), got, want):
+        assert np.linalg.norm(host(a) - b.numpy()) <= 1e-10*max(1., float(b.norm())), name
+
+    jac = torch.empty(lib.dpf_adjoint_jacobian_doubles(m), dtype=torch.float64, device=gpu.device)
+    _lib.call('dpf_adjoint_local_jacobian', *args, y_d.data_ptr(), jac.data_ptr(), gpu._stream())
+    lam[cpu.fixed] = 0.
+    lam_d, out = g(lam), torch.empty((n, 6), dtype=torch.float64, device=gpu.device)
+    _lib.call('dpf_adjoint_apply_jt', ctypes.byref(gpu._graph), jac.data_ptr(), gpu.mass.data_ptr(),
+              gpu.fixed.data_ptr(), DT, lam_d.data_ptr(), out.data_ptr(), slots.data_ptr(), gpu._stream())
+    d = rng.normal(size=(n, 6))
+    d[cpu.fixed] = 0.
+    left, right = (lam*cpu.jacobian_vector(y, d, DT, None)).sum(), (host(out)*d).sum()
+    scale = np.linalg.norm(lam)*np.linalg.norm(cpu.jacobian_vector(y, d, DT, None))
+    assert abs(left - right) <= 1e-10*scale
