@@ -172,6 +172,8 @@ SIGNATURES = {
                                    P(ParallelState), vp, vp, vp, vp]),
     'dpf_parallel_loads': (i32, [P(Graph), vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]),
     'dpf_bond_energy': (i32, [P(Graph), vp, vp, i64, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]),
+    'dpf_bond_energy_sites': (i32, [P(Graph), vp, vp, i64, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]),
+    'dpf_energy_site_doubles': (i64, [i64]),
     'dpf_energy_tangent': (i32, [P(Graph), vp, vp, i64, vp, vp, vp, vp, vp, vp]),
     'dpf_adjoint_jacobian_doubles': (i64, [i64]),
     'dpf_adjoint_slot_doubles': (i64, [i64]),
@@ -220,7 +222,7 @@ KERNELS = {
     'dpf_segment_axpy': 1, 'dpf_segment_select': 1,
     'dpf_adjoint_local_jacobian': 1, 'dpf_adjoint_apply_jt': 2, 'dpf_adjoint_bond_vjp': 2,
     'dpf_tile_pack': 2, 'dpf_tiled_hvp': 1, 'dpf_tiled_precondition': 1, 'dpf_end_pack': 2, 'dpf_end_hvp': 1,
-    'dpf_end_precondition': 1, 'dpf_bond_energy': 3, 'dpf_parallel_advance': 2, 'dpf_parallel_loads': 2,
+    'dpf_end_precondition': 1, 'dpf_bond_energy': 3, 'dpf_bond_energy_sites': 4, 'dpf_parallel_advance': 2, 'dpf_parallel_loads': 2,
     'dpf_energy_tangent': 1, 'dpf_operator_apply': 2, 'dpf_block_inverse': 1, 'dpf_block_pcg': 1, 'dpf_linear_midpoint_rhs': 1, 'dpf_linear_midpoint_advance': 1,
     'dpf_linear_sums': 1, 'dpf_anderson_gram': 1, 'dpf_anderson_mix': 1, 'dpf_barrier_selftest': 1,
     'dpf_end_precondition_f32': 1, 'dpf_mixed_jacobian_vector_f32': 3, 'dpf_arnoldi_cgs2_f32': 1,

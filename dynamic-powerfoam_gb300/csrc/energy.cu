@@ -27,9 +27,55 @@ __device__ __forceinline__ M3 quat_matrix(const double *q) {
 }
 __device__ __forceinline__ d3 mul(const M3 &R, d3 v) { return mk(dot(R.r0, v), dot(R.r1, v), dot(R.r2, v)); }
 // R^T v
-__device__ __forceinline__ d3 tmul(const M3 &R, d3 v) { return v.x * R.r0 + v.y * R.r1 + v.z * R.r2; }
+__device__ __forceinline__ d3 tmul(const M3 &R, d3 v) { return axpy(v.z, R.r2, axpy(v.y, R.r1, v.x * R.r0)); }
+__device__ __forceinline__ d3 tmul_add(d3 acc, const M3 &R, d3 v) {
+    return axpy(v.z, R.r2, axpy(v.y, R.r1, axpy(v.x, R.r0, acc)));
+}
 __device__ __forceinline__ d3 col(const M3 &R, int c) {
     return c == 0 ? mk(R.r0.x, R.r1.x, R.r2.x) : c == 1 ? mk(R.r0.y, R.r1.y, R.r2.y) : mk(R.r0.z, R.r1.z, R.r2.z);
+}
+
+// Site records (kSite doubles, 16-byte aligned): the rows of R, exp(theta/2) of
+// the four multipliers, and 1 when these products are safe from overflow.
+// Formed once a site instead of once an end: a bond's rotation matrices and
+// four exponentials were 140 of its 380 float64 operations.
+constexpr int kSite = 14;
+
+__global__ void __launch_bounds__(kThreads) energy_sites_kernel(int64_t n, const double *q, const double *theta,
+                                                                int64_t theta_stride, double *site) {
+    const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (s >= n) return;
+    const M3 R = quat_matrix(q + 4 * s);
+    double *out = site + kSite * s;
+    st3(out, R.r0);
+    st3(out + 3, R.r1);
+    st3(out + 6, R.r2);
+    double safe = 1.0;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const double t = theta[theta_stride * s + c];
+        out[9 + c] = exp(0.5 * t);
+        if (!(fabs(t) < 600.0)) safe = 0.0;
+    }
+    out[13] = safe;
+}
+
+struct SiteRecord {
+    M3 R;
+    double e[4], safe;
+};
+
+__device__ __forceinline__ SiteRecord load_site(const double *site, int64_t s) {
+    const double2 *p = reinterpret_cast<const double2 *>(site + kSite * s);
+    double v[kSite];
+#pragma unroll
+    for (int c = 0; c < kSite / 2; ++c) {
+        const double2 d = __ldg(p + c);
+        v[2 * c] = d.x;
+        v[2 * c + 1] = d.y;
+    }
+    return SiteRecord{{mk(v[0], v[1], v[2]), mk(v[3], v[4], v[5]), mk(v[6], v[7], v[8])},
+                      {v[9], v[10], v[11], v[12]}, v[13]};
 }
 
 struct BondArgs {
@@ -38,50 +84,68 @@ struct BondArgs {
     const double *base, *theta;
     int64_t theta_stride;
     const double *x, *q, *n0, *ri, *rj;
-    double *wrench;    // 9 per bond or null
-    double *partials;  // per-block energy sums or null
+    const double *site;  // site records or null
+    double *wrench;      // 9 per bond or null
+    double *partials;    // per-block energy sums or null
 };
 
-__global__ void __launch_bounds__(kThreads) bond_energy_kernel(BondArgs a) {
+// Bound by the float64 pipe: about 210 operations a bond with site records
+// (kSites), cross products and products with R as multiply-add chains, the
+// energy's own terms only where it is asked for.
+// 125k sites / 901k bonds: 565 -> 327 us.
+template <bool kSites>
+__global__ void __launch_bounds__(128) bond_energy_kernel(BondArgs a) {
     double e_sum = 0.0;
     for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < a.m; b += (int64_t)gridDim.x * blockDim.x) {
         int64_t i, j;
         edge(a.edges, b, i, j);
-        const M3 Ri = quat_matrix(a.q + 4 * i), Rj = quat_matrix(a.q + 4 * j);
+        M3 Ri, Rj;
+        double k[4];
+        const double *k0 = a.base + 4 * b;
+        bool direct = !kSites;
+        if (kSites) {
+            const SiteRecord si = load_site(a.site, i), sj = load_site(a.site, j);
+            Ri = si.R;
+            Rj = sj.R;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) k[c] = k0[c] * (si.e[c] * sj.e[c]);
+            direct = (__double_as_longlong(si.safe) & __double_as_longlong(sj.safe)) == 0;
+        } else {
+            Ri = quat_matrix(a.q + 4 * i);
+            Rj = quat_matrix(a.q + 4 * j);
+        }
+        if (direct) {
+            const double *ti = a.theta + a.theta_stride * i, *tj = a.theta + a.theta_stride * j;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) k[c] = k0[c] * exp(0.5 * (ti[c] + tj[c]));
+        }
         const d3 pi = mul(Ri, ld3(a.ri, b)), pj = mul(Rj, ld3(a.rj, b));
         const d3 D = ld3(a.x, j) + pj - ld3(a.x, i) - pi;
-        const d3 d = 0.5 * (tmul(Ri, D) + tmul(Rj, D));
+        const d3 d = 0.5 * tmul_add(tmul(Ri, D), Rj, D);
         // Psi = R_i^T R_j: Psi[r][c] = col_r(R_i) . col_c(R_j)
         const d3 ci0 = col(Ri, 0), ci1 = col(Ri, 1), ci2 = col(Ri, 2);
         const d3 cj0 = col(Rj, 0), cj1 = col(Rj, 1), cj2 = col(Rj, 2);
-        const double P00 = dot(ci0, cj0), P01 = dot(ci0, cj1), P02 = dot(ci0, cj2);
-        const double P10 = dot(ci1, cj0), P11 = dot(ci1, cj1), P12 = dot(ci1, cj2);
-        const double P20 = dot(ci2, cj0), P21 = dot(ci2, cj1), P22 = dot(ci2, cj2);
-        const d3 phi = mk(0.5 * (P21 - P12), 0.5 * (P02 - P20), 0.5 * (P10 - P01));
+        const d3 P0 = mk(dot(ci0, cj0), dot(ci0, cj1), dot(ci0, cj2));
+        const d3 P1 = mk(dot(ci1, cj0), dot(ci1, cj1), dot(ci1, cj2));
+        const d3 P2 = mk(dot(ci2, cj0), dot(ci2, cj1), dot(ci2, cj2));
+        const d3 phi = mk(0.5 * (P2.y - P1.z), 0.5 * (P0.z - P2.x), 0.5 * (P1.x - P0.y));
         const d3 n0 = ld3(a.n0, b);
-        const double *ti = a.theta + a.theta_stride * i, *tj = a.theta + a.theta_stride * j;
-        const double *k0 = a.base + 4 * b;
-        const double kn = k0[0] * exp(0.5 * (ti[0] + tj[0])), ks = k0[1] * exp(0.5 * (ti[1] + tj[1]));
-        const double kb = k0[2] * exp(0.5 * (ti[2] + tj[2])), kt = k0[3] * exp(0.5 * (ti[3] + tj[3]));
         const double dn = dot(d, n0), pn = dot(phi, n0);
-        const d3 dt = d - dn * n0, pt = phi - pn * n0;
-        e_sum += 0.5 * kn * dn * dn + 0.5 * (ks * dot(dt, dt) + kb * dot(pt, pt) + kt * pn * pn);
+        const d3 dt = axpy(-dn, n0, d), pt = axpy(-pn, n0, phi);
+        if (a.partials)
+            e_sum += 0.5 * k[0] * dn * dn + 0.5 * (k[1] * dot(dt, dt) + k[2] * dot(pt, pt) + k[3] * pn * pn);
         if (a.wrench) {
-            const d3 gd = (kn * dn) * n0 + ks * dt, gp = (kt * pn) * n0 + kb * pt;
+            const d3 gd = axpy(k[0] * dn, n0, k[1] * dt), gp = axpy(k[3] * pn, n0, k[2] * pt);
             const d3 Rgi = mul(Ri, gd), Rgj = mul(Rj, gd);
-            const d3 av = 0.5 * (Rgi + Rgj);
-            const double trace = P00 + P11 + P22;
+            const d3 av = 0.5 * (Rgi + Rgj), hD = 0.5 * D;
             // M = (tr Psi gp - Psi^T gp) / 2
-            const d3 PTgp = mk(P00 * gp.x + P10 * gp.y + P20 * gp.z, P01 * gp.x + P11 * gp.y + P21 * gp.z,
-                               P02 * gp.x + P12 * gp.y + P22 * gp.z);
-            const d3 Mv = 0.5 * (trace * gp - PTgp);
-            const d3 T = mul(Ri, Mv);
-            const d3 tjv = cross(pj, av) - 0.5 * cross(D, Rgj) + T;
-            const d3 tiv = -cross(pi, av) - 0.5 * cross(D, Rgi) - T;
+            const double trace = P0.x + P1.y + P2.z;
+            const d3 PTgp = axpy(gp.z, P2, axpy(gp.y, P1, gp.x * P0));
+            const d3 T = mul(Ri, 0.5 * axpy(trace, gp, -PTgp));
             double *w = a.wrench + 9 * b;
             st3(w, av);
-            st3(w + 3, -tiv);
-            st3(w + 6, -tjv);
+            st3(w + 3, cross_add(cross_add(T, pi, av), hD, Rgi));
+            st3(w + 6, cross_sub(cross_add(-T, hD, Rgj), pj, av));
         }
     }
     if (a.partials) {
@@ -96,36 +160,13 @@ __global__ void __launch_bounds__(kThreads) sum_partials_kernel(int count, const
 }
 
 // f_s = sum of a over i ends minus a over j ends; tau_s = -t_i / -t_j terms.
+// Two neighbouring lanes a site: its force and its torque.
 __global__ void __launch_bounds__(kThreads) site_forces_kernel(int64_t n, const int32_t *ptr, const int32_t *inc,
                                                                const double *w, double *force, double *torque) {
-    const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, s = t / 2;
     if (s >= n) return;
-    double f[3] = {0.0, 0.0, 0.0}, t[3] = {0.0, 0.0, 0.0};
-    const int e1 = ptr[s + 1];
-    for (int e = ptr[s]; e < e1; ++e) {
-        const int v = inc[e];
-        if (v >= 0) {
-            const double *p = w + 9 * (int64_t)v;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                f[c] += p[c];
-                t[c] += p[3 + c];
-            }
-        } else {
-            const double *p = w + 9 * (int64_t)(~v);
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                f[c] -= p[c];
-                t[c] += p[6 + c];
-            }
-        }
-    }
-    if (force)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) force[3 * s + c] = f[c];
-    if (torque)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) torque[3 * s + c] = t[c];
+    double *out = t & 1 ? torque : force;
+    if (out) st3(out, s, gather_half(ptr, inc, w, s, (int)(t & 1)));
 }
 
 // Frozen tangent of the bond potential at the current configuration, for
@@ -172,10 +213,10 @@ extern "C" {
 
 int64_t dpf_energy_partials_doubles(void) { return kMaxBlocks; }
 
-int dpf_bond_energy(const dpf_graph *g, const double *base, const double *theta, int64_t theta_stride,
-                    const double *x, const double *q, const double *n0, const double *ri, const double *rj,
-                    double *force, double *torque, double *energy, double *wrench, double *partials,
-                    void *stream) {
+static int bond_energy(const dpf_graph *g, const double *base, const double *theta, int64_t theta_stride,
+                       const double *x, const double *q, const double *n0, const double *ri, const double *rj,
+                       double *force, double *torque, double *energy, double *wrench, double *partials,
+                       double *site, void *stream) {
     const bool want_forces = force || torque;
     if (!g || g->n_sites <= 0 || (g->n_bonds && (!g->edges || !base || !theta || !n0 || !ri || !rj)) || !x ||
         !q || theta_stride < 4 || (want_forces && (!g->inc_ptr || (g->n_bonds && (!g->inc_bond || !wrench)))) ||
@@ -184,20 +225,45 @@ int dpf_bond_energy(const dpf_graph *g, const double *base, const double *theta,
     cudaStream_t st = (cudaStream_t)stream;
     int grid = 1;
     if (g->n_bonds) {
-        int64_t want = (g->n_bonds + kThreads - 1) / kThreads;
-        grid = (int)(want < kMaxBlocks ? want : kMaxBlocks);
-        BondArgs a{g->n_bonds, g->edges, base, theta, theta_stride, x, q, n0, ri, rj,
+        int64_t want = (g->n_bonds + 127) / 128;
+        grid = (int)(want < kMaxBlocks || !energy ? want : kMaxBlocks);
+        BondArgs a{g->n_bonds, g->edges, base, theta, theta_stride, x, q, n0, ri, rj, site,
                    want_forces ? wrench : nullptr, energy ? partials : nullptr};
-        bond_energy_kernel<<<grid, kThreads, 0, st>>>(a);
+        if (site) {
+            energy_sites_kernel<<<(int)((g->n_sites + kThreads - 1) / kThreads), kThreads, 0, st>>>(
+                g->n_sites, q, theta, theta_stride, site);
+            bond_energy_kernel<true><<<grid, 128, 0, st>>>(a);
+        } else {
+            bond_energy_kernel<false><<<grid, 128, 0, st>>>(a);
+        }
     } else if (energy) {
         cudaMemsetAsync(partials, 0, sizeof(double), st);
     }
     if (energy) sum_partials_kernel<<<1, kThreads, 0, st>>>(grid, partials, energy);
     if (want_forces)
-        site_forces_kernel<<<(int)((g->n_sites + kThreads - 1) / kThreads), kThreads, 0, st>>>(
+        site_forces_kernel<<<(int)((2 * g->n_sites + kThreads - 1) / kThreads), kThreads, 0, st>>>(
             g->n_sites, g->inc_ptr, g->inc_bond, wrench, force, torque);
     DPF_CHECK_LAUNCH();
     return DPF_OK;
+}
+
+int dpf_bond_energy(const dpf_graph *g, const double *base, const double *theta, int64_t theta_stride,
+                    const double *x, const double *q, const double *n0, const double *ri, const double *rj,
+                    double *force, double *torque, double *energy, double *wrench, double *partials,
+                    void *stream) {
+    return bond_energy(g, base, theta, theta_stride, x, q, n0, ri, rj, force, torque, energy, wrench, partials,
+                       nullptr, stream);
+}
+
+int64_t dpf_energy_site_doubles(int64_t n_sites) { return n_sites < 0 ? 0 : kSite * n_sites; }
+
+int dpf_bond_energy_sites(const dpf_graph *g, const double *base, const double *theta, int64_t theta_stride,
+                          const double *x, const double *q, const double *n0, const double *ri, const double *rj,
+                          double *force, double *torque, double *energy, double *wrench, double *partials,
+                          double *site, void *stream) {
+    if (!site || ((uintptr_t)site & 15u)) return DPF_ERR_ARGUMENT;
+    return bond_energy(g, base, theta, theta_stride, x, q, n0, ri, rj, force, torque, energy, wrench, partials,
+                       site, stream);
 }
 
 int dpf_energy_tangent(const dpf_graph *g, const double *base, const double *theta, int64_t theta_stride,

@@ -46,6 +46,7 @@ class EnergyFoam:
         self._lib = b._lib
         self._wrench = torch.empty(max(1, 9*b.n_bonds), dtype=F64, device=self.device)
         self._partials = torch.empty(self._lib.dpf_energy_partials_doubles(), dtype=F64, device=self.device)
+        self._sites = torch.empty(self._lib.dpf_energy_site_doubles(b.n_sites), dtype=F64, device=self.device)
 
     def _run(self, theta, x, q, forces, energy):
         theta = torch.as_tensor(theta, dtype=F64, device=self.device).contiguous()
@@ -60,10 +61,11 @@ class EnergyFoam:
         e = torch.empty(1, dtype=F64, device=self.device) if energy else None
         addr = lambda t: None if t is None else t.data_ptr()
         b = self._bonds
-        _lib.check(self._lib.dpf_bond_energy(
+        _lib.check(self._lib.dpf_bond_energy_sites(
             ctypes.byref(b._graph), self.base.data_ptr(), theta.data_ptr(), theta.shape[1], x.data_ptr(),
             q.data_ptr(), self.n0.data_ptr(), self.ri.data_ptr(), self.rj.data_ptr(), addr(f), addr(tau), addr(e),
-            self._wrench.data_ptr(), self._partials.data_ptr(), b._stream()), 'dpf_bond_energy')
+            self._wrench.data_ptr(), self._partials.data_ptr(), self._sites.data_ptr(), b._stream()),
+            'dpf_bond_energy_sites')
         return f, tau, e
 
     @torch.no_grad()

@@ -745,6 +745,15 @@ int dpf_bond_energy(const dpf_graph *g, const double *base, const double *theta,
                     double *force, double *torque, double *energy, double *wrench, double *partials,
                     void *stream);
 
+/* dpf_bond_energy with a scratch of dpf_energy_site_doubles(N) doubles
+ * (16-byte aligned) for the sites' rotation matrices and stiffness factors,
+ * which the bonds otherwise form once an end. */
+int64_t dpf_energy_site_doubles(int64_t n_sites);
+int dpf_bond_energy_sites(const dpf_graph *g, const double *base, const double *theta, int64_t theta_stride,
+                          const double *x, const double *q, const double *n0, const double *ri, const double *rj,
+                          double *force, double *torque, double *energy, double *wrench, double *partials,
+                          double *site, void *stream);
+
 /* Frozen tangent of the bond potential at the configuration (x, q) for the
  * Newton direction of the energy-law solver (no reference counterpart; at the
  * reference configuration it is the LinearBondsGPU stiffness, the exact
