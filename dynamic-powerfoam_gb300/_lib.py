@@ -85,7 +85,18 @@ class NewtonStep(ctypes.Structure):
                  ('committed_start', i32)])
 
 
+class Newton64(ctypes.Structure):
+    """dpf_newton64: buffers of a NewtonBonds solver for the float64 step driver."""
+    _fields_ = ([('graph', vp), ('stiffness', Stiffness)] +
+                [(k, vp) for k in ('radii', 'mass', 'fixed', 'n', 'ri', 'rj', 'diagonal', 'block', 'preconditioner',
+                                   'units', 'wrench', 'workspace', 'basis', 'transformed', 'w', 'residual', 'h',
+                                   'krylov_partials', 'partials', 'scalars', 'status', 'inner', 'barrier', 'vectors',
+                                   'host')] +
+                [('krylov_width', i32), ('elastic', i32)])
+
+
 NEWTON_VECTORS = 10
+NEWTON64_VECTORS = 7
 NEWTON_HOST_DOUBLES = 128
 NEWTON_TRACE = 32
 NEWTON_TIMERS = ('setup', 'residual', 'scaling', 'pcg', 'jvp', 'commit', 'pack', 'krylov', 'norms', 'vector', 'accept')
@@ -207,12 +218,16 @@ SIGNATURES = {
     'dpf_mixed_commit_lazy': (i32, [P(Graph), vp, vp, vp, vp, vp, vp, vp, vp, vp]),
     'dpf_mixed_fold_history': (i32, [P(Graph), vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]),
     'dpf_newton_struct_sizes': (i32, [P(ctypes.c_int64)]),
+    'dpf_commit_state': (i32, [P(Graph), P(Stiffness), P(History), vp, P(TrialOut), vp, vp]),
+    'dpf_newton64_partials_doubles': (i64, []),
+    'dpf_newton64_struct_size': (i64, []),
+    'dpf_newton64_step': (i32, [P(Newton64), P(NewtonStep), P(NewtonInfo), vp]),
 }
 
 
 # Kernels each entry point launches (the launch counter's unit).
 KERNELS = {
-    'dpf_stiffness_apply': 2, 'dpf_diagonal_blocks': 1, 'dpf_prepare_scaling': 1, 'dpf_trial': 2,
+    'dpf_stiffness_apply': 2, 'dpf_diagonal_blocks': 1, 'dpf_prepare_scaling': 1, 'dpf_trial': 2, 'dpf_commit_state': 1,
     'dpf_residual': 2, 'dpf_scale_residual': 1, 'dpf_jacobian_vector': 2, 'dpf_elastic_precondition': 1,
     'dpf_loads': 2, 'dpf_bond_setup': 2, 'dpf_accept_step': 1, 'dpf_energy': 1, 'dpf_arnoldi_cgs2': 4, 'dpf_combine_rows': 1,
     'dpf_dot_norm': 1, 'dpf_axpby': 1, 'dpf_rhs_scale': 1, 'dpf_masked_scale': 1,

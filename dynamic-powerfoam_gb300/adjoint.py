@@ -57,9 +57,8 @@ class _RecordingNewton(NewtonBonds):
 
     accepted_increment = None
 
-    def _accept(self, y, dt):
+    def _accepted(self, y):
         self.accepted_increment = y.clone()
-        super()._accept(y, dt)
 
 
 class _Rollout(torch.autograd.Function):

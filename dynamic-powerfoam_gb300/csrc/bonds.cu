@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(128) trial_bonds(TrialBondArgs a) {
     const d3 slide = ks * axpy(-dn, nm, du), bend = kb * axpy(-twist, nm, dw);
     const d3 f = axpy(fma(0.5 * kn, dn, fn_c), nm, axpy(0.5, slide, fs0));
     const d3 couple = axpy(fma(0.5 * kt, twist, mt_c), nm, axpy(0.5, bend, mb0));
-    store_wrench(a.wrench, b, f, cross_add(couple, ri, f), cross_sub(-couple, rj, f));
+    if (a.wrench) store_wrench(a.wrench, b, f, cross_add(couple, ri, f), cross_sub(-couple, rj, f));
     if (a.n) st3(a.n, b, nm);
     if (a.ri) st3(a.ri, b, ri);
     if (a.rj) st3(a.rj, b, rj);
@@ -564,14 +564,14 @@ __global__ void __launch_bounds__(kThreads) loads_bonds(int64_t m, const int64_t
     edge(edges, b, i, j);
     const d3 xi = ld3(h.x, i), xj = ld3(h.x, j);
     const d3 d = xj - xi;
-    const double length = norm(d);
-    if (length <= 1e-12 && status) atomicOr(status, DPF_ERR_COINCIDENT);
-    const d3 n = d / length;
-    const d3 c = 0.5 * (xi + xj) + (0.5 * (h.radii[i] - h.radii[j])) * n + ld3(h.offset, b);
-    const d3 ri = c - xi, rj = c - xj;
-    const d3 f = h.fn[b] * n + ld3(h.fs, b);
-    const d3 couple = h.mt[b] * n + ld3(h.mb, b);
-    store_wrench(wrench, b, f, cross(ri, f) + couple, -cross(rj, f) - couple);
+    const double d2 = dot(d, d);
+    if (d2 <= 1e-24 && status) atomicOr(status, DPF_ERR_COINCIDENT);
+    const d3 n = rsqrt(d2) * d;
+    const d3 lever = axpy(0.5 * (h.radii[i] - h.radii[j]), n, ld3(h.offset, b));
+    const d3 ri = axpy(0.5, d, lever), rj = axpy(-0.5, d, lever);
+    const d3 f = axpy(h.fn[b], n, ld3(h.fs, b));
+    const d3 couple = axpy(h.mt[b], n, ld3(h.mb, b));
+    store_wrench(wrench, b, f, cross_add(couple, ri, f), cross_sub(-couple, rj, f));
 }
 
 inline int blocks_for(int64_t n, int threads) { return (int)((n + threads - 1) / threads); }
@@ -733,6 +733,15 @@ int dpf_trial(const dpf_graph *g, const dpf_stiffness *k, const dpf_history *h, 
     a.x_end = want_end ? out->x_end : nullptr;
     a.status = status;
     site_residual<<<blocks_for(2 * g->n_sites, kThreads), kThreads, 0, st>>>(a);
+    DPF_CHECK_LAUNCH();
+    return DPF_OK;
+}
+
+int dpf_commit_state(const dpf_graph *g, const dpf_stiffness *k, const dpf_history *h, const double *y,
+                     const dpf_trial_out *out, int *status, void *stream) {
+    if (!graph_ok(g) || !k || !history_ok(h, g->n_bonds) || !y || !out || !status) return DPF_ERR_ARGUMENT;
+    cudaStream_t st = (cudaStream_t)stream;
+    launch_trial_bonds(g, k, h, y, nullptr, nullptr, 1, out, nullptr, status, st);
     DPF_CHECK_LAUNCH();
     return DPF_OK;
 }

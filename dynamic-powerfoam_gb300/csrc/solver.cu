@@ -341,57 +341,7 @@ __global__ void __launch_bounds__(kThreads) accept_kernel(int64_t n, const doubl
     const double two_over_dt = 2.0 / dt;  // one float64 division per site, not six
 #pragma unroll
     for (int c = 0; c < 6; ++c) v[6 * s + c] = two_over_dt * y[6 * s + c] - v[6 * s + c];
-    const d3 w = ld3(y + 6 * s + 3);
-    // Rodrigues coefficients A = sin(a)/a and B = (1 - cos a)/a^2 of a = |w|.
-    // Both are even in a: for a^2 < 1/4 (every step the rotation guard lets
-    // through has a <= 0.25) their Maclaurin series in a^2, 8 terms each,
-    // are exact to a few 1e-17 and need no float64 transcendental, which is
-    // slow on this part.  Larger angles take the closed form.
-    const double theta = w.x * w.x + w.y * w.y + w.z * w.z;
-    double A, B;
-    if (theta < 0.25) {
-        // Horner in theta: A = sum (-theta)^k/(2k+1)!, B = sum (-theta)^k/(2k+2)!, k = 0..7
-        A = 1.0 / 1307674368000.0;                 // 1/15!
-        A = fma(-theta, A, 1.0 / 6227020800.0);    // 1/13!
-        A = fma(-theta, A, 1.0 / 39916800.0);      // 1/11!
-        A = fma(-theta, A, 1.0 / 362880.0);        // 1/9!
-        A = fma(-theta, A, 1.0 / 5040.0);          // 1/7!
-        A = fma(-theta, A, 1.0 / 120.0);           // 1/5!
-        A = fma(-theta, A, 1.0 / 6.0);             // 1/3!
-        A = fma(-theta, A, 1.0);
-        B = 1.0 / 20922789888000.0;                // 1/16!
-        B = fma(-theta, B, 1.0 / 87178291200.0);   // 1/14!
-        B = fma(-theta, B, 1.0 / 479001600.0);     // 1/12!
-        B = fma(-theta, B, 1.0 / 3628800.0);       // 1/10!
-        B = fma(-theta, B, 1.0 / 40320.0);         // 1/8!
-        B = fma(-theta, B, 1.0 / 720.0);           // 1/6!
-        B = fma(-theta, B, 1.0 / 24.0);            // 1/4!
-        B = fma(-theta, B, 0.5);
-    } else {
-        const double angle = sqrt(theta);
-        double sh, ch;
-        sincos(0.5 * angle, &sh, &ch);
-        A = sin(angle) / angle;
-        const double q = sh / (0.5 * angle);
-        B = 0.5 * q * q;
-    }
-    const double S[9] = {0.0, -w.z, w.y, w.z, 0.0, -w.x, -w.y, w.x, 0.0};
-    double E[9];
-#pragma unroll
-    for (int p = 0; p < 3; ++p)
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-            const double ss = S[3 * p] * S[q] + S[3 * p + 1] * S[3 + q] + S[3 * p + 2] * S[6 + q];
-            E[3 * p + q] = (p == q ? 1.0 : 0.0) + A * S[3 * p + q] + B * ss;
-        }
-    double *R = rotation + 9 * s;
-    double Rn[9];
-#pragma unroll
-    for (int p = 0; p < 3; ++p)
-#pragma unroll
-        for (int q = 0; q < 3; ++q) Rn[3 * p + q] = E[3 * p] * R[q] + E[3 * p + 1] * R[3 + q] + E[3 * p + 2] * R[6 + q];
-#pragma unroll
-    for (int c = 0; c < 9; ++c) R[c] = Rn[c];
+    rotate_site(ld3(y + 6 * s + 3), rotation + 9 * s, rotation + 9 * s);
 }
 
 // Elastic + kinetic energy (bonded_dem_finite_gpu.py:122-125).

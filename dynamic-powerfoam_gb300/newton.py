@@ -93,6 +93,36 @@ def _pinned_buffers():
     return _PINNED.buffers
 
 
+def _pinned_step_host():
+    """Pinned host doubles of the float64 step driver, one set per host thread."""
+    if not hasattr(_PINNED, 'step'):
+        _PINNED.step = torch.zeros(_lib.NEWTON_HOST_DOUBLES, dtype=F64).pin_memory()
+    return _PINNED.step
+
+
+def _raise_outcome(info):
+    """The reference's exception for an unconverged step of a native driver."""
+    if info.outcome == _lib.NEWTON_CONVERGED:
+        return
+    if info.outcome == _lib.NEWTON_GUARD:
+        raise guard_error(info.guard)
+    raise SubdivideError({
+        _lib.NEWTON_NONFINITE: f'Subdivide: non-finite Newton residual ({info.relative:g}, {info.local:g})',
+        _lib.NEWTON_SINGULAR: 'Subdivide: singular Newton linear system',
+        _lib.NEWTON_KRYLOV: f'Subdivide: FGMRES did not converge ({info.krylov_relative:g})',
+        _lib.NEWTON_LINE_SEARCH: 'Subdivide: Newton line search failed',
+    }.get(info.outcome, f'Subdivide: Newton did not converge ({info.relative:g}, {info.local:g})'))
+
+
+def _step_info(info):
+    """The ``info`` of ``NewtonBonds.step`` from a native driver's."""
+    return dict(nonlinear_iterations=info.nonlinear_iterations, nonlinear_relative_residual=info.relative,
+                local_pose_defect=info.local, krylov_iterations=info.krylov_iterations,
+                cg_iterations=info.cg_iterations,
+                residual_trace=[[info.trace[2*k], info.trace[2*k + 1]] for k in range(info.trace_len)],
+                max_step_rotation=info.max_rotation)
+
+
 def bond_setup(points, radii, pairs, areas, contacts, masses, young, shear):
     """Host-side setup arithmetic of ``LinearBondsGPU.__init__``
     (``experiments/bonded_dem_linear_gpu.py:15-40``): bond normals, contact
@@ -1065,6 +1095,10 @@ class NewtonBonds(FiniteBonds):
                    self._stream())
         self.commit(state)
         self.v, self.rotation = self._v, rotation
+        self._accepted(y)
+
+    def _accepted(self, y):
+        """Called with the increment of an accepted step (a driver's workspace: clone to keep it)."""
 
     def _krylov_solve(self, operator, rhs, precondition, tolerance, rhs_norm, dt):
         """FGMRES on the scaled Newton system (``bonded_dem_newton.py:160-162``)."""
@@ -1090,6 +1124,103 @@ class NewtonBonds(FiniteBonds):
         delta.index_copy_(0, index, torch.linalg.solve(jacobian, -scaled.reshape(-1).index_select(0, index)))
         return delta.view(-1, 6)
 
+    # Drive eligible steps (FGMRES, no replaced method) from the library's float64
+    # step driver; False keeps every step on the Python control path.
+    native = True
+
+    # what the driver calls itself: a subclass or an instance that replaces one keeps the Python path
+    _NATIVE64_HOOKS = ('loads', 'trial', 'commit', 'residual', 'midpoint_force', 'jacobian_vector', '_jvp',
+                       'prepare_scaling', 'scale_residual', 'elastic_precondition', '_diagonal_blocks', 'stiffness',
+                       '_operator', 'geometry', 'assemble', '_evaluate', '_step_begin', '_iteration_residual',
+                       '_newton_operator', '_newton_preconditioner', '_line_merit', '_accept', '_krylov_solve',
+                       '_timed', '_call', '_fetch')
+
+    def _native64_ready(self, backend, preconditioning, max_iterations=12, linear_tolerance=1e-6):
+        # linear tolerances near rounding stay on the Python path: there the true residual
+        # of FGMRES carries the rounding of J x, which the driver's Arnoldi relation does not see
+        cls, own = type(self), self.__dict__
+        return (self.native and backend == 'fgmres' and preconditioning in ('elastic', 'block') and
+                linear_tolerance >= 1e-12 and 0 <= max_iterations < _lib.NEWTON_TRACE and self.profile is None and
+                own.get('call_profile') is None and self.n_sites > 0 and
+                not any(name in own or getattr(cls, name) is not getattr(NewtonBonds, name)
+                        for name in self._NATIVE64_HOOKS))
+
+    def _native64_buffers(self):
+        """Descriptor of this solver's buffers for ``dpf_newton64_step`` (cached while the
+        tensors it points to stay the same)."""
+        for name in ('mass', 'fixed', 'radii'):
+            t = getattr(self, name)
+            if not t.is_contiguous():
+                setattr(self, name, t.contiguous())
+        n, dev, lib = self.n_sites, self.device, self._lib
+        e = lambda *shape: torch.empty(shape, dtype=F64, device=dev)
+        if self.block is None or any(t is None or t.shape != (n, 6, 6) or not t.is_contiguous() for t in (
+                self.block, self.diagonal, self.preconditioner)) or self.units is None:
+            self.diagonal, self.block, self.preconditioner = e(n, 6, 6), e(n, 6, 6), e(n, 6, 6)
+            self.units = e(n, 6)
+        if self._krylov is None or self._krylov.length != 6*n:
+            self._krylov = _Krylov(6*n, 32, dev)
+        if self._pcg_workspace is None:
+            self._pcg_workspace = e(lib.dpf_elastic_workspace_doubles(n))
+        if getattr(self, '_native64_scratch', None) is None:
+            self._native64_scratch = (e(_lib.NEWTON64_VECTORS, n, 6), e(2, n, 6), e(lib.dpf_newton64_partials_doubles()))
+        vectors, pair, partials = self._native64_scratch
+        ws = self._krylov
+        held = (self.mass, self.fixed, self.radii, self.diagonal, self.block, self.preconditioner, self.units,
+                self._wrench, self._pcg_workspace, ws.basis, ws.transformed, ws.h, vectors, pair, partials,
+                self._partials, self._scalars, self._status, self._inner, self._barrier)
+        p = lambda t: t.data_ptr()
+        key = [p(t) for t in held]
+        cached = self.__dict__.get('_native64_desc')
+        if cached is not None and cached[0] == key:
+            return cached[1]
+        desc = _lib.Newton64(
+            graph=ctypes.addressof(self._graph), radii=p(self.radii), mass=p(self.mass), fixed=p(self.fixed),
+            diagonal=p(self.diagonal), block=p(self.block), preconditioner=p(self.preconditioner),
+            units=p(self.units), wrench=p(self._wrench), workspace=p(self._pcg_workspace), basis=p(ws.basis),
+            transformed=p(ws.transformed), w=p(pair[0]), residual=p(pair[1]), h=p(ws.h), krylov_partials=p(partials),
+            partials=p(self._partials), scalars=p(self._scalars), status=p(self._status), inner=p(self._inner),
+            barrier=p(self._barrier), vectors=p(vectors), krylov_width=ws.width)
+        # the descriptor holds only addresses: keep what they point into alive with it
+        self._native64_desc = (key, desc, _lib.NewtonStep(), _lib.NewtonInfo(), held)
+        return desc
+
+    def _native64_step(self, dt, external, tolerance, max_iterations, pose_tolerance, linear_tolerance, elastic):
+        """``step`` through ``dpf_newton64_step``: one library call per step."""
+        external, v0, r0 = self._vec(external), self._vec(self.v), self._vec(self.rotation)
+        history = self._history_struct()
+        desc = self._native64_buffers()
+        args, info = self._native64_desc[2:4]
+        n, m = self.n_sites, self.n_bonds
+        e = lambda *shape: torch.empty(shape, dtype=F64, device=self.device)
+        stiffness = [t.contiguous() for t in (self.kn, self.ks, self.kb, self.kt)]
+        tangent = (e(m, 3), e(m, 3), e(m, 3))
+        state = dict(x=e(n, 3), normal=e(m, 3), fn=e(m), fs=e(m, 3), mt=e(m), mb=e(m, 3), offset=e(m, 3))
+        v, rotation = torch.empty_like(v0), torch.empty_like(r0)
+        desc.stiffness = _lib.Stiffness(*(t.data_ptr() for t in stiffness))
+        desc.n, desc.ri, desc.rj = (t.data_ptr() for t in tangent)
+        host = _pinned_step_host()
+        desc.host, desc.elastic = host.data_ptr(), int(elastic)
+        args.dt, args.external, args.history = dt, external.data_ptr(), history
+        args.v, args.rotation, args.v_in, args.rotation_in = \
+            v.data_ptr(), rotation.data_ptr(), v0.data_ptr(), r0.data_ptr()
+        args.x_end, args.normal_end, args.offset_end, args.fn_end, args.fs_end, args.mt_end, args.mb_end = (
+            state[k].data_ptr() for k in ('x', 'normal', 'offset', 'fn', 'fs', 'mt', 'mb'))
+        args.tolerance, args.pose_tolerance, args.linear_tolerance = float(tolerance), float(pose_tolerance), \
+            float(linear_tolerance)
+        args.max_iterations = int(max_iterations)
+        self._inner_host = 0
+        _lib.check(self._lib.dpf_newton64_step(ctypes.byref(desc), ctypes.byref(args), ctypes.byref(info),
+                                               self._stream()), 'dpf_newton64_step')
+        _lib.LAUNCHES['count'] += info.launches
+        self.n, self.ri, self.rj = tangent
+        _raise_outcome(info)
+        self.commit(state)
+        self.v, self.rotation = v, rotation
+        self._accepted(self._native64_scratch[0][info.scaling_alternate])
+        self.time += dt
+        return info.work, _step_info(info)
+
     @torch.no_grad()
     def step(self, dt, external, tolerance=2e-7, max_iterations=12, *,
              pose_tolerance=2e-6, backend='fgmres', linear_tolerance=1e-6,
@@ -1098,6 +1229,9 @@ class NewtonBonds(FiniteBonds):
         if not np.isfinite(dt) or dt <= 0:
             raise ValueError('Positive finite dt required')
         dt = float(dt)
+        if self._native64_ready(backend, preconditioning, max_iterations, linear_tolerance):
+            return self._native64_step(dt, external, tolerance, max_iterations, pose_tolerance, linear_tolerance,
+                                       preconditioning == 'elastic')
         external = self._vec(external)
         self._v = self._vec(self.v).clone()
         y = torch.zeros_like(self._v)
@@ -1475,20 +1609,7 @@ class MixedNewtonBonds(NewtonBonds):
                 count = info.timed_launches[k]
                 if count:
                     self.profile.setdefault(key, []).extend([info.time_ms[k]/count]*count)
-        relative, local = info.relative, info.local
-        outcome = info.outcome
-        if outcome == _lib.NEWTON_GUARD:
-            raise guard_error(info.guard)
-        if outcome == _lib.NEWTON_NONFINITE:
-            raise SubdivideError(f'Subdivide: non-finite Newton residual ({relative:g}, {local:g})')
-        if outcome == _lib.NEWTON_SINGULAR:
-            raise SubdivideError('Subdivide: singular Newton linear system')
-        if outcome == _lib.NEWTON_KRYLOV:
-            raise SubdivideError(f'Subdivide: FGMRES did not converge ({info.krylov_relative:g})')
-        if outcome == _lib.NEWTON_LINE_SEARCH:
-            raise SubdivideError('Subdivide: Newton line search failed')
-        if outcome != _lib.NEWTON_CONVERGED:
-            raise SubdivideError(f'Subdivide: Newton did not converge ({relative:g}, {local:g})')
+        _raise_outcome(info)
         if self.lazy_history:
             self._commit_lazy(state['x'])
         else:
@@ -1498,11 +1619,7 @@ class MixedNewtonBonds(NewtonBonds):
         self._token = self._state_token()
         self._since_refresh += 1
         self.time += dt
-        trace = [[info.trace[2*k], info.trace[2*k + 1]] for k in range(info.trace_len)]
-        return info.work, dict(nonlinear_iterations=info.nonlinear_iterations, nonlinear_relative_residual=relative,
-                               local_pose_defect=local, krylov_iterations=info.krylov_iterations,
-                               cg_iterations=info.cg_iterations, residual_trace=trace,
-                               max_step_rotation=info.max_rotation)
+        return info.work, _step_info(info)
 
     def __init__(self, *args, **kwargs):
         super().__init__(*args, **kwargs)

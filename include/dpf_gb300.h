@@ -155,6 +155,11 @@ int dpf_trial(const dpf_graph *g, const dpf_stiffness *k, const dpf_history *h,
  * scaled residual s = P r / units and, in `norms` (3 doubles, device),
  * [|r|_2, max|s|, |s|_2].  preconditioner/units/scaled may be NULL.
  * Replaces NewtonBonds.residual + scale_residual (experiments/bonded_dem_newton.py:83-86, 104-105). */
+/* The end state of increment y (no positions, no force): the end history of
+ * dpf_trial into out's end arrays (each optional), its guards into *status. */
+int dpf_commit_state(const dpf_graph *g, const dpf_stiffness *k, const dpf_history *h, const double *y,
+                     const dpf_trial_out *out, int *status, void *stream);
+
 int dpf_residual(const dpf_graph *g, const dpf_stiffness *k, const dpf_history *h,
                  const double *y, const double *v, const double *external, const double *mass,
                  const uint8_t *fixed, double dt, const dpf_trial_out *trial,
@@ -913,6 +918,49 @@ int dpf_mixed_newton_step(const dpf_mixed_newton *solver, const dpf_newton_step 
 /* sizeof(dpf_mixed_newton), sizeof(dpf_newton_step), sizeof(dpf_newton_info)
  * into out[0..3): lets a binding check its struct layouts (host only). */
 int dpf_newton_struct_sizes(int64_t *out);
+
+/* ---- native step driver of the float64 Newton solver ---------------------
+ * One step of NewtonBonds.step with the FGMRES backend (elastic or block
+ * preconditioning) driven from host code in this library: the decisions of the
+ * Python control path on the same float64 quantities.  The residual and tangent
+ * of an accepted candidate start the next iteration; the true residual of an
+ * FGMRES cycle comes from the Arnoldi relation.  Replaces the control flow of
+ * NewtonBonds.step and fgmres (experiments/bonded_dem_newton.py:13-60, 132-201).
+ *
+ * Uses dpf_newton_step (external, history, v_in, rotation_in and the outputs v,
+ * rotation, x_end, normal_end .. mt_end, none of which may overlap the inputs;
+ * refresh, timing and committed_start are not used) and dpf_newton_info
+ * (scaling_alternate: the accepted increment is vectors + scaling_alternate 6 N;
+ * time_ms and timed_launches are zero). */
+#define DPF_NEWTON64_VECTORS 7
+
+typedef struct dpf_newton64 {
+    const dpf_graph *graph;        /* host struct */
+    dpf_stiffness stiffness;
+    const double *radii, *mass;    /* (N), (N, 6) */
+    const uint8_t *fixed;          /* (N) */
+    double *n, *ri, *rj;           /* (M, 3): the tangent of the last evaluated increment */
+    double *diagonal, *block, *preconditioner; /* (N, 6, 6) */
+    double *units;                 /* (N, 6) */
+    double *wrench;                /* 9 M */
+    double *workspace;             /* dpf_elastic_workspace_doubles(N); NULL without elastic */
+    double *basis, *transformed;   /* (width + 1, 6 N), (width, 6 N) */
+    double *w, *residual;          /* 6 N each */
+    double *h;                     /* >= width + 2 */
+    double *krylov_partials;       /* dpf_newton64_partials_doubles() */
+    double *partials;              /* dpf_partials_doubles() */
+    double *scalars;               /* >= 8 */
+    int *status, *inner;
+    unsigned *barrier;             /* 2 words */
+    double *vectors;               /* DPF_NEWTON64_VECTORS x 6 N */
+    double *host;                  /* pinned host memory, DPF_NEWTON_HOST_DOUBLES */
+    int krylov_width;              /* FGMRES restart length, <= 62 */
+    int elastic;                   /* 1: elastic PCG preconditioner, 0: block scaling only */
+} dpf_newton64;
+
+int64_t dpf_newton64_partials_doubles(void);
+int64_t dpf_newton64_struct_size(void);
+int dpf_newton64_step(const dpf_newton64 *solver, const dpf_newton_step *step, dpf_newton_info *info, void *stream);
 
 #ifdef __cplusplus
 }
