@@ -92,7 +92,7 @@ class Newton64(ctypes.Structure):
                                    'units', 'wrench', 'workspace', 'basis', 'transformed', 'w', 'residual', 'h',
                                    'krylov_partials', 'partials', 'scalars', 'status', 'inner', 'barrier', 'vectors',
                                    'host')] +
-                [('krylov_width', i32), ('elastic', i32)])
+                [('krylov_width', i32), ('elastic', i32), ('linear', vp)])
 
 
 NEWTON_VECTORS = 10
@@ -221,6 +221,7 @@ SIGNATURES = {
     'dpf_commit_state': (i32, [P(Graph), P(Stiffness), P(History), vp, P(TrialOut), vp, vp]),
     'dpf_newton64_partials_doubles': (i64, []),
     'dpf_newton64_struct_size': (i64, []),
+    'dpf_newton64_linear_doubles': (i64, [i64]),
     'dpf_newton64_step': (i32, [P(Newton64), P(NewtonStep), P(NewtonInfo), vp]),
 }
 

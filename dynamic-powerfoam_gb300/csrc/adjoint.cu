@@ -490,8 +490,8 @@ int dpf_adjoint_local_jacobian(const dpf_graph *g, const dpf_stiffness *k, const
                                double *jacobian, void *stream) {
     if (!adj_ok(g, k, h, y) || (g->n_bonds && !jacobian)) return DPF_ERR_ARGUMENT;
     if (g->n_bonds)
-        local_jacobian_kernel<<<blocks_for(g->n_bonds, 128), 128, 0, (cudaStream_t)stream>>>(
-            g->n_bonds, sources(g, k, h, y), jacobian);
+        local_jacobian_kernel<<<blocks_for(g->n_bonds, spread_threads(g->n_bonds)), spread_threads(g->n_bonds), 0,
+                                (cudaStream_t)stream>>>(g->n_bonds, sources(g, k, h, y), jacobian);
     DPF_CHECK_LAUNCH();
     return DPF_OK;
 }
@@ -520,7 +520,8 @@ int dpf_adjoint_bond_vjp(const dpf_graph *g, const dpf_stiffness *k, const dpf_h
     if (g->n_bonds) {
         VjpArgs a{g->n_bonds, sources(g, k, h, y), lam, coef, end_adjoint, with_increment ? 1 : 0,
                   history_adjoint, stiffness_adjoint, slots};
-        (end_adjoint ? vjp_kernel<true> : vjp_kernel<false>)<<<blocks_for(g->n_bonds, 128), 128, 0, st>>>(a);
+        const int threads = spread_threads(g->n_bonds);
+        (end_adjoint ? vjp_kernel<true> : vjp_kernel<false>)<<<blocks_for(g->n_bonds, threads), threads, 0, st>>>(a);
     }
     if ((y_adjoint || x_adjoint) && g->n_bonds)
         vjp_sites_kernel<<<blocks_for(g->n_sites, kThreads), kThreads, 0, st>>>(

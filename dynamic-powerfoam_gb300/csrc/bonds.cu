@@ -7,6 +7,7 @@
 // order and sums them.  Results are deterministic run to run.
 
 #include "common.cuh"
+#include "internal.cuh"
 
 namespace dpf {
 
@@ -38,6 +39,7 @@ struct TrialBondArgs {
     double *normal_end, *offset_end, *fs_end, *mb_end, *fn_end, *mt_end;
     double *wrench;
     int *status;
+    double *linear, *general;   // residual_pass: the linearisation's planes and its flag
 };
 
 // The three carried vectors where the committed normal is not a unit vector
@@ -56,6 +58,18 @@ __device__ __noinline__ void carry_general(d3 n0, d3 n1, d3 spin, d3 &a, d3 &b, 
 // end state is not wanted its guards are tested without forming it: about 240
 // float64 operations against 480 with root, divisions, sincos and rotations
 // written out.  262k sites / 1.9M bonds: 1.50 -> 0.80 ms.
+//
+// kLinearise: what jvp_linear_bonds reads, in planes of one double a bond.
+__device__ __forceinline__ void put(const TrialBondArgs &a, int plane, int64_t b, double v) {
+    a.linear[plane * a.m + b] = v;
+}
+__device__ __forceinline__ void put(const TrialBondArgs &a, int plane, int64_t b, d3 v) {
+    put(a, plane, b, v.x);
+    put(a, plane + 1, b, v.y);
+    put(a, plane + 2, b, v.z);
+}
+
+template <bool kLinearise>
 __global__ void __launch_bounds__(128) trial_bonds(TrialBondArgs a) {
     const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (b >= a.m) return;
@@ -73,7 +87,8 @@ __global__ void __launch_bounds__(128) trial_bonds(TrialBondArgs a) {
     const d3 dm = mj - mi;
     const double lm2 = dot(dm, dm);
     if (lm2 <= 1e-24) flags |= DPF_ERR_COINCIDENT;
-    const d3 nm = rsqrt(lm2) * dm;
+    const double inv = rsqrt(lm2);
+    const d3 nm = inv * dm;
     const d3 half_spin = 0.25 * (wi + wj);
     const d3 n0 = ld3(a.h.normal, b);
     d3 offset = ld3(a.h.offset, b), fs0 = ld3(a.h.fs, b), mb0 = ld3(a.h.mb, b);
@@ -82,11 +97,21 @@ __global__ void __launch_bounds__(128) trial_bonds(TrialBondArgs a) {
         if (!is_zero(offset)) offset = apply(to_mid, offset);
         fs0 = apply(to_mid, fs0);
         mb0 = apply(to_mid, mb0);
+        if (kLinearise) {
+            put(a, 4, b, to_mid.sum);
+            put(a, 7, b, 2.0 * to_mid.r * to_mid.r);
+            put(a, 8, b, 2.0 * to_mid.sh * to_mid.ch);
+            put(a, 9, b, 2.0 * to_mid.sh * to_mid.sh);
+            put(a, 10, b, to_mid.r);
+            put(a, 11, b, 2.0 * to_mid.half * to_mid.r);
+        }
     } else {
         carry_general(n0, nm, half_spin, offset, fs0, mb0, flags);
+        if (kLinearise) *a.general = 1.0;
     }
     // levers of the contact (mi + mj)/2 + (radi - radj)/2 nm + offset
-    const d3 lever = axpy(0.5 * (a.h.radii[i] - a.h.radii[j]), nm, offset);
+    const double rad = 0.5 * (a.h.radii[i] - a.h.radii[j]);
+    const d3 lever = axpy(rad, nm, offset);
     const d3 ri = axpy(0.5, dm, lever), rj = axpy(-0.5, dm, lever);
     const d3 du = cross_sub(cross_add(uj - ui, wj, rj), wi, ri);
     const d3 dw = wj - wi;
@@ -94,8 +119,30 @@ __global__ void __launch_bounds__(128) trial_bonds(TrialBondArgs a) {
     const double kn = a.k.kn[b], ks = a.k.ks[b], kb = a.k.kb[b], kt = a.k.kt[b];
     const double fn_c = a.h.fn[b], mt_c = a.h.mt[b];
     const d3 slide = ks * axpy(-dn, nm, du), bend = kb * axpy(-twist, nm, dw);
-    const d3 f = axpy(fma(0.5 * kn, dn, fn_c), nm, axpy(0.5, slide, fs0));
-    const d3 couple = axpy(fma(0.5 * kt, twist, mt_c), nm, axpy(0.5, bend, mb0));
+    const double fn_mid = fma(0.5 * kn, dn, fn_c), mt_mid = fma(0.5 * kt, twist, mt_c);
+    const d3 f = axpy(fn_mid, nm, axpy(0.5, slide, fs0));
+    const d3 couple = axpy(mt_mid, nm, axpy(0.5, bend, mb0));
+    if (kLinearise) {
+        const double hks = 0.5 * ks, hkb = 0.5 * kb;
+        put(a, 0, b, nm);
+        put(a, 3, b, 0.5 * inv);
+        put(a, 12, b, half_spin);
+        put(a, 15, b, offset);
+        put(a, 18, b, fs0);
+        put(a, 21, b, mb0);
+        put(a, 24, b, rad);
+        put(a, 25, b, ri);
+        put(a, 28, b, rj);
+        put(a, 31, b, du);
+        put(a, 34, b, dw);
+        put(a, 37, b, f);
+        put(a, 40, b, fma(-hks, dn, fn_mid));
+        put(a, 41, b, fma(-hkb, twist, mt_mid));
+        put(a, 42, b, hks);
+        put(a, 43, b, hkb);
+        put(a, 44, b, 0.5 * kn - hks);
+        put(a, 45, b, 0.5 * kt - hkb);
+    }
     if (a.wrench) store_wrench(a.wrench, b, f, cross_add(couple, ri, f), cross_sub(-couple, rj, f));
     if (a.n) st3(a.n, b, nm);
     if (a.ri) st3(a.ri, b, ri);
@@ -345,6 +392,49 @@ __global__ void __launch_bounds__(128) jvp_bonds(JvpBondArgs a) {
                  cross_sub(cross_sub(-dcouple, drj, f), rj, df));
 }
 
+// The same product from the linearisation that the residual pass at y stored:
+// everything that does not depend on the direction (geometry, transport, carried
+// forces, levers, the force itself) is read instead of formed again, about 160
+// float64 operations a bond and 46 coalesced doubles, whose loads hide behind
+// them.  With dri = e/4 + dl and drj = -e/4 + dl the spins' share of the relative
+// motion is dw x dl - spin x e.  A step's FGMRES takes two or three of these an
+// iterate for one linearisation (its stores: 5% of the trial pass).
+// 262k sites: 1.20 -> 0.56 ms; a step there 27.3 -> 23.5 ms, at 37k sites 4.5 -> 3.75 ms.
+__global__ void __launch_bounds__(128) jvp_linear_bonds(int64_t m, const int64_t *edges, const double *lin,
+                                                        const double *direction, double *wrench) {
+    const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (b >= m) return;
+    const auto get = [&](int plane) { return __ldg(lin + plane * m + b); };
+    const auto get3 = [&](int plane) { return mk(get(plane), get(plane + 1), get(plane + 2)); };
+    int64_t i, j;
+    edge(edges, b, i, j);
+    const d3 dui = ld3(direction + 6 * i), dwi = ld3(direction + 6 * i + 3);
+    const d3 duj = ld3(direction + 6 * j), dwj = ld3(direction + 6 * j + 3);
+    const d3 n = get3(0), sum = get3(4), spin = get3(12);
+    const d3 e = duj - dui, dd = get(3) * e;
+    const d3 dn = axpy(-dot(n, dd), n, dd);
+    // angular velocity of the transport (turn_rate)
+    const double r = get(10);
+    const d3 arc = get(7) * cross(sum, dn);
+    const double dth = r * dot_add(fma(-get(11), dot(sum, dn), 0.25 * dot(sum, dwi + dwj)), spin, dn);
+    const double sine = get(8);
+    const d3 side = axpy(sine, arc, get(9) * cross_add(dn, n, arc));
+    const d3 rate = cross_add(axpy(dth, n, axpy(sine, dn, arc)), n, side);
+    d3 dlever = get(24) * dn;
+    const d3 offset = get3(15);
+    if (!is_zero(offset)) dlever = cross_add(dlever, rate, offset);
+    const d3 ri = get3(25), rj = get3(28), dw = get3(34), ddw = dwj - dwi;
+    const d3 ddu = cross_sub(cross_add(cross_sub(cross_add(e, dwj, rj), dwi, ri), dw, dlever), spin, e);
+    const double dnd = dot_add(dot(get3(31), dn), ddu, n);
+    const double dtw = dot_add(dot(dw, dn), ddw, n);
+    const d3 f = get3(37);
+    const d3 df = axpy(get(40), dn, axpy(get(44) * dnd, n, cross_add(get(42) * ddu, rate, get3(18))));
+    const d3 dcouple = axpy(get(41), dn, axpy(get(45) * dtw, n, cross_add(get(43) * ddw, rate, get3(21))));
+    const d3 dri = axpy(0.25, e, dlever), drj = axpy(-0.25, e, dlever);
+    store_wrench(wrench, b, df, cross_add(cross_add(dcouple, dri, f), ri, df),
+                 cross_sub(cross_sub(-dcouple, drj, f), rj, df));
+}
+
 // Site pass of the JVP: out = M d - dt^2/2 g, fixed rows d; optional P(.)/units.
 // Two neighbouring lanes a site, as in site_residual.
 struct SiteJvpArgs {
@@ -354,6 +444,7 @@ struct SiteJvpArgs {
     const uint8_t *fixed;
     double half_dt2;
     double *out;
+    int scaled;     // the direction is in the scaled coordinates (d = units direction)
 };
 
 __global__ void __launch_bounds__(kThreads) site_jvp(SiteJvpArgs a) {
@@ -367,7 +458,7 @@ __global__ void __launch_bounds__(kThreads) site_jvp(SiteJvpArgs a) {
         d3 d = ld3(a.direction + at);
         if (a.units) {
             u = ld3(a.units + at);
-            d = mk(d.x * u.x, d.y * u.y, d.z * u.z);
+            if (a.scaled) d = mk(d.x * u.x, d.y * u.y, d.z * u.z);
         }
         const d3 m = ld3(a.mass + at);
         r = a.fixed[s] ? d
@@ -465,8 +556,11 @@ __device__ __forceinline__ void add_bond_block(BlockSum &B, d3 n, d3 r, double k
     B.kr = B.kr + kr;
 }
 
+// kLanes neighbouring lanes share a site: each sums every kLanes-th of its ends,
+// then all hold the site's block.
+template <int kLanes>
 __device__ __forceinline__ void site_diagonal(const int32_t *ptr, const int32_t *inc, const dpf_stiffness &k,
-                                              const dpf_tangent &t, int64_t s, double D[36]) {
+                                              const dpf_tangent &t, int64_t s, int lane, double D[36]) {
     BlockSum B;
 #pragma unroll
     for (int c = 0; c < 6; ++c) B.uu[c] = B.ww[c] = 0.0;
@@ -474,12 +568,20 @@ __device__ __forceinline__ void site_diagonal(const int32_t *ptr, const int32_t 
     for (int c = 0; c < 9; ++c) B.uw[c] = 0.0;
     B.k = B.w = 0.0;
     B.kr = mk(0.0, 0.0, 0.0);
-    const int e1 = ptr[s + 1];
-    for (int e = ptr[s]; e < e1; ++e) {
+    const int e1 = s < 0 ? 0 : ptr[s + 1];
+    for (int e = s < 0 ? 0 : ptr[s] + lane; e < e1; e += kLanes) {
         const int v = inc[e];
         const int64_t b = v >= 0 ? v : ~v;
         const d3 r = ld3(v >= 0 ? t.ri : t.rj, b);
         add_bond_block(B, ld3(t.n, b), r, k.kn[b], k.ks[b], k.kb[b], k.kt[b]);
+    }
+    if (kLanes > 1) {
+        double *all = reinterpret_cast<double *>(&B);
+#pragma unroll
+        for (int o = 1; o < kLanes; o <<= 1)
+#pragma unroll
+            for (int c = 0; c < (int)(sizeof(B) / sizeof(double)); ++c)
+                all[c] += __shfl_xor_sync(0xffffffffu, all[c], o);
     }
     const int at[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
     const double S[9] = {0.0, -B.kr.z, B.kr.y, B.kr.z, 0.0, -B.kr.x, -B.kr.y, B.kr.x, 0.0};
@@ -507,15 +609,30 @@ struct ScalingArgs {
     double *diagonal, *block, *P, *units;
 };
 
-__global__ void __launch_bounds__(128) scaling_sites(ScalingArgs a) {
-    const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (s >= a.n) return;
-    double D[36];
-    site_diagonal(a.ptr, a.inc, a.k, a.t, s, D);
-    if (a.diagonal) {
+// Lane `lane` of a site's kLanes writes every kLanes-th entry.
+template <int kLanes>
+__device__ __forceinline__ void put_block(double *out, int64_t s, int lane, const double M[36]) {
 #pragma unroll
-        for (int c = 0; c < 36; ++c) a.diagonal[36 * s + c] = D[c];
-    }
+    for (int c = 0; c < 36; ++c)
+        if (kLanes == 1 || c % kLanes == lane) out[36 * s + c] = M[c];
+}
+
+// One lane a site where there are sites for every scheduler; four where there
+// are not: a warp instruction of the float64 pipe takes 64 cycles of its
+// scheduler's share however few warps there are, so a site's 1,300 operations
+// one after the other took 57 us at 512 sites.  With four lanes (the ends dealt
+// among them, the inverse formed by each): 29 us; 8k sites 64 -> 43 us, 10.6k sites 60 (one
+// lane: 62).
+template <int kLanes>
+__global__ void __launch_bounds__(128) scaling_sites(ScalingArgs a) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, s = t / kLanes;
+    const int lane = (int)(t % kLanes);
+    const bool live = s < a.n;
+    if (kLanes == 1 && !live) return;
+    double D[36];
+    site_diagonal<kLanes>(a.ptr, a.inc, a.k, a.t, live ? s : -1, lane, D);
+    if (!live) return;
+    if (a.diagonal) put_block<kLanes>(a.diagonal, s, lane, D);
     if (!a.P && !a.block) return;
     const bool fx = a.fixed[s] != 0;
     double B[36];
@@ -526,32 +643,31 @@ __global__ void __launch_bounds__(128) scaling_sites(ScalingArgs a) {
             const double val = (p == q ? a.mass[6 * s + p] : 0.0) + a.alpha * D[6 * p + q];
             B[6 * p + q] = fx ? (p == q ? 1.0 : 0.0) : val;
         }
-    if (a.block) {
-#pragma unroll
-        for (int c = 0; c < 36; ++c) a.block[36 * s + c] = B[c];
-    }
+    if (a.block) put_block<kLanes>(a.block, s, lane, B);
     if (a.P) {
         double P[36];
         spd_inverse6(B, P);
-#pragma unroll
-        for (int c = 0; c < 36; ++c) a.P[36 * s + c] = P[c];
+        put_block<kLanes>(a.P, s, lane, P);
     }
-    if (a.units) {
+    if (a.units && lane == 0) {
         const double r = fx ? 1.0 : a.radii[s];
 #pragma unroll
         for (int c = 0; c < 6; ++c) a.units[6 * s + c] = c < 3 ? r : 1.0;
     }
 }
 
+template <int kLanes>
 __global__ void __launch_bounds__(128) diagonal_sites(int64_t n, const int32_t *ptr, const int32_t *inc,
                                                       dpf_stiffness k, dpf_tangent t, double *out) {
-    const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (s >= n) return;
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, s = i / kLanes;
+    const int lane = (int)(i % kLanes);
     double D[36];
-    site_diagonal(ptr, inc, k, t, s, D);
-#pragma unroll
-    for (int c = 0; c < 36; ++c) out[36 * s + c] = D[c];
+    site_diagonal<kLanes>(ptr, inc, k, t, s < n ? s : -1, lane, D);
+    if (s < n) put_block<kLanes>(out, s, lane, D);
 }
+
+// Sites from which one lane each fills the machine.
+constexpr int64_t kFewSites = 12288;
 
 // ---------------------------------------------------------------------------
 // Loads of the committed state (experiments/bonded_dem_finite_gpu.py:82-85).
@@ -660,8 +776,10 @@ int dpf_stiffness_apply(const dpf_graph *g, const dpf_stiffness *k, const dpf_ta
 int dpf_diagonal_blocks(const dpf_graph *g, const dpf_stiffness *k, const dpf_tangent *t, double *diagonal,
                         void *stream) {
     if (!graph_ok(g) || !k || !t || !diagonal) return DPF_ERR_ARGUMENT;
-    diagonal_sites<<<blocks_for(g->n_sites, 128), 128, 0, (cudaStream_t)stream>>>(
-        g->n_sites, g->inc_ptr, g->inc_bond, *k, *t, diagonal);
+    const int lanes = g->n_sites < kFewSites ? 4 : 1, threads = spread_threads(lanes * g->n_sites);
+    (lanes == 4 ? diagonal_sites<4> : diagonal_sites<1>)<<<blocks_for(lanes * g->n_sites, threads), threads, 0,
+                                                           (cudaStream_t)stream>>>(g->n_sites, g->inc_ptr, g->inc_bond,
+                                                                                   *k, *t, diagonal);
     DPF_CHECK_LAUNCH();
     return DPF_OK;
 }
@@ -672,14 +790,17 @@ int dpf_prepare_scaling(const dpf_graph *g, const dpf_stiffness *k, const dpf_ta
     if (!graph_ok(g) || !k || !t || !mass || !fixed || !radii || !preconditioner) return DPF_ERR_ARGUMENT;
     ScalingArgs a{g->n_sites, g->inc_ptr, g->inc_bond, *k, *t, mass, radii, fixed, 0.25 * dt * dt,
                   diagonal, block, preconditioner, units};
-    scaling_sites<<<blocks_for(g->n_sites, 128), 128, 0, (cudaStream_t)stream>>>(a);
+    const int lanes = g->n_sites < kFewSites ? 4 : 1, threads = spread_threads(lanes * g->n_sites);
+    (lanes == 4 ? scaling_sites<4> : scaling_sites<1>)<<<blocks_for(lanes * g->n_sites, threads), threads, 0,
+                                                         (cudaStream_t)stream>>>(a);
     DPF_CHECK_LAUNCH();
     return DPF_OK;
 }
 
 static int launch_trial_bonds(const dpf_graph *g, const dpf_stiffness *k, const dpf_history *h, const double *y,
                               const double *mid, const double *end, int want_end, const dpf_trial_out *out,
-                              double *wrench, int *status, cudaStream_t st) {
+                              double *wrench, int *status, cudaStream_t st, double *linear = nullptr,
+                              double *general = nullptr) {
     if (!g->n_bonds) return DPF_OK;
     TrialBondArgs a{};
     a.m = g->n_bonds;
@@ -703,7 +824,13 @@ static int launch_trial_bonds(const dpf_graph *g, const dpf_stiffness *k, const 
     }
     a.wrench = wrench;
     a.status = status;
-    trial_bonds<<<blocks_for(g->n_bonds, 128), 128, 0, st>>>(a);
+    a.linear = linear;
+    a.general = general;
+    const int threads = spread_threads(g->n_bonds);
+    if (linear)
+        trial_bonds<true><<<blocks_for(g->n_bonds, threads), threads, 0, st>>>(a);
+    else
+        trial_bonds<false><<<blocks_for(g->n_bonds, threads), threads, 0, st>>>(a);
     return DPF_OK;
 }
 
@@ -732,7 +859,8 @@ int dpf_trial(const dpf_graph *g, const dpf_stiffness *k, const dpf_history *h, 
     a.force = out->force;
     a.x_end = want_end ? out->x_end : nullptr;
     a.status = status;
-    site_residual<<<blocks_for(2 * g->n_sites, kThreads), kThreads, 0, st>>>(a);
+    const int threads = spread_threads(2 * g->n_sites);
+    site_residual<<<blocks_for(2 * g->n_sites, threads), threads, 0, st>>>(a);
     DPF_CHECK_LAUNCH();
     return DPF_OK;
 }
@@ -746,15 +874,15 @@ int dpf_commit_state(const dpf_graph *g, const dpf_stiffness *k, const dpf_histo
     return DPF_OK;
 }
 
-int dpf_residual(const dpf_graph *g, const dpf_stiffness *k, const dpf_history *h, const double *y,
-                 const double *v, const double *external, const double *mass, const uint8_t *fixed, double dt,
-                 const dpf_trial_out *trial, const double *preconditioner, const double *units, double *residual,
-                 double *scaled, double *norms, double *wrench, double *partials, int *status, void *stream) {
+static int residual_launch(const dpf_graph *g, const dpf_stiffness *k, const dpf_history *h, const double *y,
+                           const double *v, const double *external, const double *mass, const uint8_t *fixed,
+                           double dt, const dpf_trial_out *trial, const double *preconditioner, const double *units,
+                           double *residual, double *scaled, double *norms, double *wrench, double *partials,
+                           int *status, double *linear, double *general, cudaStream_t st) {
     if (!graph_ok(g) || !k || !history_ok(h, g->n_bonds) || !y || !v || !external || !mass || !fixed || !residual ||
         !status || (g->n_bonds && !wrench) || (norms && !partials) || (preconditioner && !units))
         return DPF_ERR_ARGUMENT;
-    cudaStream_t st = (cudaStream_t)stream;
-    launch_trial_bonds(g, k, h, y, nullptr, nullptr, 0, trial, wrench, status, st);
+    launch_trial_bonds(g, k, h, y, nullptr, nullptr, 0, trial, wrench, status, st, linear, general);
     SiteResidualArgs a{};
     a.n = g->n_sites;
     a.ptr = g->inc_ptr;
@@ -776,11 +904,20 @@ int dpf_residual(const dpf_graph *g, const dpf_stiffness *k, const dpf_history *
     a.norms = norms;
     a.partials = partials;
     a.status = status;
-    int grid = blocks_for(2 * g->n_sites, kThreads);
+    const int threads = reduce_threads(2 * g->n_sites);
+    int grid = blocks_for(2 * g->n_sites, threads);
     if (grid > kMaxReduceBlocks) grid = kMaxReduceBlocks;
-    site_residual<<<grid, kThreads, 0, st>>>(a);
+    site_residual<<<grid, threads, 0, st>>>(a);
     DPF_CHECK_LAUNCH();
     return DPF_OK;
+}
+
+int dpf_residual(const dpf_graph *g, const dpf_stiffness *k, const dpf_history *h, const double *y,
+                 const double *v, const double *external, const double *mass, const uint8_t *fixed, double dt,
+                 const dpf_trial_out *trial, const double *preconditioner, const double *units, double *residual,
+                 double *scaled, double *norms, double *wrench, double *partials, int *status, void *stream) {
+    return residual_launch(g, k, h, y, v, external, mass, fixed, dt, trial, preconditioner, units, residual, scaled,
+                           norms, wrench, partials, status, nullptr, nullptr, (cudaStream_t)stream);
 }
 
 int dpf_jacobian_vector(const dpf_graph *g, const dpf_stiffness *k, const dpf_history *h, const double *y,
@@ -793,11 +930,13 @@ int dpf_jacobian_vector(const dpf_graph *g, const dpf_stiffness *k, const dpf_hi
     cudaStream_t st = (cudaStream_t)stream;
     if (g->n_bonds) {
         JvpBondArgs a{g->n_bonds, g->edges, *k, *h, y, direction, units, wrench};
-        jvp_bonds<<<blocks_for(g->n_bonds, 128), 128, 0, st>>>(a);
+        const int threads = spread_threads(g->n_bonds);
+        jvp_bonds<<<blocks_for(g->n_bonds, threads), threads, 0, st>>>(a);
     }
     SiteJvpArgs s{g->n_sites, g->inc_ptr, g->inc_bond, wrench, direction, units, mass, preconditioner, fixed,
-                  0.5 * dt * dt, out};
-    site_jvp<<<blocks_for(2 * g->n_sites, kThreads), kThreads, 0, st>>>(s);
+                  0.5 * dt * dt, out, 1};
+    const int threads = spread_threads(2 * g->n_sites);
+    site_jvp<<<blocks_for(2 * g->n_sites, threads), threads, 0, st>>>(s);
     DPF_CHECK_LAUNCH();
     return DPF_OK;
 }
@@ -824,8 +963,7 @@ int dpf_loads(const dpf_graph *g, const dpf_history *h, double *out, double *wre
     if (!graph_ok(g) || !history_ok(h, g->n_bonds) || !out || (g->n_bonds && !wrench)) return DPF_ERR_ARGUMENT;
     cudaStream_t st = (cudaStream_t)stream;
     if (g->n_bonds)
-        loads_bonds<<<blocks_for(g->n_bonds, kThreads), kThreads, 0, st>>>(g->n_bonds, g->edges, *h, wrench,
-                                                                            nullptr);
+        loads_bonds<<<blocks_for(g->n_bonds, 128), 128, 0, st>>>(g->n_bonds, g->edges, *h, wrench, nullptr);
     site_gather<<<blocks_for(2 * g->n_sites, kThreads), kThreads, 0, st>>>(g->n_sites, g->inc_ptr, g->inc_bond,
                                                                         wrench, out);
     DPF_CHECK_LAUNCH();
@@ -833,6 +971,35 @@ int dpf_loads(const dpf_graph *g, const dpf_history *h, double *out, double *wre
 }
 
 }  // extern "C"
+
+namespace dpf {
+
+int residual_pass(const dpf_graph *g, const dpf_stiffness *k, const dpf_history *h, const double *y, const double *v,
+                  const double *external, const double *mass, const uint8_t *fixed, double dt,
+                  const dpf_trial_out *trial, const double *preconditioner, const double *units, double *residual,
+                  double *norms, double *wrench, double *partials, int *status, double *linear, double *general,
+                  cudaStream_t stream) {
+    return residual_launch(g, k, h, y, v, external, mass, fixed, dt, trial, preconditioner, units, residual, nullptr,
+                           norms, wrench, partials, status, linear, general, stream);
+}
+
+int jacobian_pass(const dpf_graph *g, const double *linear, const double *direction, const double *mass,
+                  const uint8_t *fixed, double dt, const double *units, const double *preconditioner, double *out,
+                  double *wrench, cudaStream_t stream) {
+    if (g->n_bonds) {
+        const int threads = spread_threads(g->n_bonds);
+        jvp_linear_bonds<<<blocks_for(g->n_bonds, threads), threads, 0, stream>>>(g->n_bonds, g->edges, linear,
+                                                                                  direction, wrench);
+    }
+    SiteJvpArgs s{g->n_sites, g->inc_ptr, g->inc_bond, wrench, direction, units, mass, preconditioner, fixed,
+                  0.5 * dt * dt, out, 0};
+    const int threads = spread_threads(2 * g->n_sites);
+    site_jvp<<<blocks_for(2 * g->n_sites, threads), threads, 0, stream>>>(s);
+    DPF_CHECK_LAUNCH();
+    return DPF_OK;
+}
+
+}  // namespace dpf
 
 // ---------------------------------------------------------------------------
 // K q without any allocation by anyone: the bond-wrench scratch lives in a

@@ -539,10 +539,13 @@ int dpf_block_pcg(const dpf_graph *g, const dpf_stiffness *k, const dpf_tangent 
     cudaStream_t st = (cudaStream_t)stream;
     DeviceInfo &info_d = device_info();
     if (info_d.sms <= 0 || info_d.per_sm <= 0) return DPF_ERR_CUDA;
-    const int64_t work = 2 * g->n_sites > g->n_bonds ? 2 * g->n_sites : g->n_bonds;
-    int64_t cap = (int64_t)info_d.sms * info_d.per_sm;
+    // the grid of csrc/solver.cu's elastic PCG, and why
+    const int64_t items = 2 * g->n_sites > g->n_bonds ? 2 * g->n_sites : g->n_bonds;
+    const bool few = items <= 512 * (int64_t)info_d.sms;
+    const int threads = few ? 128 : kThreads;
+    int64_t cap = (int64_t)info_d.sms * (few ? 1 : info_d.per_sm < 2 ? info_d.per_sm : 2);
     if (cap > kMaxBlocks) cap = kMaxBlocks;
-    int64_t want = blocks_for(work, kThreads);
+    const int64_t want = blocks_for(items, threads);
     const int grid = (int)(want < cap ? (want < 1 ? 1 : want) : cap);
     const int64_t n6 = 6 * g->n_sites;
     BlockPcgArgs a{};
@@ -569,7 +572,7 @@ int dpf_block_pcg(const dpf_graph *g, const dpf_stiffness *k, const dpf_tangent 
         return DPF_ERR_CUDA;
     }
     void *args[] = {&a};
-    if (cudaLaunchCooperativeKernel((const void *)block_pcg_kernel, grid, kThreads, args, 0, st) != cudaSuccess) {
+    if (cudaLaunchCooperativeKernel((const void *)block_pcg_kernel, grid, threads, args, 0, st) != cudaSuccess) {
         cudaGetLastError();
         return DPF_ERR_CUDA;
     }

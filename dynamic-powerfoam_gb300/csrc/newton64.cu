@@ -20,6 +20,7 @@
 #include <cstring>
 
 #include "common.cuh"
+#include "internal.cuh"
 
 namespace dpf {
 namespace newton64 {
@@ -116,8 +117,9 @@ struct Coefficients {
     double c[kMaxColumns];
 };
 
-// x (+)= sum c_k rows_k, then the Newton correction units x (zero rows on fixed
-// sites) and the full-step candidate y + correction.
+// x (+)= sum c_k rows_k, then the Newton correction (units x where the rows are in
+// the scaled coordinates; zero rows on fixed sites) and the full-step candidate
+// y + correction.
 __global__ void __launch_bounds__(kThreads) candidate_kernel(int64_t len, const double *rows, int64_t ld, int count,
                                                              Coefficients coef, int add, double *x,
                                                              const double *units, const uint8_t *fixed,
@@ -128,7 +130,7 @@ __global__ void __launch_bounds__(kThreads) candidate_kernel(int64_t len, const 
         for (int k = 0; k < count; ++k) v += rows[k * ld + e] * coef.c[k];
         if (add) v += x[e];
         x[e] = v;
-        const double c = fixed[e / 6] ? 0.0 : units[e] * v;
+        const double c = fixed[e / 6] ? 0.0 : units ? units[e] * v : v;
         correction[e] = c;
         candidate[e] = y[e] + c;
     }
@@ -183,19 +185,22 @@ struct Step {
     cudaStream_t st;
     int64_t n, n6, m;
     double *y, *cand, *r, *r_cand, *scaled, *x, *corr;
-    double *host;     // pinned: [0..4) norms, [4..6) scales, [16..80) h column
+    double *host;     // pinned: [0..4) norms, [4..6) scales, [6] normals without unit length, [16..80) h column
     int *host_int;    // [0] status, [1] inner
     double rhs_scale = -1.0;
     dpf_tangent tangent;
     int arnoldi_blocks = 0;
+    // elastic preconditioning with a stored linearisation: the preconditioner's rows
+    // are in the coordinates of y (x instead of x / units), as the product wants them
+    bool raw = false;
 
     int ran(int kernels, int rc) {
         if (!rc) info->launches += kernels;
         return rc;
     }
 
-    int fetch(bool scales) {
-        if (cudaMemcpyAsync(host, s->scalars, (scales ? 6 : 3) * sizeof(double), cudaMemcpyDeviceToHost, st) ||
+    int fetch(bool first) {
+        if (cudaMemcpyAsync(host, s->scalars, (first ? 7 : 3) * sizeof(double), cudaMemcpyDeviceToHost, st) ||
             cudaMemcpyAsync(host_int, s->status, sizeof(int), cudaMemcpyDeviceToHost, st))
             return DPF_ERR_CUDA;
         return cudaStreamSynchronize(st) == cudaSuccess ? DPF_OK : DPF_ERR_CUDA;
@@ -209,10 +214,11 @@ struct Step {
         t.n = s->n;
         t.ri = s->ri;
         t.rj = s->rj;
-        return ran(m ? 2 : 1, dpf_residual(s->graph, &s->stiffness, &a->history, yy, a->v_in, a->external, s->mass,
-                                           s->fixed, a->dt, &t, use_p ? s->preconditioner : nullptr,
-                                           use_p ? s->units : nullptr, out, nullptr, use_p ? s->scalars : nullptr,
-                                           s->wrench, s->partials, s->status, st));
+        return ran(m ? 2 : 1, dpf::residual_pass(s->graph, &s->stiffness, &a->history, yy, a->v_in, a->external,
+                                                 s->mass, s->fixed, a->dt, &t, use_p ? s->preconditioner : nullptr,
+                                                 use_p ? s->units : nullptr, out, use_p ? s->scalars : nullptr,
+                                                 s->wrench, s->partials, s->status, s->elastic ? s->linear : nullptr,
+                                                 s->scalars + 6, st));
     }
 
     // blocks and scaling of the tangent, then P r / units and its norms
@@ -255,14 +261,14 @@ struct Step {
         *relative = 0.0;
         *singular = false;
         if (norm == 0.0) return candidate(nullptr, nullptr, 0, false);
-        double H[65 * 64], raw[65 * 64], cs[64], sn[64], g[65], coef[64], left[65];
+        double H[65 * 64], entries[65 * 64], cs[64], sn[64], g[65], coef[64], left[65];
         const double *start = scaled;
         double sign = -1.0, g0 = norm;
         bool add = false;
         while (*krylov < 256) {
             const int width = 256 - *krylov < s->krylov_width ? 256 - *krylov : s->krylov_width;
             std::memset(H, 0, sizeof H);
-            std::memset(raw, 0, sizeof raw);
+            std::memset(entries, 0, sizeof entries);
             std::memset(g, 0, sizeof g);
             g[0] = g0;
             int rc = ran(1, dpf_axpby(n6, sign / g0, start, 0.0, start, s->basis, st));
@@ -271,15 +277,18 @@ struct Step {
             for (int j = 0; j < width; ++j) {
                 double *v = s->basis + (int64_t)j * n6, *z = s->transformed + (int64_t)j * n6;
                 if (s->elastic) {
-                    rc = ran(1, dpf_elastic_precondition(s->graph, &s->stiffness, &tangent, s->mass, s->fixed, s->block,
-                                                         s->preconditioner, s->units, v, a->dt, 0.03, 80, z, s->inner,
-                                                         s->wrench, s->workspace, s->barrier, s->status, st));
+                    rc = ran(1, dpf::elastic_pass(s->graph, &s->stiffness, &tangent, s->mass, s->fixed, s->block,
+                                                  s->preconditioner, s->units, v, a->dt, 0.03, 80, z, s->inner,
+                                                  s->wrench, s->workspace, s->barrier, s->status, raw, st));
                     if (rc) return rc;
                 } else {
                     z = v;
                 }
-                rc = ran(m ? 2 : 1, dpf_jacobian_vector(s->graph, &s->stiffness, &a->history, y, z, s->mass, s->fixed,
-                                                        a->dt, s->units, s->preconditioner, s->w, s->wrench, st));
+                rc = ran(m ? 2 : 1,
+                         raw ? dpf::jacobian_pass(s->graph, s->linear, z, s->mass, s->fixed, a->dt, s->units,
+                                                  s->preconditioner, s->w, s->wrench, st)
+                             : dpf_jacobian_vector(s->graph, &s->stiffness, &a->history, y, z, s->mass, s->fixed,
+                                                   a->dt, s->units, s->preconditioner, s->w, s->wrench, st));
                 if (rc) return rc;
                 rc = arnoldi(j);
                 if (rc) return rc;
@@ -287,7 +296,7 @@ struct Step {
                 if (cudaMemcpyAsync(column, s->h, (j + 2) * sizeof(double), cudaMemcpyDeviceToHost, st) ||
                     cudaStreamSynchronize(st))
                     return DPF_ERR_CUDA;
-                for (int i = 0; i <= j + 1; ++i) H[i * 64 + j] = raw[i * 64 + j] = column[i];
+                for (int i = 0; i <= j + 1; ++i) H[i * 64 + j] = entries[i * 64 + j] = column[i];
                 const bool breakdown = column[j + 1] < 1e-14;
                 for (int i = 0; i < j; ++i) {
                     const double hi = H[i * 64 + j], hj = H[(i + 1) * 64 + j];
@@ -320,7 +329,7 @@ struct Step {
             double sum = 0.0;
             for (int i = 0; i <= k; ++i) {
                 double acc = i == 0 ? g0 : 0.0;
-                for (int c = 0; c < k; ++c) acc -= raw[i * 64 + c] * coef[c];
+                for (int c = 0; c < k; ++c) acc -= entries[i * 64 + c] * coef[c];
                 left[i] = acc;
                 sum += acc * acc;
             }
@@ -328,7 +337,7 @@ struct Step {
             if (*relative <= 1.05 * a->linear_tolerance) return DPF_OK;
             if (*krylov >= 256) break;
             // restart from V left (a breakdown leaves no last row, whose share is below 1e-14)
-            const bool last = raw[k * 64 + k - 1] >= 1e-14;
+            const bool last = entries[k * 64 + k - 1] >= 1e-14;
             if (cudaMemsetAsync(s->residual, 0, n6 * sizeof(double), st)) return DPF_ERR_CUDA;
             rc = ran(1, dpf_combine_rows(n6, s->basis, n6, last ? k + 1 : k, left, s->residual, st));
             if (rc) return rc;
@@ -347,8 +356,8 @@ struct Step {
     int candidate(const double *rows, const double *coef, int count, bool add) {
         Coefficients c{};
         for (int k = 0; k < count; ++k) c.c[k] = coef[k];
-        candidate_kernel<<<reduce_grid(n6), kThreads, 0, st>>>(n6, rows, n6, count, c, add ? 1 : 0, x, s->units,
-                                                               s->fixed, y, corr, cand);
+        candidate_kernel<<<reduce_grid(n6), kThreads, 0, st>>>(n6, rows, n6, count, c, add ? 1 : 0, x,
+                                                               raw ? nullptr : s->units, s->fixed, y, corr, cand);
         return ran(1, cudaGetLastError() == cudaSuccess ? DPF_OK : DPF_ERR_CUDA);
     }
 
@@ -379,7 +388,8 @@ struct Step {
     int run() {
         const double dt = a->dt;
         tangent = {s->n, s->ri, s->rj};
-        if (cudaMemsetAsync(s->inner, 0, sizeof(int), st) || cudaMemsetAsync(y, 0, n6 * sizeof(double), st))
+        if (cudaMemsetAsync(s->inner, 0, sizeof(int), st) || cudaMemsetAsync(y, 0, n6 * sizeof(double), st) ||
+            cudaMemsetAsync(s->scalars + 6, 0, sizeof(double), st))
             return DPF_ERR_CUDA;
         // the step's scale (bonded_dem_newton.py:138-139), read with the first norms
         int rc = ran(m ? 2 : 1, dpf_loads(s->graph, &a->history, corr, s->wrench, st));
@@ -404,6 +414,7 @@ struct Step {
                 rhs_scale = host[4];
                 if (0.5 * dt * dt * host[5] > rhs_scale) rhs_scale = 0.5 * dt * dt * host[5];
                 if (1e-30 > rhs_scale) rhs_scale = 1e-30;
+                raw = s->elastic && s->linear && host[6] == 0.0;
             }
             const double relative = host[0] / rhs_scale, local = host[1], merit = host[2];
             info->relative = relative;
@@ -480,6 +491,8 @@ int64_t dpf_newton64_partials_doubles(void) {
     using namespace dpf::newton64;
     return (2 * (int64_t)kMaxColumns + 1) * kMaxBlocks;
 }
+
+int64_t dpf_newton64_linear_doubles(int64_t n_bonds) { return n_bonds < 0 ? 0 : dpf::kLinear * n_bonds; }
 
 int64_t dpf_newton64_struct_size(void) { return (int64_t)sizeof(dpf_newton64); }
 

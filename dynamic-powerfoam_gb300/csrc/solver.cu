@@ -2,6 +2,7 @@
 // as one cooperative launch, the FGMRES Arnoldi building blocks, reductions,
 // the accepted-step update and the energy.
 #include "common.cuh"
+#include "internal.cuh"
 
 namespace dpf {
 
@@ -59,7 +60,7 @@ struct PcgArgs {
     const double *mass, *block, *P, *units, *vector;
     const uint8_t *fixed;
     double alpha_op, tol2;
-    int max_it;
+    int max_it, raw;
     double *out;
     int *iterations;
     double *wrench, *r, *u, *p, *s, *part_a, *part_b;
@@ -170,7 +171,7 @@ __global__ void __launch_bounds__(kThreads) pcg_kernel(PcgArgs a) {
         gamma = following;
     }
     // a thread's own x: no barrier
-    for (s = first; s < a.n; s += step) {
+    for (s = first; s < a.n && !a.raw; s += step) {
         const int64_t at = 6 * s + 3 * half;
         st3(a.out + at, over_units(ld3(a.out + at), ld3(a.units + at)));
     }
@@ -599,21 +600,30 @@ extern "C" {
 
 int64_t dpf_elastic_workspace_doubles(int64_t n_sites) { return 30 * n_sites + 2 * (int64_t)kMaxPcgBlocks; }
 
-int dpf_elastic_precondition(const dpf_graph *g, const dpf_stiffness *k, const dpf_tangent *t, const double *mass,
-                             const uint8_t *fixed, const double *block, const double *preconditioner,
-                             const double *units, const double *vector, double dt, double tolerance,
-                             int max_iterations, double *out, int *iterations, double *wrench, double *workspace,
-                             unsigned *barrier, int *status, void *stream) {
+}  // extern "C"
+
+int dpf::elastic_pass(const dpf_graph *g, const dpf_stiffness *k, const dpf_tangent *t, const double *mass,
+                      const uint8_t *fixed, const double *block, const double *preconditioner, const double *units,
+                      const double *vector, double dt, double tolerance, int max_iterations, double *out,
+                      int *iterations, double *wrench, double *workspace, unsigned *barrier, int *status, bool raw,
+                      cudaStream_t st) {
     if (!g || g->n_sites <= 0 || !g->inc_ptr || (g->n_bonds && !g->inc_bond) || !k || !t || !mass || !fixed ||
         !block ||
         !preconditioner || !units || !vector || !out || !iterations || !workspace || !barrier || !status ||
         max_iterations < 1 || (g->n_bonds && (!wrench || !g->edges)))
         return DPF_ERR_ARGUMENT;
-    cudaStream_t st = (cudaStream_t)stream;
     DeviceInfo &info = device_info();
     if (info.sms <= 0 || info.pcg_blocks_per_sm <= 0) return DPF_ERR_CUDA;
-    int64_t want = blocks_for(2 * g->n_sites > g->n_bonds ? 2 * g->n_sites : g->n_bonds, kThreads);
-    int64_t cap = (int64_t)info.sms * info.pcg_blocks_per_sm;
+    // Few items: one block of 128 an SM, many: two of 256 (us an iteration: 54k
+    // bonds 24.6 with one block of 128, 32.7 with four of 256; 254k bonds 58.1 with
+    // two of 128, 58.7 with one to four of 256; 1.9M bonds 332 with four of 128,
+    // 326 with two of 256).  A grid of more warps than that only waits longer at
+    // the barriers.
+    const int64_t items = 2 * g->n_sites > g->n_bonds ? 2 * g->n_sites : g->n_bonds;
+    const bool few = items <= 512 * (int64_t)info.sms;
+    const int threads = few ? 128 : kThreads;
+    const int64_t want = blocks_for(items, threads);
+    int64_t cap = (int64_t)info.sms * (few ? 1 : info.pcg_blocks_per_sm < 2 ? info.pcg_blocks_per_sm : 2);
     if (cap > kMaxPcgBlocks) cap = kMaxPcgBlocks;
     const int grid = (int)(want < cap ? (want < 1 ? 1 : want) : cap);
     const int64_t n6 = 6 * g->n_sites;
@@ -634,6 +644,7 @@ int dpf_elastic_precondition(const dpf_graph *g, const dpf_stiffness *k, const d
     a.alpha_op = 0.25 * dt * dt;
     a.tol2 = tolerance * tolerance;
     a.max_it = max_iterations;
+    a.raw = raw ? 1 : 0;
     a.out = out;
     a.iterations = iterations;
     a.wrench = wrench;
@@ -647,11 +658,22 @@ int dpf_elastic_precondition(const dpf_graph *g, const dpf_stiffness *k, const d
     a.status = status;
     if (cudaMemsetAsync(barrier, 0, 2 * sizeof(unsigned), st) != cudaSuccess) return DPF_ERR_CUDA;
     void *args[] = {&a};
-    if (cudaLaunchCooperativeKernel((const void *)pcg_kernel, grid, kThreads, args, 0, st) != cudaSuccess) {
+    if (cudaLaunchCooperativeKernel((const void *)pcg_kernel, grid, threads, args, 0, st) != cudaSuccess) {
         cudaGetLastError();
         return DPF_ERR_CUDA;
     }
     return DPF_OK;
+}
+
+extern "C" {
+
+int dpf_elastic_precondition(const dpf_graph *g, const dpf_stiffness *k, const dpf_tangent *t, const double *mass,
+                             const uint8_t *fixed, const double *block, const double *preconditioner,
+                             const double *units, const double *vector, double dt, double tolerance,
+                             int max_iterations, double *out, int *iterations, double *wrench, double *workspace,
+                             unsigned *barrier, int *status, void *stream) {
+    return dpf::elastic_pass(g, k, t, mass, fixed, block, preconditioner, units, vector, dt, tolerance, max_iterations,
+                             out, iterations, wrench, workspace, barrier, status, false, (cudaStream_t)stream);
 }
 
 int dpf_arnoldi_cgs2(int64_t length, double *basis, int64_t ld, int j, double *w, double *h, double *partials,
@@ -764,8 +786,10 @@ int dpf_axpby(int64_t length, double alpha, const double *a, double beta, const 
 int dpf_scale_residual(int64_t n_sites, const double *preconditioner, const double *units, const double *residual,
                        double *scaled, double *norms, double *partials, void *stream) {
     if (n_sites <= 0 || !preconditioner || !units || !residual || (norms && !partials)) return DPF_ERR_ARGUMENT;
-    scale_kernel<<<reduce_grid(2 * n_sites), kThreads, 0, (cudaStream_t)stream>>>(n_sites, preconditioner, units,
-                                                                               residual, scaled, norms, partials);
+    const int threads = reduce_threads(2 * n_sites);
+    const int64_t blocks = blocks_for(2 * n_sites, threads);
+    scale_kernel<<<(int)(blocks < kMaxReduceBlocks ? blocks : kMaxReduceBlocks), threads, 0, (cudaStream_t)stream>>>(
+        n_sites, preconditioner, units, residual, scaled, norms, partials);
     DPF_CHECK_LAUNCH();
     return DPF_OK;
 }

@@ -1164,6 +1164,10 @@ class NewtonBonds(FiniteBonds):
             self._pcg_workspace = e(lib.dpf_elastic_workspace_doubles(n))
         if getattr(self, '_native64_scratch', None) is None:
             self._native64_scratch = (e(_lib.NEWTON64_VECTORS, n, 6), e(2, n, 6), e(lib.dpf_newton64_partials_doubles()))
+            try:
+                self._native64_linear = e(max(1, lib.dpf_newton64_linear_doubles(self.n_bonds)))
+            except torch.cuda.OutOfMemoryError:      # a body that fills the device: products without it
+                self._native64_linear = None
         vectors, pair, partials = self._native64_scratch
         ws = self._krylov
         held = (self.mass, self.fixed, self.radii, self.diagonal, self.block, self.preconditioner, self.units,
@@ -1180,7 +1184,8 @@ class NewtonBonds(FiniteBonds):
             units=p(self.units), wrench=p(self._wrench), workspace=p(self._pcg_workspace), basis=p(ws.basis),
             transformed=p(ws.transformed), w=p(pair[0]), residual=p(pair[1]), h=p(ws.h), krylov_partials=p(partials),
             partials=p(self._partials), scalars=p(self._scalars), status=p(self._status), inner=p(self._inner),
-            barrier=p(self._barrier), vectors=p(vectors), krylov_width=ws.width)
+            barrier=p(self._barrier), vectors=p(vectors), krylov_width=ws.width,
+            linear=_addr(self._native64_linear))
         # the descriptor holds only addresses: keep what they point into alive with it
         self._native64_desc = (key, desc, _lib.NewtonStep(), _lib.NewtonInfo(), held)
         return desc

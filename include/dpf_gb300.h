@@ -956,8 +956,11 @@ typedef struct dpf_newton64 {
     double *host;                  /* pinned host memory, DPF_NEWTON_HOST_DOUBLES */
     int krylov_width;              /* FGMRES restart length, <= 62 */
     int elastic;                   /* 1: elastic PCG preconditioner, 0: block scaling only */
+    double *linear;                /* dpf_newton64_linear_doubles(M): the linearisation at the last evaluated
+                                      increment, which a step's Jacobian products read; NULL: they form it anew */
 } dpf_newton64;
 
+int64_t dpf_newton64_linear_doubles(int64_t n_bonds);
 int64_t dpf_newton64_partials_doubles(void);
 int64_t dpf_newton64_struct_size(void);
 int dpf_newton64_step(const dpf_newton64 *solver, const dpf_newton_step *step, dpf_newton_info *info, void *stream);

@@ -60,6 +60,30 @@ def test_steps_match_the_python_path(m, contacts, preconditioning):
         _same(python, native, travel)
 
 
+@pytest.mark.parametrize('factor', [1., 1.03])
+@pytest.mark.parametrize('linear', [True, False])
+def test_prestressed_steps_with_and_without_the_stored_linearisation(factor, linear):
+    """A random history, committed normals that are unit vectors and not (the stored
+    linearisation does not hold for those), and the products formed anew."""
+    load, python, native = _pair(5, contacts=True)
+    rng = np.random.default_rng(4)
+    m = python.n_bonds
+    h = {name: rng.normal(size=(m, 3))*1e-2 for name in ('fs', 'mb')}
+    h.update({name: rng.normal(size=m)*1e-2 for name in ('fn', 'mt')}, normal=host(python.normal)*factor)
+    for s in (python, native):
+        for name, value in h.items():
+            setattr(s, name, s.tensor(value))
+    if not linear:
+        native._native64_buffers()
+        native._native64_linear = None
+        native._native64_desc = None
+    _, ip = python.step(1e-3, python.tensor(load))
+    _, inn = native.step(1e-3, native.tensor(load))
+    for key in ('nonlinear_iterations', 'krylov_iterations', 'cg_iterations'):
+        assert ip[key] == inn[key], key
+    _same(python, native, float(1e-3*python.v.abs().max()))
+
+
 def test_restarted_krylov_cycles():
     """A stiff step without the elastic preconditioner needs more than one cycle of 32."""
     load, python, native = _pair(6, young=3e7)
