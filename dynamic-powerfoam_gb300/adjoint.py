@@ -11,7 +11,7 @@ Jacobians (limited to 240 free DOFs).  Here the forward step is the CUDA
   per-bond 9 x 12 local Jacobians of the float64 trial);
 * every input adjoint (committed history, per-bond stiffness, initial
   positions, loads, velocities) comes from per-bond vector-Jacobian products
-  of the trial, evaluated with forward-mode dual numbers on the device and
+  of the trial, a hand-written reverse pass on the device, and
   summed per site in the incidence order (deterministic);
 * states are checkpointed every ``checkpoint_every`` steps together with the
   accepted increments; the backward pass replays each segment's commits from
@@ -67,6 +67,7 @@ class _Rollout(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, model, dt, stiffness, loads, *state):
+        ctx.set_materialize_grads(False)
         positions, final, checkpoints, increments = model._run(stiffness.detach(), loads.detach(),
                                                                tuple(t.detach() for t in state), dt)
         ctx.model, ctx.dt = model, dt
@@ -219,6 +220,7 @@ class DifferentiableBonds:
         zeros = lambda *shape: torch.zeros(shape, dtype=F64, device=self.device)
         g_v, g_rotation, *g_history = (g if g is not None else None for g in g_final)
         dense = lambda g: g.to(F64).contiguous().clone()
+        g_positions = zeros(steps + 1, n, 3) if g_positions is None else g_positions
         x_bar = dense(g_positions[steps])
         v_bar = dense(g_v) if g_v is not None else zeros(n, 6)
         r_bar = dense(g_rotation) if g_rotation is not None else zeros(n, 3, 3)
@@ -228,9 +230,7 @@ class DifferentiableBonds:
         load_bar = zeros(steps, n, 6)
         slots = torch.empty(max(1, lib.dpf_adjoint_slot_doubles(m)), dtype=F64, device=self.device)
         jac = torch.empty(max(1, lib.dpf_adjoint_jacobian_doubles(m)), dtype=F64, device=self.device)
-        jt_out = torch.empty((n, 6), dtype=F64, device=self.device)
-        identity = torch.eye(6, dtype=F64, device=self.device).expand(n, 6, 6).contiguous()
-        ones = torch.ones((n, 6), dtype=F64, device=self.device)
+        lam = torch.empty((n, 6), dtype=F64, device=self.device)
         krylov = _Krylov(6*n, 32, self.device)
         half = .5*dt*dt
         free = (~s.fixed)[:, None].to(F64)
@@ -245,7 +245,7 @@ class DifferentiableBonds:
                 y_bar = torch.zeros_like(y)
                 y_bar[:, :3] += x_bar
                 y_bar += (2/dt)*v_bar
-                if bool(torch.any(r_bar != 0)):
+                if g_rotation is not None and bool(torch.any(r_bar != 0)):
                     with torch.enable_grad():
                         w = y[:, 3:].clone().requires_grad_(True)
                         exp_w = exp_rotation(w)
@@ -257,9 +257,9 @@ class DifferentiableBonds:
                 self._vjp(y, None, 0., h_bar, True, h_next, stiff_bar, y_bar, x_next, slots)
                 y_bar *= free
                 # (2) the implicit solve: J^T lam = y_bar on the block-scaled system
-                trial = s.trial(y)
-                s.prepare_scaling(trial, dt)
-                lam = self._transposed_solve(y, y_bar, dt, jac, jt_out, slots, identity, ones, krylov)
+                s.prepare_scaling(s.trial(y, _check=False), dt)
+                self._transposed_solve(y, y_bar, dt, jac, lam, slots, krylov)
+                s._raise_status()
                 load_bar[t] = half*lam
                 v_next += dt*s.mass*lam
                 # (3) the residual's direct dependence on history, stiffness and positions
@@ -270,45 +270,41 @@ class DifferentiableBonds:
         normal, offset, fn, fs, mt, mb = (t.contiguous() for t in _unpack_history(h_bar))
         return stiff_bar, load_bar, x_bar, v_bar, r_bar, normal, offset, fn, fs, mt, mb
 
-    def _transposed_solve(self, y, rhs, dt, jac, jt_out, slots, identity, ones, krylov):
+    def _transposed_solve(self, y, rhs, dt, jac, lam, slots, krylov):
         """lam with J^T lam = rhs (fixed rows zero), solved as (U^-1 P J U)^T mu = U rhs."""
         s = self.solver
         lib = self._lib
         stream = s._stream()
-        _lib.check(lib.dpf_adjoint_local_jacobian(ctypes.byref(s._graph), ctypes.byref(s._stiffness_struct()),
-                                                  ctypes.byref(s._history_struct()), y.data_ptr(), jac.data_ptr(),
-                                                  stream), 'dpf_adjoint_local_jacobian')
-        units, P, block = s.units, s.preconditioner, s.block
-
-        def to_lambda(mu):
-            return torch.einsum('nij,nj->ni', P, mu/units).contiguous()
-
-        def operator(mu):
-            lam = to_lambda(mu)
-            _lib.check(lib.dpf_adjoint_apply_jt(ctypes.byref(s._graph), jac.data_ptr(), s.mass.data_ptr(),
-                                                s.fixed.data_ptr(), float(dt), lam.data_ptr(), jt_out.data_ptr(),
-                                                slots.data_ptr(), stream), 'dpf_adjoint_apply_jt')
-            return units*jt_out
-
+        graph, stiffness = ctypes.byref(s._graph), s._stiffness_struct()
+        stiffness = ctypes.byref(stiffness)
+        _lib.check(lib.dpf_adjoint_local_jacobian(graph, stiffness, ctypes.byref(s._history_struct()), y.data_ptr(),
+                                                  jac.data_ptr(), stream), 'dpf_adjoint_local_jacobian')
+        tangent = ctypes.byref(s._tangent_struct())
         if s._pcg_workspace is None:
             s._pcg_workspace = torch.empty(lib.dpf_elastic_workspace_doubles(s.n_sites), dtype=F64,
                                            device=self.device)
+        units, P = s.units, s.preconditioner
+        out, z = torch.empty_like(rhs), torch.empty_like(rhs)
+
+        def operator(mu):
+            _lib.check(lib.dpf_adjoint_operator(graph, jac.data_ptr(), s.mass.data_ptr(), s.fixed.data_ptr(),
+                                                P.data_ptr(), units.data_ptr(), float(dt), mu.data_ptr(),
+                                                out.data_ptr(), lam.data_ptr(), slots.data_ptr(), stream),
+                       'dpf_adjoint_operator')
+            return out
 
         def precondition(v):
-            r = (v/units).contiguous()
-            x = torch.empty_like(r)
-            _lib.check(lib.dpf_elastic_precondition(
-                ctypes.byref(s._graph), ctypes.byref(s._stiffness_struct()), ctypes.byref(s._tangent_struct()),
-                s.mass.data_ptr(), s.fixed.data_ptr(), identity.data_ptr(), P.data_ptr(), ones.data_ptr(),
-                r.data_ptr(), float(dt), .03, 80, x.data_ptr(), s._inner.data_ptr(), s._wrench.data_ptr(),
-                s._pcg_workspace.data_ptr(), s._barrier.data_ptr(), s._status.data_ptr(), stream),
-                'dpf_elastic_precondition')
-            return units*torch.einsum('nij,nj->ni', block, x)
+            _lib.check(lib.dpf_adjoint_precondition(
+                graph, stiffness, tangent, s.mass.data_ptr(), s.fixed.data_ptr(), s.block.data_ptr(), P.data_ptr(),
+                units.data_ptr(), v.data_ptr(), float(dt), .03, 80, z.data_ptr(), s._inner.data_ptr(),
+                s._wrench.data_ptr(), s._pcg_workspace.data_ptr(), s._barrier.data_ptr(), s._status.data_ptr(),
+                stream), 'dpf_adjoint_precondition')
+            return z
 
-        mu, info = fgmres(operator, (units*rhs).contiguous(), precondition, tolerance=self.adjoint_tolerance,
-                          workspace=krylov)
+        mu, info = fgmres(operator, units*rhs, precondition, tolerance=self.adjoint_tolerance, workspace=krylov)
         self.stats.append(dict(adjoint_krylov=info['iterations'], adjoint_relative=info['relative_residual']))
-        return to_lambda(mu)
+        _lib.check(lib.dpf_adjoint_multiplier(s.n_sites, P.data_ptr(), units.data_ptr(), mu.data_ptr(),
+                                              lam.data_ptr(), stream), 'dpf_adjoint_multiplier')
 
 
 def inverse_fit_problem(m, seed, device, steps, dt, checkpoint_every, tolerance):

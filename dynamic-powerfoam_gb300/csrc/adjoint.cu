@@ -12,6 +12,7 @@
 //     per bond, so J^T lambda costs one sparse transposed product;
 //   * dpf_adjoint_apply_jt applies J^T (free rows) for the adjoint Krylov solve.
 #include "common.cuh"
+#include "internal.cuh"
 
 namespace dpf {
 namespace adj {
@@ -346,36 +347,52 @@ __global__ void __launch_bounds__(kThreads) jt_bonds_kernel(int64_t m, const int
     }
 }
 
-// Site gather of per-bond slots of width 2K ([i-side K, j-side K]).
+// Three of the numbers of site s summed over its per-bond slots of width 2K
+// ([i-side K, j-side K]): those from `first` on.  A site's lanes take three
+// each, so that the loads of an incidence are contiguous over them.
 template <int K>
-__device__ __forceinline__ void gather_slots(const int32_t *ptr, const int32_t *inc, const double *slots, int64_t s,
-                                             double acc[K]) {
-#pragma unroll
-    for (int c = 0; c < K; ++c) acc[c] = 0.0;
+__device__ __forceinline__ d3 gather_slots(const int32_t *ptr, const int32_t *inc, const double *slots, int64_t s,
+                                           int first) {
+    d3 acc = mk(0.0, 0.0, 0.0);
     const int e1 = ptr[s + 1];
+#pragma unroll 4
     for (int e = ptr[s]; e < e1; ++e) {
-        const int v = inc[e];
-        const double *p = v >= 0 ? slots + 2 * K * (int64_t)v : slots + 2 * K * (int64_t)(~v) + K;
-#pragma unroll
-        for (int c = 0; c < K; ++c) acc[c] += p[c];
+        const int v = inc[e], j = v >> 31;
+        acc = acc + ld3(slots + 2 * K * (int64_t)(v ^ j) - (int64_t)K * j + first);
     }
+    return acc;
 }
 
-// out = M lam - h sum B^T w on free rows, lam on fixed rows (lam's fixed rows are zero).
-__global__ void __launch_bounds__(kThreads) jt_sites_kernel(int64_t n, const int32_t *ptr, const int32_t *inc,
-                                                            const double *slots, const double *mass,
-                                                            const uint8_t *fixed, double half_dt2, const double *lam,
-                                                            double *out) {
-    const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+// out = M lam - h sum B^T w on free rows, lam on fixed rows (lam's fixed rows are
+// zero); times units when given.  Two lanes a site.
+__global__ void __launch_bounds__(128) jt_sites_kernel(int64_t n, const int32_t *ptr, const int32_t *inc,
+                                                       const double *slots, const double *mass, const uint8_t *fixed,
+                                                       double half_dt2, const double *lam, const double *units,
+                                                       double *out) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, s = t / 2;
     if (s >= n) return;
-    double acc[6];
-    gather_slots<6>(ptr, inc, slots, s, acc);
-    const bool fx = fixed[s] != 0;
-#pragma unroll
-    for (int c = 0; c < 6; ++c) {
-        const double l = lam[6 * s + c];
-        out[6 * s + c] = fx ? l : mass[6 * s + c] * l - half_dt2 * acc[c];
+    const d3 acc = gather_slots<6>(ptr, inc, slots, s, 3 * (int)(t & 1)), l = ld3(lam, t), m = ld3(mass, t);
+    d3 o = fixed[s] ? l : mk(m.x * l.x - half_dt2 * acc.x, m.y * l.y - half_dt2 * acc.y, m.z * l.z - half_dt2 * acc.z);
+    if (units) {
+        const d3 u = ld3(units, t);
+        o = mk(u.x * o.x, u.y * o.y, u.z * o.z);
     }
+    st3(out, t, o);
+}
+
+// lam = P (mu / units): from the scaled adjoint system's unknown to the
+// multiplier.  Two lanes a site.  The scaled system's operator is three launches
+// (this, the bonds' transposed products, the sites' sums with the units folded in)
+// and its preconditioner one (the elastic PCG reads vector / units and writes
+// units (block x)); with the divisions, products and 6x6 products as separate
+// passes over the sites an 8k-site, 8-step rollout with its gradient took 13.4 ms,
+// with them folded in 11.1 ms.
+__global__ void __launch_bounds__(128) multiplier_kernel(int64_t n, const double *P, const double *units,
+                                                         const double *mu, double *lam) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, s = t / 2;
+    const bool live = s < n;
+    const d3 v = live ? over_units(ld3(mu, t), ld3(units, t)) : mk(0.0, 0.0, 0.0), other = other_half(v);
+    if (live) st3(lam, t, half_rows(P + 36 * s, (int)(t & 1), v, other));
 }
 
 // Input adjoints of one bond for output adjoints: wrench part = coef * (wrench
@@ -445,21 +462,15 @@ __global__ void __launch_bounds__(128) vjp_kernel(VjpArgs a) {
     ka[3] += bar.kt;
 }
 
-// Site adjoints from the VJP slots: y_adj (N, 6) and x_adj (N, 3), ADDED.
-__global__ void __launch_bounds__(kThreads) vjp_sites_kernel(int64_t n, const int32_t *ptr, const int32_t *inc,
-                                                             const double *slots, double *y_adj, double *x_adj) {
-    const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (s >= n) return;
-    double acc[9];
-    gather_slots<9>(ptr, inc, slots, s, acc);
-    if (y_adj) {
-#pragma unroll
-        for (int c = 0; c < 6; ++c) y_adj[6 * s + c] += acc[c];
-    }
-    if (x_adj) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) x_adj[3 * s + c] += acc[6 + c];
-    }
+// Site adjoints from the VJP slots: y_adj (N, 6) and x_adj (N, 3), ADDED.  Three
+// lanes a site.
+__global__ void __launch_bounds__(96) vjp_sites_kernel(int64_t n, const int32_t *ptr, const int32_t *inc,
+                                                       const double *slots, double *y_adj, double *x_adj) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, s = t / 3;
+    const int part = (int)(t - 3 * s);
+    if (s >= n || !(part < 2 ? y_adj : x_adj)) return;
+    double *out = part < 2 ? y_adj + 6 * s + 3 * part : x_adj + 3 * s;
+    st3(out, ld3(out) + gather_slots<9>(ptr, inc, slots, s, 3 * part));
 }
 
 inline int blocks_for(int64_t n, int threads) { return (int)((n + threads - 1) / threads); }
@@ -496,18 +507,51 @@ int dpf_adjoint_local_jacobian(const dpf_graph *g, const dpf_stiffness *k, const
     return DPF_OK;
 }
 
-int dpf_adjoint_apply_jt(const dpf_graph *g, const double *jacobian, const double *mass, const uint8_t *fixed,
-                         double dt, const double *lam, double *out, double *slots, void *stream) {
+static int apply_jt(const dpf_graph *g, const double *jacobian, const double *mass, const uint8_t *fixed, double dt,
+                    const double *lam, const double *units, double *out, double *slots, void *stream) {
     if (!g || g->n_sites <= 0 || !mass || !fixed || !lam || !out || (g->n_bonds && (!jacobian || !slots)))
         return DPF_ERR_ARGUMENT;
     cudaStream_t st = (cudaStream_t)stream;
     if (g->n_bonds)
         jt_bonds_kernel<<<blocks_for(g->n_bonds, kThreads), kThreads, 0, st>>>(g->n_bonds, g->edges, jacobian, lam,
                                                                                slots);
-    jt_sites_kernel<<<blocks_for(g->n_sites, kThreads), kThreads, 0, st>>>(
-        g->n_sites, g->inc_ptr, g->inc_bond, slots, mass, fixed, 0.5 * dt * dt, lam, out);
+    const int threads = spread_threads(2 * g->n_sites);
+    jt_sites_kernel<<<blocks_for(2 * g->n_sites, threads), threads, 0, st>>>(
+        g->n_sites, g->inc_ptr, g->inc_bond, slots, mass, fixed, 0.5 * dt * dt, lam, units, out);
     DPF_CHECK_LAUNCH();
     return DPF_OK;
+}
+
+int dpf_adjoint_apply_jt(const dpf_graph *g, const double *jacobian, const double *mass, const uint8_t *fixed,
+                         double dt, const double *lam, double *out, double *slots, void *stream) {
+    return apply_jt(g, jacobian, mass, fixed, dt, lam, nullptr, out, slots, stream);
+}
+
+int dpf_adjoint_multiplier(int64_t n_sites, const double *preconditioner, const double *units, const double *mu,
+                           double *lam, void *stream) {
+    if (n_sites <= 0 || !preconditioner || !units || !mu || !lam) return DPF_ERR_ARGUMENT;
+    const int threads = spread_threads(2 * n_sites);
+    multiplier_kernel<<<blocks_for(2 * n_sites, threads), threads, 0, (cudaStream_t)stream>>>(
+        n_sites, preconditioner, units, mu, lam);
+    DPF_CHECK_LAUNCH();
+    return DPF_OK;
+}
+
+int dpf_adjoint_operator(const dpf_graph *g, const double *jacobian, const double *mass, const uint8_t *fixed,
+                         const double *preconditioner, const double *units, double dt, const double *mu, double *out,
+                         double *lam, double *slots, void *stream) {
+    if (!g || !units) return DPF_ERR_ARGUMENT;
+    const int rc = dpf_adjoint_multiplier(g->n_sites, preconditioner, units, mu, lam, stream);
+    return rc ? rc : apply_jt(g, jacobian, mass, fixed, dt, lam, units, out, slots, stream);
+}
+
+int dpf_adjoint_precondition(const dpf_graph *g, const dpf_stiffness *k, const dpf_tangent *t, const double *mass,
+                             const uint8_t *fixed, const double *block, const double *preconditioner,
+                             const double *units, const double *vector, double dt, double tolerance,
+                             int max_iterations, double *out, int *iterations, double *wrench, double *workspace,
+                             unsigned *barrier, int *status, void *stream) {
+    return elastic_pass(g, k, t, mass, fixed, block, preconditioner, units, vector, dt, tolerance, max_iterations, out,
+                        iterations, wrench, workspace, barrier, status, kElasticT, (cudaStream_t)stream);
 }
 
 int dpf_adjoint_bond_vjp(const dpf_graph *g, const dpf_stiffness *k, const dpf_history *h, const double *y,
@@ -524,7 +568,7 @@ int dpf_adjoint_bond_vjp(const dpf_graph *g, const dpf_stiffness *k, const dpf_h
         (end_adjoint ? vjp_kernel<true> : vjp_kernel<false>)<<<blocks_for(g->n_bonds, threads), threads, 0, st>>>(a);
     }
     if ((y_adjoint || x_adjoint) && g->n_bonds)
-        vjp_sites_kernel<<<blocks_for(g->n_sites, kThreads), kThreads, 0, st>>>(
+        vjp_sites_kernel<<<blocks_for(3 * g->n_sites, 96), 96, 0, st>>>(
             g->n_sites, g->inc_ptr, g->inc_bond, slots, with_increment ? y_adjoint : nullptr, x_adjoint);
     DPF_CHECK_LAUNCH();
     return DPF_OK;

@@ -25,10 +25,20 @@ int jacobian_pass(const dpf_graph *g, const double *linear, const double *direct
                   const uint8_t *fixed, double dt, const double *units, const double *preconditioner, double *out,
                   double *wrench, cudaStream_t stream);
 
-// dpf_elastic_precondition; raw: the solution x itself instead of x / units.
+// One CGS2 Arnoldi step in one cooperative launch (dpf_arnoldi_cgs2_fused).
+int arnoldi_pass(int64_t length, double *basis, int64_t ld, int j, double *w, double *h, double *partials,
+                 unsigned *barrier, int *status, cudaStream_t stream);
+
+// What the elastic PCG reads and writes:
+//   kElastic    r = block (units vector), out = x / units (dpf_elastic_precondition);
+//   kElasticRaw r the same, out = x;
+//   kElasticT   r = vector / units, out = units (block x): the transposed preconditioner.
+enum ElasticForm { kElastic = 0, kElasticRaw = 1, kElasticT = 2 };
+
 int elastic_pass(const dpf_graph *g, const dpf_stiffness *k, const dpf_tangent *t, const double *mass,
                  const uint8_t *fixed, const double *block, const double *preconditioner, const double *units,
                  const double *vector, double dt, double tolerance, int max_iterations, double *out, int *iterations,
-                 double *wrench, double *workspace, unsigned *barrier, int *status, bool raw, cudaStream_t stream);
+                 double *wrench, double *workspace, unsigned *barrier, int *status, ElasticForm form,
+                 cudaStream_t stream);
 
 }  // namespace dpf

@@ -90,7 +90,10 @@ __global__ void __launch_bounds__(kThreads) arnoldi_kernel(ArnoldiArgs a) {
                     if (threadIdx.x == 0) part[(int64_t)(k0 + c) * gridDim.x + blockIdx.x] = v;
                 }
         }
-        if (!grid_barrier(a.barrier, a.status)) return;
+        if (!grid_barrier(a.barrier, a.status)) {
+            if (tid == 0) a.h[a.count] = NAN;    // no column: the solve ends without convergence
+            return;
+        }
     }
     row_totals(part2, a.count, values);
     if (blockIdx.x == 0)
@@ -104,7 +107,10 @@ __global__ void __launch_bounds__(kThreads) arnoldi_kernel(ArnoldiArgs a) {
     }
     sq = block_sum(sq);
     if (threadIdx.x == 0) part3[blockIdx.x] = sq;
-    if (!grid_barrier(a.barrier, a.status)) return;
+    if (!grid_barrier(a.barrier, a.status)) {
+        if (tid == 0) a.h[a.count] = NAN;
+        return;
+    }
     row_totals(part3, 1, values);
     const double length = sqrt(values[0]);
     if (tid == 0) a.h[a.count] = length;
@@ -189,7 +195,6 @@ struct Step {
     int *host_int;    // [0] status, [1] inner
     double rhs_scale = -1.0;
     dpf_tangent tangent;
-    int arnoldi_blocks = 0;
     // elastic preconditioning with a stored linearisation: the preconditioner's rows
     // are in the coordinates of y (x instead of x / units), as the product wants them
     bool raw = false;
@@ -230,27 +235,8 @@ struct Step {
     }
 
     int arnoldi(int j) {
-        if (!arnoldi_blocks) {
-            int dev = 0, sms = 0, per_sm = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, arnoldi_kernel, kThreads, 0);
-            if (sms < 1 || per_sm < 1) return DPF_ERR_CUDA;
-            arnoldi_blocks = sms * (per_sm < 4 ? per_sm : 4);
-            const int64_t need = (n6 + kThreads - 1) / kThreads;
-            if (arnoldi_blocks > need) arnoldi_blocks = (int)need;
-            if (arnoldi_blocks > kMaxBlocks) arnoldi_blocks = kMaxBlocks;
-        }
-        ArnoldiArgs k{n6, n6, s->basis, s->w, s->basis + (int64_t)(j + 1) * n6, s->h, s->krylov_partials, j + 1,
-                      s->barrier, s->status};
-        if (cudaMemsetAsync(s->barrier, 0, 2 * sizeof(unsigned), st)) return DPF_ERR_CUDA;
-        void *args[] = {&k};
-        if (cudaLaunchCooperativeKernel((const void *)arnoldi_kernel, arnoldi_blocks, kThreads, args, 0, st) !=
-            cudaSuccess) {
-            cudaGetLastError();
-            return DPF_ERR_CUDA;
-        }
-        return ran(1, DPF_OK);
+        return ran(1, dpf::arnoldi_pass(n6, s->basis, n6, j, s->w, s->h, s->krylov_partials, s->barrier, s->status,
+                                        st));
     }
 
     // Right-preconditioned FGMRES on the scaled system from rhs = -scaled, |rhs| =
@@ -279,7 +265,8 @@ struct Step {
                 if (s->elastic) {
                     rc = ran(1, dpf::elastic_pass(s->graph, &s->stiffness, &tangent, s->mass, s->fixed, s->block,
                                                   s->preconditioner, s->units, v, a->dt, 0.03, 80, z, s->inner,
-                                                  s->wrench, s->workspace, s->barrier, s->status, raw, st));
+                                                  s->wrench, s->workspace, s->barrier, s->status,
+                                                  raw ? dpf::kElasticRaw : dpf::kElastic, st));
                     if (rc) return rc;
                 } else {
                     z = v;
@@ -483,6 +470,35 @@ struct Step {
 };
 
 }  // namespace newton64
+
+int arnoldi_pass(int64_t length, double *basis, int64_t ld, int j, double *w, double *h, double *partials,
+                 unsigned *barrier, int *status, cudaStream_t st) {
+    using namespace newton64;
+    static int per_device[64] = {0};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    int blocks = per_device[dev & 63];
+    if (!blocks) {
+        int sms = 0, per_sm = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, arnoldi_kernel, kThreads, 0);
+        if (sms < 1 || per_sm < 1) return DPF_ERR_CUDA;
+        blocks = sms * (per_sm < 4 ? per_sm : 4);
+        if (blocks > kMaxBlocks) blocks = kMaxBlocks;
+        per_device[dev & 63] = blocks;
+    }
+    const int64_t need = (length + kThreads - 1) / kThreads;
+    if (blocks > need) blocks = (int)need;
+    ArnoldiArgs k{length, ld, basis, w, basis + (int64_t)(j + 1) * ld, h, partials, j + 1, barrier, status};
+    if (cudaMemsetAsync(barrier, 0, 2 * sizeof(unsigned), st)) return DPF_ERR_CUDA;
+    void *args[] = {&k};
+    if (cudaLaunchCooperativeKernel((const void *)arnoldi_kernel, blocks, kThreads, args, 0, st) != cudaSuccess) {
+        cudaGetLastError();
+        return DPF_ERR_CUDA;
+    }
+    return DPF_OK;
+}
+
 }  // namespace dpf
 
 extern "C" {
@@ -490,6 +506,14 @@ extern "C" {
 int64_t dpf_newton64_partials_doubles(void) {
     using namespace dpf::newton64;
     return (2 * (int64_t)kMaxColumns + 1) * kMaxBlocks;
+}
+
+int dpf_arnoldi_cgs2_fused(int64_t length, double *basis, int64_t ld, int j, double *w, double *h, double *partials,
+                           unsigned *barrier, int *status, void *stream) {
+    if (length <= 0 || !basis || !w || !h || !partials || !barrier || !status || j < 0 ||
+        j + 1 >= dpf::newton64::kMaxColumns || ld < length)
+        return DPF_ERR_ARGUMENT;
+    return dpf::arnoldi_pass(length, basis, ld, j, w, h, partials, barrier, status, (cudaStream_t)stream);
 }
 
 int64_t dpf_newton64_linear_doubles(int64_t n_bonds) { return n_bonds < 0 ? 0 : dpf::kLinear * n_bonds; }

@@ -60,7 +60,7 @@ struct PcgArgs {
     const double *mass, *block, *P, *units, *vector;
     const uint8_t *fixed;
     double alpha_op, tol2;
-    int max_it, raw;
+    int max_it, form;   // ElasticForm
     double *out;
     int *iterations;
     double *wrench, *r, *u, *p, *s, *part_a, *part_b;
@@ -84,10 +84,10 @@ __global__ void __launch_bounds__(kThreads) pcg_kernel(PcgArgs a) {
         d3 v = mk(0.0, 0.0, 0.0), r = v;
         if (live) {
             const d3 un = ld3(a.units + at), in = ld3(a.vector + at);
-            v = mk(un.x * in.x, un.y * in.y, un.z * in.z);
+            v = a.form == kElasticT ? over_units(in, un) : mk(un.x * in.x, un.y * in.y, un.z * in.z);
         }
         const d3 vo = other_half(v);
-        if (live && !a.fixed[s]) r = half_rows(a.block + 36 * s, half, v, vo);
+        if (live && !a.fixed[s]) r = a.form == kElasticT ? v : half_rows(a.block + 36 * s, half, v, vo);
         const d3 ro = other_half(r);
         if (live) {
             const d3 u = half_rows(a.P + 36 * s, half, r, ro);
@@ -171,9 +171,20 @@ __global__ void __launch_bounds__(kThreads) pcg_kernel(PcgArgs a) {
         gamma = following;
     }
     // a thread's own x: no barrier
-    for (s = first; s < a.n && !a.raw; s += step) {
+    s = first;
+    for (int64_t k = 0; k < rounds && a.form != kElasticRaw; ++k, s += step) {
+        const bool live = s < a.n;
         const int64_t at = 6 * s + 3 * half;
-        st3(a.out + at, over_units(ld3(a.out + at), ld3(a.units + at)));
+        const d3 x = live ? ld3(a.out + at) : mk(0.0, 0.0, 0.0), un = live ? ld3(a.units + at) : x;
+        if (a.form == kElasticT) {
+            const d3 xo = other_half(x);
+            if (live) {
+                const d3 v = half_rows(a.block + 36 * s, half, x, xo);
+                st3(a.out + at, mk(un.x * v.x, un.y * v.y, un.z * v.z));
+            }
+        } else if (live) {
+            st3(a.out + at, over_units(x, un));
+        }
     }
     if (tid == 0) atomicAdd(a.iterations, it < a.max_it ? it + 1 : a.max_it);
 }
@@ -605,8 +616,8 @@ int64_t dpf_elastic_workspace_doubles(int64_t n_sites) { return 30 * n_sites + 2
 int dpf::elastic_pass(const dpf_graph *g, const dpf_stiffness *k, const dpf_tangent *t, const double *mass,
                       const uint8_t *fixed, const double *block, const double *preconditioner, const double *units,
                       const double *vector, double dt, double tolerance, int max_iterations, double *out,
-                      int *iterations, double *wrench, double *workspace, unsigned *barrier, int *status, bool raw,
-                      cudaStream_t st) {
+                      int *iterations, double *wrench, double *workspace, unsigned *barrier, int *status,
+                      ElasticForm form, cudaStream_t st) {
     if (!g || g->n_sites <= 0 || !g->inc_ptr || (g->n_bonds && !g->inc_bond) || !k || !t || !mass || !fixed ||
         !block ||
         !preconditioner || !units || !vector || !out || !iterations || !workspace || !barrier || !status ||
@@ -644,7 +655,7 @@ int dpf::elastic_pass(const dpf_graph *g, const dpf_stiffness *k, const dpf_tang
     a.alpha_op = 0.25 * dt * dt;
     a.tol2 = tolerance * tolerance;
     a.max_it = max_iterations;
-    a.raw = raw ? 1 : 0;
+    a.form = form;
     a.out = out;
     a.iterations = iterations;
     a.wrench = wrench;
@@ -673,7 +684,8 @@ int dpf_elastic_precondition(const dpf_graph *g, const dpf_stiffness *k, const d
                              int max_iterations, double *out, int *iterations, double *wrench, double *workspace,
                              unsigned *barrier, int *status, void *stream) {
     return dpf::elastic_pass(g, k, t, mass, fixed, block, preconditioner, units, vector, dt, tolerance, max_iterations,
-                             out, iterations, wrench, workspace, barrier, status, false, (cudaStream_t)stream);
+                             out, iterations, wrench, workspace, barrier, status, kElastic,
+                             (cudaStream_t)stream);
 }
 
 int dpf_arnoldi_cgs2(int64_t length, double *basis, int64_t ld, int j, double *w, double *h, double *partials,

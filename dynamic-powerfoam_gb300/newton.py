@@ -809,6 +809,9 @@ def fgmres(operator, rhs, precondition, tolerance=1e-6, restart=32, max_iteratio
     length = b.numel()
     partials = torch.zeros(lib.dpf_partials_doubles(), dtype=F64, device=device)
     scal = torch.zeros(2, dtype=F64, device=device)
+    arnoldi = torch.empty(lib.dpf_newton64_partials_doubles(), dtype=F64, device=device)
+    barrier = torch.zeros(4, dtype=torch.int32, device=device)
+    host_h = torch.empty(72, dtype=F64, pin_memory=True)
 
     def norm_of(v):
         _lib.check(lib.dpf_dot_norm(length, v.data_ptr(), None, scal.data_ptr(), partials.data_ptr(), stream),
@@ -838,9 +841,12 @@ def fgmres(operator, rhs, precondition, tolerance=1e-6, restart=32, max_iteratio
             w = operator(ws.transformed[j].reshape(shape)).reshape(-1).to(F64).contiguous()
             if w.data_ptr() == ws.transformed[j].data_ptr():
                 w = w.clone()
-            _lib.check(lib.dpf_arnoldi_cgs2(length, ws.basis.data_ptr(), length, j, w.data_ptr(), ws.h.data_ptr(),
-                                            partials.data_ptr(), stream), 'dpf_arnoldi_cgs2')
-            column = ws.h[:j+2].cpu().numpy()
+            _lib.check(lib.dpf_arnoldi_cgs2_fused(length, ws.basis.data_ptr(), length, j, w.data_ptr(),
+                                                  ws.h.data_ptr(), arnoldi.data_ptr(), barrier.data_ptr(),
+                                                  barrier[2:].data_ptr(), stream), 'dpf_arnoldi_cgs2_fused')
+            host_h.copy_(ws.h, non_blocking=True)
+            torch.cuda.current_stream(device).synchronize()
+            column = host_h.numpy()
             h[:j+1, j] = column[:j+1]
             h[j+1, j] = column[j+1]
             breakdown = h[j+1, j] < 1e-14

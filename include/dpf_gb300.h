@@ -237,6 +237,12 @@ int dpf_energy(const dpf_graph *g, const dpf_stiffness *k, const dpf_history *h,
 /* Size in doubles of the reduction partials used by the vector kernels. */
 int64_t dpf_partials_doubles(void);
 
+/* dpf_arnoldi_cgs2 in one cooperative launch: partials
+ * dpf_newton64_partials_doubles() doubles, barrier 2 unsigned ints (device,
+ * zeroed by the call on its stream); h[j+1] is NaN after a barrier timeout. */
+int dpf_arnoldi_cgs2_fused(int64_t length, double *basis, int64_t ld, int j, double *w, double *h, double *partials,
+                           unsigned *barrier, int *status, void *stream);
+
 /* Twice-iterated classical Gram-Schmidt of w against basis rows 0..j
  * (row stride ld) followed by h[0..j] = projections, h[j+1] = |w|, and, when
  * |w| >= 1e-14, basis row j+1 = w / |w|.  h is a device array of j+2 doubles.
@@ -587,6 +593,23 @@ int dpf_adjoint_local_jacobian(const dpf_graph *g, const dpf_stiffness *k, const
 int dpf_adjoint_apply_jt(const dpf_graph *g, const double *jacobian, const double *mass,
                          const uint8_t *fixed, double dt, const double *lam, double *out,
                          double *slots, void *stream);
+
+/* The adjoint Krylov solve's system (U^-1 P J U)^T mu = U rhs with U = diag(units),
+ * P the 6x6 block inverses of dpf_prepare_scaling:
+ *   multiplier    lam = P (mu / units);
+ *   operator      out = units J^T lam with lam = P (mu / units) (lam: 6 N scratch);
+ *   precondition  out = units (block x) with (M + dt^2/4 K) x = vector / units on free
+ *                 sites by the elastic PCG (arguments of dpf_elastic_precondition). */
+int dpf_adjoint_multiplier(int64_t n_sites, const double *preconditioner, const double *units, const double *mu,
+                           double *lam, void *stream);
+int dpf_adjoint_operator(const dpf_graph *g, const double *jacobian, const double *mass, const uint8_t *fixed,
+                         const double *preconditioner, const double *units, double dt, const double *mu, double *out,
+                         double *lam, double *slots, void *stream);
+int dpf_adjoint_precondition(const dpf_graph *g, const dpf_stiffness *k, const dpf_tangent *t, const double *mass,
+                             const uint8_t *fixed, const double *block, const double *preconditioner,
+                             const double *units, const double *vector, double dt, double tolerance,
+                             int max_iterations, double *out, int *iterations, double *wrench, double *workspace,
+                             unsigned *barrier, int *status, void *stream);
 
 /* Vector-Jacobian product of the trial at increment y for the output adjoints
  * coef * (wrench adjoint of the site vector lam) + end_adjoint (M x 14, the

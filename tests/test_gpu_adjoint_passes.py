@@ -92,3 +92,78 @@ def test_input_adjoints_and_transposed_product(n, m, contacts, unit, end):
     left, right = (lam*cpu.jacobian_vector(y, d, DT, None)).sum(), (host(out)*d).sum()
     scale = np.linalg.norm(lam)*np.linalg.norm(cpu.jacobian_vector(y, d, DT, None))
     assert abs(left - right) <= 1e-10*scale
+
+
+@pytest.mark.parametrize('n,m', [(2, 1), (15, 31), (17, 33), (65, 255), (700, 2049)])
+def test_scaled_adjoint_system(n, m):
+    """The fused operator, multiplier and preconditioner against their definitions (sums of 6: 1e-12; the
+    PCG run to 1e-13 on systems of condition below 1e3: 1e-9)."""
+    import torch
+    from dpf_gb300 import _lib
+    gpu, cpu, rng = _pair(n, m, seed=n)
+    lib, empty = _lib.load(), lambda *s: torch.empty(s, dtype=torch.float64, device=gpu.device)
+    y = gpu.tensor(rng.normal(0, .02, (n, 6)))
+    gpu.prepare_scaling(gpu.trial(y), DT)
+    units, P, block = gpu.units, gpu.preconditioner, gpu.block
+    mu = rng.normal(size=(n, 6))
+    mu[cpu.fixed] = 0.
+    mu = gpu.tensor(mu)
+    jac, slots = empty(max(1, lib.dpf_adjoint_jacobian_doubles(m))), empty(max(1, lib.dpf_adjoint_slot_doubles(m)))
+    graph, stream = ctypes.byref(gpu._graph), gpu._stream()
+    _lib.call('dpf_adjoint_local_jacobian', graph, ctypes.byref(gpu._stiffness_struct()),
+              ctypes.byref(gpu._history_struct()), y.data_ptr(), jac.data_ptr(), stream)
+    lam, out, plain = empty(n, 6), empty(n, 6), empty(n, 6)
+    _lib.call('dpf_adjoint_operator', graph, jac.data_ptr(), gpu.mass.data_ptr(), gpu.fixed.data_ptr(), P.data_ptr(),
+              units.data_ptr(), DT, mu.data_ptr(), out.data_ptr(), lam.data_ptr(), slots.data_ptr(), stream)
+    want = (P@(mu/units)[:, :, None])[:, :, 0].contiguous()
+    rel = lambda a, b: float(torch.linalg.vector_norm(a - b)/torch.linalg.vector_norm(b).clamp_min(1e-300))
+    assert rel(lam, want) <= 1e-12
+    _lib.call('dpf_adjoint_multiplier', n, P.data_ptr(), units.data_ptr(), mu.data_ptr(), plain.data_ptr(), stream)
+    assert torch.equal(plain, lam)
+    _lib.call('dpf_adjoint_apply_jt', graph, jac.data_ptr(), gpu.mass.data_ptr(), gpu.fixed.data_ptr(), DT,
+              lam.data_ptr(), plain.data_ptr(), slots.data_ptr(), stream)
+    assert rel(out, units*plain) <= 1e-12
+
+    work = empty(lib.dpf_elastic_workspace_doubles(n))
+    def pcg(name, block, units, vector, out):
+        _lib.call(name, graph, ctypes.byref(gpu._stiffness_struct()), ctypes.byref(gpu._tangent_struct()),
+                  gpu.mass.data_ptr(), gpu.fixed.data_ptr(), block.data_ptr(), P.data_ptr(), units.data_ptr(),
+                  vector.data_ptr(), DT, 1e-13, 400, out.data_ptr(), gpu._inner.data_ptr(), gpu._wrench.data_ptr(),
+                  work.data_ptr(), gpu._barrier.data_ptr(), gpu._status.data_ptr(), stream)
+    gpu._status.zero_()
+    pcg('dpf_adjoint_precondition', block, units, mu, out)
+    identity, ones = torch.eye(6, dtype=block.dtype, device=gpu.device).repeat(n, 1, 1), torch.ones_like(units)
+    pcg('dpf_elastic_precondition', identity, ones, mu/units, plain)
+    assert int(gpu._status[0]) == 0
+    assert rel(out, units*(block@plain[:, :, None])[:, :, 0]) <= 1e-9
+
+
+@pytest.mark.parametrize('length,j', [(2, 0), (6, 4), (257, 8), (257, 62), (70001, 31)])
+def test_fused_arnoldi_step(length, j):
+    """One cooperative launch against the four-pass step: the same column and next row (dot products of
+    unit rows, 1e-12 of |w|; the next row is divided by a remainder of the order of |w|)."""
+    import torch
+    from dpf_gb300 import _lib
+    lib, dev = _lib.load(), torch.device('cuda')
+    rng = np.random.default_rng(length + j)
+    rows = np.linalg.qr(rng.normal(size=(length, j + 1)))[0].T
+    got = []
+    for name in ('dpf_arnoldi_cgs2', 'dpf_arnoldi_cgs2_fused'):
+        basis = torch.zeros((j + 2, length), dtype=torch.float64, device=dev)
+        basis[:j + 1] = torch.as_tensor(rows)
+        w = torch.as_tensor(np.random.default_rng(j).normal(size=length)).to(dev)
+        h = torch.zeros(72, dtype=torch.float64, device=dev)
+        partials = torch.zeros(max(lib.dpf_partials_doubles(), lib.dpf_newton64_partials_doubles()),
+                               dtype=torch.float64, device=dev)
+        barrier = torch.ones(4, dtype=torch.int32, device=dev)
+        barrier[2:] = 0
+        extra = () if name == 'dpf_arnoldi_cgs2' else (barrier.data_ptr(), barrier[2:].data_ptr())
+        _lib.call(name, length, basis.data_ptr(), length, j, w.data_ptr(), h.data_ptr(), partials.data_ptr(), *extra,
+                  torch.cuda.current_stream(dev).cuda_stream)
+        assert int(barrier[2]) == 0
+        got.append((host(h), host(basis), host(w)))
+    size = np.sqrt(length)
+    (h0, b0, w0), (h1, b1, w1) = got
+    assert np.abs(h0 - h1).max() <= 1e-12*size and np.abs(w0 - w1).max() <= 1e-12*size
+    assert h0[j + 1] > 1e-3*size
+    assert np.abs(b0 - b1).max() <= 1e-12*size/h0[j + 1]*10
