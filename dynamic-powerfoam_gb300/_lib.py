@@ -95,7 +95,7 @@ class Newton64(ctypes.Structure):
                 [('krylov_width', i32), ('elastic', i32), ('linear', vp)])
 
 
-NEWTON_VECTORS = 10
+NEWTON_VECTORS = 9
 NEWTON64_VECTORS = 7
 NEWTON_HOST_DOUBLES = 128
 NEWTON_TRACE = 32
@@ -243,7 +243,7 @@ KERNELS = {
     'dpf_to_float': 1, 'dpf_mixed_precondition': 1, 'dpf_mixed_commit': 3, 'dpf_mixed_begin': 1, 'dpf_mixed_residual_segmented': 2, 'dpf_segment_norms': 2,
     'dpf_segment_axpy': 1, 'dpf_segment_select': 1,
     'dpf_adjoint_local_jacobian': 1, 'dpf_adjoint_apply_jt': 2, 'dpf_adjoint_bond_vjp': 2,
-    'dpf_tile_pack': 2, 'dpf_tiled_hvp': 1, 'dpf_tiled_precondition': 1, 'dpf_end_pack': 2, 'dpf_end_hvp': 1,
+    'dpf_tile_pack': 2, 'dpf_tiled_hvp': 1, 'dpf_tiled_precondition': 1, 'dpf_end_pack': 1, 'dpf_end_hvp': 1,
     'dpf_end_precondition': 1, 'dpf_bond_energy': 3, 'dpf_bond_energy_sites': 4, 'dpf_parallel_advance': 2, 'dpf_parallel_loads': 2,
     'dpf_energy_tangent': 1, 'dpf_operator_apply': 2, 'dpf_block_inverse': 1, 'dpf_block_pcg': 1, 'dpf_linear_midpoint_rhs': 1, 'dpf_linear_midpoint_advance': 1,
     'dpf_linear_sums': 1, 'dpf_anderson_gram': 1, 'dpf_anderson_mix': 1, 'dpf_barrier_selftest': 1,

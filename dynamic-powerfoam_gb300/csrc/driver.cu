@@ -2,39 +2,65 @@
 // NewtonBonds.step and fgmres (experiments/bonded_dem_newton.py:13-60,
 // 132-201) as host code that launches this library's entry points directly.
 //
-// The Python control path (MixedNewtonBonds.step) and this driver issue the
-// same entry points in the same order with the same arguments, and take the
-// same host decisions in float64 (Givens rotations with hypot, back
-// substitution, convergence tests, Armijo line search), so a step gives
-// bit-identical results either way.  What changes is the host cost between
-// launches: a few microseconds of C++ instead of Python, which matters after
-// each of the step's small device reads (the FGMRES Hessenberg column, the
-// residual norms), when the GPU idles until the next launch arrives.
-#include <cuda_runtime.h>
-
+// The Python control path (MixedNewtonBonds.step) and this driver do the same
+// arithmetic on every entry in the same order and take the same host decisions
+// in float64 (Givens rotations with hypot, back substitution, convergence
+// tests, Armijo line search), so a step gives bit-identical results either way.
+// What changes is what lies between: the host's C++ instead of Python, passes
+// over whole vectors joined into one (the start of a step, the end of a Krylov
+// cycle, the end state), and results written to pinned host memory by the
+// kernels instead of copied.  A 4k-site step is bound by the launches and by the
+// waits: 62 launches, copies and memsets took 735 us, 22 launches take 578 us; at
+// 262k sites the joined passes save the traffic of whole vectors (5186 us a step,
+// now 4874).
 #include <cmath>
 #include <cstring>
 #include <vector>
 
-#include "dpf_gb300.h"
+#include "common.cuh"
+#include "internal.cuh"
 
 namespace dpf {
 namespace driver {
 
-// max over sites of |y_w| (the rotation part of the increment); non-negative
-// doubles order like their bit patterns, so an integer atomicMax is exact.
-__global__ void max_rotation_kernel(int64_t n, const double *y, unsigned long long *out) {
-    double best = 0.0;
-    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < n; s += (int64_t)gridDim.x * blockDim.x) {
-        const double *w = y + 6 * s + 3;
-        const double v = sqrt(w[0] * w[0] + w[1] * w[1] + w[2] * w[2]);
-        best = v > best ? v : best;
+// The end of an accepted step: x_end = x + u, v_end = 2 y / dt - v, R_end = exp(y_w) R
+// (each as dpf_mixed_commit and dpf_accept_step form it), and the largest |y_w|,
+// with the PCG's iteration count, to the host.
+struct AcceptArgs {
+    int64_t n;
+    const double *x, *y, *v, *rotation;
+    double two_over_dt;
+    double *x_end, *v_end, *rotation_end, *partials, *turn;
+    const int *inner;
+    int *inner_to;
+};
+
+__global__ void __launch_bounds__(kThreads) accept_kernel(AcceptArgs a) {
+    double turn = 0.0;
+    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < a.n; s += (int64_t)gridDim.x * blockDim.x) {
+        const double2 *yp = reinterpret_cast<const double2 *>(a.y + 6 * s);
+        const double2 y0 = yp[0], y1 = yp[1], y2 = yp[2];
+        const double y[6] = {y0.x, y0.y, y1.x, y1.y, y2.x, y2.y};
+        const d3 u = mk(y[0], y[1], y[2]), w = mk(y[3], y[4], y[5]);
+        double v[6];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) v[c] = a.two_over_dt * y[c] - a.v[6 * s + c];
+        st3(a.x_end, s, ld3(a.x, s) + u);
+#pragma unroll
+        for (int c = 0; c < 6; ++c) a.v_end[6 * s + c] = v[c];
+        rotate_site(w, a.rotation + 9 * s, a.rotation_end + 9 * s);
+        turn = fmax(turn, dot(w, w));
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        const double other = __shfl_xor_sync(0xffffffffu, best, o);
-        best = other > best ? other : best;
+    turn = block_max(turn);
+    double *part = a.partials + 8;
+    if (threadIdx.x == 0) part[blockIdx.x] = turn;
+    if (last_block(reinterpret_cast<unsigned *>(a.partials) + 1)) {
+        const double most = block_max_array(part, gridDim.x, 1);
+        if (threadIdx.x == 0) {
+            *a.turn = sqrt(most);
+            *a.inner_to = *a.inner;
+        }
     }
-    if ((threadIdx.x & 31) == 0 && best > 0.0) atomicMax(out, (unsigned long long)__double_as_longlong(best));
 }
 
 // launch categories timed with step->timing (the order of DPF_NEWTON_TIMERS)
@@ -92,9 +118,11 @@ struct Step {
     dpf_newton_info *info;
     cudaStream_t st;
     int64_t n, n6, m;
-    double *y, *cand, *r, *r_cand, *scaled, *rhs, *x, *res, *corr, *ax;
-    double *host;     // pinned: [0..8) scalars, [8..10) scales, [12] a norm, [16..80) h column
+    double *y, *cand, *r, *r_cand, *scaled, *rhs, *x, *res, *corr;
+    double *host;     // pinned, written by the kernels: [0..3) a residual's norms, [4..7) the scaled residual's,
+                      // [8..10) scales, [12..14) the true Krylov residual's, [14..16) work, [16..80) h column
     int *host_int;    // pinned ints after the doubles: [0] status, [1] inner
+    const double *v0, *rotation0;   // the step's start
     Timing timing;
     bool packed = false;
     double rhs_scale = -1.0;
@@ -115,46 +143,47 @@ struct Step {
         return rc;
     }
 
-    // copy `count` device scalars (and optionally the status word and the
-    // step's scales) to pinned memory, then wait for the stream
-    int fetch(int count, bool status, bool scales) {
-        if (count && cudaMemcpyAsync(host, s->scalars, count * sizeof(double), cudaMemcpyDeviceToHost, st))
-            return DPF_ERR_CUDA;
+    // wait for the stream, after copying the status word when no kernel reported it
+    int wait(bool status = false) {
         if (status && cudaMemcpyAsync(host_int, s->status, sizeof(int), cudaMemcpyDeviceToHost, st))
-            return DPF_ERR_CUDA;
-        if (scales && cudaMemcpyAsync(host + 8, s->scales, 2 * sizeof(double), cudaMemcpyDeviceToHost, st))
             return DPF_ERR_CUDA;
         return cudaStreamSynchronize(st) == cudaSuccess ? DPF_OK : DPF_ERR_CUDA;
     }
 
-    int residual(const double *yy, double *out, bool use_p) {
-        int rc = call(kVector, 1, [&] { return dpf_to_float(n6, yy, s->y32, st); });
-        if (rc) return rc;
-        if (cudaMemsetAsync(s->status, 0, sizeof(int), st)) return DPF_ERR_CUDA;
+    // prepared: y32 = (float)yy and the cleared status word are there already
+    int residual(const double *yy, double *out, bool use_p, bool prepared) {
+        if (!prepared) {
+            const int rc = call(kVector, 1, [&] { return dpf_to_float(n6, yy, s->y32, st); });
+            if (rc) return rc;
+            if (cudaMemsetAsync(s->status, 0, sizeof(int), st)) return DPF_ERR_CUDA;
+        }
         return call(kResidual, m ? 2 : 1, [&] {
             return dpf_mixed_residual(s->graph, s->bond_data, yy, s->y32, s->mass, s->fixed, a->dt, s->r0, 1,
                                       use_p ? cur.p32 : nullptr, use_p ? cur.units32 : nullptr, out, nullptr,
-                                      use_p ? s->scalars : nullptr, s->wrench32, s->partials, s->status, st);
+                                      use_p ? host : nullptr, s->wrench32, s->partials, s->status, st);
         });
     }
 
     // blocks and scaling of the tangent in bond_data into `into`, then the
-    // scaled residual of rr and its norms [|r|, max |s|, |s|] into norms
-    int scaling_norms(const Scaling &into, const double *rr, double *norms) {
+    // scaled residual of rr and its norms [|r|, max |s|, |s|] into norms, with
+    // the report and the status word
+    int scaling_norms(const Scaling &into, const double *rr, double *norms, Report report) {
         int rc = call(kScaling, 1, [&] {
             return dpf_mixed_scaling(s->graph, s->bond_data, s->mass32, s->fixed, s->radii, a->dt, into.block32,
                                      into.p32, into.units, into.units32, st);
         });
         if (rc) return rc;
+        report.status = s->status;
+        report.status_to = host_int;
         return call(kNorms, 1, [&] {
-            return dpf_mixed_scale_residual(n, into.p32, into.units32, rr, scaled, norms, s->partials, st);
+            return scale_residual_pass(n, into.p32, into.units32, rr, scaled, norms, s->partials, report, st);
         });
     }
 
-    // the elastic PCG on a float32 Krylov vector
+    // the elastic PCG on a float32 Krylov vector; d32 = units * out for the JVP
     int precondition(const float *vector, float *out) {
         if (!packed) {
-            const int rc = call(kPack, 2, [&] {
+            const int rc = call(kPack, 1, [&] {
                 return dpf_end_pack(s->graph, s->bond_data, 0.25 * a->dt * a->dt, cur.p32, s->mass32, s->fixed,
                                     s->ends, s->p24, s->site4, st);
             });
@@ -162,50 +191,42 @@ struct Step {
             packed = true;
         }
         return call(kPcg, 1, [&] {
-            return dpf_end_precondition_f32(s->graph, s->ends, s->site4, s->fixed, cur.block32, s->p24, cur.units32,
-                                            vector, 0.03, 80, out, s->inner, s->end_workspace, s->end_partials,
-                                            s->barrier, s->status, s->end_variant, st);
+            return end_precondition32_pass(s->graph, s->ends, s->site4, s->fixed, cur.block32, s->p24, cur.units32,
+                                           vector, 0.03, 80, out, s->d32, s->inner, s->end_workspace,
+                                           s->end_partials, s->barrier, s->barrier + 1, s->status, s->end_variant,
+                                           st);
         });
     }
 
-    // J d on float32 Krylov vectors
-    int jvp32(const float *direction, float *out) {
-        return call(kJvp, m ? 3 : 2, [&] {
-            return dpf_mixed_jacobian_vector_f32(s->graph, s->bond_data, s->y32, direction, s->mass32, s->fixed,
-                                                 a->dt, cur.units32, cur.p32, out, s->d32, s->wrench32, st);
-        });
-    }
-
-    // J d on a float64 vector (the Newton direction)
-    int jvp(const double *direction, double *out) {
-        return call(kJvp, m ? 3 : 2, [&] {
-            return dpf_mixed_jacobian_vector(s->graph, s->bond_data, s->y32, direction, s->mass32, s->fixed, a->dt,
-                                             cur.units32, cur.p32, out, s->d32, s->wrench32, nullptr, nullptr, st);
+    // J d on d32
+    int jvp32(float *out) {
+        return call(kJvp, m ? 2 : 1, [&] {
+            return jvp32_pass(s->graph, s->bond_data, s->y32, s->mass32, s->fixed, a->dt, cur.units32, cur.p32, out,
+                              s->d32, s->wrench32, st);
         });
     }
 
     // One restart cycle of the right-preconditioned FGMRES with CGS2 Arnoldi
-    // (MixedNewtonBonds._fgmres32 in newton.py) from `start` with |start| = g0:
-    // x += the cycle's correction, then J x (from the kept products J z_k), the
-    // true residual res = rhs - J x and its norm (krylov_scalars[1]) are
-    // enqueued but not read: the caller fetches that norm together with the
-    // speculative line-search values.  The Krylov vectors are float32 (the PCG
-    // and JVP outputs carry float32 precision), their sums exact float32
-    // pairs; x, rhs and the true residual are float64.  *krylov counts the
-    // Arnoldi steps; *singular reports a zero Givens denominator.
-    int fgmres_cycle(const double *start, double g0, double norm, double tolerance, int width, int *krylov,
-                     bool *singular) {
+    // (MixedNewtonBonds._fgmres32 in newton.py)
+    // from sign * `start` with |start| = g0; the caller forms the correction, the
+    // true residual (from the kept products J z_k) and its norm from the `columns`
+    // coefficients.  The Krylov vectors are float32 (the PCG and JVP outputs carry
+    // float32 precision), their sums exact float32 pairs; x and the true residual
+    // are float64.  *krylov counts the Arnoldi steps; *singular reports a zero
+    // Givens denominator.
+    int fgmres_cycle(const double *start, double sign, double g0, double norm, double tolerance, int width,
+                     int *krylov, bool *singular, double *coef, int *columns) {
         *singular = false;
         if (width > s->krylov_width) return DPF_ERR_ARGUMENT;
         const int ldh = width;  // H is (width + 1) x width, row-major
         double H[64 * 63];
-        double cs[64], sn[64], g[65], coef[64];
+        double cs[64], sn[64], g[65];
         std::memset(H, 0, sizeof(double) * (width + 1) * width);
         std::memset(cs, 0, sizeof(double) * width);
         std::memset(sn, 0, sizeof(double) * width);
         std::memset(g, 0, sizeof(double) * (width + 1));
         g[0] = g0;
-        int rc = call(kKrylov, 1, [&] { return dpf_scale_to_float(n6, 1.0 / g[0], start, s->basis, st); });
+        int rc = call(kKrylov, 1, [&] { return dpf_scale_to_float(n6, sign / g[0], start, s->basis, st); });
         if (rc) return rc;
         for (int j = 0; j < width; ++j) {
             float *bj = s->basis + (int64_t)j * n6;
@@ -213,17 +234,16 @@ struct Step {
             float *pj = s->products + (int64_t)j * n6;
             rc = precondition(bj, tj);
             if (rc) return rc;
-            rc = jvp32(tj, pj);
+            rc = jvp32(pj);
             if (rc) return rc;
             rc = call(kKrylov, 1, [&] {
-                return dpf_arnoldi_cgs2_f32(n6, s->basis, n6, j, pj, s->w32, s->h, s->krylov_partials, s->barrier,
-                                            s->status, st);
+                return arnoldi32_pass(n6, s->basis, n6, j, pj, s->w32, host + 16, s->krylov_partials,
+                                      s->barrier + 1, s->barrier, s->status, st);
             });
             if (rc) return rc;
-            double *column = host + 16;
-            if (cudaMemcpyAsync(column, s->h, (j + 2) * sizeof(double), cudaMemcpyDeviceToHost, st) ||
-                cudaStreamSynchronize(st))
-                return DPF_ERR_CUDA;
+            rc = wait();
+            if (rc) return rc;
+            const double *column = host + 16;
             for (int k = 0; k <= j + 1; ++k) H[k * ldh + j] = column[k];
             const bool breakdown = H[(j + 1) * ldh + j] < 1e-14;
             for (int k = 0; k < j; ++k) {
@@ -252,74 +272,64 @@ struct Step {
                     for (int c = i + 1; c < k; ++c) acc -= H[i * ldh + c] * coef[c];
                     coef[i] = acc / H[i * ldh + i];
                 }
-                rc = call(kKrylov, 1, [&] { return dpf_combine_rows_f32(n6, s->transformed, n6, k, coef, x, st); });
-                if (rc) return rc;
-                // J x = sum_k c_k J z_k from the stored products (J is linear)
-                if (cudaMemsetAsync(ax, 0, n6 * sizeof(double), st)) return DPF_ERR_CUDA;
-                rc = call(kKrylov, 1, [&] { return dpf_combine_rows_f32(n6, s->products, n6, k, coef, ax, st); });
-                if (rc) return rc;
-                rc = call(kVector, 1, [&] { return dpf_axpby(n6, 1.0, rhs, -1.0, ax, res, st); });
-                if (rc) return rc;
-                return call(kKrylov, 1, [&] {
-                    return dpf_dot_norm(n6, res, nullptr, s->krylov_scalars, s->krylov_partials, st);
-                });
+                *columns = k;
+                return DPF_OK;
             }
         }
         return DPF_OK;
     }
 
+    // the end state (y32 is the accepted increment's already)
     int accept() {
-        int rc = call(kVector, 1, [&] { return dpf_to_float(n6, y, s->y32, st); });
-        if (rc) return rc;
         const dpf_history &h = a->history;
-        rc = call(kCommit, m ? 3 : 1, [&] {
-            if (s->history_corrections)
-                return dpf_mixed_commit_lazy(s->graph, s->bond_data, h.x, y, s->y32, a->x_end, s->history_corrections,
-                                             s->wrench32, s->loads, st);
-            return dpf_mixed_commit(s->graph, s->bond_data, &h, y, s->y32, a->x_end, a->normal_end, a->offset_end,
-                                    a->fn_end, a->fs_end, a->mt_end, a->mb_end, s->wrench32, s->loads, st);
-        });
-        if (rc) return rc;
-        rc = call(kAccept, 1, [&] { return dpf_accept_step(n, y, a->dt, a->v, a->rotation, st); });
-        if (rc) return rc;
-        rc = call(kAccept, 1, [&] { return dpf_dot_norm(n6, a->external, y, s->scalars, s->partials, st); });
-        if (rc) return rc;
-        if (cudaMemsetAsync(s->scalars + 2, 0, sizeof(double), st)) return DPF_ERR_CUDA;
-        rc = call(kAccept, 1, [&] {
-            const int grid = (int)((n + 255) / 256 < 1024 ? (n + 255) / 256 : 1024);
-            max_rotation_kernel<<<grid, 256, 0, st>>>(n, y, reinterpret_cast<unsigned long long *>(s->scalars + 2));
+        int rc = call(kAccept, 1, [&] {
+            const int threads = reduce_threads(n);
+            const int64_t want = (n + threads - 1) / threads;
+            AcceptArgs k{n, h.x, y, v0, rotation0, 2.0 / a->dt, a->x_end, a->v, a->rotation, s->partials, host + 2,
+                         s->inner, host_int + 1};
+            accept_kernel<<<(int)(want < 1024 ? want : 1024), threads, 0, st>>>(k);
             return cudaGetLastError() == cudaSuccess ? DPF_OK : DPF_ERR_CUDA;
         });
         if (rc) return rc;
-        if (cudaMemcpyAsync(host_int + 1, s->inner, sizeof(int), cudaMemcpyDeviceToHost, st)) return DPF_ERR_CUDA;
-        rc = fetch(3, false, false);
+        if (m) {
+            rc = call(kCommit, 2, [&] {
+                return mixed_commit_pass(s->graph, s->bond_data, &h, s->y32, a->x_end, a->normal_end, a->offset_end,
+                                         a->fn_end, a->fs_end, a->mt_end, a->mb_end, s->history_corrections,
+                                         s->wrench32, s->loads, st);
+            });
+            if (rc) return rc;
+        }
+        rc = call(kAccept, 1, [&] { return dpf_dot_norm(n6, a->external, y, host + 14, s->partials, st); });
         if (rc) return rc;
-        info->work = host[0];
+        rc = wait();
+        if (rc) return rc;
+        info->work = host[14];
         info->max_rotation = host[2];
         info->cg_iterations = host_int[1];
         return DPF_OK;
     }
 
     int run() {
-        if (cudaMemsetAsync(s->inner, 0, sizeof(int), st) || cudaMemsetAsync(s->status, 0, sizeof(int), st) ||
-            cudaMemsetAsync(y, 0, n6 * sizeof(double), st))
-            return DPF_ERR_CUDA;
-        if ((a->v_in && cudaMemcpyAsync(a->v, a->v_in, n6 * sizeof(double), cudaMemcpyDeviceToDevice, st)) ||
-            (a->rotation_in &&
-             cudaMemcpyAsync(a->rotation, a->rotation_in, 9 * n * sizeof(double), cudaMemcpyDeviceToDevice, st)))
-            return DPF_ERR_CUDA;
+        const bool committed = a->committed_start && !a->refresh;
         int rc;
-        if (a->refresh) {
-            const dpf_history &h = a->history;
-            rc = call(kSetup, m ? 2 : 1, [&] {
-                return dpf_mixed_setup(s->graph, &s->stiffness, &h, s->mass, a->v, a->external, s->fixed, a->dt,
-                                       s->bond_data, s->r0, s->loads, s->scales, s->wrench64,
-                                       s->history_corrections, s->partials, s->status, st);
+        if (committed) {
+            rc = call(kSetup, 1, [&] {
+                return mixed_start_pass(n, s->loads, s->mass, v0, a->external, s->fixed, a->dt, s->r0, s->scales,
+                                        s->partials, y, s->y32, r, s->status, s->inner, s->barrier, st);
             });
         } else {
-            rc = call(kSetup, 1, [&] {
-                return dpf_mixed_begin(n, s->loads, s->mass, a->v, a->external, s->fixed, a->dt, s->r0, s->scales,
-                                       s->partials, st);
+            if (cudaMemsetAsync(s->inner, 0, sizeof(int), st) || cudaMemsetAsync(s->status, 0, sizeof(int), st) ||
+                cudaMemsetAsync(s->barrier, 0, 2 * sizeof(unsigned), st) ||
+                cudaMemsetAsync(y, 0, n6 * sizeof(double), st))
+                return DPF_ERR_CUDA;
+            rc = call(kSetup, !a->refresh ? 1 : m ? 2 : 1, [&] {
+                if (!a->refresh)
+                    return dpf_mixed_begin(n, s->loads, s->mass, v0, a->external, s->fixed, a->dt, s->r0, s->scales,
+                                           s->partials, st);
+                const dpf_history &h = a->history;
+                return dpf_mixed_setup(s->graph, &s->stiffness, &h, s->mass, v0, a->external, s->fixed, a->dt,
+                                       s->bond_data, s->r0, s->loads, s->scales, s->wrench64,
+                                       s->history_corrections, s->partials, s->status, st);
             });
         }
         if (rc) return rc;
@@ -335,18 +345,15 @@ struct Step {
                 local = pre[1];
                 merit = pre[2];
             } else {
-                if (iteration == 0 && a->committed_start && !a->refresh) {
-                    if (cudaMemsetAsync(s->status, 0, sizeof(int), st)) return DPF_ERR_CUDA;
-                    rc = call(kResidual, 1,
-                              [&] { return dpf_mixed_initial_residual(n, s->r0, s->fixed, s->y32, r, st); });
-                    if (rc) return rc;
-                } else if (!cached) {
-                    rc = residual(y, r, false);
+                if (!cached && !(iteration == 0 && committed)) {
+                    rc = residual(y, r, false, false);
                     if (rc) return rc;
                 }
-                rc = scaling_norms(cur, r, s->scalars);
+                Report report;
+                if (first) report = {s->scales, host + 8, 2};
+                rc = scaling_norms(cur, r, host, report);
                 if (rc) return rc;
-                rc = fetch(3, !cached, first);
+                rc = wait();
                 if (rc) return rc;
                 const int status = cached ? 0 : host_int[0];
                 if (status) {
@@ -388,8 +395,13 @@ struct Step {
                 return DPF_OK;
             }
             if (iteration == a->max_iterations) break;
-            rc = call(kVector, 1, [&] { return dpf_axpby(n6, -1.0, scaled, 0.0, scaled, rhs, st); });
-            if (rc) return rc;
+            // the right-hand side is -rhs (the scaled residual of the iterate); the
+            // candidate's goes to the other vector
+            {
+                double *t = rhs;
+                rhs = scaled;
+                scaled = t;
+            }
             // FGMRES cycles (restart 32, at most 256 Arnoldi steps).  Each cycle's
             // true-residual norm is fetched together with a speculative first
             // line-search step (factor 1) and the scaling and norms of that
@@ -397,38 +409,37 @@ struct Step {
             // one wait instead of three.  A failed guess costs work, not results:
             // the iterate's scaling stays in `cur`, and y32 is restored before a
             // restart's JVPs.
-            if (cudaMemsetAsync(x, 0, n6 * sizeof(double), st)) return DPF_ERR_CUDA;
             int krylov = 0;
             const double *start = rhs;
-            double g0 = merit;
-            bool speculated = false;
+            double g0 = merit, sign = -1.0;
+            bool speculated = false, again = false;
             for (;;) {
+                double coef[64];
+                int columns = 0;
                 if (merit != 0.0) {
                     const int width = 256 - krylov < 32 ? 256 - krylov : 32;
                     bool singular;
-                    rc = fgmres_cycle(start, g0, merit, a->linear_tolerance, width, &krylov, &singular);
+                    rc = fgmres_cycle(start, sign, g0, merit, a->linear_tolerance, width, &krylov, &singular, coef,
+                                      &columns);
                     if (rc) return rc;
                     if (singular) {
                         info->outcome = DPF_NEWTON_SINGULAR;
                         return DPF_OK;
                     }
                 }
-                rc = call(kVector, 1, [&] { return dpf_masked_scale(n, x, cur.units, s->fixed, corr, st); });
+                rc = call(kVector, 1, [&] {
+                    return mixed_correction_pass(n, s->transformed, s->products, columns, coef, again, rhs, cur.units,
+                                                 s->fixed, y, x, res, corr, cand, s->y32, s->krylov_scalars,
+                                                 s->krylov_partials, s->status, st);
+                });
                 if (rc) return rc;
-                rc = call(kVector, 1, [&] { return dpf_axpby(n6, 1.0, y, 1.0, corr, cand, st); });
+                rc = residual(cand, r_cand, true, true);
                 if (rc) return rc;
-                rc = residual(cand, r_cand, true);
+                rc = scaling_norms(alt, r_cand, host + 4, {s->krylov_scalars, host + 12, 2});
                 if (rc) return rc;
-                rc = scaling_norms(alt, r_cand, s->scalars + 4);
+                rc = wait();
                 if (rc) return rc;
-                if (merit != 0.0 &&
-                    cudaMemcpyAsync(host + 12, s->krylov_scalars + 1, sizeof(double), cudaMemcpyDeviceToHost, st))
-                    return DPF_ERR_CUDA;
-                if (cudaMemcpyAsync(host + 4, s->scalars + 4, 3 * sizeof(double), cudaMemcpyDeviceToHost, st))
-                    return DPF_ERR_CUDA;
-                rc = fetch(3, true, false);
-                if (rc) return rc;
-                const double krylov_relative = merit != 0.0 ? host[12] / merit : 0.0;
+                const double krylov_relative = merit != 0.0 ? host[13] / merit : 0.0;
                 info->krylov_relative = krylov_relative;
                 if (krylov_relative <= 1.05 * a->linear_tolerance) {
                     speculated = true;
@@ -442,7 +453,9 @@ struct Step {
                 rc = call(kVector, 1, [&] { return dpf_to_float(n6, y, s->y32, st); });
                 if (rc) return rc;
                 start = res;
-                g0 = host[12];
+                sign = 1.0;
+                again = true;
+                g0 = host[13];
             }
             info->krylov_iterations += krylov;
             bool accepted = false;
@@ -451,9 +464,9 @@ struct Step {
                 if (power > 0 || !speculated) {
                     rc = call(kVector, 1, [&] { return dpf_axpby(n6, 1.0, y, factor, corr, cand, st); });
                     if (rc) return rc;
-                    rc = residual(cand, r_cand, true);
+                    rc = residual(cand, r_cand, true, false);
                     if (rc) return rc;
-                    rc = fetch(3, true, false);
+                    rc = wait(true);
                     if (rc) return rc;
                 }
                 if (host_int[0]) continue;
@@ -514,16 +527,31 @@ extern "C" int dpf_mixed_newton_step(const dpf_mixed_newton *solver, const dpf_n
     run.n6 = 6 * run.n;
     run.m = solver->graph->n_bonds;
     double *v = solver->vectors;
-    double **slots[DPF_NEWTON_VECTORS] = {&run.y, &run.cand, &run.r, &run.r_cand, &run.scaled,
-                                          &run.rhs, &run.x, &run.res, &run.corr, &run.ax};
-    for (int k = 0; k < DPF_NEWTON_VECTORS; ++k) *slots[k] = v + (int64_t)k * run.n6;
+    double **slots[] = {&run.y, &run.cand, &run.r, &run.r_cand, &run.scaled, &run.rhs, &run.x, &run.res, &run.corr};
+    static_assert(sizeof(slots) / sizeof(slots[0]) <= DPF_NEWTON_VECTORS, "vectors of a step");
+    for (size_t k = 0; k < sizeof(slots) / sizeof(slots[0]); ++k) *slots[k] = v + (int64_t)k * run.n6;
+    // the address at which the device writes the pinned block
+    void *mapped = nullptr;
+    if (cudaHostGetDevicePointer(&mapped, solver->host, 0) != cudaSuccess || mapped != (void *)solver->host) {
+        cudaGetLastError();
+        return DPF_ERR_ARGUMENT;
+    }
     run.host = solver->host;
     run.host_int = reinterpret_cast<int *>(solver->host + 96);
     run.cur = {solver->block32, solver->p32, solver->units32, solver->units};
     run.alt = {solver->block32_b, solver->p32_b, solver->units32_b, solver->units_b};
     run.timing.on = step->timing != 0;
     run.timing.stream = run.st;
-    const int rc = run.run();
+    run.v0 = step->v_in ? step->v_in : step->v;
+    run.rotation0 = step->rotation_in ? step->rotation_in : step->rotation;
+    int rc = run.run();
+    // a step that did not commit leaves the start values
+    if (!rc && info->outcome != DPF_NEWTON_CONVERGED &&
+        ((step->v_in && cudaMemcpyAsync(step->v, step->v_in, run.n6 * sizeof(double), cudaMemcpyDeviceToDevice,
+                                        run.st)) ||
+         (step->rotation_in && cudaMemcpyAsync(step->rotation, step->rotation_in, 9 * run.n * sizeof(double),
+                                               cudaMemcpyDeviceToDevice, run.st))))
+        rc = DPF_ERR_CUDA;
     if (!run.timing.events.empty() && cudaStreamSynchronize(run.st) == cudaSuccess) run.timing.collect(info);
     return rc;
 }

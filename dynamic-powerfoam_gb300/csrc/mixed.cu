@@ -10,6 +10,7 @@
 // only (normal change, transport increments, lever changes; see mixed.cuh)
 // and summed per site in float64.  The JVP is the forward-mode derivative of
 // the same float32 increment.  Site sums walk the incidence CSR (no atomics).
+#include "internal.cuh"
 #include "mixed.cuh"
 
 namespace dpf {
@@ -374,7 +375,7 @@ __device__ __forceinline__ void matvec6f(const float *P, const float x[6], float
 // instead of a float64 add per shuffle level), then in the last block the
 // grid totals.
 __device__ __forceinline__ void finish_norms(double sum_r, float max_s, float s_hi, float s_lo, double *partials,
-                                             int slot, double *norms, int *status) {
+                                             int slot, double *norms, int *status, const Report &report = Report()) {
     const float r_hi = (float)sum_r, r_lo = (float)(sum_r - (double)r_hi);
     const float2 r2 = block_pair_sum(r_hi, r_lo);
     const float mx = block_max_float(max_s);
@@ -394,6 +395,8 @@ __device__ __forceinline__ void finish_norms(double sum_r, float max_s, float s_
             norms[1] = mx;
             norms[2] = sqrt(s2);
             if (status && (!isfinite(r2) || !isfinite(s2))) atomicOr(status, DPF_ERR_NONFINITE);
+            for (int k = 0; k < report.count; ++k) report.to[k] = report.from[k];
+            if (report.status) *report.status_to = *report.status;
         }
     }
 }
@@ -500,7 +503,7 @@ __global__ void __launch_bounds__(kThreads) residual_sites(ResidualSiteArgs a) {
 // float32 once), the 36-float P block, the six units; s = P r / units.
 __global__ void __launch_bounds__(kThreads) scale_sites_f32(int64_t n, const float *P, const float *units32,
                                                             const double *r, double *scaled, double *norms,
-                                                            double *partials) {
+                                                            double *partials, Report report) {
     double sum_r = 0.0;
     float max_s = 0.0f;
     float s_hi = 0.0f, s_lo = 0.0f;
@@ -546,7 +549,7 @@ __global__ void __launch_bounds__(kThreads) scale_sites_f32(int64_t n, const flo
         }
     }
     if (!norms) return;
-    finish_norms(sum_r, max_s, s_hi, s_lo, partials, 7, norms, nullptr);
+    finish_norms(sum_r, max_s, s_hi, s_lo, partials, 7, norms, nullptr, report);
 }
 
 // ---------------------------------------------------------------------------
@@ -1334,17 +1337,30 @@ struct BeginArgs {
     const uint8_t *fixed;
     double dt, half_dt2;
     double *r0, *scales, *partials;
+    double *y, *residual;      // kStart: the rest of a step's start (mixed_start_pass)
+    float *y32;
+    int *status, *inner;
+    unsigned *barrier;
 };
 
+template <bool kStart>
 __global__ void __launch_bounds__(kThreads) begin_sites(BeginArgs a) {
     double a2 = 0.0, l2 = 0.0;
+    if (kStart && blockIdx.x == 0 && threadIdx.x == 0) *a.status = *a.inner = a.barrier[0] = a.barrier[1] = 0;
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < 6 * a.n; e += (int64_t)gridDim.x * blockDim.x) {
         const double mv = a.dt * a.mass[e] * a.v[e];
         const double rhs = mv + a.half_dt2 * a.external[e];
         a2 += rhs * rhs;
         const double L = a.loads[e];
-        if (!a.fixed[e / 6]) l2 += L * L;
-        a.r0[e] = -mv - a.half_dt2 * (L + a.external[e]);
+        const bool fx = a.fixed[e / 6] != 0;
+        if (!fx) l2 += L * L;
+        const double r0 = -mv - a.half_dt2 * (L + a.external[e]);
+        a.r0[e] = r0;
+        if (kStart) {
+            a.residual[e] = fx ? 0.0 : r0;
+            a.y[e] = 0.0;
+            a.y32[e] = 0.0f;
+        }
     }
     a2 = block_sum(a2);
     l2 = block_sum(l2);
@@ -1535,30 +1551,42 @@ int dpf_mixed_scaling(const dpf_graph *g, float *bond_data, const float *mass32,
 
 int dpf_mixed_scale_residual(int64_t n_sites, const float *preconditioner, const float *units32,
                              const double *residual, double *scaled, double *norms, double *partials, void *stream) {
+    return dpf::scale_residual_pass(n_sites, preconditioner, units32, residual, scaled, norms, partials, dpf::Report(),
+                                    (cudaStream_t)stream);
+}
+
+}  // extern "C"
+
+int dpf::scale_residual_pass(int64_t n_sites, const float *preconditioner, const float *units32,
+                             const double *residual, double *scaled, double *norms, double *partials,
+                             const Report &report, cudaStream_t st) {
     // P in 16-byte quads, units in 8-byte pairs, residual and scaled in 16-byte pairs
     if (n_sites <= 0 || !preconditioner || !units32 || !residual || (norms && !partials) ||
         ((uintptr_t)preconditioner & 15u) || ((uintptr_t)units32 & 7u) || ((uintptr_t)residual & 15u) ||
         ((uintptr_t)scaled & 15u))
         return DPF_ERR_ARGUMENT;
-    scale_sites_f32<<<reduce_grid(n_sites), kThreads, 0, (cudaStream_t)stream>>>(n_sites, preconditioner, units32,
-                                                                                  residual, scaled, norms, partials);
+    scale_sites_f32<<<reduce_grid(n_sites), kThreads, 0, st>>>(n_sites, preconditioner, units32, residual, scaled,
+                                                               norms, partials, report);
     DPF_CHECK_LAUNCH();
     return DPF_OK;
 }
+
+extern "C" {
 
 static int mixed_jvp(const dpf_graph *g, float *bond_data, const float *y32, const double *direction,
                      const float *direction32, const float *mass32, const uint8_t *fixed, double dt,
                      const float *units32, const float *preconditioner, double *out, float *out32, float *d32,
                      float *wrench, const int32_t *seg_bond, const uint8_t *active, void *stream) {
-    if (!mixed_graph_ok(g) || !bond_data || !y32 || (!direction && !direction32) || !mass32 || !fixed ||
-        (!out && !out32) || !d32 || (g->n_bonds && !wrench) || (preconditioner && !units32) ||
+    // neither direction: d32 holds units * direction already
+    if (!mixed_graph_ok(g) || !bond_data || !y32 || !mass32 || !fixed || (!out && !out32) || !d32 || (g->n_bonds && !wrench) || (preconditioner && !units32) ||
         (active && !seg_bond) || ((uintptr_t)preconditioner & 7u) ||  // rows of P are read in 8-byte pairs
         !aligned16(wrench))
         return DPF_ERR_ARGUMENT;
     cudaStream_t st = (cudaStream_t)stream;
     const int64_t n6 = 6 * g->n_sites;
-    prepare_direction<<<blocks_for(n6, kThreads), kThreads, 0, st>>>(n6, direction32 ? nullptr : direction,
-                                                                     direction32, units32, d32);
+    if (direction || direction32)
+        prepare_direction<<<blocks_for(n6, kThreads), kThreads, 0, st>>>(n6, direction32 ? nullptr : direction,
+                                                                         direction32, units32, d32);
     if (g->n_bonds) {
         JvpArgs a{g->n_bonds, split_bond_data(bond_data, g->n_bonds), y32, d32, wrench, seg_bond, active};
         jvp_bonds_mixed<<<blocks_for(g->n_bonds, kThreads), kThreads, 0, st>>>(a);
@@ -1693,10 +1721,24 @@ int dpf_mixed_commit(const dpf_graph *g, float *bond_data, const dpf_history *h,
         return DPF_ERR_ARGUMENT;
     cudaStream_t st = (cudaStream_t)stream;
     end_positions<<<blocks_for(3 * g->n_sites, kThreads), kThreads, 0, st>>>(g->n_sites, h->x, y, x_end);
+    return dpf::mixed_commit_pass(g, bond_data, h, y32, x_end, normal_end, offset_end, fn_end, fs_end, mt_end, mb_end,
+                                  nullptr, dloads, loads, st);
+}
+
+}  // extern "C"
+
+int dpf::mixed_commit_pass(const dpf_graph *g, float *bond_data, const dpf_history *h, const float *y32,
+                           const double *x_end, double *normal_end, double *offset_end, double *fn_end, double *fs_end,
+                           double *mt_end, double *mb_end, float *corrections, float *dloads, double *loads,
+                           cudaStream_t st) {
     if (g->n_bonds) {
         CommitArgs a{g->n_bonds, split_bond_data(bond_data, g->n_bonds), *h, y32, x_end, normal_end, offset_end,
-                     fs_end, mb_end, fn_end, mt_end, dloads, nullptr};
-        commit_bonds<false><<<blocks_for(g->n_bonds, kThreads), kThreads, 0, st>>>(a);
+                     fs_end, mb_end, fn_end, mt_end, dloads, reinterpret_cast<float4 *>(corrections)};
+        const int blocks = blocks_for(g->n_bonds, kThreads);
+        if (corrections)
+            commit_bonds<true><<<blocks, kThreads, 0, st>>>(a);
+        else
+            commit_bonds<false><<<blocks, kThreads, 0, st>>>(a);
         if (dloads)
             commit_sites<<<blocks_for(kGroupJ * g->n_sites, kThreads), kThreads, 0, st>>>(
                 g->n_sites, g->inc_ptr, g->inc_bond, dloads, loads);
@@ -1704,6 +1746,8 @@ int dpf_mixed_commit(const dpf_graph *g, float *bond_data, const dpf_history *h,
     DPF_CHECK_LAUNCH();
     return DPF_OK;
 }
+
+extern "C" {
 
 int dpf_mixed_initial_residual(int64_t n_sites, const double *r0, const uint8_t *fixed, float *y32, double *residual,
                                void *stream) {
@@ -1736,17 +1780,10 @@ int dpf_mixed_commit_lazy(const dpf_graph *g, float *bond_data, const double *x,
         return DPF_ERR_ARGUMENT;
     cudaStream_t st = (cudaStream_t)stream;
     end_positions<<<blocks_for(3 * g->n_sites, kThreads), kThreads, 0, st>>>(g->n_sites, x, y, x_end);
-    if (g->n_bonds) {
-        dpf_history h{};
-        h.x = x;
-        CommitArgs a{g->n_bonds, split_bond_data(bond_data, g->n_bonds), h, y32, x_end, nullptr, nullptr, nullptr,
-                     nullptr, nullptr, nullptr, dloads, reinterpret_cast<float4 *>(corrections)};
-        commit_bonds<true><<<blocks_for(g->n_bonds, kThreads), kThreads, 0, st>>>(a);
-        commit_sites<<<blocks_for(kGroupJ * g->n_sites, kThreads), kThreads, 0, st>>>(g->n_sites, g->inc_ptr,
-                                                                                       g->inc_bond, dloads, loads);
-    }
-    DPF_CHECK_LAUNCH();
-    return DPF_OK;
+    dpf_history h{};
+    h.x = x;
+    return dpf::mixed_commit_pass(g, bond_data, &h, y32, x_end, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
+                                  corrections, dloads, loads, st);
 }
 
 int dpf_mixed_fold_history(const dpf_graph *g, const double *x, const float *bond_data, const float *corrections,
@@ -1768,11 +1805,37 @@ int dpf_mixed_begin(int64_t n_sites, const double *loads, const double *mass, co
                     const uint8_t *fixed, double dt, double *r0, double *scales, double *partials, void *stream) {
     if (n_sites <= 0 || !loads || !mass || !v || !external || !fixed || !r0 || !scales || !partials)
         return DPF_ERR_ARGUMENT;
-    BeginArgs a{n_sites, loads, mass, v, external, fixed, dt, 0.5 * dt * dt, r0, scales, partials};
-    begin_sites<<<reduce_grid(6 * n_sites), kThreads, 0, (cudaStream_t)stream>>>(a);
+    BeginArgs a{n_sites, loads, mass, v, external, fixed, dt, 0.5 * dt * dt, r0, scales, partials,
+                nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+    begin_sites<false><<<reduce_grid(6 * n_sites), kThreads, 0, (cudaStream_t)stream>>>(a);
     DPF_CHECK_LAUNCH();
     return DPF_OK;
 }
+
+}  // extern "C"
+
+int dpf::mixed_start_pass(int64_t n_sites, const double *loads, const double *mass, const double *v,
+                          const double *external, const uint8_t *fixed, double dt, double *r0, double *scales,
+                          double *partials, double *y, float *y32, double *residual, int *status, int *inner,
+                          unsigned *barrier, cudaStream_t st) {
+    if (n_sites <= 0 || !loads || !mass || !v || !external || !fixed || !r0 || !scales || !partials || !y || !y32 ||
+        !residual || !status || !inner || !barrier)
+        return DPF_ERR_ARGUMENT;
+    BeginArgs a{n_sites, loads, mass, v, external, fixed, dt, 0.5 * dt * dt, r0, scales, partials,
+                y, residual, y32, status, inner, barrier};
+    begin_sites<true><<<reduce_grid(6 * n_sites), kThreads, 0, st>>>(a);
+    DPF_CHECK_LAUNCH();
+    return DPF_OK;
+}
+
+int dpf::jvp32_pass(const dpf_graph *g, float *bond_data, const float *y32, const float *mass32, const uint8_t *fixed,
+                    double dt, const float *units32, const float *preconditioner, float *out, const float *d32,
+                    float *wrench, cudaStream_t st) {
+    return mixed_jvp(g, bond_data, y32, nullptr, nullptr, mass32, fixed, dt, units32, preconditioner, nullptr, out,
+                     const_cast<float *>(d32), wrench, nullptr, nullptr, st);
+}
+
+extern "C" {
 
 int64_t dpf_segment_partials_doubles(int n_segments) { return n_segments < 0 ? 0 : 3LL * kSegChunks * n_segments; }
 

@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "internal.cuh"
 
 namespace dpf {
 namespace tiles {
@@ -539,23 +540,30 @@ __global__ void __launch_bounds__(kThreads) pack_entries_kernel(PackArgs a) {
 
 // P (36 floats, symmetric) -> 21 upper-triangle floats padded to 24; site
 // records (m, I, 1, 0), fixed sites (1, 1, 0, 0).
-__global__ void __launch_bounds__(kThreads) pack_sites_kernel(int64_t n, const float *P36, const float *mass32,
-                                                              const uint8_t *fixed, float4 *P24, float4 *site) {
-    const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+// A site's P packed to its upper triangle and its operator record; either output may be NULL.
+__device__ __forceinline__ void pack_site(int64_t s, int64_t n, const float *P36, const float *mass32,
+                                          const uint8_t *fixed, float4 *P24, float4 *site) {
     if (s >= n) return;
-    const float *p = P36 + 36 * s;
-    float u[24];
-    int k = 0;
+    if (P24) {
+        const float *p = P36 + 36 * s;
+        float u[24];
+        int k = 0;
 #pragma unroll
-    for (int r = 0; r < 6; ++r)
+        for (int r = 0; r < 6; ++r)
 #pragma unroll
-        for (int c = r; c < 6; ++c) u[k++] = p[6 * r + c];
-    u[21] = u[22] = u[23] = 0.0f;
+            for (int c = r; c < 6; ++c) u[k++] = p[6 * r + c];
+        u[21] = u[22] = u[23] = 0.0f;
 #pragma unroll
-    for (int q = 0; q < 6; ++q) P24[6 * s + q] = make_float4(u[4 * q], u[4 * q + 1], u[4 * q + 2], u[4 * q + 3]);
+        for (int q = 0; q < 6; ++q) P24[6 * s + q] = make_float4(u[4 * q], u[4 * q + 1], u[4 * q + 2], u[4 * q + 3]);
+    }
     if (site)
         site[s] = fixed[s] ? make_float4(1.0f, 1.0f, 0.0f, 0.0f)
                            : make_float4(mass32[6 * s], mass32[6 * s + 3], 1.0f, 0.0f);
+}
+
+__global__ void __launch_bounds__(kThreads) pack_sites_kernel(int64_t n, const float *P36, const float *mass32,
+                                                              const uint8_t *fixed, float4 *P24, float4 *site) {
+    pack_site(blockIdx.x * (int64_t)blockDim.x + threadIdx.x, n, P36, mass32, fixed, P24, site);
 }
 
 __device__ __forceinline__ void sym6(const float4 *P24, float P[21]) {
@@ -788,6 +796,11 @@ __global__ void __launch_bounds__(kEndThreads, B) end_hvp_kernel(EndGraph G, con
 // v = inc_bond[k] (v >= 0: s is its i end; ~v: its j end).
 struct EndPackArgs {
     int64_t n_inc;
+    int end_blocks;                   // the blocks from here on pack the sites
+    int64_t n;
+    const float *P36, *mass32;
+    const uint8_t *fixed;
+    float4 *P24, *site;
     const int32_t *inc_bond;
     const int64_t *edges;
     const float4 *t0, *t1, *t2, *t3;  // tangent records (n, kn), (ri, ks), (rj, kb), (kt, -, -, -)
@@ -796,6 +809,11 @@ struct EndPackArgs {
 };
 
 __global__ void __launch_bounds__(kThreads) pack_ends_kernel(EndPackArgs a) {
+    if ((int)blockIdx.x >= a.end_blocks) {
+        pack_site(((int)blockIdx.x - a.end_blocks) * (int64_t)blockDim.x + threadIdx.x, a.n, a.P36, a.mass32, a.fixed,
+                  a.P24, a.site);
+        return;
+    }
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= a.n_inc) return;
     const int v = a.inc_bond[k];
@@ -834,6 +852,8 @@ struct PcgArgs {
     int max_it;
     double *out;
     float *out32;           // float32 output instead of out (one of the two)
+    float *direction;       // with out32: units * out32 (the JVP's direction), or NULL
+    unsigned *clear;        // the next launch's barrier word, or NULL
     int *iterations;
     float *x, *r, *u, *p, *s, *w;  // (N, 6) each
     double *part_a, *part_b;
@@ -865,15 +885,22 @@ __device__ __forceinline__ void mv36(const float *B, const float x[6], float y[6
 
 // One site of the single-reduction update: p = u + beta p, x += alpha p,
 // s = w + beta s, r -= alpha s, u = P r; returns (r, u).  Every load of the
-// site comes before any store.
+// site comes before any store.  kFirst: x = p = s = 0, neither stored before nor
+// read here.
+template <bool kFirst>
 __device__ __forceinline__ float update_site(const PcgArgs &a, int64_t s, float fa, float fb) {
     float uv[6], pv[6], xv[6], wv[6], sv[6], rv[6], Pm[21];
     const uint64_t pol = keep_policy();
     ld6_keep(a.u + 6 * s, uv, pol);
-    ld6_keep(a.p + 6 * s, pv, pol);
-    ld6_keep(a.x + 6 * s, xv, pol);
     ld6_keep(a.w + 6 * s, wv, pol);
-    ld6_keep(a.s + 6 * s, sv, pol);
+    if (kFirst) {
+#pragma unroll
+        for (int c = 0; c < 6; ++c) pv[c] = xv[c] = sv[c] = 0.0f;
+    } else {
+        ld6_keep(a.p + 6 * s, pv, pol);
+        ld6_keep(a.x + 6 * s, xv, pol);
+        ld6_keep(a.s + 6 * s, sv, pol);
+    }
     ld6_keep(a.r + 6 * s, rv, pol);
     {
         float q24[24];
@@ -912,10 +939,10 @@ template <bool kTiles, int L>
 __device__ __forceinline__ void pcg_body(PcgArgs &a, unsigned char *smem) {
     const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    const float zero6[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    if (a.clear && tid == 0) *a.clear = 0u;
     Pipe P;
     if (kTiles) P = pipe_init(smem, a.L, ((int)blockDim.x - 64) / 32);
-    // r0 = B (units v) with fixed rows zero, u0 = P r0, x = p = s = 0
+    // r0 = B (units v) with fixed rows zero, u0 = P r0
     float pf = 0.0f;
     for (int64_t s = tid; s < a.n; s += stride) {
         float v[6], rr[6], zz[6], Pm[21];
@@ -932,9 +959,6 @@ __device__ __forceinline__ void pcg_body(PcgArgs &a, unsigned char *smem) {
         sym_mv6(Pm, rr, zz);
         st6(a.r + 6 * s, rr);
         st6(a.u + 6 * s, zz);
-        st6(a.x + 6 * s, zero6);
-        st6(a.p + 6 * s, zero6);
-        st6(a.s + 6 * s, zero6);
 #pragma unroll
         for (int c = 0; c < 6; ++c) pf = fmaf(rr[c], zz[c], pf);
     }
@@ -950,6 +974,7 @@ __device__ __forceinline__ void pcg_body(PcgArgs &a, unsigned char *smem) {
                 a.out32[e] = 0.0f;
             else
                 a.out[e] = 0.0;
+            if (a.direction) a.direction[e] = 0.0f;
         }
         return;
     }
@@ -986,7 +1011,10 @@ __device__ __forceinline__ void pcg_body(PcgArgs &a, unsigned char *smem) {
         const double alpha = shared_ab[0], beta = shared_ab[1];
         const float fa = (float)alpha, fb = (float)beta;
         pf = 0.0f;
-        for (int64_t s = tid; s < a.n; s += stride) pf += update_site(a, s, fa, fb);
+        if (it == 0)
+            for (int64_t s = tid; s < a.n; s += stride) pf += update_site<true>(a, s, fa, fb);
+        else
+            for (int64_t s = tid; s < a.n; s += stride) pf += update_site<false>(a, s, fa, fb);
         block_pair_partial(pf, part_b);
         if (!grid_barrier(a.barrier, a.status)) return;
         const double following = pair_total(part_b, gridDim.x);
@@ -1000,11 +1028,12 @@ __device__ __forceinline__ void pcg_body(PcgArgs &a, unsigned char *smem) {
         ld6(a.x + 6 * s, xv);
 #pragma unroll
         for (int c = 0; c < 6; ++c) {
-            const float v = xv[c] / a.units32[6 * s + c];
+            const float un = a.units32[6 * s + c], v = xv[c] / un;
             if (a.out32)
                 a.out32[6 * s + c] = v;
             else
                 a.out[6 * s + c] = (double)v;
+            if (a.direction) a.direction[6 * s + c] = v * un;
         }
     }
     if (tid == 0) atomicAdd(a.iterations, it < a.max_it ? it + 1 : a.max_it);
@@ -1420,18 +1449,16 @@ int dpf_end_pack(const dpf_graph *g, const float *bond_data, double alpha, const
                                                                 !aligned16(bond_data) || !aligned16(ends))) ||
         (P24 && (!P36 || !aligned16(P24))) || (site4 && (!mass32 || !fixed || !aligned16(site4))))
         return DPF_ERR_ARGUMENT;
-    cudaStream_t st = (cudaStream_t)stream;
     const int64_t m = g->n_bonds, n_inc = 2 * m;
-    if (m) {
-        const float4 *base = reinterpret_cast<const float4 *>(bond_data);
-        float4 *e = reinterpret_cast<float4 *>(ends);
-        EndPackArgs a{n_inc, g->inc_bond, g->edges, base + 7 * m, base + 8 * m, base + 9 * m, base + 10 * m,
-                      (float)alpha, e, e + n_inc, e + 2 * n_inc};
-        pack_ends_kernel<<<blocks_for(n_inc, kThreads), kThreads, 0, st>>>(a);
-    }
-    if (P24 || site4)
-        pack_sites_kernel<<<blocks_for(g->n_sites, kThreads), kThreads, 0, st>>>(
-            g->n_sites, P36, mass32, fixed, reinterpret_cast<float4 *>(P24), reinterpret_cast<float4 *>(site4));
+    const float4 *base = reinterpret_cast<const float4 *>(bond_data);
+    float4 *e = reinterpret_cast<float4 *>(ends);
+    const int end_blocks = blocks_for(n_inc, kThreads);
+    const int blocks = end_blocks + (P24 || site4 ? blocks_for(g->n_sites, kThreads) : 0);
+    if (!blocks) return DPF_OK;
+    EndPackArgs a{n_inc, end_blocks, g->n_sites, P36, mass32, fixed, reinterpret_cast<float4 *>(P24),
+                  reinterpret_cast<float4 *>(site4), g->inc_bond, g->edges,
+                  base + 7 * m, base + 8 * m, base + 9 * m, base + 10 * m, (float)alpha, e, e + n_inc, e + 2 * n_inc};
+    pack_ends_kernel<<<blocks, kThreads, 0, (cudaStream_t)stream>>>(a);
     DPF_CHECK_LAUNCH();
     return DPF_OK;
 }
@@ -1472,7 +1499,8 @@ static int end_precondition(const dpf_graph *g, const float *ends, const float *
                             const float *block32, const float *P24, const float *units32, const double *vector,
                             const float *vector32, double tolerance, int max_iterations, double *out, float *out32,
                             int *iterations, float *workspace, double *partials, unsigned *barrier, int *status,
-                            const int32_t *seg_site, const uint8_t *active, int variant, void *stream) {
+                            const int32_t *seg_site, const uint8_t *active, int variant, void *stream,
+                            float *direction = nullptr, unsigned *clear = nullptr) {
     if (!g || g->n_sites <= 0 || !g->inc_ptr || (g->n_bonds && (!ends || !aligned16(ends))) || !site4 || !fixed ||
         !block32 || !P24 || !units32 || (!vector && !vector32) || (!out && !out32) || !iterations || !workspace ||
         !partials || !barrier || !status || max_iterations < 1 || !aligned16(workspace) || !aligned16(P24) ||
@@ -1505,10 +1533,12 @@ static int end_precondition(const dpf_graph *g, const float *ends, const float *
     a.w = workspace + 5 * n6;
     a.part_a = partials;
     a.part_b = partials + kMaxPcgBlocksTiled;
+    a.direction = direction;
+    a.clear = clear;
     a.barrier = barrier;
     a.status = status;
     // a wait that timed out in an earlier launch leaves a partial arrival count
-    if (cudaMemsetAsync(barrier, 0, 2 * sizeof(unsigned), (cudaStream_t)stream) != cudaSuccess) {
+    if (!clear && cudaMemsetAsync(barrier, 0, 2 * sizeof(unsigned), (cudaStream_t)stream) != cudaSuccess) {
         cudaGetLastError();
         return DPF_ERR_CUDA;
     }
@@ -1544,3 +1574,14 @@ int dpf_end_precondition_f32(const dpf_graph *g, const float *ends, const float 
 }
 
 }  // extern "C"
+
+int dpf::end_precondition32_pass(const dpf_graph *g, const float *ends, const float *site4, const uint8_t *fixed,
+                                 const float *block32, const float *P24, const float *units32, const float *vector,
+                                 double tolerance, int max_iterations, float *out, float *direction, int *iterations,
+                                 float *workspace, double *partials, unsigned *barrier, unsigned *clear, int *status,
+                                 int variant, cudaStream_t st) {
+    if (!vector || !out) return DPF_ERR_ARGUMENT;
+    return end_precondition(g, ends, site4, fixed, block32, P24, units32, nullptr, vector, tolerance, max_iterations,
+                            nullptr, out, iterations, workspace, partials, barrier, status, nullptr, nullptr, variant,
+                            st, direction, clear);
+}

@@ -843,7 +843,7 @@ int dpf_parallel_loads(const dpf_graph *g, const double *radii, const double *x,
  * (experiments/bonded_dem_newton.py:13-60, 132-201).
  *
  * Device pointers unless noted; float64 vectors are (N, 6) = 6 N doubles. */
-#define DPF_NEWTON_VECTORS 10      /* scratch vectors of 6 N doubles in `vectors` */
+#define DPF_NEWTON_VECTORS 9       /* scratch vectors of 6 N doubles in `vectors` */
 #define DPF_NEWTON_HOST_DOUBLES 128 /* pinned host doubles in `host` */
 #define DPF_NEWTON_TRACE 32         /* residual trace entries kept */
 #define DPF_NEWTON_TIMERS 11        /* setup, residual, scaling, pcg, jvp, commit, pack, krylov, norms, vector, accept */

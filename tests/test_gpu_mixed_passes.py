@@ -1,0 +1,74 @@
+"""The mixed-precision step driver's joined passes: bit-identical to the Python
+control path at sizes off every block and warp edge, for lazy and eager commits,
+committed and refreshed starts; and the packed bond-end records against their
+definition (copies and single float32 products: exact)."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from tests.helpers import host
+from tests.test_gpu_driver import assert_same_info, assert_same_state, pair
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize('m', [2, 3, 7, 17])
+@pytest.mark.parametrize('lazy', [False, True])
+def test_driver_equals_python_path(m, lazy):
+    import dpf_gb300
+    foam, python, native = pair(m=m, seed=m, refresh=2)
+    load = dpf_gb300.gravity_load(foam)*4.0
+    for s in (python, native):
+        s.lazy_history = lazy
+    for step in range(5):
+        out = [s.step(2e-3, s.tensor(load), tolerance=1e-6) for s in (python, native)]
+        assert out[0][0] == out[1][0]
+        assert_same_info(out[0][1], out[1][1])
+        assert_same_state(python, native)
+
+
+@pytest.mark.parametrize('n,m', [(2, 1), (17, 33), (129, 400)])
+@pytest.mark.parametrize('sites', [False, True])
+def test_packed_ends(n, m, sites):
+    import torch
+    from dpf_gb300 import _lib
+    from tests.test_gpu_float64_passes import _pair
+    gpu, cpu, rng = _pair(n, m, seed=n)
+    lib, alpha = _lib.load(), .37
+    dev = lambda a: torch.as_tensor(np.ascontiguousarray(a)).to(gpu.device)
+    data = rng.normal(size=lib.dpf_mixed_bond_floats(m)).astype(np.float32)
+    P = rng.normal(size=(n, 6, 6)).astype(np.float32)
+    mass = rng.uniform(1, 2, (n, 6)).astype(np.float32)
+    data_d, P_d, mass_d = dev(data), dev(P), dev(mass)
+    ends, p24, site4 = (torch.full((k,), -7., dtype=torch.float32, device=gpu.device)
+                        for k in (lib.dpf_end_floats(m), 24*n, 4*n))
+    _lib.call('dpf_end_pack', ctypes.byref(gpu._graph), data_d.data_ptr(), alpha, P_d.data_ptr(), mass_d.data_ptr(),
+              gpu.fixed.data_ptr(), ends.data_ptr(), p24.data_ptr() if sites else None,
+              site4.data_ptr() if sites else None, gpu._stream())
+    t = data[28*m:44*m].reshape(4, m, 4)
+    got = host(ends).reshape(3, 2*m, 4)
+    order = [(s, b, end) for s in range(n) for b in range(m) for end in (0, 1) if (cpu.i, cpu.j)[end][b] == s]
+    assert len(order) == 2*m
+    rows = {}
+    for k in range(2*m):
+        rows.setdefault(tuple(np.abs(got[0, k, :3])), []).append(k)
+    a = np.float32(alpha)
+    for s, b, end in order:
+        sign = np.float32(1 - 2*end)
+        want = np.concatenate((sign*t[0, b, :3], t[1 + end, b, :3]))
+        near = [k for k in rows[tuple(np.abs(t[0, b, :3]))]
+                if np.array_equal(np.concatenate((got[0, k], got[1, k, :2])), want)]
+        assert len(near) == 1
+        k = near[0]
+        assert got[1, k, 3] == a*t[0, b, 3]
+        assert np.array_equal(got[2, k, :3], a*np.array([t[1, b, 3], t[2, b, 3], t[3, b, 0]]))
+        assert got[2, k, 3].view(np.int32) == (cpu.j, cpu.i)[end][b]
+    if sites:
+        r, c = np.triu_indices(6)
+        assert np.array_equal(host(p24).reshape(n, 24)[:, :21], P[:, r, c])
+        fixed = host(gpu.fixed).astype(bool)
+        want = np.where(fixed[:, None], [1, 1, 0, 0], np.stack((mass[:, 0], mass[:, 3], np.ones(n), np.zeros(n)), 1))
+        assert np.array_equal(host(site4).reshape(n, 4), want.astype(np.float32))
+    else:
+        assert (host(p24) == -7).all() and (host(site4) == -7).all()
