@@ -243,9 +243,9 @@ __global__ void __launch_bounds__(kThreads) site_residual(SiteResidualArgs a) {
         part[3 * blockIdx.x + 2] = sum_s;
     }
     if (last_block(counter_slot(a.partials, 0))) {
-        const double r2 = block_sum_array(part + 0, gridDim.x, 3);
-        const double mx = block_max_array(part + 1, gridDim.x, 3);
-        const double s2 = block_sum_array(part + 2, gridDim.x, 3);
+        double totals[3];
+        block_arrays<3, 2u>(part, gridDim.x, totals);
+        const double r2 = totals[0], mx = totals[1], s2 = totals[2];
         if (threadIdx.x == 0) {
             a.norms[0] = sqrt(r2);
             a.norms[1] = mx;

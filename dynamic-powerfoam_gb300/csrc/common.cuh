@@ -433,6 +433,15 @@ inline int reduce_threads(int64_t work) {
     return work >= (int64_t)kThreads * kSMs ? kThreads : spread_threads(work);
 }
 
+// Blocks of a grid-stride pass: no more than are resident at once, `resident` of
+// kThreads threads an SM (the kernel's launch bounds).  With 1024 blocks a kernel of
+// six blocks an SM ran a second wave of 112 blocks, nearly empty and as long as the
+// first (residual pass of 262k sites 83 us, now 64).
+inline int wave_grid(int64_t work, int resident, int threads = kThreads) {
+    const int64_t g = (work + threads - 1) / threads, cap = (int64_t)kSMs * resident * kThreads / threads;
+    return (int)(g < 1 ? 1 : g < cap ? g : cap);
+}
+
 // ---- reductions -----------------------------------------------------------
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -496,9 +505,49 @@ __device__ __forceinline__ double block_max(double v) {
     return buf[kThreads];
 }
 
-// Sum of `count` values spaced `stride` apart, in a fixed order (every block
-// that calls this with the same data gets the bit-identical result); one warp
-// adds, the others wait.
+// Sum or maximum of `count` partials by one warp, valid in every lane.  A lane has
+// 16 loads in flight (one to four at a time, 1024 partials cost a last block 8 to 32
+// round trips to L2: the norms of 262k sites 32.5 us, now 28.6); the sums go through
+// four accumulators in a fixed order.
+__device__ __forceinline__ double warp_array(const double *p, int count, int stride, bool most) {
+    const int lane = threadIdx.x & 31;
+    const double none = most ? -INFINITY : 0.0;
+    double s[4] = {none, none, none, none};
+    for (int base = 0; base < count; base += 512) {
+        double v[16];
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+            const int k = base + 32 * c + lane;
+            v[c] = k < count ? p[(int64_t)k * stride] : none;
+        }
+#pragma unroll
+        for (int c = 0; c < 16; ++c)
+            if (base + 32 * c < count) s[c & 3] = most ? fmax(s[c & 3], v[c]) : s[c & 3] + v[c];
+    }
+    return most ? warp_max(fmax(fmax(s[0], s[1]), fmax(s[2], s[3]))) : warp_sum((s[0] + s[1]) + (s[2] + s[3]));
+}
+
+// The K interleaved partial arrays p[k + K b] reduced over b, array k a maximum where
+// bit k of kMaxMask is set; a warp an array.  Every thread gets the totals.
+template <int K, unsigned kMaxMask>
+__device__ __forceinline__ void block_arrays(const double *p, int count, double (&out)[K]) {
+    __shared__ double total[K];
+    __syncthreads();
+    const int warps = (blockDim.x + 31) >> 5;
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+        if ((int)(threadIdx.x >> 5) == k % warps) {
+            const double v = warp_array(p + k, count, K, ((kMaxMask >> k) & 1u) != 0);
+            if ((threadIdx.x & 31) == 0) total[k] = v;
+        }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < K; ++k) out[k] = total[k];
+}
+
+// Sum of `count` values spaced `stride` apart, in a fixed order (every block that
+// calls this with the same data gets the bit-identical result); one warp adds, the
+// others wait.  For the few hundred partials of a grid barrier.
 __device__ __forceinline__ double block_sum_array(const double *p, int count, int stride = 1) {
     __shared__ double total;
     __syncthreads();
@@ -519,13 +568,33 @@ __device__ __forceinline__ double block_max_array(const double *p, int count, in
     __shared__ double total;
     __syncthreads();
     if (threadIdx.x < 32) {
-        double m = -INFINITY;
-        for (int k = threadIdx.x; k < count; k += 32) m = fmax(m, p[(int64_t)k * stride]);
-        m = warp_max(m);
+        const double m = warp_array(p, count, stride, true);
         if (threadIdx.x == 0) total = m;
     }
     __syncthreads();
     return total;
+}
+
+// ---- conversions between float32 and float64 in integer arithmetic ------------
+// The conversion instructions run on the float64 pipe, which takes a warp's
+// instruction in 16 cycles; re-biasing the exponent and moving the fraction are a
+// handful of integer instructions.  Same results as the casts: what is neither zero
+// nor normal in both formats takes the cast.
+
+__device__ __forceinline__ double widen(float f) {
+    const unsigned u = __float_as_uint(f), t = u & 0x7fffffffu;
+    if (t != 0u && t - 0x00800000u >= 0x7f000000u) return (double)f;  // subnormal, infinite, not a number
+    const unsigned hi = (u & 0x80000000u) | (t ? (t >> 3) + 0x38000000u : 0u);
+    return __hiloint2double((int)hi, (int)(u << 29));
+}
+
+// round to nearest, ties to even
+__device__ __forceinline__ float narrow(double d) {
+    const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d), t = hi & 0x7fffffffu;
+    if ((t | lo) != 0u && t - 0x38100000u >= 0x0fe00000u) return (float)d;  // outside float32's normal range
+    const unsigned m = ((t - 0x38000000u) << 3) | (lo >> 29);
+    const unsigned up = ((lo & 0x1fffffffu) + 0x0fffffffu + (m & 1u)) >> 29;
+    return __uint_as_float((hi & 0x80000000u) | ((t | lo) ? m + up : 0u));
 }
 
 // ---- sums as float32 pairs ---------------------------------------------------
@@ -595,19 +664,29 @@ __device__ __forceinline__ void block_pair_partial(float v, float2 *part) {
     if (threadIdx.x == 0) part[blockIdx.x] = t;
 }
 
+// Sum of `count` partial pairs in float64 by one warp, valid in its lane 0; 8 loads
+// in flight a lane.
+__device__ __forceinline__ double warp_pair_array(const float2 *part, int count) {
+    float hi = 0.0f, lo = 0.0f;
+    for (int k0 = threadIdx.x & 31; k0 < count; k0 += 256) {
+        float2 p[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) p[c] = k0 + 32 * c < count ? part[k0 + 32 * c] : make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) pair_add(hi, lo, p[c].x, p[c].y);
+    }
+    warp_pair_sum(hi, lo);
+    return (double)hi + (double)lo;
+}
+
 // Sum of `count` block partial pairs, in float64, the same in every block
 // (one warp adds them in a fixed order; the others wait at the block barrier).
 __device__ __forceinline__ double pair_total(const float2 *part, int count) {
     __shared__ double total;
     __syncthreads();  // the previous total has been read
     if (threadIdx.x < 32) {
-        float hi = 0.0f, lo = 0.0f;
-        for (int k = threadIdx.x; k < count; k += 32) {
-            const float2 p = part[k];
-            pair_add(hi, lo, p.x, p.y);
-        }
-        warp_pair_sum(hi, lo);
-        if (threadIdx.x == 0) total = (double)hi + (double)lo;
+        const double v = warp_pair_array(part, count);
+        if (threadIdx.x == 0) total = v;
     }
     __syncthreads();
     return total;

@@ -121,9 +121,11 @@ struct Reducer {
             p[3 * blockIdx.x + 2] = m2;
         }
         if (!grid_barrier(barrier, status)) return false;
-        out[0] = block_sum_array(p, gridDim.x, 3);
-        out[1] = block_sum_array(p + 1, gridDim.x, 3);
-        out[2] = block_max_array(p + 2, gridDim.x, 3);
+        double totals[3];
+        block_arrays<3, 4u>(p, gridDim.x, totals);
+        out[0] = totals[0];
+        out[1] = totals[1];
+        out[2] = totals[2];
         buf ^= 1;  // the other buffer: no block still reads it after the next barrier
         return true;
     }
@@ -365,8 +367,9 @@ __global__ void __launch_bounds__(kThreads) pair_sums_kernel(int64_t len, const 
         part[2 * blockIdx.x + 1] = en;
     }
     if (last_block(reinterpret_cast<unsigned *>(partials))) {
-        const double s_ab = block_sum_array(part, gridDim.x, 2);
-        const double s_en = block_sum_array(part + 1, gridDim.x, 2);
+        double totals[2];
+        block_arrays<2, 0u>(part, gridDim.x, totals);
+        const double s_ab = totals[0], s_en = totals[1];
         if (threadIdx.x == 0) {
             out[0] = s_ab;
             out[1] = 0.5 * s_en;

@@ -238,7 +238,7 @@ struct SetupSiteArgs {
     double *r0, *loads, *scales, *partials;
 };
 
-__global__ void __launch_bounds__(kThreads) setup_sites(SetupSiteArgs a) {
+__global__ void __launch_bounds__(kThreads, 5) setup_sites(SetupSiteArgs a) {
     double a2 = 0.0, l2 = 0.0;
     for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < a.n; s += (int64_t)gridDim.x * blockDim.x) {
         double acc[6];
@@ -281,8 +281,9 @@ __global__ void __launch_bounds__(kThreads) setup_sites(SetupSiteArgs a) {
         part[2 * blockIdx.x + 1] = l2;
     }
     if (last_block(counter_slot(a.partials, 5))) {
-        const double sa = block_sum_array(part, gridDim.x, 2);
-        const double sl = block_sum_array(part + 1, gridDim.x, 2);
+        double totals[2];
+        block_arrays<2, 0u>(part, gridDim.x, totals);
+        const double sa = totals[0], sl = totals[1];
         if (threadIdx.x == 0) {
             a.scales[0] = sqrt(sa);
             a.scales[1] = sqrt(sl);
@@ -376,20 +377,38 @@ __device__ __forceinline__ void matvec6f(const float *P, const float x[6], float
 // grid totals.
 __device__ __forceinline__ void finish_norms(double sum_r, float max_s, float s_hi, float s_lo, double *partials,
                                              int slot, double *norms, int *status, const Report &report = Report()) {
-    const float r_hi = (float)sum_r, r_lo = (float)(sum_r - (double)r_hi);
-    const float2 r2 = block_pair_sum(r_hi, r_lo);
-    const float mx = block_max_float(max_s);
-    const float2 s2 = block_pair_sum(s_hi, s_lo);
+    float r_hi = (float)sum_r, r_lo = (float)(sum_r - (double)r_hi);
+    // the three reductions side by side: one wait for the block
+    __shared__ float4 pairs[kThreads / 32];
+    __shared__ float most[kThreads / 32];
+    const int lane = threadIdx.x & 31, warps = (blockDim.x + 31) >> 5;
+    warp_pair_sum(r_hi, r_lo);
+    warp_pair_sum(s_hi, s_lo);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) max_s = fmaxf(max_s, __shfl_xor_sync(0xffffffffu, max_s, o));
+    if (lane == 0) {
+        pairs[threadIdx.x >> 5] = make_float4(r_hi, r_lo, s_hi, s_lo);
+        most[threadIdx.x >> 5] = max_s;
+    }
+    __syncthreads();
     double *part = partials + kPartialsOffset;
-    if (threadIdx.x == 0) {
-        part[3 * blockIdx.x] = (double)r2.x + (double)r2.y;
-        part[3 * blockIdx.x + 1] = mx;
-        part[3 * blockIdx.x + 2] = (double)s2.x + (double)s2.y;
+    if (threadIdx.x < 32) {
+        float4 v = lane < warps ? pairs[lane] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        float mx = lane < warps ? most[lane] : 0.0f;
+        warp_pair_sum(v.x, v.y);
+        warp_pair_sum(v.z, v.w);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        if (lane == 0) {
+            part[3 * blockIdx.x] = (double)v.x + (double)v.y;
+            part[3 * blockIdx.x + 1] = mx;
+            part[3 * blockIdx.x + 2] = (double)v.z + (double)v.w;
+        }
     }
     if (last_block(counter_slot(partials, slot))) {
-        const double r2 = block_sum_array(part, gridDim.x, 3);
-        const double mx = block_max_array(part + 1, gridDim.x, 3);
-        const double s2 = block_sum_array(part + 2, gridDim.x, 3);
+        double totals[3];
+        block_arrays<3, 2u>(part, gridDim.x, totals);
+        const double r2 = totals[0], mx = totals[1], s2 = totals[2];
         if (threadIdx.x == 0) {
             norms[0] = sqrt(r2);
             norms[1] = mx;
@@ -426,11 +445,19 @@ __device__ __forceinline__ void add_square(float &hi, float &lo, float v) {
     lo += e;
 }
 
+// Components 2 lane and 2 lane + 1 of a group's sums (lanes 0-2).
+__device__ __forceinline__ void lane_pair(const float v[6], int lane, float &a, float &b) {
+    a = lane == 0 ? v[0] : (lane == 1 ? v[2] : v[4]);
+    b = lane == 0 ? v[1] : (lane == 1 ? v[3] : v[5]);
+}
+
 // A group of kGroupJ lanes per site: the lanes gather the site's bond
 // wrench, lanes 0-2 then form two residual components each (16-byte loads and
 // stores), the group exchanges them by shuffles, and with a preconditioner
-// lane l scales rows l, l + kGroupJ, ... of the six.
-__global__ void __launch_bounds__(kThreads) residual_sites(ResidualSiteArgs a) {
+// lane l scales rows l, l + kGroupJ, ... of the six.  The float64 pipe takes the
+// four operations of an entry; conversions stay off it (with them 20 instructions
+// of a warp instead of 8).  262k sites: 86 us, in one wave of blocks 64 us.
+__global__ void __launch_bounds__(kThreads, 6) residual_sites(ResidualSiteArgs a) {
     double sum_r = 0.0;
     float max_s = 0.0f;
     float s_hi = 0.0f, s_lo = 0.0f;
@@ -443,25 +470,28 @@ __global__ void __launch_bounds__(kThreads) residual_sites(ResidualSiteArgs a) {
         float hi[6], lo[6];
         group_gather9c_j(a.ptr, a.inc, a.wrench, s, valid, lane, hi, lo);
         double r0v = 0.0, r1v = 0.0;
+        float y0 = 0.0f, y1 = 0.0f;
         if (valid && lane < 3) {
-            const float h0 = lane == 0 ? hi[0] : (lane == 1 ? hi[2] : hi[4]);
-            const float l0 = lane == 0 ? lo[0] : (lane == 1 ? lo[2] : lo[4]);
-            const float h1 = lane == 0 ? hi[1] : (lane == 1 ? hi[3] : hi[5]);
-            const float l1 = lane == 0 ? lo[1] : (lane == 1 ? lo[3] : lo[5]);
+            float h0, h1, l0, l1;
+            lane_pair(hi, lane, h0, h1);
+            lane_pair(lo, lane, l0, l1);
             const int64_t e = 6 * s + 2 * lane;
             const double2 yv = *reinterpret_cast<const double2 *>(a.y + e);
             const double2 mv = *reinterpret_cast<const double2 *>(a.mass + e);
             const double2 rv = *reinterpret_cast<const double2 *>(a.r0 + e);
             const bool fx = a.fixed[s] != 0;
-            r0v = fx ? yv.x : fma(mv.x, yv.x, rv.x) - a.half_dt2 * ((double)h0 + (double)l0);
-            r1v = fx ? yv.y : fma(mv.y, yv.y, rv.y) - a.half_dt2 * ((double)h1 + (double)l1);
+            r0v = fx ? yv.x : fma(mv.x, yv.x, rv.x) - a.half_dt2 * (widen(h0) + widen(l0));
+            r1v = fx ? yv.y : fma(mv.y, yv.y, rv.y) - a.half_dt2 * (widen(h1) + widen(l1));
             *reinterpret_cast<double2 *>(a.residual + e) = make_double2(r0v, r1v);
             sum_r = fma(r0v, r0v, sum_r);
             sum_r = fma(r1v, r1v, sum_r);
+            y0 = narrow(yv.x);
+            y1 = narrow(yv.y);
         }
+        // the rotation guard: lane 1 holds y[3], lane 2 y[4] and y[5]
+        const float w0 = __shfl_sync(0xffffffffu, y1, 1, kGroupJ), w1 = __shfl_sync(0xffffffffu, y0, 2, kGroupJ),
+                    w2 = __shfl_sync(0xffffffffu, y1, 2, kGroupJ);
         if (valid && lane == 0) {
-            const double *ys = a.y + 6 * s;
-            const float w0 = (float)ys[3], w1 = (float)ys[4], w2 = (float)ys[5];
             if (sqrtf(w0 * w0 + w1 * w1 + w2 * w2) > 0.25f) {
                 if (a.seg)
                     atomicOr(a.status + a.seg[s], DPF_ERR_ROTATION);
@@ -471,7 +501,7 @@ __global__ void __launch_bounds__(kThreads) residual_sites(ResidualSiteArgs a) {
         }
         if (a.P) {  // uniform over the grid: every lane takes part in the shuffles
             // lanes 0-2 round their two entries to float32, the group shares them
-            const float f0 = (float)r0v, f1 = (float)r1v;
+            const float f0 = narrow(r0v), f1 = narrow(r1v);
             float rf[6];
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
@@ -486,7 +516,7 @@ __global__ void __launch_bounds__(kThreads) residual_sites(ResidualSiteArgs a) {
                     const int row = lane + kGroupJ * k;
                     if (row < 6) {
                         const float v = scale_row(P, rf, row, u[row]);
-                        if (a.scaled) a.scaled[6 * s + row] = v;
+                        if (a.scaled) a.scaled[6 * s + row] = widen(v);
                         max_s = fmaxf(max_s, fabsf(v));
                         add_square(s_hi, s_lo, v);
                     }
@@ -500,8 +530,9 @@ __global__ void __launch_bounds__(kThreads) residual_sites(ResidualSiteArgs a) {
 }
 
 // One thread per site, 16-byte loads: the six residual entries (rounded to
-// float32 once), the 36-float P block, the six units; s = P r / units.
-__global__ void __launch_bounds__(kThreads) scale_sites_f32(int64_t n, const float *P, const float *units32,
+// float32 once), the 36-float P block, the six units; s = P r / units.  262k sites:
+// 32.5 us in three waves of blocks with conversions on the float64 pipe, now 20.
+__global__ void __launch_bounds__(kThreads, 3) scale_sites_f32(int64_t n, const float *P, const float *units32,
                                                             const double *r, double *scaled, double *norms,
                                                             double *partials, Report report) {
     double sum_r = 0.0;
@@ -515,7 +546,7 @@ __global__ void __launch_bounds__(kThreads) scale_sites_f32(int64_t n, const flo
 #pragma unroll
         for (int c = 0; c < 6; ++c) {
             sum_r = fma(rr[c], rr[c], sum_r);
-            rf[c] = (float)rr[c];
+            rf[c] = narrow(rr[c]);
         }
         const float4 *pp = reinterpret_cast<const float4 *>(P + 36 * s);
         float pm[36];
@@ -539,7 +570,7 @@ __global__ void __launch_bounds__(kThreads) scale_sites_f32(int64_t n, const flo
             v = v / un[row];
             max_s = fmaxf(max_s, fabsf(v));
             add_square(s_hi, s_lo, v);
-            out[row] = (double)v;
+            out[row] = widen(v);
         }
         if (scaled) {
             double2 *sp = reinterpret_cast<double2 *>(scaled + 6 * s);
@@ -652,7 +683,7 @@ __global__ void __launch_bounds__(kThreads) jvp_sites_mixed(JvpSiteArgs a) {
             if (a.out32)
                 a.out32[6 * s + row] = v;
             else
-                a.out[6 * s + row] = (double)v;
+                a.out[6 * s + row] = widen(v);
         }
     }
 }
@@ -681,7 +712,7 @@ __global__ void __launch_bounds__(kThreads) stiffness_bonds_f32(int64_t m, BondD
 
 __global__ void __launch_bounds__(kThreads) to_f32(int64_t n, const double *a, float *out) {
     const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (e < n) out[e] = (float)a[e];
+    if (e < n) out[e] = narrow(a[e]);
 }
 
 __global__ void __launch_bounds__(kThreads) gather_to_f64(int64_t n, const int32_t *ptr, const int32_t *inc,
@@ -1260,7 +1291,9 @@ __global__ void __launch_bounds__(kThreads, 3) commit_bonds(CommitArgs a) {
     a.bd.rec.r5[b] = make_float4(offr.x, offr.y, offr.z, B.ks);
 }
 
-// loads += site sum of the load increments.
+// loads += site sum of the load increments, lanes 0-2 of a group two entries each
+// (lane 0 alone, with conversions: 24 float64 instructions of a warp, now four; 55
+// us at 262k sites, now 45; 258 and 178 at 1.4M).
 __global__ void __launch_bounds__(kThreads) commit_sites(int64_t n, const int32_t *ptr, const int32_t *inc,
                                                          const float *dloads, double *loads) {
     const int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kGroupJ;
@@ -1268,9 +1301,14 @@ __global__ void __launch_bounds__(kThreads) commit_sites(int64_t n, const int32_
     const bool valid = g < n;
     float hi[6], lo[6];
     group_gather9c_j(ptr, inc, dloads, g, valid, lane, hi, lo);
-    if (valid && lane == 0) {
-#pragma unroll
-        for (int c = 0; c < 6; ++c) loads[6 * g + c] += (double)hi[c] + (double)lo[c];
+    if (valid && lane < 3) {
+        float h0, h1, l0, l1;
+        lane_pair(hi, lane, h0, h1);
+        lane_pair(lo, lane, l0, l1);
+        double *p = loads + 6 * g + 2 * lane;
+        const double v0 = p[0], v1 = p[1];
+        p[0] = v0 + (widen(h0) + widen(l0));
+        p[1] = v1 + (widen(h1) + widen(l1));
     }
 }
 
@@ -1344,7 +1382,7 @@ struct BeginArgs {
 };
 
 template <bool kStart>
-__global__ void __launch_bounds__(kThreads) begin_sites(BeginArgs a) {
+__global__ void __launch_bounds__(kThreads, 5) begin_sites(BeginArgs a) {
     double a2 = 0.0, l2 = 0.0;
     if (kStart && blockIdx.x == 0 && threadIdx.x == 0) *a.status = *a.inner = a.barrier[0] = a.barrier[1] = 0;
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < 6 * a.n; e += (int64_t)gridDim.x * blockDim.x) {
@@ -1370,8 +1408,9 @@ __global__ void __launch_bounds__(kThreads) begin_sites(BeginArgs a) {
         part[2 * blockIdx.x + 1] = l2;
     }
     if (last_block(counter_slot(a.partials, 5))) {
-        const double sa = block_sum_array(part, gridDim.x, 2);
-        const double sl = block_sum_array(part + 1, gridDim.x, 2);
+        double totals[2];
+        block_arrays<2, 0u>(part, gridDim.x, totals);
+        const double sa = totals[0], sl = totals[1];
         if (threadIdx.x == 0) {
             a.scales[0] = sqrt(sa);
             a.scales[1] = sqrt(sl);
@@ -1489,7 +1528,7 @@ int dpf_mixed_setup(const dpf_graph *g, const dpf_stiffness *k, const dpf_histor
     }
     SetupSiteArgs s{g->n_sites, g->inc_ptr, g->inc_bond, wrench, mass, v, external, fixed, dt, 0.5 * dt * dt,
                     r0, loads, scales, partials};
-    setup_sites<<<reduce_grid(g->n_sites), kThreads, 0, st>>>(s);
+    setup_sites<<<wave_grid(g->n_sites, 5), kThreads, 0, st>>>(s);
     DPF_CHECK_LAUNCH();
     return DPF_OK;
 }
@@ -1532,7 +1571,7 @@ int dpf_mixed_residual_segmented(const dpf_graph *g, float *bond_data, const dou
     }
     ResidualSiteArgs s{g->n_sites, g->inc_ptr, g->inc_bond, wrench, y, mass, r0, fixed, 0.5 * dt * dt,
                        preconditioner, units32, residual, scaled, norms, partials, status, seg_site};
-    residual_sites<<<reduce_grid(kGroupJ * g->n_sites), kThreads, 0, st>>>(s);
+    residual_sites<<<wave_grid(kGroupJ * g->n_sites, 6), kThreads, 0, st>>>(s);
     DPF_CHECK_LAUNCH();
     return DPF_OK;
 }
@@ -1565,7 +1604,7 @@ int dpf::scale_residual_pass(int64_t n_sites, const float *preconditioner, const
         ((uintptr_t)preconditioner & 15u) || ((uintptr_t)units32 & 7u) || ((uintptr_t)residual & 15u) ||
         ((uintptr_t)scaled & 15u))
         return DPF_ERR_ARGUMENT;
-    scale_sites_f32<<<reduce_grid(n_sites), kThreads, 0, st>>>(n_sites, preconditioner, units32, residual, scaled,
+    scale_sites_f32<<<wave_grid(n_sites, 3), kThreads, 0, st>>>(n_sites, preconditioner, units32, residual, scaled,
                                                                norms, partials, report);
     DPF_CHECK_LAUNCH();
     return DPF_OK;
@@ -1807,7 +1846,7 @@ int dpf_mixed_begin(int64_t n_sites, const double *loads, const double *mass, co
         return DPF_ERR_ARGUMENT;
     BeginArgs a{n_sites, loads, mass, v, external, fixed, dt, 0.5 * dt * dt, r0, scales, partials,
                 nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-    begin_sites<false><<<reduce_grid(6 * n_sites), kThreads, 0, (cudaStream_t)stream>>>(a);
+    begin_sites<false><<<wave_grid(6 * n_sites, 5), kThreads, 0, (cudaStream_t)stream>>>(a);
     DPF_CHECK_LAUNCH();
     return DPF_OK;
 }
@@ -1823,7 +1862,7 @@ int dpf::mixed_start_pass(int64_t n_sites, const double *loads, const double *ma
         return DPF_ERR_ARGUMENT;
     BeginArgs a{n_sites, loads, mass, v, external, fixed, dt, 0.5 * dt * dt, r0, scales, partials,
                 y, residual, y32, status, inner, barrier};
-    begin_sites<true><<<reduce_grid(6 * n_sites), kThreads, 0, st>>>(a);
+    begin_sites<true><<<wave_grid(6 * n_sites, 5), kThreads, 0, st>>>(a);
     DPF_CHECK_LAUNCH();
     return DPF_OK;
 }

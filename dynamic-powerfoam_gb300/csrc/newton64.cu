@@ -171,7 +171,9 @@ __global__ void __launch_bounds__(kThreads) accept_state_kernel(AcceptArgs a) {
         part[2 * blockIdx.x + 1] = turn;
     }
     if (last_block(reinterpret_cast<unsigned *>(a.partials) + 1)) {
-        const double sum = block_sum_array(part, gridDim.x, 2), most = block_max_array(part + 1, gridDim.x, 2);
+        double totals[2];
+        block_arrays<2, 2u>(part, gridDim.x, totals);
+        const double sum = totals[0], most = totals[1];
         if (threadIdx.x == 0) {
             a.out[0] = sum;
             a.out[1] = sqrt(most);

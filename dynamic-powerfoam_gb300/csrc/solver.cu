@@ -12,6 +12,7 @@ constexpr int kMaxArnoldi = 64;
 constexpr int kMaxPcgBlocks = 4096;
 
 inline int blocks_for(int64_t n, int threads) { return (int)((n + threads - 1) / threads); }
+constexpr int kNormResident = 5;   // dot_norm_kernel and correction_kernel: the same grid, the same sums
 inline int reduce_grid(int64_t n) {
     int g = blocks_for(n, kThreads);
     if (g > kMaxReduceBlocks) g = kMaxReduceBlocks;
@@ -269,7 +270,7 @@ __global__ void __launch_bounds__(kThreads) combine_rows_kernel(int64_t len, con
     }
 }
 
-__global__ void __launch_bounds__(kThreads) dot_norm_kernel(int64_t len, const double *a, const double *b,
+__global__ void __launch_bounds__(kThreads, kNormResident) dot_norm_kernel(int64_t len, const double *a, const double *b,
                                                             double *result, double *partials) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     double ab = 0.0, aa = 0.0;
@@ -286,8 +287,9 @@ __global__ void __launch_bounds__(kThreads) dot_norm_kernel(int64_t len, const d
         part[2 * blockIdx.x + 1] = aa;
     }
     if (last_block(counter_slot(partials, 1))) {
-        const double s_ab = block_sum_array(part, gridDim.x, 2);
-        const double s_aa = block_sum_array(part + 1, gridDim.x, 2);
+        double totals[2];
+        block_arrays<2, 0u>(part, gridDim.x, totals);
+        const double s_ab = totals[0], s_aa = totals[1];
         if (threadIdx.x == 0) {
             result[0] = s_ab;
             result[1] = sqrt(s_aa);
@@ -334,9 +336,9 @@ __global__ void __launch_bounds__(kThreads) scale_kernel(int64_t n, const double
         part[3 * blockIdx.x + 2] = sum_s;
     }
     if (last_block(counter_slot(partials, 2))) {
-        const double r2 = block_sum_array(part, gridDim.x, 3);
-        const double mx = block_max_array(part + 1, gridDim.x, 3);
-        const double s2 = block_sum_array(part + 2, gridDim.x, 3);
+        double totals[3];
+        block_arrays<3, 2u>(part, gridDim.x, totals);
+        const double r2 = totals[0], mx = totals[1], s2 = totals[2];
         if (threadIdx.x == 0) {
             norms[0] = sqrt(r2);
             norms[1] = mx;
@@ -377,8 +379,9 @@ __global__ void __launch_bounds__(kThreads) energy_kernel(int64_t m, int64_t n, 
         part[2 * blockIdx.x + 1] = kin;
     }
     if (last_block(counter_slot(partials, 3))) {
-        const double se = block_sum_array(part, gridDim.x, 2);
-        const double sk = block_sum_array(part + 1, gridDim.x, 2);
+        double totals[2];
+        block_arrays<2, 0u>(part, gridDim.x, totals);
+        const double se = totals[0], sk = totals[1];
         if (threadIdx.x == 0) *energy = 0.5 * se + 0.5 * sk;
     }
 }
@@ -403,8 +406,9 @@ __global__ void __launch_bounds__(kThreads) rhs_scale_kernel(int64_t n, const do
         part[2 * blockIdx.x + 1] = l2;
     }
     if (last_block(counter_slot(partials, 4))) {
-        const double sa = block_sum_array(part, gridDim.x, 2);
-        const double sl = block_sum_array(part + 1, gridDim.x, 2);
+        double totals[2];
+        block_arrays<2, 0u>(part, gridDim.x, totals);
+        const double sa = totals[0], sl = totals[1];
         if (threadIdx.x == 0) {
             out[0] = sqrt(sa);
             out[1] = sqrt(sl);
@@ -512,7 +516,7 @@ struct CorrectionArgs {
     int *status;
 };
 
-__global__ void __launch_bounds__(kThreads) correction_kernel(CorrectionArgs a) {
+__global__ void __launch_bounds__(kThreads, kNormResident) correction_kernel(CorrectionArgs a) {
     __shared__ float chi[kMaxArnoldi], clo[kMaxArnoldi];
     if (threadIdx.x < a.count) ff_split(a.coef.c[threadIdx.x], chi[threadIdx.x], clo[threadIdx.x]);
     if (blockIdx.x == 0 && threadIdx.x == 0) *a.status = 0;
@@ -530,13 +534,15 @@ __global__ void __launch_bounds__(kThreads) correction_kernel(CorrectionArgs a) 
             ff_add_product(jh, jl, chi[k], j);
             jl = fmaf(clo[k], j, jl);
         }
-        const double xv = (a.add ? a.x[e] : 0.0) + ff_value(zh, zl), rv = -s - ff_value(jh, jl);
+        double xv = widen(zh) + widen(zl);
+        if (a.add) xv += a.x[e];
+        const double rv = -s - (widen(jh) + widen(jl));
         const double c = fx ? 0.0 : __dmul_rn(un, xv), y1 = yv + c;   // rounded as masked_scale_kernel does
         a.x[e] = xv;
         a.res[e] = rv;
         a.correction[e] = c;
         a.candidate[e] = y1;
-        a.y32[e] = (float)y1;
+        a.y32[e] = narrow(y1);
         aa += rv * rv;
     }
     aa = block_sum(aa);
@@ -600,10 +606,11 @@ __device__ __forceinline__ void arnoldi_dots_pass(const Arnoldi32Args &a, const 
 __device__ __forceinline__ void arnoldi_project(const Arnoldi32Args &a, const float2 *in, const double *part,
                                                bool second, float &sq_hi, float &sq_lo) {
     __shared__ float vhi[kMaxArnoldi], vlo[kMaxArnoldi];
-    __shared__ double column[kMaxArnoldi];   // thread 0 of block 0: h may be host memory, which is only written
-    for (int k = 0; k < a.count; ++k) {
-        const double v = pair_total(reinterpret_cast<const float2 *>(part) + k * gridDim.x, gridDim.x);
-        if (threadIdx.x == 0) {
+    __shared__ double column[kMaxArnoldi];   // kept for the second pass: h may be host memory, which is only written
+    // a warp a row (one warp for all of them: 5 us a row more at 262k sites)
+    for (int k = threadIdx.x >> 5; k < a.count; k += kThreads / 32) {
+        const double v = warp_pair_array(reinterpret_cast<const float2 *>(part) + k * gridDim.x, gridDim.x);
+        if ((threadIdx.x & 31) == 0) {
             ff_split(v, vhi[k], vlo[k]);
             column[k] = second ? column[k] + v : v;
             if (second && blockIdx.x == 0) a.h[k] = column[k];
@@ -663,7 +670,7 @@ __global__ void __launch_bounds__(kThreads) scale_to_float_kernel(int64_t len, d
                                                                   float *out) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < len; e += stride)
-        out[e] = (float)(alpha * a[e]);
+        out[e] = narrow(alpha * a[e]);
 }
 
 }  // namespace dpf
@@ -848,7 +855,7 @@ int dpf::mixed_correction_pass(int64_t n_sites, const float *transformed, const 
     a.norm = norm;
     a.partials = partials;
     a.status = status;
-    correction_kernel<<<reduce_grid(a.len), kThreads, 0, st>>>(a);
+    correction_kernel<<<wave_grid(a.len, kNormResident), kThreads, 0, st>>>(a);
     DPF_CHECK_LAUNCH();
     return DPF_OK;
 }
@@ -886,7 +893,7 @@ int dpf_combine_rows(int64_t length, const double *rows, int64_t ld, int count, 
 
 int dpf_dot_norm(int64_t length, const double *a, const double *b, double *result, double *partials, void *stream) {
     if (length <= 0 || !a || !result || !partials) return DPF_ERR_ARGUMENT;
-    dot_norm_kernel<<<reduce_grid(length), kThreads, 0, (cudaStream_t)stream>>>(length, a, b, result, partials);
+    dot_norm_kernel<<<wave_grid(length, kNormResident), kThreads, 0, (cudaStream_t)stream>>>(length, a, b, result, partials);
     DPF_CHECK_LAUNCH();
     return DPF_OK;
 }

@@ -72,3 +72,39 @@ def test_packed_ends(n, m, sites):
         assert np.array_equal(host(site4).reshape(n, 4), want.astype(np.float32))
     else:
         assert (host(p24) == -7).all() and (host(site4) == -7).all()
+
+
+def test_conversions_equal_the_casts():
+    """Every class of value: normal, ties, carries into the exponent, both ends of float32's range,
+    subnormal, zero, infinite and not a number; the same bits as the casts."""
+    import torch
+    from dpf_gb300 import _lib
+    rng = np.random.default_rng(5)
+    bits = rng.integers(0, 2**64, 40000, dtype=np.uint64)
+    near = (rng.integers(890, 1155, 40000).astype(np.uint64) << np.uint64(52)) | (bits & np.uint64(0x800fffffffffffff))
+    tie = (near & ~np.uint64(0x1fffffff)) | np.uint64(0x10000000)
+    edge = np.array([0., -0., np.inf, -np.inf, np.nan, 1., 2.**-126, 2.**-126*(1 - 2.**-25), 2.**-149, 2.**-150, 2.**-1074,
+                     3.4028234663852886e38, 3.4028235677973366e38, 1e300, -1e-300, 1 - 2.**-25, 1 + 2.**-24])
+    v = np.concatenate((bits.view(np.float64), near.view(np.float64), tie.view(np.float64),
+                        (tie + np.uint64(1)).view(np.float64), (tie - np.uint64(1)).view(np.float64), edge))
+    stream = torch.cuda.current_stream().cuda_stream
+    d = torch.as_tensor(v).cuda()
+    out = torch.empty(len(v), dtype=torch.float32, device='cuda')
+    _lib.call('dpf_to_float', len(v), d.data_ptr(), out.data_ptr(), stream)
+    with np.errstate(over='ignore', invalid='ignore', under='ignore'):
+        want = v.astype(np.float32)
+    got = host(out)
+    number = ~np.isnan(v)
+    assert np.array_equal(got[number].view(np.uint32), want[number].view(np.uint32)) and np.isnan(got[~number]).all()
+
+    # s = P r / units with P = 1, one entry a site: (double)(float)r
+    n = len(v)
+    r = torch.zeros((n, 6), dtype=torch.float64, device='cuda')
+    at = torch.arange(n, device='cuda') % 6
+    r[torch.arange(n, device='cuda'), at] = d
+    eye = torch.eye(6, dtype=torch.float32, device='cuda').repeat(n, 1, 1)
+    units, scaled = torch.ones((n, 6), dtype=torch.float32, device='cuda'), torch.empty_like(r)
+    _lib.call('dpf_mixed_scale_residual', n, eye.data_ptr(), units.data_ptr(), r.data_ptr(), scaled.data_ptr(), None,
+              None, stream)
+    got = host(scaled[torch.arange(n, device='cuda'), at])
+    assert np.array_equal(got[number], want[number].astype(np.float64)) and np.isnan(got[~number]).all()
