@@ -551,7 +551,7 @@ int dpf_adjoint_precondition(const dpf_graph *g, const dpf_stiffness *k, const d
                              int max_iterations, double *out, int *iterations, double *wrench, double *workspace,
                              unsigned *barrier, int *status, void *stream) {
     return elastic_pass(g, k, t, mass, fixed, block, preconditioner, units, vector, dt, tolerance, max_iterations, out,
-                        iterations, wrench, workspace, barrier, status, kElasticT, (cudaStream_t)stream);
+                        iterations, wrench, workspace, barrier, nullptr, status, kElasticT, (cudaStream_t)stream);
 }
 
 int dpf_adjoint_bond_vjp(const dpf_graph *g, const dpf_stiffness *k, const dpf_history *h, const double *y,

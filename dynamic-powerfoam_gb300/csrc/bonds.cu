@@ -233,24 +233,21 @@ __global__ void __launch_bounds__(kThreads) site_residual(SiteResidualArgs a) {
     }
     if (flags) atomicOr(a.status, flags);
     if (!a.norms) return;
-    sum_r = block_sum(sum_r);
-    max_s = block_max(max_s);
-    sum_s = block_sum(sum_s);
+    double v[3] = {sum_r, max_s, sum_s};
+    block_reduce<3, 2u>(v);
     double *part = a.partials + kPartialsOffset;
     if (threadIdx.x == 0) {
-        part[3 * blockIdx.x + 0] = sum_r;
-        part[3 * blockIdx.x + 1] = max_s;
-        part[3 * blockIdx.x + 2] = sum_s;
+        part[3 * blockIdx.x + 0] = v[0];
+        part[3 * blockIdx.x + 1] = v[1];
+        part[3 * blockIdx.x + 2] = v[2];
     }
     if (last_block(counter_slot(a.partials, 0))) {
-        double totals[3];
-        block_arrays<3, 2u>(part, gridDim.x, totals);
-        const double r2 = totals[0], mx = totals[1], s2 = totals[2];
+        block_arrays<3, 2u>(part, gridDim.x, v);
         if (threadIdx.x == 0) {
-            a.norms[0] = sqrt(r2);
-            a.norms[1] = mx;
-            a.norms[2] = sqrt(s2);
-            if (!isfinite(r2) || !isfinite(s2)) atomicOr(a.status, DPF_ERR_NONFINITE);
+            a.norms[0] = sqrt(v[0]);
+            a.norms[1] = v[1];
+            a.norms[2] = sqrt(v[2]);
+            if (!isfinite(v[0]) || !isfinite(v[2])) atomicOr(a.status, DPF_ERR_NONFINITE);
         }
     }
 }
@@ -962,8 +959,8 @@ int dpf_bond_setup(int64_t n_sites, int64_t n_bonds, const int64_t *edges, const
 int dpf_loads(const dpf_graph *g, const dpf_history *h, double *out, double *wrench, void *stream) {
     if (!graph_ok(g) || !history_ok(h, g->n_bonds) || !out || (g->n_bonds && !wrench)) return DPF_ERR_ARGUMENT;
     cudaStream_t st = (cudaStream_t)stream;
-    if (g->n_bonds)
-        loads_bonds<<<blocks_for(g->n_bonds, 128), 128, 0, st>>>(g->n_bonds, g->edges, *h, wrench, nullptr);
+    const int rc = dpf::loads_bonds_pass(g, h, wrench, st);
+    if (rc) return rc;
     site_gather<<<blocks_for(2 * g->n_sites, kThreads), kThreads, 0, st>>>(g->n_sites, g->inc_ptr, g->inc_bond,
                                                                         wrench, out);
     DPF_CHECK_LAUNCH();
@@ -973,6 +970,14 @@ int dpf_loads(const dpf_graph *g, const dpf_history *h, double *out, double *wre
 }  // extern "C"
 
 namespace dpf {
+
+int loads_bonds_pass(const dpf_graph *g, const dpf_history *h, double *wrench, cudaStream_t st) {
+    if (!graph_ok(g) || !history_ok(h, g->n_bonds) || (g->n_bonds && !wrench)) return DPF_ERR_ARGUMENT;
+    if (g->n_bonds)
+        loads_bonds<<<blocks_for(g->n_bonds, 128), 128, 0, st>>>(g->n_bonds, g->edges, *h, wrench, nullptr);
+    DPF_CHECK_LAUNCH();
+    return DPF_OK;
+}
 
 int residual_pass(const dpf_graph *g, const dpf_stiffness *k, const dpf_history *h, const double *y, const double *v,
                   const double *external, const double *mass, const uint8_t *fixed, double dt,

@@ -505,6 +505,36 @@ __device__ __forceinline__ double block_max(double v) {
     return buf[kThreads];
 }
 
+// K reductions over the block's threads (at most kThreads), number k a maximum where
+// bit k of kMaxMask is set; every thread gets the totals.  A warp takes an array, as
+// block_sum does for one, so three cost little more than one (a float64 instruction
+// holds its scheduler for 64 cycles: one after the other they took 1.1 us a block).
+template <int K, unsigned kMaxMask>
+__device__ __forceinline__ void block_reduce(double (&v)[K]) {
+    __shared__ double buf[K][kThreads];
+    __shared__ double total[K];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < K; ++k) buf[k][threadIdx.x] = v[k];
+    __syncthreads();
+    const int warps = (blockDim.x + 31) >> 5;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        if ((int)(threadIdx.x >> 5) != k % warps) continue;
+        const bool most = ((kMaxMask >> k) & 1u) != 0;
+        double s = most ? -INFINITY : 0.0, t = s;
+        for (int e = threadIdx.x & 31; e < (int)blockDim.x; e += 64) {
+            s = most ? fmax(s, buf[k][e]) : s + buf[k][e];
+            if (e + 32 < (int)blockDim.x) t = most ? fmax(t, buf[k][e + 32]) : t + buf[k][e + 32];
+        }
+        s = most ? warp_max(fmax(s, t)) : warp_sum(s + t);
+        if ((threadIdx.x & 31) == 0) total[k] = s;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < K; ++k) v[k] = total[k];
+}
+
 // Sum or maximum of `count` partials by one warp, valid in every lane.  A lane has
 // 16 loads in flight (one to four at a time, 1024 partials cost a last block 8 to 32
 // round trips to L2: the norms of 262k sites 32.5 us, now 28.6); the sums go through

@@ -545,6 +545,7 @@ extern "C" int dpf_mixed_newton_step(const dpf_mixed_newton *solver, const dpf_n
     run.v0 = step->v_in ? step->v_in : step->v;
     run.rotation0 = step->rotation_in ? step->rotation_in : step->rotation;
     int rc = run.run();
+    if (rc) cudaStreamSynchronize(run.st);   // no launch writes the pinned block after the call
     // a step that did not commit leaves the start values
     if (!rc && info->outcome != DPF_NEWTON_CONVERGED &&
         ((step->v_in && cudaMemcpyAsync(step->v, step->v_in, run.n6 * sizeof(double), cudaMemcpyDeviceToDevice,

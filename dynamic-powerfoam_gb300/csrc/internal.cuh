@@ -25,37 +25,52 @@ int jacobian_pass(const dpf_graph *g, const double *linear, const double *direct
                   const uint8_t *fixed, double dt, const double *units, const double *preconditioner, double *out,
                   double *wrench, cudaStream_t stream);
 
-// One CGS2 Arnoldi step in one cooperative launch (dpf_arnoldi_cgs2_fused).
-int arnoldi_pass(int64_t length, double *basis, int64_t ld, int j, double *w, double *h, double *partials,
-                 unsigned *barrier, int *status, cudaStream_t stream);
+// The bonds' wrenches of the committed state (dpf_loads without the sites' sums).
+int loads_bonds_pass(const dpf_graph *g, const dpf_history *h, double *wrench, cudaStream_t stream);
 
-// What the elastic PCG reads and writes:
-//   kElastic    r = block (units vector), out = x / units (dpf_elastic_precondition);
-//   kElasticRaw r the same, out = x;
-//   kElasticT   r = vector / units, out = units (block x): the transposed preconditioner.
-enum ElasticForm { kElastic = 0, kElasticRaw = 1, kElasticT = 2 };
-
-int elastic_pass(const dpf_graph *g, const dpf_stiffness *k, const dpf_tangent *t, const double *mass,
-                 const uint8_t *fixed, const double *block, const double *preconditioner, const double *units,
-                 const double *vector, double dt, double tolerance, int max_iterations, double *out, int *iterations,
-                 double *wrench, double *workspace, unsigned *barrier, int *status, ElasticForm form,
-                 cudaStream_t stream);
-
-// ---- passes of the mixed-precision step driver -------------------------------
-//
-// The driver's launches are shared or joined where the entry points of the same
-// passes each read and write whole vectors; every entry gets the same arithmetic
-// in the same order, so a step gives the same bits either way.  `host` pointers
-// are pinned memory that the device writes (read after the stream is waited for).
-
-// Words the last block of a pass copies to the host beside its own results.
+// A step driver's launches write what the host decides on straight to pinned memory
+// (`host` pointers, read after the stream is waited for).  Report: words that the last
+// block of a pass copies there beside its own results.
 struct Report {
     const double *from = nullptr;
     double *to = nullptr;
     int count = 0;
     const int *status = nullptr;
     int *status_to = nullptr;
+    __device__ void send() const {
+        for (int k = 0; k < count; ++k) to[k] = from[k];
+        if (status) *status_to = *status;
+    }
 };
+
+// One CGS2 Arnoldi step in one cooperative launch (dpf_arnoldi_cgs2_fused); h may be
+// pinned host memory.  clear: the next cooperative launch's barrier word, which this
+// launch clears; with it the own word is clean already, without it a memset cleans it.
+int arnoldi_pass(int64_t length, double *basis, int64_t ld, int j, double *w, double *h, double *partials,
+                 unsigned *barrier, unsigned *clear, int *status, cudaStream_t stream);
+
+// dpf_scale_residual with a report.
+int scale_residual64_pass(int64_t n_sites, const double *preconditioner, const double *units, const double *residual,
+                          double *scaled, double *norms, double *partials, const Report &report, cudaStream_t stream);
+
+// What the elastic PCG reads and writes:
+//   kElastic    r = block (units vector), out = x / units (dpf_elastic_precondition);
+//   kElasticRaw r the same, out = x;
+//   kElasticT   r = vector / units, out = units (block x): the transposed preconditioner.
+// clear as arnoldi_pass.
+enum ElasticForm { kElastic = 0, kElasticRaw = 1, kElasticT = 2 };
+
+int elastic_pass(const dpf_graph *g, const dpf_stiffness *k, const dpf_tangent *t, const double *mass,
+                 const uint8_t *fixed, const double *block, const double *preconditioner, const double *units,
+                 const double *vector, double dt, double tolerance, int max_iterations, double *out, int *iterations,
+                 double *wrench, double *workspace, unsigned *barrier, unsigned *clear, int *status, ElasticForm form,
+                 cudaStream_t stream);
+
+// ---- passes of the mixed-precision step driver -------------------------------
+//
+// The driver's launches are shared or joined where the entry points of the same
+// passes each read and write whole vectors; every entry gets the same arithmetic
+// in the same order, so a step gives the same bits either way.
 
 // dpf_mixed_begin, and the start of a step whose records come from the last
 // commit: y = y32 = 0, residual = r0 on free sites, cleared status, counter and

@@ -111,22 +111,29 @@ struct Reducer {
     // Block partials (sum, sum, max) -> grid barrier -> the same totals in every block.
     __device__ __forceinline__ bool operator()(double s0, double s1, double m2, unsigned *barrier, int *status,
                                                double out[3]) {
-        s0 = block_sum(s0);
-        s1 = block_sum(s1);
-        m2 = block_max(m2);
+        double v[3] = {s0, s1, m2};
+        block_reduce<3, 4u>(v);
         double *p = part + (int64_t)buf * 3 * kMaxBlocks;
         if (threadIdx.x == 0) {
-            p[3 * blockIdx.x] = s0;
-            p[3 * blockIdx.x + 1] = s1;
-            p[3 * blockIdx.x + 2] = m2;
+            p[3 * blockIdx.x] = v[0];
+            p[3 * blockIdx.x + 1] = v[1];
+            p[3 * blockIdx.x + 2] = v[2];
         }
         if (!grid_barrier(barrier, status)) return false;
-        double totals[3];
-        block_arrays<3, 4u>(p, gridDim.x, totals);
-        out[0] = totals[0];
-        out[1] = totals[1];
-        out[2] = totals[2];
+        block_arrays<3, 4u>(p, gridDim.x, v);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) out[k] = v[k];
         buf ^= 1;  // the other buffer: no block still reads it after the next barrier
+        return true;
+    }
+    // the first sum alone
+    __device__ __forceinline__ bool one(double s0, unsigned *barrier, int *status, double out[3]) {
+        s0 = block_sum(s0);
+        double *p = part + (int64_t)buf * 3 * kMaxBlocks;
+        if (threadIdx.x == 0) p[blockIdx.x] = s0;
+        if (!grid_barrier(barrier, status)) return false;
+        out[0] = block_sum_array(p, gridDim.x);
+        buf ^= 1;
         return true;
     }
 };
@@ -217,9 +224,10 @@ __global__ void __launch_bounds__(kThreads) block_pcg_kernel(BlockPcgArgs a) {
             st3(a.s + at, q);
             ps = dot_add(ps, p, q);
         }
-        if (!reduce(ps, 0.0, 0.0, a.barrier, a.status, tot)) return;
+        if (!reduce.one(ps, a.barrier, a.status, tot)) return;
         const double alpha = block_divide(gamma, tot[0]);
-        // x += alpha p, r -= alpha s, u = P r; (r, u), |r|^2, max |u / scale|
+        // x += alpha p, r -= alpha s, u = P r; (r, u), and where they are tested |r|^2, max |u / scale|
+        const bool tested = it % 10 == 0;
         double rr2 = 0.0, umax = 0.0;
         ru = 0.0;
         s = first;
@@ -231,19 +239,20 @@ __global__ void __launch_bounds__(kThreads) block_pcg_kernel(BlockPcgArgs a) {
                 r = axpy(-alpha, ld3(a.s + at), ld3(a.r + at));
                 st3(a.x + at, axpy(alpha, ld3(a.p + at), ld3(a.x + at)));
                 st3(a.r + at, r);
-                rr2 = dot_add(rr2, r, r);
+                if (tested) rr2 = dot_add(rr2, r, r);
             }
             const d3 ro = other_half(r);
             if (live) {
                 const d3 u = half_rows(a.P + 36 * s, half, r, ro);
                 st3(a.u + at, u);
                 ru = dot_add(ru, r, u);
-                umax = scaled_max(a, at, u, umax);
+                if (tested) umax = scaled_max(a, at, u, umax);
             }
         }
-        if (!reduce(ru, rr2, umax, a.barrier, a.status, tot)) return;
+        if (!(tested ? reduce(ru, rr2, umax, a.barrier, a.status, tot) : reduce.one(ru, a.barrier, a.status, tot)))
+            return;
         ru = tot[0];
-        if (it % 10 == 0) {
+        if (tested) {
             relative = sqrt(tot[1]) / norm;
             if (a.mode == kLinear) {
                 if (relative < a.tol) {
@@ -288,7 +297,7 @@ __global__ void __launch_bounds__(kThreads) block_pcg_kernel(BlockPcgArgs a) {
             const d3 res = rhs_half(a, s, half) - operator_rows<false>(a.A, a.x, s, half);
             e2 = dot_add(e2, res, res);
         }
-        if (!reduce(e2, 0.0, 0.0, a.barrier, a.status, tot)) return;
+        if (!reduce.one(e2, a.barrier, a.status, tot)) return;
         relative = sqrt(tot[0]) / norm;
     }
     if (tid == 0) {

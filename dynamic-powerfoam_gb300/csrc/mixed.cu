@@ -414,8 +414,7 @@ __device__ __forceinline__ void finish_norms(double sum_r, float max_s, float s_
             norms[1] = mx;
             norms[2] = sqrt(s2);
             if (status && (!isfinite(r2) || !isfinite(s2))) atomicOr(status, DPF_ERR_NONFINITE);
-            for (int k = 0; k < report.count; ++k) report.to[k] = report.from[k];
-            if (report.status) *report.status_to = *report.status;
+            report.send();
         }
     }
 }

@@ -11,7 +11,11 @@
 //   * the true residual of an FGMRES cycle comes from the Arnoldi relation,
 //     b - J x = V (g0 e_1 - H c) with orthonormal V (CGS2): its norm is that of
 //     the host's coefficient vector, and no J x is formed;
-//   * the accepted increment's end state needs no force.
+//   * the accepted increment's end state needs no force;
+//   * the blocks, inverses and scaled norms of a line-search candidate are formed
+//     behind its residual, before it is accepted, so that the next iteration starts
+//     without a wait of its own (a rejected candidate costs the iterate's again);
+//   * what the host decides on is written to pinned memory by the kernels.
 // What the host does between launches (about a hundred library calls a step from
 // Python) is a few microseconds here; at 512 sites that was most of a step.
 // A step of two Newton iterations, before and after: 512 sites 3.7 -> 1.4 ms,
@@ -36,7 +40,7 @@ struct ArnoldiArgs {
     const double *basis;
     double *w, *next, *h, *part;
     int count;
-    unsigned *barrier;
+    unsigned *barrier, *clear;
     int *status;
 };
 
@@ -62,12 +66,13 @@ __global__ void __launch_bounds__(kThreads) arnoldi_kernel(ArnoldiArgs a) {
     __shared__ double values[kMaxColumns];
     const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
     double *part2 = a.part + (int64_t)kMaxColumns * kMaxBlocks, *part3 = part2 + (int64_t)kMaxColumns * kMaxBlocks;
+    if (a.clear && tid == 0) *a.clear = 0u;
+    double first = 0.0;      // thread k of block 0: column entry k of the first pass (h is only written)
     for (int pass = 0; pass < 2; ++pass) {
         double *part = pass ? part2 : a.part;
         if (pass) {
             row_totals(a.part, a.count, values);
-            if (blockIdx.x == 0)
-                for (int k = threadIdx.x; k < a.count; k += blockDim.x) a.h[k] = values[k];
+            if (threadIdx.x < a.count) first = values[threadIdx.x];
         }
         for (int k0 = 0; k0 < a.count; k0 += kRows) {
             double p[kRows];
@@ -96,8 +101,7 @@ __global__ void __launch_bounds__(kThreads) arnoldi_kernel(ArnoldiArgs a) {
         }
     }
     row_totals(part2, a.count, values);
-    if (blockIdx.x == 0)
-        for (int k = threadIdx.x; k < a.count; k += blockDim.x) a.h[k] += values[k];
+    if (blockIdx.x == 0 && threadIdx.x < a.count) a.h[threadIdx.x] = first + values[threadIdx.x];
     double sq = 0.0;
     for (int64_t e = tid; e < a.len; e += stride) {
         double wv = a.w[e];
@@ -125,12 +129,14 @@ struct Coefficients {
 
 // x (+)= sum c_k rows_k, then the Newton correction (units x where the rows are in
 // the scaled coordinates; zero rows on fixed sites) and the full-step candidate
-// y + correction.
+// y + correction; clears the status word.
 __global__ void __launch_bounds__(kThreads) candidate_kernel(int64_t len, const double *rows, int64_t ld, int count,
                                                              Coefficients coef, int add, double *x,
                                                              const double *units, const uint8_t *fixed,
-                                                             const double *y, double *correction, double *candidate) {
+                                                             const double *y, double *correction, double *candidate,
+                                                             int *status) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < len; e += stride) {
         double v = 0.0;
         for (int k = 0; k < count; ++k) v += rows[k * ld + e] * coef.c[k];
@@ -150,6 +156,8 @@ struct AcceptArgs {
     const double *x, *y, *v, *rotation, *external;
     double two_over_dt;
     double *x_end, *v_end, *rotation_end, *out, *partials;
+    const int *inner;
+    int *inner_to;
 };
 
 __global__ void __launch_bounds__(kThreads) accept_state_kernel(AcceptArgs a) {
@@ -177,6 +185,55 @@ __global__ void __launch_bounds__(kThreads) accept_state_kernel(AcceptArgs a) {
         if (threadIdx.x == 0) {
             a.out[0] = sum;
             a.out[1] = sqrt(most);
+            *a.inner_to = *a.inner;
+        }
+    }
+}
+
+// The start of a step: its scale [|dt M v + dt^2/2 ext|, |loads on free sites|]
+// (bonded_dem_newton.py:138-139) with the sites' loads summed here from the bonds'
+// wrenches, y = 0 and the cleared words.  Two lanes a site.
+struct StartArgs {
+    int64_t n;
+    const int32_t *ptr, *inc;
+    const double *wrench, *mass, *v, *external;
+    const uint8_t *fixed;
+    double dt, half_dt2;
+    double *y, *scales, *partials, *general;
+    int *status, *inner;
+    unsigned *barrier;
+};
+
+__global__ void __launch_bounds__(kThreads) start_kernel(StartArgs a) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *a.status = *a.inner = a.barrier[0] = a.barrier[1] = 0;
+        *a.general = 0.0;
+    }
+    double sums[2] = {0.0, 0.0};
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < 2 * a.n; t += stride) {
+        const int64_t s = t / 2;
+        const d3 m = ld3(a.mass, t), v = ld3(a.v, t), ext = ld3(a.external, t);
+        const d3 rhs = mk(a.dt * m.x * v.x + a.half_dt2 * ext.x, a.dt * m.y * v.y + a.half_dt2 * ext.y,
+                          a.dt * m.z * v.z + a.half_dt2 * ext.z);
+        sums[0] = dot_add(sums[0], rhs, rhs);
+        if (!a.fixed[s]) {
+            const d3 loads = gather_half(a.ptr, a.inc, a.wrench, s, (int)(t & 1));
+            sums[1] = dot_add(sums[1], loads, loads);
+        }
+        st3(a.y, t, mk(0.0, 0.0, 0.0));
+    }
+    block_reduce<2, 0u>(sums);
+    double *part = a.partials + 8;
+    if (threadIdx.x == 0) {
+        part[2 * blockIdx.x] = sums[0];
+        part[2 * blockIdx.x + 1] = sums[1];
+    }
+    if (last_block(reinterpret_cast<unsigned *>(a.partials) + 1)) {
+        block_arrays<2, 0u>(part, gridDim.x, sums);
+        if (threadIdx.x == 0) {
+            a.scales[0] = sqrt(sums[0]);
+            a.scales[1] = sqrt(sums[1]);
         }
     }
 }
@@ -193,7 +250,8 @@ struct Step {
     cudaStream_t st;
     int64_t n, n6, m;
     double *y, *cand, *r, *r_cand, *scaled, *x, *corr;
-    double *host;     // pinned: [0..4) norms, [4..6) scales, [6] normals without unit length, [16..80) h column
+    double *host;     // pinned, written by the kernels: [0..3) a residual's norms, [4..6) scales, [6] normals without
+                      // unit length, [8..11) the scaled residual's norms, [12..14) a restart's, [16..80) h column
     int *host_int;    // [0] status, [1] inner
     double rhs_scale = -1.0;
     dpf_tangent tangent;
@@ -206,39 +264,42 @@ struct Step {
         return rc;
     }
 
-    int fetch(bool first) {
-        if (cudaMemcpyAsync(host, s->scalars, (first ? 7 : 3) * sizeof(double), cudaMemcpyDeviceToHost, st) ||
-            cudaMemcpyAsync(host_int, s->status, sizeof(int), cudaMemcpyDeviceToHost, st))
+    // wait for the stream, after copying the status word when no kernel reported it
+    int wait(bool status = false) {
+        if (status && cudaMemcpyAsync(host_int, s->status, sizeof(int), cudaMemcpyDeviceToHost, st))
             return DPF_ERR_CUDA;
         return cudaStreamSynchronize(st) == cudaSuccess ? DPF_OK : DPF_ERR_CUDA;
     }
 
     // residual of yy with every trial guard and the tangent there; use_p: also
-    // the norms of P r / units
-    int residual(const double *yy, double *out, bool use_p) {
-        if (cudaMemsetAsync(s->status, 0, sizeof(int), st)) return DPF_ERR_CUDA;
+    // the norms of P r / units; cleared: the status word is
+    int residual(const double *yy, double *out, bool use_p, bool cleared) {
+        if (!cleared && cudaMemsetAsync(s->status, 0, sizeof(int), st)) return DPF_ERR_CUDA;
         dpf_trial_out t{};
         t.n = s->n;
         t.ri = s->ri;
         t.rj = s->rj;
         return ran(m ? 2 : 1, dpf::residual_pass(s->graph, &s->stiffness, &a->history, yy, a->v_in, a->external,
                                                  s->mass, s->fixed, a->dt, &t, use_p ? s->preconditioner : nullptr,
-                                                 use_p ? s->units : nullptr, out, use_p ? s->scalars : nullptr,
+                                                 use_p ? s->units : nullptr, out, use_p ? host : nullptr,
                                                  s->wrench, s->partials, s->status, s->elastic ? s->linear : nullptr,
                                                  s->scalars + 6, st));
     }
 
-    // blocks and scaling of the tangent, then P r / units and its norms
+    // blocks and scaling of the tangent, then P r / units and its norms (host[8..11)),
+    // with the status word and the flag of the normals
     int scaling(const double *rr) {
         int rc = ran(1, dpf_prepare_scaling(s->graph, &s->stiffness, &tangent, s->mass, s->fixed, s->radii, a->dt,
                                             s->diagonal, s->block, s->preconditioner, s->units, st));
         if (rc) return rc;
-        return ran(1, dpf_scale_residual(n, s->preconditioner, s->units, rr, scaled, s->scalars, s->partials, st));
+        return ran(1, dpf::scale_residual64_pass(n, s->preconditioner, s->units, rr, scaled, host + 8, s->partials,
+                                                 dpf::Report{s->scalars + 6, host + 6, 1, s->status, host_int}, st));
     }
 
+    // the elastic PCG and the Arnoldi step clear each other's barrier word
     int arnoldi(int j) {
-        return ran(1, dpf::arnoldi_pass(n6, s->basis, n6, j, s->w, s->h, s->krylov_partials, s->barrier, s->status,
-                                        st));
+        return ran(1, dpf::arnoldi_pass(n6, s->basis, n6, j, s->w, host + 16, s->krylov_partials, s->barrier + 1,
+                                        s->elastic ? s->barrier : nullptr, s->status, st));
     }
 
     // Right-preconditioned FGMRES on the scaled system from rhs = -scaled, |rhs| =
@@ -267,7 +328,7 @@ struct Step {
                 if (s->elastic) {
                     rc = ran(1, dpf::elastic_pass(s->graph, &s->stiffness, &tangent, s->mass, s->fixed, s->block,
                                                   s->preconditioner, s->units, v, a->dt, 0.03, 80, z, s->inner,
-                                                  s->wrench, s->workspace, s->barrier, s->status,
+                                                  s->wrench, s->workspace, s->barrier, s->barrier + 1, s->status,
                                                   raw ? dpf::kElasticRaw : dpf::kElastic, st));
                     if (rc) return rc;
                 } else {
@@ -281,10 +342,9 @@ struct Step {
                 if (rc) return rc;
                 rc = arnoldi(j);
                 if (rc) return rc;
-                double *column = host + 16;
-                if (cudaMemcpyAsync(column, s->h, (j + 2) * sizeof(double), cudaMemcpyDeviceToHost, st) ||
-                    cudaStreamSynchronize(st))
-                    return DPF_ERR_CUDA;
+                rc = wait();
+                if (rc) return rc;
+                const double *column = host + 16;
                 for (int i = 0; i <= j + 1; ++i) H[i * 64 + j] = entries[i * 64 + j] = column[i];
                 const bool breakdown = column[j + 1] < 1e-14;
                 for (int i = 0; i < j; ++i) {
@@ -330,13 +390,13 @@ struct Step {
             if (cudaMemsetAsync(s->residual, 0, n6 * sizeof(double), st)) return DPF_ERR_CUDA;
             rc = ran(1, dpf_combine_rows(n6, s->basis, n6, last ? k + 1 : k, left, s->residual, st));
             if (rc) return rc;
-            rc = ran(1, dpf_dot_norm(n6, s->residual, nullptr, s->scalars, s->partials, st));
+            rc = ran(1, dpf_dot_norm(n6, s->residual, nullptr, host + 12, s->partials, st));
             if (rc) return rc;
-            rc = fetch(false);
+            rc = wait();
             if (rc) return rc;
             start = s->residual;
             sign = 1.0;
-            g0 = host[1];
+            g0 = host[13];
             add = true;
         }
         return DPF_OK;
@@ -346,7 +406,8 @@ struct Step {
         Coefficients c{};
         for (int k = 0; k < count; ++k) c.c[k] = coef[k];
         candidate_kernel<<<reduce_grid(n6), kThreads, 0, st>>>(n6, rows, n6, count, c, add ? 1 : 0, x,
-                                                               raw ? nullptr : s->units, s->fixed, y, corr, cand);
+                                                               raw ? nullptr : s->units, s->fixed, y, corr, cand,
+                                                               s->status);
         return ran(1, cudaGetLastError() == cudaSuccess ? DPF_OK : DPF_ERR_CUDA);
     }
 
@@ -361,12 +422,11 @@ struct Step {
         int rc = ran(m ? 1 : 0, dpf_commit_state(s->graph, &s->stiffness, &a->history, y, &t, s->status, st));
         if (rc) return rc;
         AcceptArgs k{n, a->history.x, y, a->v_in, a->rotation_in, a->external, 2.0 / a->dt,
-                     a->x_end, a->v, a->rotation, s->scalars, s->partials};
+                     a->x_end, a->v, a->rotation, host, s->partials, s->inner, host_int + 1};
         accept_state_kernel<<<reduce_grid(n), kThreads, 0, st>>>(k);
         rc = ran(1, cudaGetLastError() == cudaSuccess ? DPF_OK : DPF_ERR_CUDA);
         if (rc) return rc;
-        if (cudaMemcpyAsync(host_int + 1, s->inner, sizeof(int), cudaMemcpyDeviceToHost, st)) return DPF_ERR_CUDA;
-        rc = fetch(false);
+        rc = wait();
         if (rc) return rc;
         info->work = host[0];
         info->max_rotation = host[1];
@@ -377,23 +437,29 @@ struct Step {
     int run() {
         const double dt = a->dt;
         tangent = {s->n, s->ri, s->rj};
-        if (cudaMemsetAsync(s->inner, 0, sizeof(int), st) || cudaMemsetAsync(y, 0, n6 * sizeof(double), st) ||
-            cudaMemsetAsync(s->scalars + 6, 0, sizeof(double), st))
-            return DPF_ERR_CUDA;
-        // the step's scale (bonded_dem_newton.py:138-139), read with the first norms
-        int rc = ran(m ? 2 : 1, dpf_loads(s->graph, &a->history, corr, s->wrench, st));
+        int rc = ran(m ? 1 : 0, dpf::loads_bonds_pass(s->graph, &a->history, s->wrench, st));
         if (rc) return rc;
-        rc = ran(1, dpf_rhs_scale(n, s->mass, a->v_in, a->external, corr, s->fixed, dt, s->scalars + 4, s->partials,
-                                  st));
+        {
+            StartArgs k{n, s->graph->inc_ptr, s->graph->inc_bond, s->wrench, s->mass, a->v_in, a->external, s->fixed,
+                        dt, 0.5 * dt * dt, y, host + 4, s->partials, s->scalars + 6, s->status, s->inner, s->barrier};
+            const int threads = reduce_threads(2 * n);
+            const int64_t want = (2 * n + threads - 1) / threads;
+            start_kernel<<<(int)(want < kMaxBlocks ? want : kMaxBlocks), threads, 0, st>>>(k);
+            rc = ran(1, cudaGetLastError() == cudaSuccess ? DPF_OK : DPF_ERR_CUDA);
+            if (rc) return rc;
+        }
+        rc = residual(y, r, false, true);
         if (rc) return rc;
-        rc = residual(y, r, false);
-        if (rc) return rc;
+        bool prefetched = false;
         for (int iteration = 0; iteration <= a->max_iterations; ++iteration) {
-            rc = scaling(r);
-            if (rc) return rc;
             const bool first = rhs_scale < 0.0;
-            rc = fetch(first);
-            if (rc) return rc;
+            if (!prefetched) {
+                rc = scaling(r);
+                if (rc) return rc;
+                rc = wait();
+                if (rc) return rc;
+            }
+            prefetched = false;
             if (first && host_int[0]) {
                 info->outcome = DPF_NEWTON_GUARD;
                 info->guard = host_int[0];
@@ -405,7 +471,7 @@ struct Step {
                 if (1e-30 > rhs_scale) rhs_scale = 1e-30;
                 raw = s->elastic && s->linear && host[6] == 0.0;
             }
-            const double relative = host[0] / rhs_scale, local = host[1], merit = host[2];
+            const double relative = host[8] / rhs_scale, local = host[9], merit = host[10];
             info->relative = relative;
             info->local = local;
             info->nonlinear_iterations = iteration;
@@ -447,9 +513,13 @@ struct Step {
                     rc = ran(1, dpf_axpby(n6, 1.0, y, factor, corr, cand, st));
                     if (rc) return rc;
                 }
-                rc = residual(cand, r_cand, true);
+                rc = residual(cand, r_cand, true, power == 0);
                 if (rc) return rc;
-                rc = fetch(false);
+                if (power == 0) {
+                    rc = scaling(r_cand);
+                    if (rc) return rc;
+                }
+                rc = wait(power > 0);
                 if (rc) return rc;
                 if (!host_int[0] && host[2] < (1.0 - 1e-4 * factor) * merit) {
                     double *t = y;
@@ -459,6 +529,13 @@ struct Step {
                     r = r_cand;
                     r_cand = t;
                     accepted = true;
+                    prefetched = power == 0;
+                } else if (power == 0) {
+                    // the iterate's tangent, blocks and inverses again for the other candidates
+                    rc = residual(y, r, false, false);
+                    if (rc) return rc;
+                    rc = scaling(r);
+                    if (rc) return rc;
                 }
             }
             if (!accepted) {
@@ -474,7 +551,7 @@ struct Step {
 }  // namespace newton64
 
 int arnoldi_pass(int64_t length, double *basis, int64_t ld, int j, double *w, double *h, double *partials,
-                 unsigned *barrier, int *status, cudaStream_t st) {
+                 unsigned *barrier, unsigned *clear, int *status, cudaStream_t st) {
     using namespace newton64;
     static int per_device[64] = {0};
     int dev = 0;
@@ -491,8 +568,8 @@ int arnoldi_pass(int64_t length, double *basis, int64_t ld, int j, double *w, do
     }
     const int64_t need = (length + kThreads - 1) / kThreads;
     if (blocks > need) blocks = (int)need;
-    ArnoldiArgs k{length, ld, basis, w, basis + (int64_t)(j + 1) * ld, h, partials, j + 1, barrier, status};
-    if (cudaMemsetAsync(barrier, 0, 2 * sizeof(unsigned), st)) return DPF_ERR_CUDA;
+    ArnoldiArgs k{length, ld, basis, w, basis + (int64_t)(j + 1) * ld, h, partials, j + 1, barrier, clear, status};
+    if (!clear && cudaMemsetAsync(barrier, 0, sizeof(unsigned), st)) return DPF_ERR_CUDA;
     void *args[] = {&k};
     if (cudaLaunchCooperativeKernel((const void *)arnoldi_kernel, blocks, kThreads, args, 0, st) != cudaSuccess) {
         cudaGetLastError();
@@ -515,7 +592,7 @@ int dpf_arnoldi_cgs2_fused(int64_t length, double *basis, int64_t ld, int j, dou
     if (length <= 0 || !basis || !w || !h || !partials || !barrier || !status || j < 0 ||
         j + 1 >= dpf::newton64::kMaxColumns || ld < length)
         return DPF_ERR_ARGUMENT;
-    return dpf::arnoldi_pass(length, basis, ld, j, w, h, partials, barrier, status, (cudaStream_t)stream);
+    return dpf::arnoldi_pass(length, basis, ld, j, w, h, partials, barrier, nullptr, status, (cudaStream_t)stream);
 }
 
 int64_t dpf_newton64_linear_doubles(int64_t n_bonds) { return n_bonds < 0 ? 0 : dpf::kLinear * n_bonds; }
@@ -542,9 +619,16 @@ int dpf_newton64_step(const dpf_newton64 *solver, const dpf_newton_step *step, d
     run.m = solver->graph->n_bonds;
     double **slots[DPF_NEWTON64_VECTORS] = {&run.y, &run.cand, &run.r, &run.r_cand, &run.scaled, &run.x, &run.corr};
     for (int k = 0; k < DPF_NEWTON64_VECTORS; ++k) *slots[k] = solver->vectors + (int64_t)k * run.n6;
+    // the address at which the device writes the pinned block
+    void *mapped = nullptr;
+    if (cudaHostGetDevicePointer(&mapped, solver->host, 0) != cudaSuccess || mapped != (void *)solver->host) {
+        cudaGetLastError();
+        return DPF_ERR_ARGUMENT;
+    }
     run.host = solver->host;
     run.host_int = reinterpret_cast<int *>(solver->host + 96);
     const int rc = run.run();
+    if (rc) cudaStreamSynchronize(run.st);   // no launch writes the pinned block after the call
     info->scaling_alternate = run.y == solver->vectors ? 0 : 1;
     return rc;
 }

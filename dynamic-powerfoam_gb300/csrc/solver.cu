@@ -65,7 +65,7 @@ struct PcgArgs {
     double *out;
     int *iterations;
     double *wrench, *r, *u, *p, *s, *part_a, *part_b;
-    unsigned *barrier;
+    unsigned *barrier, *clear;   // clear: the next cooperative launch's word, or NULL
     int *status;
 };
 
@@ -74,6 +74,7 @@ __global__ void __launch_bounds__(kThreads) pcg_kernel(PcgArgs a) {
     const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     const int half = threadIdx.x & 1;
+    if (a.clear && tid == 0) *a.clear = 0u;
     // site loops: lanes 2k and 2k + 1 of a warp share site s and run the same rounds
     const int64_t first = tid / 2, step = stride / 2, rounds = (a.n + step - 1) / step;
     double *mine = stage + 9 * (threadIdx.x & ~31);
@@ -307,7 +308,7 @@ __global__ void __launch_bounds__(kThreads) axpby_kernel(int64_t len, double alp
 // Scaled residual s = P r / units and [|r|, max|s|, |s|] (bonded_dem_newton.py:104-105, 147).
 __global__ void __launch_bounds__(kThreads) scale_kernel(int64_t n, const double *P, const double *units,
                                                          const double *r, double *scaled, double *norms,
-                                                         double *partials) {
+                                                         double *partials, Report report) {
     double sum_r = 0.0, max_s = 0.0, sum_s = 0.0;
     const int half = threadIdx.x & 1;    // two neighbouring lanes a site: its force rows and its torque rows
     const int64_t step = (int64_t)gridDim.x * (blockDim.x / 2), rounds = (n + step - 1) / step;
@@ -326,23 +327,21 @@ __global__ void __launch_bounds__(kThreads) scale_kernel(int64_t n, const double
         }
     }
     if (!norms) return;
-    sum_r = block_sum(sum_r);
-    max_s = block_max(max_s);
-    sum_s = block_sum(sum_s);
+    double v[3] = {sum_r, max_s, sum_s};
+    block_reduce<3, 2u>(v);
     double *part = partials + kPartialsOffset;
     if (threadIdx.x == 0) {
-        part[3 * blockIdx.x] = sum_r;
-        part[3 * blockIdx.x + 1] = max_s;
-        part[3 * blockIdx.x + 2] = sum_s;
+        part[3 * blockIdx.x] = v[0];
+        part[3 * blockIdx.x + 1] = v[1];
+        part[3 * blockIdx.x + 2] = v[2];
     }
     if (last_block(counter_slot(partials, 2))) {
-        double totals[3];
-        block_arrays<3, 2u>(part, gridDim.x, totals);
-        const double r2 = totals[0], mx = totals[1], s2 = totals[2];
+        block_arrays<3, 2u>(part, gridDim.x, v);
         if (threadIdx.x == 0) {
-            norms[0] = sqrt(r2);
-            norms[1] = mx;
-            norms[2] = sqrt(s2);
+            norms[0] = sqrt(v[0]);
+            norms[1] = v[1];
+            norms[2] = sqrt(v[2]);
+            report.send();
         }
     }
 }
@@ -684,8 +683,8 @@ int64_t dpf_elastic_workspace_doubles(int64_t n_sites) { return 30 * n_sites + 2
 int dpf::elastic_pass(const dpf_graph *g, const dpf_stiffness *k, const dpf_tangent *t, const double *mass,
                       const uint8_t *fixed, const double *block, const double *preconditioner, const double *units,
                       const double *vector, double dt, double tolerance, int max_iterations, double *out,
-                      int *iterations, double *wrench, double *workspace, unsigned *barrier, int *status,
-                      ElasticForm form, cudaStream_t st) {
+                      int *iterations, double *wrench, double *workspace, unsigned *barrier, unsigned *clear,
+                      int *status, ElasticForm form, cudaStream_t st) {
     if (!g || g->n_sites <= 0 || !g->inc_ptr || (g->n_bonds && !g->inc_bond) || !k || !t || !mass || !fixed ||
         !block ||
         !preconditioner || !units || !vector || !out || !iterations || !workspace || !barrier || !status ||
@@ -724,6 +723,7 @@ int dpf::elastic_pass(const dpf_graph *g, const dpf_stiffness *k, const dpf_tang
     a.tol2 = tolerance * tolerance;
     a.max_it = max_iterations;
     a.form = form;
+    a.clear = clear;
     a.out = out;
     a.iterations = iterations;
     a.wrench = wrench;
@@ -735,7 +735,7 @@ int dpf::elastic_pass(const dpf_graph *g, const dpf_stiffness *k, const dpf_tang
     a.part_b = workspace + 5 * n6 + kMaxPcgBlocks;
     a.barrier = barrier;
     a.status = status;
-    if (cudaMemsetAsync(barrier, 0, 2 * sizeof(unsigned), st) != cudaSuccess) return DPF_ERR_CUDA;
+    if (!clear && cudaMemsetAsync(barrier, 0, 2 * sizeof(unsigned), st) != cudaSuccess) return DPF_ERR_CUDA;
     void *args[] = {&a};
     if (cudaLaunchCooperativeKernel((const void *)pcg_kernel, grid, threads, args, 0, st) != cudaSuccess) {
         cudaGetLastError();
@@ -752,7 +752,7 @@ int dpf_elastic_precondition(const dpf_graph *g, const dpf_stiffness *k, const d
                              int max_iterations, double *out, int *iterations, double *wrench, double *workspace,
                              unsigned *barrier, int *status, void *stream) {
     return dpf::elastic_pass(g, k, t, mass, fixed, block, preconditioner, units, vector, dt, tolerance, max_iterations,
-                             out, iterations, wrench, workspace, barrier, status, kElastic,
+                             out, iterations, wrench, workspace, barrier, nullptr, status, kElastic,
                              (cudaStream_t)stream);
 }
 
@@ -908,14 +908,25 @@ int dpf_axpby(int64_t length, double alpha, const double *a, double beta, const 
 
 int dpf_scale_residual(int64_t n_sites, const double *preconditioner, const double *units, const double *residual,
                        double *scaled, double *norms, double *partials, void *stream) {
+    return dpf::scale_residual64_pass(n_sites, preconditioner, units, residual, scaled, norms, partials, Report(),
+                                      (cudaStream_t)stream);
+}
+
+}  // extern "C"
+
+int dpf::scale_residual64_pass(int64_t n_sites, const double *preconditioner, const double *units,
+                               const double *residual, double *scaled, double *norms, double *partials,
+                               const Report &report, cudaStream_t st) {
     if (n_sites <= 0 || !preconditioner || !units || !residual || (norms && !partials)) return DPF_ERR_ARGUMENT;
     const int threads = reduce_threads(2 * n_sites);
     const int64_t blocks = blocks_for(2 * n_sites, threads);
-    scale_kernel<<<(int)(blocks < kMaxReduceBlocks ? blocks : kMaxReduceBlocks), threads, 0, (cudaStream_t)stream>>>(
-        n_sites, preconditioner, units, residual, scaled, norms, partials);
+    scale_kernel<<<(int)(blocks < kMaxReduceBlocks ? blocks : kMaxReduceBlocks), threads, 0, st>>>(
+        n_sites, preconditioner, units, residual, scaled, norms, partials, report);
     DPF_CHECK_LAUNCH();
     return DPF_OK;
 }
+
+extern "C" {
 
 int dpf_accept_step(int64_t n_sites, const double *y, double dt, double *v, double *rotation, void *stream) {
     if (n_sites <= 0 || !y || !v || !rotation) return DPF_ERR_ARGUMENT;
