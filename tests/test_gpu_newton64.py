@@ -125,3 +125,20 @@ def test_replaced_methods_keep_the_python_path():
     load[-1, 2] = -1.
     native.step(1e-3, native.tensor(load))
     assert calls
+
+
+@pytest.mark.parametrize('iterations', [1, 2, 3])
+@pytest.mark.parametrize('preconditioning', ['elastic', 'block'])
+def test_rejected_full_steps(iterations, preconditioning):
+    """A pull whose first Newton corrections are halved: the iterate's tangent, blocks and inverses are
+    there again for the shorter candidates.  The step is cut off after a few iterations and its message
+    carries the residual and the pose defect of the last iterate in six digits (one unit of the last)."""
+    import dpf_gb300
+    load, python, native = _pair(3)
+    load[:, :3] += np.random.default_rng(1).normal(size=(len(load), 3))*100*np.abs(load).max()
+    values = []
+    for s in (python, native):
+        with pytest.raises(dpf_gb300.SubdivideError, match='did not converge') as error:
+            s.step(1e-2, s.tensor(load), max_iterations=iterations, preconditioning=preconditioning)
+        values.append([float(v) for v in str(error.value).split('(')[1].rstrip(')').split(',')])
+    assert np.allclose(values[0], values[1], rtol=2e-5, atol=0), values
