@@ -769,21 +769,28 @@ __device__ __forceinline__ unsigned long long global_ns() {
 // have arrived (and the low bits return to where they were); a block waits
 // until the bit differs from the value its own add returned.  Release add and
 // acquire loads order the blocks' writes before and after the barrier.
-// barrier[0] starts at 0 (the launching entry point clears it); barrier[1] is
-// unused.  Returns false when the wait ran past timeout_ns (the status word
+// barrier[0] starts at 0 (the launching entry point clears it).  Returns false when the wait ran past timeout_ns (the status word
 // then carries the error).  parties: arrivals that release the barrier (0 =
 // every block of the grid).
-__device__ __forceinline__ bool grid_barrier(unsigned *barrier, int *status,
-                                             unsigned long long timeout_ns = kBarrierTimeoutNs,
-                                             unsigned parties = 0) {
-    __shared__ int ok;
+//
+// grid_arrive and grid_wait are its halves: thread 0 may work between them while
+// the other blocks arrive.
+__device__ __forceinline__ unsigned grid_arrive(unsigned *barrier, unsigned parties = 0) {
     __syncthreads();
+    unsigned old = 0;
     if (threadIdx.x == 0) {
-        ok = 1;
         const unsigned n = parties ? parties : gridDim.x;
         const unsigned add = blockIdx.x == 0 ? 0x80000000u - (n - 1) : 1u;
-        unsigned old;
         asm volatile("atom.add.release.gpu.global.u32 %0, [%1], %2;" : "=r"(old) : "l"(barrier), "r"(add) : "memory");
+    }
+    return old;
+}
+
+__device__ __forceinline__ bool grid_wait(unsigned *barrier, unsigned old, int *status,
+                                          unsigned long long timeout_ns = kBarrierTimeoutNs) {
+    __shared__ int ok;
+    if (threadIdx.x == 0) {
+        ok = 1;
         unsigned polls = 0;
         const unsigned long long t0 = global_ns();
         while (((ld_acquire(barrier) ^ old) & 0x80000000u) == 0) {
@@ -796,6 +803,13 @@ __device__ __forceinline__ bool grid_barrier(unsigned *barrier, int *status,
     }
     __syncthreads();
     return ok != 0;
+}
+
+__device__ __forceinline__ bool grid_barrier(unsigned *barrier, int *status,
+                                             unsigned long long timeout_ns = kBarrierTimeoutNs,
+                                             unsigned parties = 0) {
+    const unsigned old = grid_arrive(barrier, parties);
+    return grid_wait(barrier, old, status, timeout_ns);
 }
 
 }  // namespace dpf

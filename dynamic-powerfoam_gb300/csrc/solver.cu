@@ -70,7 +70,7 @@ struct PcgArgs {
 };
 
 __global__ void __launch_bounds__(kThreads) pcg_kernel(PcgArgs a) {
-    __shared__ double stage[9 * kThreads];
+    __shared__ double stage[9 * kThreads], over_gamma;
     const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     const int half = threadIdx.x & 1;
@@ -166,10 +166,12 @@ __global__ void __launch_bounds__(kThreads) pcg_kernel(PcgArgs a) {
         }
         part = block_sum(part);
         if (threadIdx.x == 0) a.part_b[blockIdx.x] = part;
-        if (!grid_barrier(a.barrier, a.status)) return;
+        const unsigned old = grid_arrive(a.barrier);
+        if (threadIdx.x == 0) over_gamma = 1.0 / gamma;     // while the other blocks arrive
+        if (!grid_wait(a.barrier, old, a.status)) return;
         const double following = block_sum_array(a.part_b, gridDim.x);
         if (it % 5 == 0 && following <= a.tol2 * initial) break;
-        beta = block_divide(following, gamma);
+        beta = following * over_gamma;
         gamma = following;
     }
     // a thread's own x: no barrier
@@ -556,11 +558,14 @@ __global__ void __launch_bounds__(kThreads, kNormResident) correction_kernel(Cor
     }
 }
 
-// CGS2 of one Arnoldi step in one cooperative launch: dots, projection,
-// dots, projection and norm, normalisation, with grid barriers between them
-// and pairs of floats per access.  Block partials are float32 pairs; every
+// CGS2 of one Arnoldi step in one cooperative launch with three grid barriers:
+// dots; projection with the second pass's dots (a thread reads back only its own
+// elements); second projection with the norm; normalisation.  Pairs of floats per
+// access, two of them in flight a thread.  Block partials are float32 pairs; every
 // block sums them in the same order, so all take the same values.  Partials:
-// part1 = count x grid, part2 = count x grid, part3 = grid pairs.
+// part1 = count x grid, part2 = count x grid, part3 = grid pairs.  262k sites, rows
+// of 1.6M floats, one to three rows: 40 us on average with four barriers and two
+// passes over w more, now 33.5; 160 and 110 us at 1.4M sites.
 struct Arnoldi32Args {
     int64_t half;        // length / 2 (the length is even: 6 per site)
     const float2 *basis;  // rows of ld2 float2
@@ -574,82 +579,134 @@ struct Arnoldi32Args {
     int *status;
 };
 
-// per-thread float32-pair dots of rows 0..count-1 with x, reduced per block
-// into part[k * gridDim.x + blockIdx.x]
-__device__ __forceinline__ void arnoldi_dots_pass(const Arnoldi32Args &a, const float2 *x, double *part) {
-    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int k0 = 0; k0 < a.count; k0 += 4) {
-        float hi[4] = {0.0f, 0.0f, 0.0f, 0.0f}, lo[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        const int kn = a.count - k0 < 4 ? a.count - k0 : 4;
-        for (int64_t e = tid; e < a.half; e += stride) {
-            const float2 xv = x[e];
+constexpr int kArnoldiRows = 4;   // rows whose dots a pass keeps in registers
+
+// this thread's pairs of rows k0.. reduced per block into part[k * gridDim.x + blockIdx.x]
+__device__ __forceinline__ void store_row_partials(const float hi[kArnoldiRows], const float lo[kArnoldiRows], int k0,
+                                                   int count, double *part) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                if (q < kn) {
-                    const float2 b = a.basis[(k0 + q) * a.ld2 + e];
-                    ff_add_product(hi[q], lo[q], b.x, xv.x);
-                    ff_add_product(hi[q], lo[q], b.y, xv.y);
-                }
-            }
-        }
-        for (int q = 0; q < kn; ++q) {
+    for (int q = 0; q < kArnoldiRows; ++q)
+        if (k0 + q < count) {
             const float2 p = block_pair_sum(hi[q], lo[q]);
             if (threadIdx.x == 0) reinterpret_cast<float2 *>(part)[(k0 + q) * gridDim.x + blockIdx.x] = p;
         }
-    }
 }
 
-// w = in - sum_k values_k basis_k (values from the partials of the last pass),
-// the projection as float32 pairs; returns this thread's |w|^2 pair
-__device__ __forceinline__ void arnoldi_project(const Arnoldi32Args &a, const float2 *in, const double *part,
-                                               bool second, float &sq_hi, float &sq_lo) {
-    __shared__ float vhi[kMaxArnoldi], vlo[kMaxArnoldi];
-    __shared__ double column[kMaxArnoldi];   // kept for the second pass: h may be host memory, which is only written
+// Column values of a pass from its partials, split into floats, in shared memory.
+struct ArnoldiColumn {
+    float hi[kMaxArnoldi], lo[kMaxArnoldi];
+    double total[kMaxArnoldi];   // both passes' (h may be host memory, which is only written)
+};
+
+__device__ __forceinline__ void read_column(const Arnoldi32Args &a, const double *part, bool second,
+                                            ArnoldiColumn &col) {
+    __syncthreads();
     // a warp a row (one warp for all of them: 5 us a row more at 262k sites)
     for (int k = threadIdx.x >> 5; k < a.count; k += kThreads / 32) {
         const double v = warp_pair_array(reinterpret_cast<const float2 *>(part) + k * gridDim.x, gridDim.x);
         if ((threadIdx.x & 31) == 0) {
-            ff_split(v, vhi[k], vlo[k]);
-            column[k] = second ? column[k] + v : v;
-            if (second && blockIdx.x == 0) a.h[k] = column[k];
+            ff_split(v, col.hi[k], col.lo[k]);
+            col.total[k] = second ? col.total[k] + v : v;
+            if (second && blockIdx.x == 0) a.h[k] = col.total[k];
         }
     }
     __syncthreads();
-    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t e = tid; e < a.half; e += stride) {
-        float2 ph = make_float2(0.0f, 0.0f), pl = make_float2(0.0f, 0.0f);
-        for (int k = 0; k < a.count; ++k) {
-            const float2 b = a.basis[k * a.ld2 + e];
-            ff_add_product(ph.x, pl.x, vhi[k], b.x);
-            ff_add_product(ph.y, pl.y, vhi[k], b.y);
-            pl.x = fmaf(vlo[k], b.x, pl.x);
-            pl.y = fmaf(vlo[k], b.y, pl.y);
-        }
-        const float2 iv = in[e];
+}
+
+// in - sum_k column_k basis_k at pair e, the projection as float32 pairs
+struct Projection {
+    float2 ph, pl;
+    __device__ __forceinline__ void add(const ArnoldiColumn &col, int k, float2 b) {
+        ff_add_product(ph.x, pl.x, col.hi[k], b.x);
+        ff_add_product(ph.y, pl.y, col.hi[k], b.y);
+        pl.x = fmaf(col.lo[k], b.x, pl.x);
+        pl.y = fmaf(col.lo[k], b.y, pl.y);
+    }
+    __device__ __forceinline__ float2 from(float2 iv) const {
         float dx = iv.x, ex = 0.0f, dy = iv.y, ey = 0.0f;
         ff_two_sum(dx, ex, -ph.x);
         ff_two_sum(dy, ey, -ph.y);
-        const float2 wv = make_float2(dx + (ex - pl.x), dy + (ey - pl.y));
-        a.w[e] = wv;
-        ff_add_product(sq_hi, sq_lo, wv.x, wv.x);
-        ff_add_product(sq_hi, sq_lo, wv.y, wv.y);
+        return make_float2(dx + (ex - pl.x), dy + (ey - pl.y));
     }
-}
+};
 
-__global__ void __launch_bounds__(kThreads) arnoldi32_fused_kernel(Arnoldi32Args a) {
-    if (a.clear && blockIdx.x == 0 && threadIdx.x == 0) *a.clear = 0u;
-    arnoldi_dots_pass(a, a.v, a.part1);
+__global__ void __launch_bounds__(kThreads, 4) arnoldi32_fused_kernel(Arnoldi32Args a) {
+    __shared__ ArnoldiColumn col;
+    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    if (a.clear && tid == 0) *a.clear = 0u;
+    // dots of the rows with v
+    for (int k0 = 0; k0 < a.count; k0 += kArnoldiRows) {
+        float hi[kArnoldiRows] = {}, lo[kArnoldiRows] = {};
+        const int kn = a.count - k0;
+        for (int64_t e = tid; e < a.half; e += 2 * stride) {
+            const int64_t f = e + stride;
+            const bool two = f < a.half;
+            const float2 x0 = __ldg(a.v + e), x1 = two ? __ldg(a.v + f) : make_float2(0.0f, 0.0f);
+            float2 b0[kArnoldiRows], b1[kArnoldiRows];
+#pragma unroll
+            for (int q = 0; q < kArnoldiRows; ++q)
+                if (q < kn) {
+                    b0[q] = __ldg(a.basis + (k0 + q) * a.ld2 + e);
+                    b1[q] = two ? __ldg(a.basis + (k0 + q) * a.ld2 + f) : make_float2(0.0f, 0.0f);
+                }
+#pragma unroll
+            for (int q = 0; q < kArnoldiRows; ++q)
+                if (q < kn) {
+                    ff_add_product(hi[q], lo[q], b0[q].x, x0.x);
+                    ff_add_product(hi[q], lo[q], b0[q].y, x0.y);
+                    ff_add_product(hi[q], lo[q], b1[q].x, x1.x);
+                    ff_add_product(hi[q], lo[q], b1[q].y, x1.y);
+                }
+        }
+        store_row_partials(hi, lo, k0, a.count, a.part1);
+    }
     if (!grid_barrier(a.barrier, a.status)) return;
+    // projection, and the dots of the rows with what it leaves
+    read_column(a, a.part1, false, col);
+    for (int k0 = 0; k0 < a.count; k0 += kArnoldiRows) {
+        float hi[kArnoldiRows] = {}, lo[kArnoldiRows] = {};
+        const int kn = a.count - k0;
+        for (int64_t e = tid; e < a.half; e += stride) {
+            float2 b[kArnoldiRows], w;
+#pragma unroll
+            for (int q = 0; q < kArnoldiRows; ++q)
+                if (q < kn) b[q] = __ldg(a.basis + (k0 + q) * a.ld2 + e);
+            if (k0 == 0) {
+                const float2 iv = __ldg(a.v + e);
+                Projection p{};
+#pragma unroll
+                for (int q = 0; q < kArnoldiRows; ++q)
+                    if (q < kn) p.add(col, q, b[q]);
+                for (int k = kArnoldiRows; k < a.count; ++k) p.add(col, k, __ldg(a.basis + k * a.ld2 + e));
+                w = p.from(iv);
+                a.w[e] = w;
+            } else {
+                w = a.w[e];
+            }
+#pragma unroll
+            for (int q = 0; q < kArnoldiRows; ++q)
+                if (q < kn) {
+                    ff_add_product(hi[q], lo[q], b[q].x, w.x);
+                    ff_add_product(hi[q], lo[q], b[q].y, w.y);
+                }
+        }
+        store_row_partials(hi, lo, k0, a.count, a.part2);
+    }
+    if (!grid_barrier(a.barrier, a.status)) return;
+    // second projection and the norm of what it leaves
+    read_column(a, a.part2, true, col);
     float sh = 0.0f, sl = 0.0f;
-    arnoldi_project(a, a.v, a.part1, false, sh, sl);
-    // the second pass reads w only after every block has written it
-    if (!grid_barrier(a.barrier, a.status)) return;
-    arnoldi_dots_pass(a, a.w, a.part2);
-    if (!grid_barrier(a.barrier, a.status)) return;
-    sh = sl = 0.0f;
-    arnoldi_project(a, a.w, a.part2, true, sh, sl);
+    for (int64_t e = tid; e < a.half; e += stride) {
+        const float2 iv = a.w[e];
+        Projection p{};
+#pragma unroll 4
+        for (int k = 0; k < a.count; ++k) p.add(col, k, __ldg(a.basis + k * a.ld2 + e));
+        const float2 w = p.from(iv);
+        a.w[e] = w;
+        ff_add_product(sh, sl, w.x, w.x);
+        ff_add_product(sh, sl, w.y, w.y);
+    }
     const float2 sq = block_pair_sum(sh, sl);
     if (threadIdx.x == 0) reinterpret_cast<float2 *>(a.part3)[blockIdx.x] = sq;
     if (!grid_barrier(a.barrier, a.status)) return;
@@ -657,8 +714,6 @@ __global__ void __launch_bounds__(kThreads) arnoldi32_fused_kernel(Arnoldi32Args
     if (blockIdx.x == 0 && threadIdx.x == 0) a.h[a.count] = nrm;
     if (!(nrm >= 1e-14)) return;
     const float inv = (float)(1.0 / nrm);
-    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t e = tid; e < a.half; e += stride) {
         const float2 wv = a.w[e];
         a.next[e] = make_float2(wv.x * inv, wv.y * inv);

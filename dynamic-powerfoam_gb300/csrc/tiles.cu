@@ -853,6 +853,7 @@ struct PcgArgs {
     double *out;
     float *out32;           // float32 output instead of out (one of the two)
     float *direction;       // with out32: units * out32 (the JVP's direction), or NULL
+    int wide;               // float32 in and out, rows aligned to 8 bytes, blocks to 16
     unsigned *clear;        // the next launch's barrier word, or NULL
     int *iterations;
     float *x, *r, *u, *p, *s, *w;  // (N, 6) each
@@ -942,16 +943,37 @@ __device__ __forceinline__ void pcg_body(PcgArgs &a, unsigned char *smem) {
     if (a.clear && tid == 0) *a.clear = 0u;
     Pipe P;
     if (kTiles) P = pipe_init(smem, a.L, ((int)blockDim.x - 64) / 32);
-    // r0 = B (units v) with fixed rows zero, u0 = P r0
+    // r0 = B (units v) with fixed rows zero, u0 = P r0.  Site rows in 16- and 8-byte
+    // accesses where the caller's arrays allow them (a.wide).
     float pf = 0.0f;
     for (int64_t s = tid; s < a.n; s += stride) {
         float v[6], rr[6], zz[6], Pm[21];
+        if (a.wide) {
+            float in[6];
+            ld6(a.units32 + 6 * s, v);
+            ld6(a.vector32 + 6 * s, in);
 #pragma unroll
-        for (int c = 0; c < 6; ++c)
-            v[c] = a.units32[6 * s + c] * (a.vector32 ? a.vector32[6 * s + c] : (float)a.vector[6 * s + c]);
+            for (int c = 0; c < 6; ++c) v[c] *= in[c];
+        } else {
+#pragma unroll
+            for (int c = 0; c < 6; ++c)
+                v[c] = a.units32[6 * s + c] * (a.vector32 ? a.vector32[6 * s + c] : (float)a.vector[6 * s + c]);
+        }
         if (a.fixed[s]) {
 #pragma unroll
             for (int c = 0; c < 6; ++c) rr[c] = 0.0f;
+        } else if (a.wide) {
+            const float4 *B = reinterpret_cast<const float4 *>(a.block + 36 * s);
+#pragma unroll
+            for (int c = 0; c < 6; ++c) rr[c] = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 9; ++k) {
+                const float4 q = __ldg(B + k);
+                rr[4 * k / 6] = fmaf(q.x, v[4 * k % 6], rr[4 * k / 6]);
+                rr[(4 * k + 1) / 6] = fmaf(q.y, v[(4 * k + 1) % 6], rr[(4 * k + 1) / 6]);
+                rr[(4 * k + 2) / 6] = fmaf(q.z, v[(4 * k + 2) % 6], rr[(4 * k + 2) / 6]);
+                rr[(4 * k + 3) / 6] = fmaf(q.w, v[(4 * k + 3) % 6], rr[(4 * k + 3) / 6]);
+            }
         } else {
             mv36(a.block + 36 * s, v, rr);
         }
@@ -990,22 +1012,22 @@ __device__ __forceinline__ void pcg_body(PcgArgs &a, unsigned char *smem) {
             for_ends<L, false>(a.E, a.u, epi);
         block_pair_partial(epi.dot, part_a);
         if (!ok) return;
-        if (!grid_barrier(a.barrier, a.status)) return;
-        const double delta = pair_total(part_a, gridDim.x);
-        // the recurrence's three float64 divisions once per block (thread 0),
-        // not once per thread: float64 division is slow on this part
+        const unsigned old = grid_arrive(a.barrier);
+        // the recurrence's float64 divisions once per block (thread 0), not once per
+        // thread: float64 division is slow on this part.  The two that do not need
+        // delta run while the other blocks arrive (4k sites 10.4 -> 9.9 us an iteration,
+        // 1.4M sites 316 -> 305).
         __shared__ double shared_ab[2];
+        double beta0 = 0.0, carried = 0.0;
+        if (threadIdx.x == 0 && it > 0) {
+            beta0 = gamma / gamma_prev;
+            carried = beta0 * gamma / alpha_prev;
+        }
+        if (!grid_wait(a.barrier, old, a.status)) return;
+        const double delta = pair_total(part_a, gridDim.x);
         if (threadIdx.x == 0) {
-            double beta, alpha;
-            if (it == 0) {
-                beta = 0.0;
-                alpha = gamma / delta;
-            } else {
-                beta = gamma / gamma_prev;
-                alpha = gamma / (delta - beta * gamma / alpha_prev);
-            }
-            shared_ab[0] = alpha;
-            shared_ab[1] = beta;
+            shared_ab[0] = gamma / (delta - carried);
+            shared_ab[1] = beta0;
         }
         __syncthreads();
         const double alpha = shared_ab[0], beta = shared_ab[1];
@@ -1024,16 +1046,28 @@ __device__ __forceinline__ void pcg_body(PcgArgs &a, unsigned char *smem) {
         alpha_prev = alpha;
     }
     for (int64_t s = tid; s < a.n; s += stride) {
-        float xv[6];
+        float xv[6], un[6];
         ld6(a.x + 6 * s, xv);
+        if (a.wide) {
+            ld6(a.units32 + 6 * s, un);
+#pragma unroll
+            for (int c = 0; c < 6; ++c) xv[c] = xv[c] / un[c];
+            st6(a.out32 + 6 * s, xv);
+            if (a.direction) {
+#pragma unroll
+                for (int c = 0; c < 6; ++c) xv[c] *= un[c];
+                st6(a.direction + 6 * s, xv);
+            }
+            continue;
+        }
 #pragma unroll
         for (int c = 0; c < 6; ++c) {
-            const float un = a.units32[6 * s + c], v = xv[c] / un;
+            const float unit = a.units32[6 * s + c], v = xv[c] / unit;
             if (a.out32)
                 a.out32[6 * s + c] = v;
             else
                 a.out[6 * s + c] = (double)v;
-            if (a.direction) a.direction[6 * s + c] = v * un;
+            if (a.direction) a.direction[6 * s + c] = v * unit;
         }
     }
     if (tid == 0) atomicAdd(a.iterations, it < a.max_it ? it + 1 : a.max_it);
@@ -1534,6 +1568,8 @@ static int end_precondition(const dpf_graph *g, const float *ends, const float *
     a.part_a = partials;
     a.part_b = partials + kMaxPcgBlocksTiled;
     a.direction = direction;
+    a.wide = vector32 && out32 && aligned16(block32) &&
+             !(((uintptr_t)units32 | (uintptr_t)vector32 | (uintptr_t)out32 | (uintptr_t)direction) & 7u);
     a.clear = clear;
     a.barrier = barrier;
     a.status = status;
