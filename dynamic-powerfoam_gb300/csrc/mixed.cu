@@ -305,17 +305,12 @@ struct ResidualBondArgs {
     const uint8_t *active;   // optional per-segment flag: bonds of inactive segments are skipped
 };
 
-__device__ __forceinline__ void load_y(const float *y, int s, V3<float> &u, V3<float> &w) {
-    const float *p = y + 6 * (int64_t)s;
-    u = {p[0], p[1], p[2]};
-    w = {p[3], p[4], p[5]};
-}
-
 __device__ __forceinline__ void store_zero9(float *w, int64_t b) {
     float4 *p = reinterpret_cast<float4 *>(w + kWrenchFloats * b);
     p[0] = p[1] = p[2] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 }
 
+template <bool kPairs>
 __global__ void __launch_bounds__(kThreads) residual_bonds(ResidualBondArgs a) {
     const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (b >= a.m) return;
@@ -325,8 +320,8 @@ __global__ void __launch_bounds__(kThreads) residual_bonds(ResidualBondArgs a) {
     }
     const Bond B = load_bond(a.bd.rec, b);
     V3<float> ui, wi, uj, wj;
-    load_y(a.y, B.i, ui, wi);
-    load_y(a.y, B.j, uj, wj);
+    load_row<kPairs>(a.y, B.i, ui, wi);
+    load_row<kPairs>(a.y, B.j, uj, wj);
     const BondIncrement<float> o = bond_increment<float>(B, ui, wi, uj, wj);
     store9(a.wrench, b, o.dF, o.dTi, o.dTj);
     int flags = 0;
@@ -609,21 +604,30 @@ __global__ void __launch_bounds__(kThreads) prepare_direction(int64_t count, con
     d32[e] = units32 ? d * units32[e] : d;
 }
 
-// Resident 256-thread blocks per SM the JVP bond pass is compiled for (the
-// dual-number increment is register heavy); 0 leaves the register count to
-// the compiler (99 registers, 2 blocks).  3 blocks (80 registers, 88 bytes of
-// spills) measured 156 us per JVP on the 64^3 foam against 168 us for 2 and
-// 164 us for 4 (64 registers).  The build may set it.
-#ifndef DPF_JVP_BLOCKS_PER_SM
-#define DPF_JVP_BLOCKS_PER_SM 3
-#endif
-#if DPF_JVP_BLOCKS_PER_SM > 0
-#define DPF_JVP_BOUNDS __launch_bounds__(kThreads, DPF_JVP_BLOCKS_PER_SM)
-#else
-#define DPF_JVP_BOUNDS __launch_bounds__(kThreads)
-#endif
+// The derivative with dual numbers, for a committed normal that is not a unit vector
+// (a state assigned from outside).
+__device__ __noinline__ void jvp_bond_general(JvpArgs a, int64_t b) {
+    const Bond B = load_bond(a.bd.rec, b);
+    V3<float> ui, wi, uj, wj, dui, dwi, duj, dwj;
+    load_row<false>(a.y, B.i, ui, wi);
+    load_row<false>(a.y, B.j, uj, wj);
+    load_row<false>(a.d, B.i, dui, dwi);
+    load_row<false>(a.d, B.j, duj, dwj);
+    const BondIncrement<Dual> o =
+        bond_increment<Dual>(B, dual3(ui, dui), dual3(wi, dwi), dual3(uj, duj), dual3(wj, dwj));
+    store9(a.wrench, b, der3(o.dF), der3(o.dTi), der3(o.dTj));
+}
 
-__global__ void DPF_JVP_BOUNDS jvp_bonds_mixed(JvpArgs a) {
+// The derivative is written out (bond_jvp): with dual numbers it took 1081 instructions
+// a warp and the issue slots bound it (68% busy with three blocks of 256 threads and 80
+// registers).  With 620 instructions it waited on loads that the compiler had placed
+// late; with every load first (load_bond, load_row) it is bound by memory.  1.9M bonds:
+// 82 us, written out 65, loads first 54; 10.3M bonds 420 -> 278 us.  128 threads: five to
+// eight blocks an SM 591, 557, 474, 495 us for the whole product of 10.3M bonds.
+constexpr int kJvpThreads = 128, kJvpBlocks = 7;
+
+template <bool kPairs>
+__global__ void __launch_bounds__(kJvpThreads, kJvpBlocks) jvp_bonds_mixed(JvpArgs a) {
     const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (b >= a.m) return;
     if (a.active && !a.active[a.seg[b]]) {
@@ -631,14 +635,18 @@ __global__ void DPF_JVP_BOUNDS jvp_bonds_mixed(JvpArgs a) {
         return;
     }
     const Bond B = load_bond(a.bd.rec, b);
-    V3<float> ui, wi, uj, wj, dui, dwi, duj, dwj;
-    load_y(a.y, B.i, ui, wi);
-    load_y(a.y, B.j, uj, wj);
-    load_y(a.d, B.i, dui, dwi);
-    load_y(a.d, B.j, duj, dwj);
-    const BondIncrement<Dual> o =
-        bond_increment<Dual>(B, dual3(ui, dui), dual3(wi, dwi), dual3(uj, duj), dual3(wj, dwj));
-    store9(a.wrench, b, der3(o.dF), der3(o.dTi), der3(o.dTj));
+    V3<float> ui, wi, uj, wj, dui, dwi, duj, dwj, F, Ti, Tj;
+    load_row<kPairs>(a.y, B.i, ui, wi);
+    load_row<kPairs>(a.y, B.j, uj, wj);
+    load_row<kPairs>(a.d, B.i, dui, dwi);
+    load_row<kPairs>(a.d, B.j, duj, dwj);
+    const V3<float> n0 = lift3<float>(B.n0);
+    if (!(fabsf(dot(n0, n0) - 1.0f) < 1e-6f)) {
+        jvp_bond_general(a, b);
+        return;
+    }
+    bond_jvp(B, uj - ui, wi, wj, duj - dui, dwi, dwj, F, Ti, Tj);
+    store9(a.wrench, b, F, Ti, Tj);
 }
 
 struct JvpSiteArgs {
@@ -1205,14 +1213,14 @@ __device__ __forceinline__ d3 end_normal(const double *x, int64_t i, int64_t j, 
 
 // kLazy: the float64 end state is not written; the records' rounding errors
 // go to the corrections a.corr (dpf_mixed_fold_history forms the history).
-template <bool kLazy>
+template <bool kLazy, bool kPairs>
 __global__ void __launch_bounds__(kThreads, 3) commit_bonds(CommitArgs a) {
     const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (b >= a.m) return;
     const Bond B = load_bond(a.bd.rec, b);
     V3<float> ui, wi, uj, wj;
-    load_y(a.y32, B.i, ui, wi);
-    load_y(a.y32, B.j, uj, wj);
+    load_row<kPairs>(a.y32, B.i, ui, wi);
+    load_row<kPairs>(a.y32, B.j, uj, wj);
     const BondIncrement<float> o = bond_increment<float>(B, ui, wi, uj, wj);
     const float dfn = B.kn * value(o.dn), dmt = B.kt * value(o.tw);
     if (!kLazy) {
@@ -1505,6 +1513,9 @@ int64_t dpf_mixed_workspace_floats(int64_t n_sites, int64_t n_bonds) {
     return 40 * n_sites + 12 * n_bonds + 4 * (int64_t)kMaxPcgBlocks;
 }
 
+// rows of the float32 (N, 6) arrays can be read in 8-byte pairs
+static bool pairs_ok(const float *y, const float *d = nullptr) { return !(((uintptr_t)y | (uintptr_t)d) & 7u); }
+
 static bool mixed_graph_ok(const dpf_graph *g) {
     return g && g->n_sites > 0 && g->n_bonds >= 0 && g->n_bonds < (int64_t(1) << 31) && g->inc_ptr &&
            (g->n_bonds == 0 || g->inc_bond);
@@ -1566,7 +1577,10 @@ int dpf_mixed_residual_segmented(const dpf_graph *g, float *bond_data, const dou
     if (g->n_bonds) {
         ResidualBondArgs a{g->n_bonds, split_bond_data(bond_data, g->n_bonds), y32, want_tangent, wrench, status,
                            seg_bond, active};
-        residual_bonds<<<blocks_for(g->n_bonds, kThreads), kThreads, 0, st>>>(a);
+        if (pairs_ok(y32))
+            residual_bonds<true><<<blocks_for(g->n_bonds, kThreads), kThreads, 0, st>>>(a);
+        else
+            residual_bonds<false><<<blocks_for(g->n_bonds, kThreads), kThreads, 0, st>>>(a);
     }
     ResidualSiteArgs s{g->n_sites, g->inc_ptr, g->inc_bond, wrench, y, mass, r0, fixed, 0.5 * dt * dt,
                        preconditioner, units32, residual, scaled, norms, partials, status, seg_site};
@@ -1627,7 +1641,11 @@ static int mixed_jvp(const dpf_graph *g, float *bond_data, const float *y32, con
                                                                          direction32, units32, d32);
     if (g->n_bonds) {
         JvpArgs a{g->n_bonds, split_bond_data(bond_data, g->n_bonds), y32, d32, wrench, seg_bond, active};
-        jvp_bonds_mixed<<<blocks_for(g->n_bonds, kThreads), kThreads, 0, st>>>(a);
+        const int blocks = blocks_for(g->n_bonds, kJvpThreads);
+        if (pairs_ok(y32, d32))
+            jvp_bonds_mixed<true><<<blocks, kJvpThreads, 0, st>>>(a);
+        else
+            jvp_bonds_mixed<false><<<blocks, kJvpThreads, 0, st>>>(a);
     }
     JvpSiteArgs s{g->n_sites, g->inc_ptr, g->inc_bond, wrench, d32, mass32, preconditioner, units32, fixed,
                   (float)(0.5 * dt * dt), out32 ? nullptr : out, out32};
@@ -1773,10 +1791,15 @@ int dpf::mixed_commit_pass(const dpf_graph *g, float *bond_data, const dpf_histo
         CommitArgs a{g->n_bonds, split_bond_data(bond_data, g->n_bonds), *h, y32, x_end, normal_end, offset_end,
                      fs_end, mb_end, fn_end, mt_end, dloads, reinterpret_cast<float4 *>(corrections)};
         const int blocks = blocks_for(g->n_bonds, kThreads);
-        if (corrections)
-            commit_bonds<true><<<blocks, kThreads, 0, st>>>(a);
+        const bool pairs = pairs_ok(y32);
+        if (corrections && pairs)
+            commit_bonds<true, true><<<blocks, kThreads, 0, st>>>(a);
+        else if (corrections)
+            commit_bonds<true, false><<<blocks, kThreads, 0, st>>>(a);
+        else if (pairs)
+            commit_bonds<false, true><<<blocks, kThreads, 0, st>>>(a);
         else
-            commit_bonds<false><<<blocks, kThreads, 0, st>>>(a);
+            commit_bonds<false, false><<<blocks, kThreads, 0, st>>>(a);
         if (dloads)
             commit_sites<<<blocks_for(kGroupJ * g->n_sites, kThreads), kThreads, 0, st>>>(
                 g->n_sites, g->inc_ptr, g->inc_bond, dloads, loads);

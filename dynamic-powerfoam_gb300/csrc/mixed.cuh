@@ -133,9 +133,40 @@ struct Bond {
     int i, j;
 };
 
+// Loads that keep their place: a bond pass issues its record, then its sites' rows,
+// and only then computes.  Left to the compiler, which moves a load next to its
+// first use to save registers, a bond paid the latency of memory several times.
+__device__ __forceinline__ float4 load4(const float4 *p) {
+    float4 v;
+    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float2 load2(const float *p) {
+    float2 v;
+    asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+
+// Row s of a float32 (N, 6) array; kPairs: the array is aligned to 8 bytes.
+template <bool kPairs>
+__device__ __forceinline__ void load_row(const float *y, int s, V3<float> &u, V3<float> &w) {
+    const float *p = y + 6 * (int64_t)s;
+    if (kPairs) {
+        const float2 a = load2(p), b = load2(p + 2), c = load2(p + 4);
+        u = {a.x, a.y, b.x};
+        w = {b.y, c.x, c.y};
+    } else {
+        u = {__ldg(p), __ldg(p + 1), __ldg(p + 2)};
+        w = {__ldg(p + 3), __ldg(p + 4), __ldg(p + 5)};
+    }
+}
+
 __device__ __forceinline__ Bond load_bond(const Records &R, int64_t b) {
-    const float4 a = __ldg(R.r0 + b), c = __ldg(R.r1 + b), e = __ldg(R.r2 + b), f = __ldg(R.r3 + b);
-    const float4 g = __ldg(R.r4 + b), h = __ldg(R.r5 + b), k = __ldg(R.r6 + b);
+    const float4 k = load4(R.r6 + b);      // the endpoints first: their rows wait for them
+    const float4 a = load4(R.r0 + b), c = load4(R.r1 + b), e = load4(R.r2 + b), f = load4(R.r3 + b);
+    const float4 g = load4(R.r4 + b), h = load4(R.r5 + b);
     Bond o;
     o.n0 = make_float3(a.x, a.y, a.z);
     o.L0 = a.w;
@@ -242,6 +273,72 @@ __device__ __forceinline__ BondIncrement<T> bond_increment(const Bond &B, V3<T> 
     o.dTi = cross(dri, f) + cross(ri_x, o.dF) + dcp;
     o.dTj = -(cross(drj, f) + cross(rj_x, o.dF) + dcp);
     return o;
+}
+
+// acc + a x b, acc - a x b, acc + a . b and acc + s a, each step one FMA
+__device__ __forceinline__ V3<float> cross_add(V3<float> acc, V3<float> a, V3<float> b) {
+    return {fmaf(-a.z, b.y, fmaf(a.y, b.z, acc.x)), fmaf(-a.x, b.z, fmaf(a.z, b.x, acc.y)),
+            fmaf(-a.y, b.x, fmaf(a.x, b.y, acc.z))};
+}
+__device__ __forceinline__ V3<float> cross_sub(V3<float> acc, V3<float> a, V3<float> b) {
+    return cross_add(acc, b, a);
+}
+__device__ __forceinline__ float dot_add(float acc, V3<float> a, V3<float> b) {
+    return fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, acc)));
+}
+__device__ __forceinline__ V3<float> axpy(float s, V3<float> a, V3<float> acc) {
+    return {fmaf(s, a.x, acc.x), fmaf(s, a.y, acc.y), fmaf(s, a.z, acc.z)};
+}
+
+// The derivative of the bond increment in one direction, written out for a
+// committed normal of unit length: ey = u_j - u_i and e, dwi, dwj the direction's
+// share.  The transport is a quaternion (the form of common.cuh's Turn) and what it
+// carries turns with its angular velocity, so the three carried vectors share the
+// derivative; with every operation as a dual number it is twice the instructions.
+// Small terms are summed before the large ones.
+__device__ __forceinline__ void bond_jvp(const Bond &B, V3<float> ey, V3<float> wi, V3<float> wj, V3<float> e,
+                                         V3<float> dwi, V3<float> dwj, V3<float> &F, V3<float> &Ti, V3<float> &Tj) {
+    using F3 = V3<float>;
+    const F3 n0 = lift3<float>(B.n0), dn0 = lift3<float>(B.dn0), nx = n0 + dn0;
+    float length;
+    const F3 dn_x = normal_change(B.L0, nx, 0.5f * ey, length);
+    const F3 turn = dn_x + dn0, n = n0 + turn;
+    const F3 spin = 0.25f * (wi + wj);
+    const float turn2 = dot(turn, turn);
+    const F3 sum = axpy(2.0f, n0, turn);
+    const float r = rsqrtf(4.0f - turn2), half = 0.5f * r * dot(spin, sum);
+    float sh, omc;
+    sin_omc(half, sh, omc);
+    const float ch = 1.0f - omc, rc = r * ch, w = rc * (2.0f - 0.5f * turn2);
+    const F3 v = axpy(r * sh, sum, rc * cross(n0, turn)), v2 = v + v;
+    const auto moved = [&](F3 a) {      // the carried vector minus the vector
+        const F3 x = cross(v2, a);
+        return cross_add(w * x, v, x);
+    };
+    // the normal's derivative and the transport's angular velocity
+    const F3 dd = (0.5f / length) * e, dn = axpy(-dot(n, dd), n, dd);
+    const float sine = 2.0f * sh * ch, versine = 2.0f * sh * sh;
+    const F3 arc = (2.0f * r * r) * cross(sum, dn);
+    const float dth = r * dot_add(fmaf(-(2.0f * half * r), dot(sum, dn), 0.25f * dot(sum, dwi + dwj)), spin, dn);
+    const F3 side = axpy(sine, arc, versine * cross_add(dn, n, arc));
+    const F3 rate = cross_add(axpy(dth, n, axpy(sine, dn, arc)), n, side);
+    // levers
+    const F3 off = lift3<float>(B.off), doff = moved(off), lever = axpy(B.rh, dn_x, doff), ri_x = lift3<float>(B.ri_x);
+    const F3 ri = ri_x + axpy(0.25f, ey, lever), rj = axpy(-B.L0, nx, ri_x) + axpy(-0.25f, ey, lever);
+    const F3 dlever = cross_add(B.rh * dn, rate, off + doff);
+    // relative motion and its derivative
+    const F3 du = cross_sub(cross_add(ey, wj, rj), wi, ri), dw = wj - wi, ddw = dwj - dwi;
+    const F3 ddu = cross_sub(cross_add(cross_sub(cross(dw, dlever), spin, e) + e, dwj, rj), dwi, ri);
+    const float nd = dot(du, n), tw = dot(dw, n);
+    const float dnd = dot_add(dot(du, dn), ddu, n), dtw = dot_add(dot(dw, dn), ddw, n);
+    const float hkn = 0.5f * B.kn, hks = 0.5f * B.ks, hkb = 0.5f * B.kb, hkt = 0.5f * B.kt;
+    const F3 fs0 = lift3<float>(B.fs), mb0 = lift3<float>(B.mb), fs = fs0 + moved(fs0), mb = mb0 + moved(mb0);
+    const float fn = fmaf(hkn, nd, B.fn), mt = fmaf(hkt, tw, B.mt);
+    const F3 f = axpy(fn, n, axpy(hks, axpy(-nd, n, du), fs));
+    F = axpy(hks, ddu, axpy((hkn - hks) * dnd, n, cross_add(fmaf(-hks, nd, fn) * dn, rate, fs)));
+    const F3 couple = axpy(hkb, ddw, axpy((hkt - hkb) * dtw, n, cross_add(fmaf(-hkb, tw, mt) * dn, rate, mb)));
+    Ti = cross_add(cross_add(couple, axpy(0.25f, e, dlever), f), ri, F);
+    Tj = -cross_add(cross_add(couple, axpy(-0.25f, e, dlever), f), rj, F);
 }
 
 }  // namespace mp

@@ -108,3 +108,42 @@ def test_conversions_equal_the_casts():
               None, stream)
     got = host(scaled[torch.arange(n, device='cuda'), at])
     assert np.array_equal(got[number], want[number].astype(np.float64)) and np.isnan(got[~number]).all()
+
+
+@pytest.mark.parametrize('n,m', [(2, 1), (17, 127), (40, 129), (300, 2049)])
+@pytest.mark.parametrize('unit', [True, False])
+@pytest.mark.parametrize('shift', [0, 1])
+def test_float32_jacobian_vector(n, m, unit, shift):
+    """J d of the float32 passes against the float64 product, for committed normals that are unit vectors and
+    not, and for float32 rows aligned to 8 bytes and not (shift).  A bond's wrench takes some 60 roundings of
+    2^-24 to its terms, which a site adds with random signs: 1e-6 of the whole."""
+    import torch
+    import dpf_gb300
+    from dpf_gb300 import _lib
+    rng = np.random.default_rng(n)
+    side = int(np.ceil(n**(1/3)))
+    points = np.stack(np.meshgrid(*[np.arange(side)]*3, indexing='ij'), -1).reshape(-1, 3)[:n] + rng.uniform(-.2, .2, (n, 3))
+    i = rng.integers(0, n, m)
+    pairs = np.stack((i, (i + rng.integers(1, n, m)) % n), 1)
+    given = points[pairs].mean(1) + rng.normal(0, .1, (m, 3))
+    s = dpf_gb300.MixedNewtonBonds(points, rng.uniform(.3, .6, n), pairs, rng.uniform(.5, 1., m),
+                                   rng.uniform(.5, 2., n), np.arange(n) % 5 == 3, contacts=given)
+    for name, shape in (('fn', m), ('mt', m), ('fs', (m, 3)), ('mb', (m, 3))):
+        setattr(s, name, s.tensor(rng.normal(size=shape)))
+    if not unit:
+        s.normal = s.normal*s.tensor(1 + .1*rng.random((m, 1)))
+    dt, y, d = 1e-1, s.tensor(rng.normal(0, .02, (n, 6))), s.tensor(rng.normal(size=(n, 6)))
+    y[s.fixed] = 0.
+    d[s.fixed] = 0.
+    external = torch.zeros_like(y)
+    s._v = s._vec(s.v).clone()
+    s._step_begin(dt, external)
+    s._iteration_residual(y, dt, external)
+    y32, d32 = (torch.empty(6*n + 1, dtype=torch.float32, device=s.device)[shift:shift + 6*n] for _ in range(2))
+    y32.copy_(y.reshape(-1))
+    out = torch.empty_like(y)
+    _lib.call('dpf_mixed_jacobian_vector', ctypes.byref(s._graph), s._bond_data.data_ptr(), y32.data_ptr(),
+              d.data_ptr(), s._mass32.data_ptr(), s.fixed.data_ptr(), dt, None, None, out.data_ptr(), d32.data_ptr(),
+              s._wrench32.data_ptr(), None, None, s._stream())
+    want = dpf_gb300.NewtonBonds.jacobian_vector(s, y, d, dt, external)
+    assert float(torch.linalg.vector_norm(out - want)) <= 1e-6*float(torch.linalg.vector_norm(want))
