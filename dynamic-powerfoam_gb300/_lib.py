@@ -218,8 +218,12 @@ SIGNATURES = {
     'dpf_mixed_commit_lazy': (i32, [P(Graph), vp, vp, vp, vp, vp, vp, vp, vp, vp]),
     'dpf_mixed_fold_history': (i32, [P(Graph), vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]),
     'dpf_newton_struct_sizes': (i32, [P(ctypes.c_int64)]),
+    'dpf_pinned_writable': (i32, [vp]),
     'dpf_arnoldi_cgs2_fused': (i32, [i64, vp, i64, i32, vp, vp, vp, vp, vp, vp]),
     'dpf_adjoint_multiplier': (i32, [i64, vp, vp, vp, vp, vp]),
+    'dpf_adjoint_commit_map': (i32, [i64, f64, vp, vp, vp, vp, vp, vp, vp]),
+    'dpf_adjoint_rhs': (i32, [i64, vp, vp, vp, vp, vp]),
+    'dpf_adjoint_loads': (i32, [i64, f64, vp, vp, vp, vp, vp]),
     'dpf_adjoint_operator': (i32, [P(Graph), vp, vp, vp, vp, vp, f64, vp, vp, vp, vp, vp]),
     'dpf_adjoint_precondition': (i32, [P(Graph), P(Stiffness), P(Tangent), vp, vp, vp, vp, vp, vp, f64, f64, i32,
                                        vp, vp, vp, vp, vp, vp, vp]),
@@ -236,7 +240,8 @@ KERNELS = {
     'dpf_stiffness_apply': 2, 'dpf_diagonal_blocks': 1, 'dpf_prepare_scaling': 1, 'dpf_trial': 2, 'dpf_commit_state': 1,
     'dpf_residual': 2, 'dpf_scale_residual': 1, 'dpf_jacobian_vector': 2, 'dpf_elastic_precondition': 1,
     'dpf_loads': 2, 'dpf_bond_setup': 2, 'dpf_accept_step': 1, 'dpf_energy': 1, 'dpf_arnoldi_cgs2': 4, 'dpf_combine_rows': 1,
-    'dpf_arnoldi_cgs2_fused': 1, 'dpf_adjoint_multiplier': 1, 'dpf_adjoint_operator': 3, 'dpf_adjoint_precondition': 1,
+    'dpf_arnoldi_cgs2_fused': 1, 'dpf_adjoint_multiplier': 1, 'dpf_adjoint_commit_map': 1, 'dpf_adjoint_rhs': 1, 'dpf_adjoint_loads': 1,
+    'dpf_adjoint_operator': 3, 'dpf_adjoint_precondition': 1,
     'dpf_dot_norm': 1, 'dpf_axpby': 1, 'dpf_rhs_scale': 1, 'dpf_masked_scale': 1,
     'dpf_stiffness_apply_static': 2, 'dpf_mixed_setup': 2, 'dpf_mixed_residual': 2, 'dpf_mixed_scaling': 1,
     'dpf_mixed_scale_residual': 1, 'dpf_mixed_jacobian_vector': 3, 'dpf_mixed_stiffness_apply': 2,

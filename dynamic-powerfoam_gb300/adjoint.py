@@ -24,7 +24,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .newton import F64, NewtonBonds, _Krylov, _addr, fgmres
+from .newton import F64, NewtonBonds, _InPlace, _Krylov, _addr, fgmres
 
 STATE_NAMES = ('x', 'v', 'rotation', 'normal', 'offset', 'fn', 'fs', 'mt', 'mb')
 STIFFNESS_NAMES = ('kn', 'ks', 'kb', 'kt')
@@ -220,7 +220,7 @@ class DifferentiableBonds:
         zeros = lambda *shape: torch.zeros(shape, dtype=F64, device=self.device)
         g_v, g_rotation, *g_history = (g if g is not None else None for g in g_final)
         dense = lambda g: g.to(F64).contiguous().clone()
-        g_positions = zeros(steps + 1, n, 3) if g_positions is None else g_positions
+        g_positions = zeros(steps + 1, n, 3) if g_positions is None else g_positions.to(F64).contiguous()
         x_bar = dense(g_positions[steps])
         v_bar = dense(g_v) if g_v is not None else zeros(n, 6)
         r_bar = dense(g_rotation) if g_rotation is not None else zeros(n, 3, 3)
@@ -232,8 +232,8 @@ class DifferentiableBonds:
         jac = torch.empty(max(1, lib.dpf_adjoint_jacobian_doubles(m)), dtype=F64, device=self.device)
         lam = torch.empty((n, 6), dtype=F64, device=self.device)
         krylov = _Krylov(6*n, 32, self.device)
+        y_bar, rhs = torch.empty_like(lam), torch.empty_like(lam)
         half = .5*dt*dt
-        free = (~s.fixed)[:, None].to(F64)
         starts = sorted(checkpoints)
         for c, start in reversed(list(enumerate(starts))):
             stop = starts[c+1] if c+1 < len(starts) else steps
@@ -242,9 +242,10 @@ class DifferentiableBonds:
                 state, y = states[t-start], increments[t]
                 self._set_history(state)
                 # (1) the commit map: x' = x + u, v' = 2y/dt - v, R' = exp(w) R, history' = trial end
-                y_bar = torch.zeros_like(y)
-                y_bar[:, :3] += x_bar
-                y_bar += (2/dt)*v_bar
+                x_next, v_next = torch.empty_like(x_bar), torch.empty_like(v_bar)
+                _lib.check(lib.dpf_adjoint_commit_map(n, dt, x_bar.data_ptr(), v_bar.data_ptr(),
+                                                      g_positions[t].data_ptr(), y_bar.data_ptr(), x_next.data_ptr(),
+                                                      v_next.data_ptr(), stream), 'dpf_adjoint_commit_map')
                 if g_rotation is not None and bool(torch.any(r_bar != 0)):
                     with torch.enable_grad():
                         w = y[:, 3:].clone().requires_grad_(True)
@@ -252,26 +253,25 @@ class DifferentiableBonds:
                         w_bar, = torch.autograd.grad(exp_w@state[2], (w,), r_bar)
                     y_bar[:, 3:] += w_bar
                     r_bar = exp_w.detach().transpose(1, 2)@r_bar
-                x_next, v_next = x_bar.clone(), -v_bar
                 h_next = torch.zeros_like(h_bar)
                 self._vjp(y, None, 0., h_bar, True, h_next, stiff_bar, y_bar, x_next, slots)
-                y_bar *= free
                 # (2) the implicit solve: J^T lam = y_bar on the block-scaled system
                 s.prepare_scaling(s.trial(y, _check=False), dt)
-                self._transposed_solve(y, y_bar, dt, jac, lam, slots, krylov)
+                _lib.check(lib.dpf_adjoint_rhs(n, y_bar.data_ptr(), s.units.data_ptr(), s.fixed.data_ptr(),
+                                               rhs.data_ptr(), stream), 'dpf_adjoint_rhs')
+                self._transposed_solve(y, rhs, dt, jac, lam, slots, krylov)
                 s._raise_status()
-                load_bar[t] = half*lam
-                v_next += dt*s.mass*lam
+                _lib.check(lib.dpf_adjoint_loads(n, dt, s.mass.data_ptr(), lam.data_ptr(), load_bar[t].data_ptr(),
+                                                 v_next.data_ptr(), stream), 'dpf_adjoint_loads')
                 # (3) the residual's direct dependence on history, stiffness and positions
                 self._vjp(y, lam, half, None, False, h_next, stiff_bar, None, x_next, slots)
                 x_bar, v_bar, h_bar = x_next, v_next, h_next
-                x_bar += g_positions[t]
         self._set(stiffness, checkpoints[0])
         normal, offset, fn, fs, mt, mb = (t.contiguous() for t in _unpack_history(h_bar))
         return stiff_bar, load_bar, x_bar, v_bar, r_bar, normal, offset, fn, fs, mt, mb
 
     def _transposed_solve(self, y, rhs, dt, jac, lam, slots, krylov):
-        """lam with J^T lam = rhs (fixed rows zero), solved as (U^-1 P J U)^T mu = U rhs."""
+        """lam with J^T lam = U^-1 rhs (fixed rows zero), solved as (U^-1 P J U)^T mu = rhs."""
         s = self.solver
         lib = self._lib
         stream = s._stream()
@@ -284,7 +284,7 @@ class DifferentiableBonds:
             s._pcg_workspace = torch.empty(lib.dpf_elastic_workspace_doubles(s.n_sites), dtype=F64,
                                            device=self.device)
         units, P = s.units, s.preconditioner
-        out, z = torch.empty_like(rhs), torch.empty_like(rhs)
+        out = torch.empty_like(rhs)
 
         def operator(mu):
             _lib.check(lib.dpf_adjoint_operator(graph, jac.data_ptr(), s.mass.data_ptr(), s.fixed.data_ptr(),
@@ -293,15 +293,14 @@ class DifferentiableBonds:
                        'dpf_adjoint_operator')
             return out
 
-        def precondition(v):
+        def precondition(v, z):
             _lib.check(lib.dpf_adjoint_precondition(
                 graph, stiffness, tangent, s.mass.data_ptr(), s.fixed.data_ptr(), s.block.data_ptr(), P.data_ptr(),
                 units.data_ptr(), v.data_ptr(), float(dt), .03, 80, z.data_ptr(), s._inner.data_ptr(),
                 s._wrench.data_ptr(), s._pcg_workspace.data_ptr(), s._barrier.data_ptr(), s._status.data_ptr(),
                 stream), 'dpf_adjoint_precondition')
-            return z
 
-        mu, info = fgmres(operator, units*rhs, precondition, tolerance=self.adjoint_tolerance, workspace=krylov)
+        mu, info = fgmres(operator, rhs, _InPlace(precondition), tolerance=self.adjoint_tolerance, workspace=krylov)
         self.stats.append(dict(adjoint_krylov=info['iterations'], adjoint_relative=info['relative_residual']))
         _lib.check(lib.dpf_adjoint_multiplier(s.n_sites, P.data_ptr(), units.data_ptr(), mu.data_ptr(),
                                               lam.data_ptr(), stream), 'dpf_adjoint_multiplier')

@@ -530,12 +530,7 @@ extern "C" int dpf_mixed_newton_step(const dpf_mixed_newton *solver, const dpf_n
     double **slots[] = {&run.y, &run.cand, &run.r, &run.r_cand, &run.scaled, &run.rhs, &run.x, &run.res, &run.corr};
     static_assert(sizeof(slots) / sizeof(slots[0]) <= DPF_NEWTON_VECTORS, "vectors of a step");
     for (size_t k = 0; k < sizeof(slots) / sizeof(slots[0]); ++k) *slots[k] = v + (int64_t)k * run.n6;
-    // the address at which the device writes the pinned block
-    void *mapped = nullptr;
-    if (cudaHostGetDevicePointer(&mapped, solver->host, 0) != cudaSuccess || mapped != (void *)solver->host) {
-        cudaGetLastError();
-        return DPF_ERR_ARGUMENT;
-    }
+    if (!dpf_pinned_writable(solver->host)) return DPF_ERR_ARGUMENT;
     run.host = solver->host;
     run.host_int = reinterpret_cast<int *>(solver->host + 96);
     run.cur = {solver->block32, solver->p32, solver->units32, solver->units};

@@ -582,6 +582,13 @@ int arnoldi_pass(int64_t length, double *basis, int64_t ld, int j, double *w, do
 
 extern "C" {
 
+int dpf_pinned_writable(const void *host) {
+    void *mapped = nullptr;
+    if (host && cudaHostGetDevicePointer(&mapped, const_cast<void *>(host), 0) == cudaSuccess) return mapped == host;
+    cudaGetLastError();
+    return 0;
+}
+
 int64_t dpf_newton64_partials_doubles(void) {
     using namespace dpf::newton64;
     return (2 * (int64_t)kMaxColumns + 1) * kMaxBlocks;
@@ -619,12 +626,7 @@ int dpf_newton64_step(const dpf_newton64 *solver, const dpf_newton_step *step, d
     run.m = solver->graph->n_bonds;
     double **slots[DPF_NEWTON64_VECTORS] = {&run.y, &run.cand, &run.r, &run.r_cand, &run.scaled, &run.x, &run.corr};
     for (int k = 0; k < DPF_NEWTON64_VECTORS; ++k) *slots[k] = solver->vectors + (int64_t)k * run.n6;
-    // the address at which the device writes the pinned block
-    void *mapped = nullptr;
-    if (cudaHostGetDevicePointer(&mapped, solver->host, 0) != cudaSuccess || mapped != (void *)solver->host) {
-        cudaGetLastError();
-        return DPF_ERR_ARGUMENT;
-    }
+    if (!dpf_pinned_writable(solver->host)) return DPF_ERR_ARGUMENT;
     run.host = solver->host;
     run.host_int = reinterpret_cast<int *>(solver->host + 96);
     const int rc = run.run();

@@ -754,6 +754,27 @@ class _Krylov:
         self.transformed = torch.empty((width, length), dtype=F64, device=device)
         self.h = torch.zeros(72, dtype=F64, device=device)
 
+    def scratch(self):
+        """Reduction partials, barrier words and pinned results of ``fgmres`` (kept with the workspace)."""
+        kept = self.__dict__.get('_scratch')
+        if kept is None:
+            lib, device = _lib.load(), self.basis.device
+            kept = self._scratch = (torch.zeros(lib.dpf_partials_doubles(), dtype=F64, device=device),
+                                    torch.empty(lib.dpf_newton64_partials_doubles(), dtype=F64, device=device),
+                                    torch.zeros(4, dtype=torch.int32, device=device),
+                                    torch.empty(80, dtype=F64, pin_memory=True))
+            if not lib.dpf_pinned_writable(kept[3].data_ptr()):
+                self._scratch = None
+                raise RuntimeError('pinned memory is not mapped at its host address')
+        return kept
+
+
+class _InPlace:
+    """A preconditioner of ``fgmres`` that writes its result to its second argument."""
+
+    def __init__(self, apply):
+        self.apply = apply
+
 
 class _Krylov32:
     """Float32 Krylov vectors of the mixed Newton path's FGMRES (basis,
@@ -803,50 +824,55 @@ def fgmres(operator, rhs, precondition, tolerance=1e-6, restart=32, max_iteratio
     """
     lib = _lib.load()
     device = rhs.device
-    stream = torch.cuda.current_stream(device).cuda_stream
+    current = torch.cuda.current_stream(device)
+    stream = current.cuda_stream
     shape = rhs.shape
     b = rhs.reshape(-1).to(F64).contiguous()
     length = b.numel()
-    partials = torch.zeros(lib.dpf_partials_doubles(), dtype=F64, device=device)
-    scal = torch.zeros(2, dtype=F64, device=device)
-    arnoldi = torch.empty(lib.dpf_newton64_partials_doubles(), dtype=F64, device=device)
-    barrier = torch.zeros(4, dtype=torch.int32, device=device)
-    host_h = torch.empty(72, dtype=F64, pin_memory=True)
+    ws = workspace
+    if ws is None or ws.length != length or ws.width < min(restart, max_iterations):
+        ws = _Krylov(length, min(restart, max_iterations), device)
+    # the kernels write norms and Hessenberg columns straight to pinned memory
+    partials, arnoldi, barrier, host = ws.scratch()
+    results = host.numpy()
+    in_place = isinstance(precondition, _InPlace)
 
     def norm_of(v):
-        _lib.check(lib.dpf_dot_norm(length, v.data_ptr(), None, scal.data_ptr(), partials.data_ptr(), stream),
+        _lib.check(lib.dpf_dot_norm(length, v.data_ptr(), None, host[72:].data_ptr(), partials.data_ptr(), stream),
                    'dpf_dot_norm')
-        return float(scal[1])
+        current.synchronize()
+        return float(results[73])
 
     norm = norm_of(b) if rhs_norm is None else float(rhs_norm)
     x = torch.zeros_like(b)
     if norm == 0:
         return x.reshape(shape), dict(iterations=0, relative_residual=0.)
-    residual = b.clone(); iterations = 0
+    start, residual, iterations = b, None, 0
     relative = float('nan')
     residual_norm = norm      # the first cycle starts from x = 0
     while iterations < max_iterations:
         width = min(restart, max_iterations - iterations)
-        ws = workspace if (workspace is not None and workspace.width >= width and workspace.length == length) \
-            else _Krylov(length, width, device)
         h = np.zeros((width+1, width)); cs, sn = np.zeros(width), np.zeros(width)
-        g = np.zeros(width+1); g[0] = residual_norm if residual_norm is not None else norm_of(residual)
+        g = np.zeros(width+1); g[0] = residual_norm if residual_norm is not None else norm_of(start)
         residual_norm = None
-        _lib.check(lib.dpf_axpby(length, 1./g[0], residual.data_ptr(), 0., residual.data_ptr(),
+        _lib.check(lib.dpf_axpby(length, 1./g[0], start.data_ptr(), 0., start.data_ptr(),
                                  ws.basis[0].data_ptr(), stream), 'dpf_axpby')
         for j in range(width):
-            z = precondition(ws.basis[j].reshape(shape)).reshape(-1).to(F64).contiguous()
-            _lib.check(lib.dpf_axpby(length, 1., z.data_ptr(), 0., z.data_ptr(), ws.transformed[j].data_ptr(),
-                                     stream), 'dpf_axpby')
-            w = operator(ws.transformed[j].reshape(shape)).reshape(-1).to(F64).contiguous()
-            if w.data_ptr() == ws.transformed[j].data_ptr():
+            row = ws.transformed[j]
+            if in_place:
+                precondition.apply(ws.basis[j], row)
+            else:
+                z = precondition(ws.basis[j].reshape(shape)).reshape(-1).to(F64).contiguous()
+                _lib.check(lib.dpf_axpby(length, 1., z.data_ptr(), 0., z.data_ptr(), row.data_ptr(), stream),
+                           'dpf_axpby')
+            w = operator(row.reshape(shape)).reshape(-1).to(F64).contiguous()
+            if w.data_ptr() == row.data_ptr():
                 w = w.clone()
             _lib.check(lib.dpf_arnoldi_cgs2_fused(length, ws.basis.data_ptr(), length, j, w.data_ptr(),
-                                                  ws.h.data_ptr(), arnoldi.data_ptr(), barrier.data_ptr(),
+                                                  host.data_ptr(), arnoldi.data_ptr(), barrier.data_ptr(),
                                                   barrier[2:].data_ptr(), stream), 'dpf_arnoldi_cgs2_fused')
-            host_h.copy_(ws.h, non_blocking=True)
-            torch.cuda.current_stream(device).synchronize()
-            column = host_h.numpy()
+            current.synchronize()
+            column = results
             h[:j+1, j] = column[:j+1]
             h[j+1, j] = column[j+1]
             breakdown = h[j+1, j] < 1e-14
@@ -865,8 +891,10 @@ def fgmres(operator, rhs, precondition, tolerance=1e-6, restart=32, max_iteratio
                                                 coefficients.ctypes.data_as(ctypes.POINTER(ctypes.c_double)),
                                                 x.data_ptr(), stream), 'dpf_combine_rows')
                 ax = operator(x.reshape(shape)).reshape(-1).to(F64).contiguous()
+                residual = torch.empty_like(b) if residual is None else residual
                 _lib.check(lib.dpf_axpby(length, 1., b.data_ptr(), -1., ax.data_ptr(), residual.data_ptr(), stream),
                            'dpf_axpby')
+                start = residual
                 relative = norm_of(residual)/norm
                 if relative <= 1.05*tolerance:
                     return x.reshape(shape), dict(iterations=iterations, relative_residual=relative)

@@ -237,6 +237,10 @@ int dpf_energy(const dpf_graph *g, const dpf_stiffness *k, const dpf_history *h,
 /* Size in doubles of the reduction partials used by the vector kernels. */
 int64_t dpf_partials_doubles(void);
 
+/* 1 when the device writes pinned host memory at its host address (so that a call's
+ * results may go there directly: dpf_dot_norm, dpf_arnoldi_cgs2_fused), else 0. */
+int dpf_pinned_writable(const void *host);
+
 /* dpf_arnoldi_cgs2 in one cooperative launch: partials
  * dpf_newton64_partials_doubles() doubles, barrier 2 unsigned ints (device,
  * zeroed by the call on its stream); h[j+1] is NaN after a barrier timeout. */
@@ -593,6 +597,18 @@ int dpf_adjoint_local_jacobian(const dpf_graph *g, const dpf_stiffness *k, const
 int dpf_adjoint_apply_jt(const dpf_graph *g, const double *jacobian, const double *mass,
                          const uint8_t *fixed, double dt, const double *lam, double *out,
                          double *slots, void *stream);
+
+/* Site passes of a step's adjoint, (N, 6) arrays unless said otherwise:
+ *   commit_map  y_bar = [x_bar, 0] + (2/dt) v_bar, x_next = x_bar + g, v_next = -v_bar
+ *               (x_bar, g, x_next: (N, 3));
+ *   rhs         rhs = units y_bar, zero rows on fixed sites;
+ *   loads       load_bar = dt^2/2 lam, v_next += dt mass lam. */
+int dpf_adjoint_commit_map(int64_t n_sites, double dt, const double *x_bar, const double *v_bar, const double *g,
+                           double *y_bar, double *x_next, double *v_next, void *stream);
+int dpf_adjoint_rhs(int64_t n_sites, const double *y_bar, const double *units, const uint8_t *fixed, double *rhs,
+                    void *stream);
+int dpf_adjoint_loads(int64_t n_sites, double dt, const double *mass, const double *lam, double *load_bar,
+                      double *v_next, void *stream);
 
 /* The adjoint Krylov solve's system (U^-1 P J U)^T mu = U rhs with U = diag(units),
  * P the 6x6 block inverses of dpf_prepare_scaling:

@@ -167,3 +167,28 @@ def test_fused_arnoldi_step(length, j):
     assert np.abs(h0 - h1).max() <= 1e-12*size and np.abs(w0 - w1).max() <= 1e-12*size
     assert h0[j + 1] > 1e-3*size
     assert np.abs(b0 - b1).max() <= 1e-12*size/h0[j + 1]*10
+
+
+@pytest.mark.parametrize('n', [1, 16, 17, 700])
+def test_adjoint_site_passes(n):
+    """The joined site passes against the same sums in torch (one or two roundings of each: 1e-15)."""
+    import torch
+    from dpf_gb300 import _lib
+    dev, dt = torch.device('cuda'), 3e-3
+    rng = np.random.default_rng(n)
+    t = lambda *s: torch.as_tensor(rng.normal(size=s)).to(dev)
+    x_bar, v_bar, g, units, mass, lam, v = t(n, 3), t(n, 6), t(n, 3), t(n, 6), t(n, 6), t(n, 6), t(n, 6)
+    fixed = torch.as_tensor(np.arange(n) % 3 == 1).to(dev)
+    y_bar, x_next, v_next, rhs, load = (torch.full(s, np.nan, dtype=torch.float64, device=dev)
+                                        for s in ((n, 6), (n, 3), (n, 6), (n, 6), (n, 6)))
+    p, stream = (lambda a: a.data_ptr()), torch.cuda.current_stream(dev).cuda_stream
+    _lib.call('dpf_adjoint_commit_map', n, dt, p(x_bar), p(v_bar), p(g), p(y_bar), p(x_next), p(v_next), stream)
+    want = (2/dt)*v_bar
+    want[:, :3] += x_bar
+    close = lambda a, b: bool((a - b).abs().max() <= 1e-15*b.abs().max())
+    assert close(y_bar, want) and torch.equal(x_next, x_bar + g) and torch.equal(v_next, -v_bar)
+    _lib.call('dpf_adjoint_rhs', n, p(y_bar), p(units), p(fixed), p(rhs), stream)
+    assert torch.equal(rhs, torch.where(fixed[:, None], torch.zeros_like(rhs), units*y_bar))
+    v0 = v.clone()
+    _lib.call('dpf_adjoint_loads', n, dt, p(mass), p(lam), p(load), p(v), stream)
+    assert close(load, .5*dt*dt*lam) and close(v, v0 + dt*mass*lam)
