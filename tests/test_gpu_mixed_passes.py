@@ -147,3 +147,34 @@ def test_float32_jacobian_vector(n, m, unit, shift):
               s._wrench32.data_ptr(), None, None, s._stream())
     want = dpf_gb300.NewtonBonds.jacobian_vector(s, y, d, dt, external)
     assert float(torch.linalg.vector_norm(out - want)) <= 1e-6*float(torch.linalg.vector_norm(want))
+
+
+@pytest.mark.parametrize('m', [2, 5])
+@pytest.mark.parametrize('shift', [1, 2, 4])
+def test_end_pcg_alignment(m, shift):
+    """The PCG's first and last site rows in wide accesses against scalar ones (arrays shifted by floats):
+    the same arithmetic, the same bits."""
+    import torch
+    import dpf_gb300
+    from dpf_gb300 import _lib
+    foam = dpf_gb300.jittered_lattice_foam(m, seed=m)
+    s = dpf_gb300.MixedNewtonBonds(*(foam[k] for k in ('points', 'radii', 'pairs', 'areas', 'masses', 'fixed')),
+                                   young=foam['young'], shear=foam['shear'])
+    load = s.tensor(dpf_gb300.gravity_load(foam)*4.)
+    s.step(2e-3, load, tolerance=1e-6)
+    s._pack_ends(2e-3)
+    n, rng = s.n_sites, np.random.default_rng(m)
+    vector = torch.as_tensor(rng.normal(size=6*n).astype(np.float32)).to(s.device)
+    outs = []
+    for k in (0, shift):
+        place = lambda t: torch.cat((torch.zeros(k, dtype=torch.float32, device=s.device), t.reshape(-1)))[k:]
+        block, units, v = place(s._block32), place(s._units32), place(vector)
+        out = place(torch.zeros_like(vector))
+        s._status.zero_()
+        _lib.call('dpf_end_precondition_f32', ctypes.byref(s._graph), s._ends.data_ptr(), s._site4.data_ptr(),
+                  s.fixed.data_ptr(), block.data_ptr(), s._p24.data_ptr(), units.data_ptr(), v.data_ptr(), .03, 80,
+                  out.data_ptr(), s._inner.data_ptr(), s._tiled_workspace.data_ptr(), s._tiled_partials.data_ptr(),
+                  s._barrier.data_ptr(), s._status.data_ptr(), 0, s._stream())
+        assert int(s._status[0]) == 0
+        outs.append(host(out))
+    assert np.array_equal(*outs) and np.abs(outs[0]).max() > 0
