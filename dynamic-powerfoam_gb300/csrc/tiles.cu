@@ -935,6 +935,75 @@ __device__ __forceinline__ float update_site(const PcgArgs &a, int64_t s, float 
     return dot;
 }
 
+// Site s of the PCG's start: r0 = B (units v), zero on fixed rows.  Site rows in 16- and
+// 8-byte accesses where the caller's arrays allow them (a.wide).
+__device__ __forceinline__ void first_residual(const PcgArgs &a, int64_t s, float rr[6]) {
+    float v[6];
+    if (a.wide) {
+        float in[6];
+        ld6(a.units32 + 6 * s, v);
+        ld6(a.vector32 + 6 * s, in);
+#pragma unroll
+        for (int c = 0; c < 6; ++c) v[c] *= in[c];
+    } else {
+#pragma unroll
+        for (int c = 0; c < 6; ++c)
+            v[c] = a.units32[6 * s + c] * (a.vector32 ? a.vector32[6 * s + c] : (float)a.vector[6 * s + c]);
+    }
+    if (a.fixed[s]) {
+#pragma unroll
+        for (int c = 0; c < 6; ++c) rr[c] = 0.0f;
+    } else if (a.wide) {
+        const float4 *B = reinterpret_cast<const float4 *>(a.block + 36 * s);
+#pragma unroll
+        for (int c = 0; c < 6; ++c) rr[c] = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            const float4 q = __ldg(B + k);
+            rr[4 * k / 6] = fmaf(q.x, v[4 * k % 6], rr[4 * k / 6]);
+            rr[(4 * k + 1) / 6] = fmaf(q.y, v[(4 * k + 1) % 6], rr[(4 * k + 1) / 6]);
+            rr[(4 * k + 2) / 6] = fmaf(q.z, v[(4 * k + 2) % 6], rr[(4 * k + 2) / 6]);
+            rr[(4 * k + 3) / 6] = fmaf(q.w, v[(4 * k + 3) % 6], rr[(4 * k + 3) / 6]);
+        }
+    } else {
+        mv36(a.block + 36 * s, v, rr);
+    }
+}
+
+// Site s of the PCG's result: x / units, and the direction units * (x / units).
+__device__ __forceinline__ void write_solution(const PcgArgs &a, int64_t s, float xv[6]) {
+    float un[6];
+    if (a.wide) {
+        ld6(a.units32 + 6 * s, un);
+#pragma unroll
+        for (int c = 0; c < 6; ++c) xv[c] = xv[c] / un[c];
+        st6(a.out32 + 6 * s, xv);
+        if (a.direction) {
+#pragma unroll
+            for (int c = 0; c < 6; ++c) xv[c] *= un[c];
+            st6(a.direction + 6 * s, xv);
+        }
+        return;
+    }
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+        const float unit = a.units32[6 * s + c], v = xv[c] / unit;
+        if (a.out32)
+            a.out32[6 * s + c] = v;
+        else
+            a.out[6 * s + c] = (double)v;
+        if (a.direction) a.direction[6 * s + c] = v * unit;
+    }
+}
+
+__device__ __forceinline__ void write_zeros(const PcgArgs &a, int64_t e) {
+    if (a.out32)
+        a.out32[e] = 0.0f;
+    else
+        a.out[e] = 0.0;
+    if (a.direction) a.direction[e] = 0.0f;
+}
+
 // kTiles: w = A u by the tiled sweep, else by the bond-end sweep.
 template <bool kTiles, int L>
 __device__ __forceinline__ void pcg_body(PcgArgs &a, unsigned char *smem) {
@@ -943,40 +1012,11 @@ __device__ __forceinline__ void pcg_body(PcgArgs &a, unsigned char *smem) {
     if (a.clear && tid == 0) *a.clear = 0u;
     Pipe P;
     if (kTiles) P = pipe_init(smem, a.L, ((int)blockDim.x - 64) / 32);
-    // r0 = B (units v) with fixed rows zero, u0 = P r0.  Site rows in 16- and 8-byte
-    // accesses where the caller's arrays allow them (a.wide).
+    // r0 and u0 = P r0
     float pf = 0.0f;
     for (int64_t s = tid; s < a.n; s += stride) {
-        float v[6], rr[6], zz[6], Pm[21];
-        if (a.wide) {
-            float in[6];
-            ld6(a.units32 + 6 * s, v);
-            ld6(a.vector32 + 6 * s, in);
-#pragma unroll
-            for (int c = 0; c < 6; ++c) v[c] *= in[c];
-        } else {
-#pragma unroll
-            for (int c = 0; c < 6; ++c)
-                v[c] = a.units32[6 * s + c] * (a.vector32 ? a.vector32[6 * s + c] : (float)a.vector[6 * s + c]);
-        }
-        if (a.fixed[s]) {
-#pragma unroll
-            for (int c = 0; c < 6; ++c) rr[c] = 0.0f;
-        } else if (a.wide) {
-            const float4 *B = reinterpret_cast<const float4 *>(a.block + 36 * s);
-#pragma unroll
-            for (int c = 0; c < 6; ++c) rr[c] = 0.0f;
-#pragma unroll
-            for (int k = 0; k < 9; ++k) {
-                const float4 q = __ldg(B + k);
-                rr[4 * k / 6] = fmaf(q.x, v[4 * k % 6], rr[4 * k / 6]);
-                rr[(4 * k + 1) / 6] = fmaf(q.y, v[(4 * k + 1) % 6], rr[(4 * k + 1) / 6]);
-                rr[(4 * k + 2) / 6] = fmaf(q.z, v[(4 * k + 2) % 6], rr[(4 * k + 2) / 6]);
-                rr[(4 * k + 3) / 6] = fmaf(q.w, v[(4 * k + 3) % 6], rr[(4 * k + 3) / 6]);
-            }
-        } else {
-            mv36(a.block + 36 * s, v, rr);
-        }
+        float rr[6], zz[6], Pm[21];
+        first_residual(a, s, rr);
         sym6(a.P24 + 6 * s, Pm);
         sym_mv6(Pm, rr, zz);
         st6(a.r + 6 * s, rr);
@@ -991,13 +1031,7 @@ __device__ __forceinline__ void pcg_body(PcgArgs &a, unsigned char *smem) {
     double gamma = pair_total(part_b, gridDim.x);
     const double initial = gamma;
     if (initial == 0.0) {
-        for (int64_t e = tid; e < 6 * a.n; e += stride) {
-            if (a.out32)
-                a.out32[e] = 0.0f;
-            else
-                a.out[e] = 0.0;
-            if (a.direction) a.direction[e] = 0.0f;
-        }
+        for (int64_t e = tid; e < 6 * a.n; e += stride) write_zeros(a, e);
         return;
     }
     double alpha_prev = 1.0, gamma_prev = 1.0;
@@ -1046,29 +1080,9 @@ __device__ __forceinline__ void pcg_body(PcgArgs &a, unsigned char *smem) {
         alpha_prev = alpha;
     }
     for (int64_t s = tid; s < a.n; s += stride) {
-        float xv[6], un[6];
+        float xv[6];
         ld6(a.x + 6 * s, xv);
-        if (a.wide) {
-            ld6(a.units32 + 6 * s, un);
-#pragma unroll
-            for (int c = 0; c < 6; ++c) xv[c] = xv[c] / un[c];
-            st6(a.out32 + 6 * s, xv);
-            if (a.direction) {
-#pragma unroll
-                for (int c = 0; c < 6; ++c) xv[c] *= un[c];
-                st6(a.direction + 6 * s, xv);
-            }
-            continue;
-        }
-#pragma unroll
-        for (int c = 0; c < 6; ++c) {
-            const float unit = a.units32[6 * s + c], v = xv[c] / unit;
-            if (a.out32)
-                a.out32[6 * s + c] = v;
-            else
-                a.out[6 * s + c] = (double)v;
-            if (a.direction) a.direction[6 * s + c] = v * unit;
-        }
+        write_solution(a, s, xv);
     }
     if (tid == 0) atomicAdd(a.iterations, it < a.max_it ? it + 1 : a.max_it);
 }
@@ -1076,6 +1090,119 @@ __device__ __forceinline__ void pcg_body(PcgArgs &a, unsigned char *smem) {
 __global__ void __launch_bounds__(kTileThreadsMax + 64, DPF_TILE_MIN_BLOCKS) tiled_pcg_kernel(PcgArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     pcg_body<true, 8>(a, smem);
+}
+
+// The same PCG where every site has its own group of L lanes for the whole launch (n
+// sites in n / (32 / L) warps): the group's first lane keeps r, u, p, s, x and the block
+// inverse in registers, w never leaves it, and only u goes through memory.  An
+// iteration of the loop above at 4k sites is two waits of the grid and four round trips
+// to L2 beside them; this one has two of the four.  Measured there: 9.9 -> 6.8 us an
+// iteration, 67 -> 45 us a launch.
+template <int L>
+__global__ void __launch_bounds__(kEndPcgThreads, 2) end_pcg_small_kernel(PcgArgs a) {
+    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, s = tid / L;
+    const int lane = (int)threadIdx.x & (L - 1);
+    if (a.clear && tid == 0) *a.clear = 0u;
+    const bool valid = s < a.n, head = valid && lane == 0;
+    const bool live = valid && !(a.E.active && !a.E.active[a.E.seg[s]]);
+    const int k0 = live ? a.E.ptr[s] : 0, k1 = live ? a.E.ptr[s + 1] : 0;
+    float r[6], u[6], p[6], sv[6], x[6], Pm[21];
+#pragma unroll
+    for (int c = 0; c < 6; ++c) r[c] = u[c] = p[c] = sv[c] = x[c] = 0.0f;
+    float4 rec = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float pf = 0.0f;
+    if (head) {
+        rec = a.E.site[s];
+        sym6(a.P24 + 6 * s, Pm);
+        first_residual(a, s, r);
+        sym_mv6(Pm, r, u);
+        st6(a.u + 6 * s, u);
+#pragma unroll
+        for (int c = 0; c < 6; ++c) pf = fmaf(r[c], u[c], pf);
+    }
+    float2 *part_a = reinterpret_cast<float2 *>(a.part_a), *part_b = reinterpret_cast<float2 *>(a.part_b);
+    block_pair_partial(pf, part_b);
+    if (!grid_barrier(a.barrier, a.status)) return;
+    double gamma = pair_total(part_b, gridDim.x);
+    const double initial = gamma;
+    if (initial == 0.0) {
+        for (int64_t e = tid; e < 6 * a.n; e += (int64_t)gridDim.x * blockDim.x) write_zeros(a, e);
+        return;
+    }
+    double alpha_prev = 1.0, gamma_prev = 1.0;
+    int it = 0;
+    for (; it < a.max_it; ++it) {
+        float qs[6], acc[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (int c = 0; c < 6; ++c) qs[c] = __shfl_sync(0xffffffffu, u[c], 0, L);
+        for (int k = k0 + lane; k < k1; k += 2 * L) {
+            const int k2 = k + L;
+            const bool two = k2 < k1;
+            // read again every iteration: the records of a small graph stay in L1
+            const float4 e0 = __ldg(a.E.e0 + k), e1 = __ldg(a.E.e1 + k), e2 = __ldg(a.E.e2 + k);
+            float4 f0 = e0, f1 = e1, f2 = e2;
+            if (two) {
+                f0 = __ldg(a.E.e0 + k2);
+                f1 = __ldg(a.E.e1 + k2);
+                f2 = __ldg(a.E.e2 + k2);
+            }
+            float qo[6], qo2[6];
+            load_q<false>(a.u, (int64_t)__float_as_int(e2.w), qo);
+            load_q<false>(a.u, (int64_t)__float_as_int(f2.w), qo2);
+            end_wrench(e0, e1, e2, qs, qo, acc);
+            if (two) end_wrench(f0, f1, f2, qs, qo2, acc);
+        }
+#pragma unroll
+        for (int o = 1; o < L; o <<= 1)
+#pragma unroll
+            for (int c = 0; c < 6; ++c) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+        float w[6], dot = 0.0f;
+        operator_row(rec, u, acc, w);
+        if (head) {
+#pragma unroll
+            for (int c = 0; c < 6; ++c) dot = fmaf(w[c], u[c], dot);
+        }
+        block_pair_partial(dot, part_a);
+        const unsigned old = grid_arrive(a.barrier);
+        __shared__ double shared_ab[2];
+        double beta0 = 0.0, carried = 0.0;
+        if (threadIdx.x == 0 && it > 0) {
+            beta0 = gamma / gamma_prev;
+            carried = beta0 * gamma / alpha_prev;
+        }
+        if (!grid_wait(a.barrier, old, a.status)) return;
+        const double delta = pair_total(part_a, gridDim.x);
+        if (threadIdx.x == 0) {
+            shared_ab[0] = gamma / (delta - carried);
+            shared_ab[1] = beta0;
+        }
+        __syncthreads();
+        const double alpha = shared_ab[0];
+        const float fa = (float)alpha, fb = (float)shared_ab[1];
+        pf = 0.0f;
+        if (head) {
+#pragma unroll
+            for (int c = 0; c < 6; ++c) {
+                p[c] = fmaf(fb, p[c], u[c]);
+                x[c] = fmaf(fa, p[c], x[c]);
+                sv[c] = fmaf(fb, sv[c], w[c]);
+                r[c] = fmaf(-fa, sv[c], r[c]);
+            }
+            sym_mv6(Pm, r, u);
+            st6(a.u + 6 * s, u);
+#pragma unroll
+            for (int c = 0; c < 6; ++c) pf = fmaf(r[c], u[c], pf);
+        }
+        block_pair_partial(pf, part_b);
+        if (!grid_barrier(a.barrier, a.status)) return;
+        const double following = pair_total(part_b, gridDim.x);
+        if (it % 5 == 0 && following <= a.tol2 * initial) break;
+        gamma_prev = gamma;
+        gamma = following;
+        alpha_prev = alpha;
+    }
+    if (head) write_solution(a, s, x);
+    if (tid == 0) atomicAdd(a.iterations, it < a.max_it ? it + 1 : a.max_it);
 }
 
 template <int L, int B>
@@ -1540,10 +1667,29 @@ static int end_precondition(const dpf_graph *g, const float *ends, const float *
         !partials || !barrier || !status || max_iterations < 1 || !aligned16(workspace) || !aligned16(P24) ||
         !aligned16(site4) || (active && !seg_site) || variant < 0 || variant >= kEndVariants)
         return DPF_ERR_ARGUMENT;
-    int grid = 0;
-    const EndPcgKernel kernel = end_pcg_variant(variant);
-    int rc = persistent_grid(kernel, kEndPcgThreads, 0, INT32_MAX, kMaxPcgBlocksTiled, grid, false);
-    if (rc) return rc;
+    int grid = 0, rc;
+    EndPcgKernel kernel = end_pcg_variant(variant);
+    // sites that fit the resident groups of a shape of two blocks an SM: a group a site (8
+    // lanes up to 9728 sites, 4 up to 19456; the autotuner picks the shape).  us an
+    // iteration, looping and not: 4k sites 9.9 and 6.8, 10.6k (4 lanes) 9.9 and 6.3, 17.6k
+    // 14.5 and 8.8
+    bool small = false;
+    if (kEndVariantBlocks[variant] == 2) {
+        const int lanes = kEndVariantLanes[variant];
+        const EndPcgKernel own = lanes == 4 ? end_pcg_small_kernel<4> : end_pcg_small_kernel<8>;
+        const int64_t need = (lanes * g->n_sites + kEndPcgThreads - 1) / kEndPcgThreads;
+        rc = persistent_grid(own, kEndPcgThreads, 0, INT32_MAX, kMaxPcgBlocksTiled, grid, false);
+        if (rc) return rc;
+        if (need <= grid) {
+            kernel = own;
+            grid = (int)need;
+            small = true;
+        }
+    }
+    if (!small) {
+        rc = persistent_grid(kernel, kEndPcgThreads, 0, INT32_MAX, kMaxPcgBlocksTiled, grid, false);
+        if (rc) return rc;
+    }
     const int64_t n6 = 6 * g->n_sites;
     PcgArgs a{};
     a.n = g->n_sites;

@@ -178,3 +178,45 @@ def test_end_pcg_alignment(m, shift):
         assert int(s._status[0]) == 0
         outs.append(host(out))
     assert np.array_equal(*outs) and np.abs(outs[0]).max() > 0
+
+
+@pytest.mark.parametrize('m', [2, 3, 5, 16, 21, 22])
+@pytest.mark.parametrize('masked', [False, True])
+def test_pcg_of_small_graphs(m, masked):
+    """The PCG with a group of lanes a site (the (8, 2) shape up to 9728 sites: 21^3, not 22^3; the (4, 2)
+    shape up to 19456: both) against the looping kernel after six iterations: a float32 operator (2e-6) applied six times, 2e-5; with requests
+    whose ends are skipped."""
+    import torch
+    import dpf_gb300
+    from dpf_gb300 import _lib
+    foam = dpf_gb300.jittered_lattice_foam(m, seed=m)
+    s = dpf_gb300.MixedNewtonBonds(*(foam[k] for k in ('points', 'radii', 'pairs', 'areas', 'masses', 'fixed')),
+                                   young=foam['young'], shear=foam['shear'])
+    load = s.tensor(dpf_gb300.gravity_load(foam)*4.)
+    s.step(2e-3, load, tolerance=1e-6)
+    s._pack_ends(2e-3)
+    n, rng = s.n_sites, np.random.default_rng(m)
+    vector = rng.normal(size=(n, 6))
+    seg = np.zeros(n, np.int32)
+    active = np.ones(2, np.uint8)
+    if masked:        # the second half of the sites frozen: zero rows, ends skipped
+        seg[n//2:] = 1
+        active[1] = 0
+        vector[n//2:] = 0.
+    vector, seg, active = s.tensor(vector), torch.as_tensor(seg).to(s.device), torch.as_tensor(active).to(s.device)
+    outs, counts = [], []
+    for variant in (0, 4, 5):
+        out, inner = torch.full_like(vector, np.nan), torch.zeros(1, dtype=torch.int32, device=s.device)
+        s._status.zero_()
+        _lib.call('dpf_end_precondition', ctypes.byref(s._graph), s._ends.data_ptr(), s._site4.data_ptr(),
+                  s.fixed.data_ptr(), s._block32.data_ptr(), s._p24.data_ptr(), s._units32.data_ptr(),
+                  vector.data_ptr(), 0., 6, out.data_ptr(), inner.data_ptr(), s._tiled_workspace.data_ptr(),
+                  s._tiled_partials.data_ptr(), s._barrier.data_ptr(), s._status.data_ptr(),
+                  seg.data_ptr() if masked else None, active.data_ptr() if masked else None, variant, s._stream())
+        assert int(s._status[0]) == 0
+        outs.append(host(out))
+        counts.append(int(inner[0]))
+    for out, count in zip(outs[1:], counts[1:]):
+        assert counts[0] == count
+        assert np.linalg.norm(outs[0] - out) <= 2e-5*np.linalg.norm(outs[0])
+        assert not masked or not out[n//2:].any()
