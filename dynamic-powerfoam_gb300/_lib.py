@@ -218,6 +218,7 @@ SIGNATURES = {
     'dpf_mixed_commit_lazy': (i32, [P(Graph), vp, vp, vp, vp, vp, vp, vp, vp, vp]),
     'dpf_mixed_fold_history': (i32, [P(Graph), vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]),
     'dpf_newton_struct_sizes': (i32, [P(ctypes.c_int64)]),
+    'dpf_end_variant_for': (i32, [i64]),
     'dpf_pinned_writable': (i32, [vp]),
     'dpf_arnoldi_cgs2_fused': (i32, [i64, vp, i64, i32, vp, vp, vp, vp, vp, vp]),
     'dpf_adjoint_multiplier': (i32, [i64, vp, vp, vp, vp, vp]),

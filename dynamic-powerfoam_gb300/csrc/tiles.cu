@@ -1634,6 +1634,13 @@ static EndGraph end_graph(const dpf_graph *g, const float *ends, const float *si
 
 int dpf_end_variant_count(void) { return kEndVariants; }
 
+// A group of lanes for every site where the grid has one (end_pcg_small_kernel, the
+// fastest there: see end_precondition), the default shape beyond.
+int dpf_end_variant_for(int64_t n_sites) {
+    const int64_t lanes = (int64_t)kSMs * 2 * kEndPcgThreads;
+    return 8 * n_sites <= lanes ? 5 : 4 * n_sites <= lanes ? 4 : 0;
+}
+
 int dpf_end_variant_shape(int variant, int *lanes, int *blocks_per_sm) {
     if (variant < 0 || variant >= kEndVariants) return DPF_ERR_ARGUMENT;
     if (lanes) *lanes = kEndVariantLanes[variant];

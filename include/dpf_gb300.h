@@ -740,6 +740,8 @@ int dpf_end_pack(const dpf_graph *g, const float *bond_data, double alpha, const
  * thread).  Variant 0 (8 lanes, 4 CTAs) is the default; an autotuner may
  * pick another per graph size.  Output pointers may be NULL. */
 int dpf_end_variant_count(void);
+/* Launch shape for a PCG whose shapes are not timed: by the site count alone. */
+int dpf_end_variant_for(int64_t n_sites);
 int dpf_end_variant_shape(int variant, int *lanes, int *blocks_per_sm);
 
 /* y = (diag M + alpha K) q in float32 from the end records; q, y (N, 6)
@@ -851,10 +853,11 @@ int dpf_parallel_loads(const dpf_graph *g, const double *radii, const double *x,
 
 /* ---- native step driver of the mixed-precision Newton solver -------------
  * One implicit step of MixedNewtonBonds.step (bond-end PCG, FGMRES, elastic
- * preconditioning) driven from host code in this library: the same entry
- * points, in the same order, with the same arguments and the same host
+ * preconditioning) driven from host code in this library: the Python control
+ * path's arithmetic on every entry in the same order and the same host
  * decisions (convergence tests, Givens rotations, triangular solve, line
- * search) as the Python control path, so both give bit-identical results.
+ * search), so both give bit-identical results; passes over whole vectors are
+ * joined and results go to pinned memory without copies.
  * Replaces the control flow of NewtonBonds.step and fgmres
  * (experiments/bonded_dem_newton.py:13-60, 132-201).
  *

@@ -220,3 +220,9 @@ def test_pcg_of_small_graphs(m, masked):
         assert counts[0] == count
         assert np.linalg.norm(outs[0] - out) <= 2e-5*np.linalg.norm(outs[0])
         assert not masked or not out[n//2:].any()
+
+
+@pytest.mark.parametrize('n,variant', [(1, 5), (9728, 5), (9729, 4), (19456, 4), (19457, 0), (10**7, 0)])
+def test_shape_by_site_count(n, variant):
+    from dpf_gb300 import _lib
+    assert _lib.load().dpf_end_variant_for(n) == variant
