@@ -1425,9 +1425,9 @@ class MixedNewtonBonds(NewtonBonds):
     sweep = 'ends'
 
     # Drive eligible steps (bond-end sweep, FGMRES, elastic preconditioning, no
-    # overridden hook) from the library's host step driver: the same launches
+    # overridden hook) from the library's host step driver: the same arithmetic
     # and decisions as the Python control path, bit for bit, without Python
-    # between the launches.  False keeps every step on the Python path.
+    # between the launches and with passes over whole vectors joined.  False keeps every step on the Python path.
     native = True
 
     # the hooks the native driver replaces; a subclass that overrides one keeps the Python path
@@ -1516,7 +1516,7 @@ class MixedNewtonBonds(NewtonBonds):
         (``bonded_dem_newton.py:13-60``), except that the true residual's J x
         is sum_k c_k J z_k from the kept products (J is linear; the reference
         applies the operator to x once more, a fourth JVP per two Arnoldi
-        steps).  The library's step driver runs the same launches."""
+        steps).  The library's step driver gives the same bits."""
         lib, stream = self._lib, self._stream()
         n6 = 6*self.n_sites
         ws = self._krylov_workspace32()
