@@ -100,10 +100,11 @@ int end_precondition32_pass(const dpf_graph *g, const float *ends, const float *
 int arnoldi32_pass(int64_t length, float *basis, int64_t ld, int j, const float *v, float *w, double *h,
                    double *partials, unsigned *barrier, unsigned *clear, int *status, cudaStream_t stream);
 
-// The end of a restart cycle: x (+)= sum c_k z_k, the true residual res = -scaled -
-// sum c_k (J z_k) with its norm in norm[1], the Newton correction (units x, zero
-// rows on fixed sites), the full step y + correction and its float32 copy; clears
-// the status word.
+// The end of a restart cycle: x = sum c_k z_k and the true residual res = -scaled -
+// sum c_k (J z_k), or with `add` (a later cycle) x += sum c_k z_k and res -= sum c_k
+// (J z_k); the residual's norm in norm[1], the Newton correction (units x, zero rows
+// on fixed sites), the full step y + correction and its float32 copy; clears the
+// status word.
 int mixed_correction_pass(int64_t n_sites, const float *transformed, const float *products, int count,
                           const double *coefficients, bool add, const double *scaled, const double *units,
                           const uint8_t *fixed, const double *y, double *x, double *res, double *correction,

@@ -502,7 +502,8 @@ __global__ void __launch_bounds__(kThreads) combine32_kernel(int64_t len, const 
 // as eight launches (two row combinations into cleared vectors, the residual and its
 // norm, the masked scaling, the candidate, its float32 copy) that each read and
 // write whole float64 vectors it took 97 us at 262k sites, as one 49 us.  The sums
-// over entries run in dot_norm_kernel's order.
+// over entries run in dot_norm_kernel's order.  The residual is -scaled - J z of the
+// first cycle and from then on the kept residual minus the cycle's own J z.
 struct CorrectionArgs {
     int64_t len;
     const float *z, *jz;
@@ -537,7 +538,7 @@ __global__ void __launch_bounds__(kThreads, kNormResident) correction_kernel(Cor
         }
         double xv = widen(zh) + widen(zl);
         if (a.add) xv += a.x[e];
-        const double rv = -s - (widen(jh) + widen(jl));
+        const double rv = (a.add ? a.res[e] : -s) - (widen(jh) + widen(jl));
         const double c = fx ? 0.0 : __dmul_rn(un, xv), y1 = yv + c;   // rounded as masked_scale_kernel does
         a.x[e] = xv;
         a.res[e] = rv;

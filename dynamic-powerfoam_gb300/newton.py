@@ -1516,7 +1516,8 @@ class MixedNewtonBonds(NewtonBonds):
         (``bonded_dem_newton.py:13-60``), except that the true residual's J x
         is sum_k c_k J z_k from the kept products (J is linear; the reference
         applies the operator to x once more, a fourth JVP per two Arnoldi
-        steps).  The library's step driver gives the same bits."""
+        steps), each cycle's subtracted from the residual it started from.
+        The library's step driver gives the same bits."""
         lib, stream = self._lib, self._stream()
         n6 = 6*self.n_sites
         ws = self._krylov_workspace32()
@@ -1582,7 +1583,7 @@ class MixedNewtonBonds(NewtonBonds):
                     ax = ws.product
                     ax.zero_()
                     self._call('dpf_combine_rows_f32', n6, ws.products.data_ptr(), n6, j+1, c, ax.data_ptr(), stream)
-                    self._call('dpf_axpby', n6, 1., b.data_ptr(), -1., ax.data_ptr(), res.data_ptr(), stream)
+                    self._call('dpf_axpby', n6, 1., start.data_ptr(), -1., ax.data_ptr(), res.data_ptr(), stream)
                     relative = norm_of(res)/norm
                     if relative <= 1.05*tolerance:
                         return x.view(-1, 6), dict(iterations=iterations, relative_residual=relative)
