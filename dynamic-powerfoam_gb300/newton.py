@@ -1161,6 +1161,9 @@ class NewtonBonds(FiniteBonds):
     # Drive eligible steps (FGMRES, no replaced method) from the library's float64
     # step driver; False keeps every step on the Python control path.
     native = True
+    # Store the linearisation (46 doubles a bond, for the duration of a step) that the step's products
+    # J d read; false where it did not fit beside the body, whose products are then formed anew.
+    _native64_linear = True
 
     # what the driver calls itself: a subclass or an instance that replaces one keeps the Python path
     _NATIVE64_HOOKS = ('loads', 'trial', 'commit', 'residual', 'midpoint_force', 'jacobian_vector', '_jvp',
@@ -1198,10 +1201,6 @@ class NewtonBonds(FiniteBonds):
             self._pcg_workspace = e(lib.dpf_elastic_workspace_doubles(n))
         if getattr(self, '_native64_scratch', None) is None:
             self._native64_scratch = (e(_lib.NEWTON64_VECTORS, n, 6), e(2, n, 6), e(lib.dpf_newton64_partials_doubles()))
-            try:
-                self._native64_linear = e(max(1, lib.dpf_newton64_linear_doubles(self.n_bonds)))
-            except torch.cuda.OutOfMemoryError:      # a body that fills the device: products without it
-                self._native64_linear = None
         vectors, pair, partials = self._native64_scratch
         ws = self._krylov
         held = (self.mass, self.fixed, self.radii, self.diagonal, self.block, self.preconditioner, self.units,
@@ -1218,8 +1217,7 @@ class NewtonBonds(FiniteBonds):
             units=p(self.units), wrench=p(self._wrench), workspace=p(self._pcg_workspace), basis=p(ws.basis),
             transformed=p(ws.transformed), w=p(pair[0]), residual=p(pair[1]), h=p(ws.h), krylov_partials=p(partials),
             partials=p(self._partials), scalars=p(self._scalars), status=p(self._status), inner=p(self._inner),
-            barrier=p(self._barrier), vectors=p(vectors), krylov_width=ws.width,
-            linear=_addr(self._native64_linear))
+            barrier=p(self._barrier), vectors=p(vectors), krylov_width=ws.width)
         # the descriptor holds only addresses: keep what they point into alive with it
         self._native64_desc = (key, desc, _lib.NewtonStep(), _lib.NewtonInfo(), held)
         return desc
@@ -1233,13 +1231,26 @@ class NewtonBonds(FiniteBonds):
         n, m = self.n_sites, self.n_bonds
         e = lambda *shape: torch.empty(shape, dtype=F64, device=self.device)
         stiffness = [t.contiguous() for t in (self.kn, self.ks, self.kb, self.kt)]
-        tangent = (e(m, 3), e(m, 3), e(m, 3))
-        state = dict(x=e(n, 3), normal=e(m, 3), fn=e(m), fs=e(m, 3), mt=e(m), mb=e(m, 3), offset=e(m, 3))
-        v, rotation = torch.empty_like(v0), torch.empty_like(r0)
+        # The linearisation goes back to the allocator behind the step: what a gradient or another solver
+        # needs between steps is not held here.  Where it leaves too little for the step's other tensors,
+        # it is left out.
+        for stored in ((True, False) if elastic and self._native64_linear else (False,)):
+            try:
+                linear = e(max(1, self._lib.dpf_newton64_linear_doubles(m))) if stored else None
+                tangent = (e(m, 3), e(m, 3), e(m, 3))
+                state = dict(x=e(n, 3), normal=e(m, 3), fn=e(m), fs=e(m, 3), mt=e(m), mb=e(m, 3), offset=e(m, 3))
+                v, rotation = torch.empty_like(v0), torch.empty_like(r0)
+                break
+            except torch.cuda.OutOfMemoryError:
+                if not stored:
+                    raise
+                linear = tangent = state = None
+                self._native64_linear = False
         desc.stiffness = _lib.Stiffness(*(t.data_ptr() for t in stiffness))
         desc.n, desc.ri, desc.rj = (t.data_ptr() for t in tangent)
         host = _pinned_step_host()
         desc.host, desc.elastic = host.data_ptr(), int(elastic)
+        desc.linear = _addr(linear)
         args.dt, args.external, args.history = dt, external.data_ptr(), history
         args.v, args.rotation, args.v_in, args.rotation_in = \
             v.data_ptr(), rotation.data_ptr(), v0.data_ptr(), r0.data_ptr()
@@ -1251,6 +1262,7 @@ class NewtonBonds(FiniteBonds):
         self._inner_host = 0
         _lib.check(self._lib.dpf_newton64_step(ctypes.byref(desc), ctypes.byref(args), ctypes.byref(info),
                                                self._stream()), 'dpf_newton64_step')
+        linear = desc.linear = None
         _lib.LAUNCHES['count'] += info.launches
         self.n, self.ri, self.rj = tangent
         _raise_outcome(info)
