@@ -1177,7 +1177,8 @@ class NewtonBonds(FiniteBonds):
         # of FGMRES carries the rounding of J x, which the driver's Arnoldi relation does not see
         cls, own = type(self), self.__dict__
         return (self.native and backend == 'fgmres' and preconditioning in ('elastic', 'block') and
-                linear_tolerance >= 1e-12 and 0 <= max_iterations < _lib.NEWTON_TRACE and self.profile is None and
+                linear_tolerance >= 1e-12 and isinstance(max_iterations, (int, np.integer)) and
+                0 <= max_iterations < _lib.NEWTON_TRACE and self.profile is None and
                 own.get('call_profile') is None and self.n_sites > 0 and
                 not any(name in own or getattr(cls, name) is not getattr(NewtonBonds, name)
                         for name in self._NATIVE64_HOOKS))
