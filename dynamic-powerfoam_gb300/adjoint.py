@@ -187,7 +187,7 @@ class DifferentiableBonds:
         for y in increments[:-1]:
             self._set_history(state)
             trial = s.trial(y)
-            # the forward's own accept kernel: replayed states are bit-identical
+            # the arithmetic of the forward's accept kernel (one device function each): the same bits
             v, rotation = state[1].clone(), state[2].contiguous().clone()
             _lib.check(self._lib.dpf_accept_step(s.n_sites, y.data_ptr(), dt, v.data_ptr(), rotation.data_ptr(),
                                                  s._stream()), 'dpf_accept_step')

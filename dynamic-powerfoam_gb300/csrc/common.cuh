@@ -361,6 +361,17 @@ __device__ __forceinline__ void spd_inverse6(const double A[36], double P[36]) {
         }
 }
 
+// The midpoint step's end velocity 2 y / dt - v (bonded_dem_newton.py:150).  Every kernel
+// that accepts a step takes it from here: a step committed again from its increment gives
+// the bits of the first time.
+__device__ __forceinline__ double end_velocity(double two_over_dt, double y, double v) {
+    return fma(two_over_dt, y, -v);
+}
+__device__ __forceinline__ d3 end_velocity(double two_over_dt, d3 y, d3 v) {
+    return {end_velocity(two_over_dt, y.x, v.x), end_velocity(two_over_dt, y.y, v.y),
+            end_velocity(two_over_dt, y.z, v.z)};
+}
+
 // out = exp([w]x) R of one body (bonded_dem_finite_gpu.py:35-43); out may be R.
 __device__ __forceinline__ void rotate_site(d3 w, const double *R, double *out) {
     // Rodrigues coefficients A = sin(a)/a and B = (1 - cos a)/a^2 of a = |w|.

@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(kThreads) accept_kernel(AcceptArgs a) {
         const d3 u = mk(y[0], y[1], y[2]), w = mk(y[3], y[4], y[5]);
         double v[6];
 #pragma unroll
-        for (int c = 0; c < 6; ++c) v[c] = a.two_over_dt * y[c] - a.v[6 * s + c];
+        for (int c = 0; c < 6; ++c) v[c] = end_velocity(a.two_over_dt, y[c], a.v[6 * s + c]);
         st3(a.x_end, s, ld3(a.x, s) + u);
 #pragma unroll
         for (int c = 0; c < 6; ++c) a.v_end[6 * s + c] = v[c];

@@ -165,8 +165,8 @@ __global__ void __launch_bounds__(kThreads) accept_state_kernel(AcceptArgs a) {
     for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < a.n; s += (int64_t)gridDim.x * blockDim.x) {
         const d3 u = ld3(a.y + 6 * s), w = ld3(a.y + 6 * s + 3);
         st3(a.x_end, s, ld3(a.x, s) + u);
-        st3(a.v_end + 6 * s, axpy(a.two_over_dt, u, -ld3(a.v + 6 * s)));
-        st3(a.v_end + 6 * s + 3, axpy(a.two_over_dt, w, -ld3(a.v + 6 * s + 3)));
+        st3(a.v_end + 6 * s, end_velocity(a.two_over_dt, u, ld3(a.v + 6 * s)));
+        st3(a.v_end + 6 * s + 3, end_velocity(a.two_over_dt, w, ld3(a.v + 6 * s + 3)));
         rotate_site(w, a.rotation + 9 * s, a.rotation_end + 9 * s);
         work = dot_add(dot_add(work, ld3(a.external + 6 * s), u), ld3(a.external + 6 * s + 3), w);
         turn = fmax(turn, dot(w, w));

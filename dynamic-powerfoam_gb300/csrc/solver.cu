@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(kThreads) accept_kernel(int64_t n, const doubl
     if (s >= n) return;
     const double two_over_dt = 2.0 / dt;  // one float64 division per site, not six
 #pragma unroll
-    for (int c = 0; c < 6; ++c) v[6 * s + c] = two_over_dt * y[6 * s + c] - v[6 * s + c];
+    for (int c = 0; c < 6; ++c) v[6 * s + c] = end_velocity(two_over_dt, y[6 * s + c], v[6 * s + c]);
     rotate_site(ld3(y + 6 * s + 3), rotation + 9 * s, rotation + 9 * s);
 }
 
