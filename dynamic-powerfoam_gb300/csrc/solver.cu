@@ -524,9 +524,12 @@ __global__ void __launch_bounds__(kThreads, kNormResident) correction_kernel(Cor
     if (blockIdx.x == 0 && threadIdx.x == 0) *a.status = 0;
     __syncthreads();
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    // what the cycle started from: -scaled or the kept residual (the sign off the float64 pipe)
+    const double *start = a.add ? a.res : a.scaled;
+    const long long flip = a.add ? 0ll : (long long)(1ull << 63);
     double aa = 0.0;
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < a.len; e += stride) {
-        const double s = a.scaled[e], un = a.units[e], yv = a.y[e];
+        const double kept = start[e], un = a.units[e], yv = a.y[e];
         const bool fx = a.fixed[e / 6] != 0;
         float zh = 0.0f, zl = 0.0f, jh = 0.0f, jl = 0.0f;
         for (int k = 0; k < a.count; ++k) {
@@ -538,7 +541,7 @@ __global__ void __launch_bounds__(kThreads, kNormResident) correction_kernel(Cor
         }
         double xv = widen(zh) + widen(zl);
         if (a.add) xv += a.x[e];
-        const double rv = (a.add ? a.res[e] : -s) - (widen(jh) + widen(jl));
+        const double rv = __longlong_as_double(__double_as_longlong(kept) ^ flip) - (widen(jh) + widen(jl));
         const double c = fx ? 0.0 : __dmul_rn(un, xv), y1 = yv + c;   // rounded as masked_scale_kernel does
         a.x[e] = xv;
         a.res[e] = rv;
