@@ -3,7 +3,7 @@
 // The per-bond constitutive trial (experiments/bonded_dem_finite_gpu.py:87-116:
 // midpoint wrench and end-of-step history) is differentiated by hand, in
 // reverse: bond_reverse contracts given adjoints of its outputs with its
-// derivative in every input, at about three times the trial's own operations.
+// derivative in every input, at three to four times the trial's own operations.
 //   * dpf_adjoint_bond_vjp returns input adjoints per bond (history,
 //     stiffness) and per site (increment, position; a deterministic incidence
 //     gather) for output adjoints (wrench adjoints from a site vector,
@@ -258,7 +258,7 @@ __device__ __noinline__ void jacobian_rows(const Bond &a, double *B) {
 // B_b (9 x 12, row-major by output) for every bond, bound by the float64 pipe.
 // The wrench depends on u_i and u_j through u_j - u_i alone (three columns,
 // the others their negatives), and on a rotation through its lever and one
-// scalar, the spin angle: about 1,000 operations a bond against twelve
+// scalar, the spin angle: 990 float64 instructions a bond (ncu) against twelve
 // forward-mode passes of the whole trial at 1,200 each.
 // 8k sites / 55k bonds: 978 -> 106 us.
 __global__ void __launch_bounds__(128) local_jacobian_kernel(int64_t m, BondSources s, double *B) {
@@ -453,9 +453,10 @@ struct VjpArgs {
     double *slots;            // (M, 18) written
 };
 
-// One reverse pass of the trial a bond (about 1,000 float64 operations, the
-// float64 pipe's rate) where one forward-mode pass for each of 36 inputs was
-// taken before.  8k sites / 55k bonds: 4.35 ms -> 0.13 ms.
+// One reverse pass of the trial a bond (by ncu 1,210 float64 instructions with
+// end-history adjoints, 740 without, at 85-87% of the float64 pipe) where one
+// forward-mode pass for each of 36 inputs was taken before.  8k sites / 55k bonds:
+// 4.35 ms -> 0.13 ms.
 template <bool kEnd>
 __global__ void __launch_bounds__(128) vjp_kernel(VjpArgs a) {
     const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;

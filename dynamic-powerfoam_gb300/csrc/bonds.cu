@@ -55,9 +55,10 @@ __device__ __noinline__ void carry_general(d3 n0, d3 n1, d3 spin, d3 &a, d3 &b, 
 // comes from one reciprocal root, the transport is a quaternion (make_turn)
 // whose application costs 15 operations, an offset of exactly zero (classical
 // contacts, which every transport keeps at zero) is not rotated, and where the
-// end state is not wanted its guards are tested without forming it: about 240
-// float64 operations against 480 with root, divisions, sincos and rotations
-// written out.  262k sites / 1.9M bonds: 1.50 -> 0.80 ms.
+// end state is not wanted its guards are tested without forming it: 230 to 250
+// float64 instructions (ncu's count; 280 to 310 with the end state) against 480
+// operations with root, divisions, sincos and rotations written out.  262k sites /
+// 1.9M bonds: 1.50 -> 0.79 ms, with the end state 0.96 ms.
 //
 // kLinearise: what jvp_linear_bonds reads, in planes of one double a bond.
 __device__ __forceinline__ void put(const TrialBondArgs &a, int plane, int64_t b, double v) {
@@ -330,9 +331,9 @@ __device__ __noinline__ void carry_jvp_general(d3 n0, d3 n, d3 dn, d3 spin, d3 d
 
 // One thread per bond; bound by the float64 pipe.  A transported vector's
 // derivative is one cross product with the transport's angular velocity
-// (turn_rate), so the three vectors share what the derivative costs: about
-// 370 float64 operations a bond against 770 with every vector's derivative
-// written out.  262k sites / 1.9M bonds: 2.46 -> 1.20 ms; 101k sites with
+// (turn_rate), so the three vectors share what the derivative costs: 380
+// float64 instructions a bond (ncu, given contacts) against 770 with every vector's
+// derivative written out.  262k sites / 1.9M bonds: 2.46 -> 1.20 ms; 101k sites with
 // given contacts: 0.95 -> 0.49 ms.
 __global__ void __launch_bounds__(128) jvp_bonds(JvpBondArgs a) {
     const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -391,12 +392,12 @@ __global__ void __launch_bounds__(128) jvp_bonds(JvpBondArgs a) {
 
 // The same product from the linearisation that the residual pass at y stored:
 // everything that does not depend on the direction (geometry, transport, carried
-// forces, levers, the force itself) is read instead of formed again, about 160
-// float64 operations a bond and 46 coalesced doubles, whose loads hide behind
+// forces, levers, the force itself) is read instead of formed again, 170 float64
+// instructions a bond (ncu) and 46 coalesced doubles, whose loads hide behind
 // them.  With dri = e/4 + dl and drj = -e/4 + dl the spins' share of the relative
 // motion is dw x dl - spin x e.  A step's FGMRES takes two or three of these an
 // iterate for one linearisation (its stores: 5% of the trial pass).
-// 262k sites: 1.20 -> 0.56 ms; a step there 27.3 -> 23.5 ms, at 37k sites 4.5 -> 3.75 ms.
+// 262k sites: 1.20 -> 0.55 ms; a step there 27.0 -> 23.2 ms, at 37k sites 3.72 -> 3.33 ms.
 __global__ void __launch_bounds__(128) jvp_linear_bonds(int64_t m, const int64_t *edges, const double *lin,
                                                         const double *direction, double *wrench) {
     const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;

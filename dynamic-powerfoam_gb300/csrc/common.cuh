@@ -428,8 +428,9 @@ __device__ __forceinline__ void rotate_site(d3 w, const double *R, double *out) 
 // Threads a block for `work` independent items of a float64-bound kernel: the
 // largest of 128, 64 and 32 that still gives every SM four blocks (the float64
 // pipe belongs to the SM, so a few items packed into few blocks leave most
-// pipes idle and an uneven last wave costs whole blocks), else 32.  A step at
-// 512 sites / 3k bonds 1.37 -> 1.33 ms, the adjoint's passes at 8k sites 3%.
+// pipes idle and an uneven last wave costs whole blocks), else 32.  Against blocks
+// of 128 throughout: 3% of a float64 step at 512 sites / 3k bonds (40 us), 3% of the
+// adjoint's passes at 8k sites.
 constexpr int kSMs = 152;
 inline int spread_threads(int64_t work) {
     for (int t = 128; t > 32; t /= 2)

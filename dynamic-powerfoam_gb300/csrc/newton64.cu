@@ -18,8 +18,10 @@
 //   * what the host decides on is written to pinned memory by the kernels.
 // What the host does between launches (about a hundred library calls a step from
 // Python) is a few microseconds here; at 512 sites that was most of a step.
-// A step of two Newton iterations, before and after: 512 sites 3.7 -> 1.4 ms,
-// 37k sites 7.1 -> 4.5 ms, 262k sites 33.9 -> 27.4 ms.
+// A step of two Newton iterations, Python control path and here: 512 sites 3.07
+// and 1.04 ms, 37k sites 5.86 and 3.33 ms, 262k sites 33.2 and 23.2 ms (with the
+// products formed from the state instead of a stored linearisation 1.09, 3.72 and
+// 27.0 ms).
 #include <cmath>
 #include <cstring>
 
@@ -59,9 +61,9 @@ __device__ __forceinline__ void row_totals(const double *part, int count, double
 
 // One cooperative launch with three grid barriers: dot products; projection and
 // the second pass's dot products (a thread reads back only its own elements, so
-// no barrier between them); second projection with |w|^2; normalisation.  As
-// four launches of one pass each: 46 us a step at 37k sites, 98 us at 262k;
-// fused: 36 and 98 us.
+// no barrier between them); second projection with |w|^2; normalisation.  One, two
+// and three rows, as four launches of one pass each (dpf_arnoldi_cgs2) and fused: 37k
+// sites 47, 66, 83 us and 34, 37, 40 us; 262k sites 87, 128, 164 us and 86, 94, 100 us.
 __global__ void __launch_bounds__(kThreads) arnoldi_kernel(ArnoldiArgs a) {
     __shared__ double values[kMaxColumns];
     const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;

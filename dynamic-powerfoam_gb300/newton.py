@@ -919,7 +919,9 @@ class NewtonBonds(FiniteBonds):
         self._krylov = None
         self.block = None
         self.units = None
-        # Optional {name: [(start_event, end_event), ...]} timing of the hot launches.
+        # Optional {name: [(start_event, end_event), ...]} timing of the hot launches.  Float64 steps with
+        # it run on the Python control path, whose launches it times: products from the state, not the
+        # driver's from a stored linearisation.
         self.profile = None
 
     def _timed(self, key, fn):

@@ -150,16 +150,16 @@ int dpf_trial(const dpf_graph *g, const dpf_stiffness *k, const dpf_history *h,
               const double *y, const double *mid_positions, const double *end_positions,
               int want_end, const dpf_trial_out *out, double *wrench, int *status, void *stream);
 
-/* Midpoint residual r = M (y - dt v) - dt^2/2 (f_mid(y) + external), fixed
- * rows r = y, computed with the guards of a full trial; optionally also the
- * scaled residual s = P r / units and, in `norms` (3 doubles, device),
- * [|r|_2, max|s|, |s|_2].  preconditioner/units/scaled may be NULL.
- * Replaces NewtonBonds.residual + scale_residual (experiments/bonded_dem_newton.py:83-86, 104-105). */
 /* The end state of increment y (no positions, no force): the end history of
  * dpf_trial into out's end arrays (each optional), its guards into *status. */
 int dpf_commit_state(const dpf_graph *g, const dpf_stiffness *k, const dpf_history *h, const double *y,
                      const dpf_trial_out *out, int *status, void *stream);
 
+/* Midpoint residual r = M (y - dt v) - dt^2/2 (f_mid(y) + external), fixed
+ * rows r = y, computed with the guards of a full trial; optionally also the
+ * scaled residual s = P r / units and, in `norms` (3 doubles, device),
+ * [|r|_2, max|s|, |s|_2].  preconditioner/units/scaled may be NULL.
+ * Replaces NewtonBonds.residual + scale_residual (experiments/bonded_dem_newton.py:83-86, 104-105). */
 int dpf_residual(const dpf_graph *g, const dpf_stiffness *k, const dpf_history *h,
                  const double *y, const double *v, const double *external, const double *mass,
                  const uint8_t *fixed, double dt, const dpf_trial_out *trial,
@@ -250,6 +250,8 @@ int dpf_arnoldi_cgs2_fused(int64_t length, double *basis, int64_t ld, int j, dou
 /* Twice-iterated classical Gram-Schmidt of w against basis rows 0..j
  * (row stride ld) followed by h[0..j] = projections, h[j+1] = |w|, and, when
  * |w| >= 1e-14, basis row j+1 = w / |w|.  h is a device array of j+2 doubles.
+ * Four plain launches, for callers that cannot launch cooperatively; fgmres and
+ * the step drivers use the fused form.
  * Replaces the Arnoldi body of fgmres (experiments/bonded_dem_newton.py:35-43). */
 int dpf_arnoldi_cgs2(int64_t length, double *basis, int64_t ld, int j, double *w, double *h,
                      double *partials, void *stream);
@@ -791,7 +793,7 @@ int dpf_bond_energy(const dpf_graph *g, const double *base, const double *theta,
                     double *force, double *torque, double *energy, double *wrench, double *partials,
                     void *stream);
 
-/* dpf_bond_energy with a scratch of dpf_energy_site_doubles(N) doubles
+/* dpf_bond_energy (which is for callers without that scratch) with a scratch of dpf_energy_site_doubles(N) doubles
  * (16-byte aligned) for the sites' rotation matrices and stiffness factors,
  * which the bonds otherwise form once an end. */
 int64_t dpf_energy_site_doubles(int64_t n_sites);
@@ -896,7 +898,7 @@ typedef struct dpf_mixed_newton {
     float *basis, *transformed;    /* float32 Krylov vectors (width + 1, 6 N), (width, 6 N) */
     float *products;               /* float32 J z_k of the transformed rows, (width, 6 N) */
     float *w32;                    /* 6 N floats */
-    double *h;                     /* >= width + 2 */
+    double *h;                     /* >= width + 2, not NULL; not used (columns go to `host`) */
     int krylov_width;              /* FGMRES restart length, <= 62 */
     double *krylov_partials;       /* dpf_partials_doubles() */
     double *krylov_scalars;        /* 2 */
@@ -988,7 +990,7 @@ typedef struct dpf_newton64 {
     double *workspace;             /* dpf_elastic_workspace_doubles(N); NULL without elastic */
     double *basis, *transformed;   /* (width + 1, 6 N), (width, 6 N) */
     double *w, *residual;          /* 6 N each */
-    double *h;                     /* >= width + 2 */
+    double *h;                     /* >= width + 2, not NULL; not used (columns go to `host`) */
     double *krylov_partials;       /* dpf_newton64_partials_doubles() */
     double *partials;              /* dpf_partials_doubles() */
     double *scalars;               /* >= 8 */
@@ -998,7 +1000,7 @@ typedef struct dpf_newton64 {
     double *host;                  /* pinned host memory, DPF_NEWTON_HOST_DOUBLES */
     int krylov_width;              /* FGMRES restart length, <= 62 */
     int elastic;                   /* 1: elastic PCG preconditioner, 0: block scaling only */
-    double *linear;                /* dpf_newton64_linear_doubles(M): the linearisation at the last evaluated
+    double *linear;                /* dpf_newton64_linear_doubles(M), used during a step: the linearisation at the evaluated
                                       increment, which a step's Jacobian products read; NULL: they form it anew */
 } dpf_newton64;
 
