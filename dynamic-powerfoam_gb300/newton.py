@@ -1174,11 +1174,13 @@ class NewtonBonds(FiniteBonds):
                        '_newton_operator', '_newton_preconditioner', '_line_merit', '_accept', '_krylov_solve',
                        '_timed', '_call', '_fetch')
 
-    def _native64_ready(self, backend, preconditioning, max_iterations=12, linear_tolerance=1e-6):
+    def _native64_ready(self, backend, preconditioning, max_iterations=12, linear_tolerance=1e-6, tolerances=()):
         # linear tolerances near rounding stay on the Python path: there the true residual
-        # of FGMRES carries the rounding of J x, which the driver's Arnoldi relation does not see
+        # of FGMRES carries the rounding of J x, which the driver's Arnoldi relation does not see.
+        # What is not a number goes there too, to be refused by its comparisons.
         cls, own = type(self), self.__dict__
         return (self.native and backend == 'fgmres' and preconditioning in ('elastic', 'block') and
+                all(isinstance(t, (int, float, np.number, torch.Tensor)) for t in (linear_tolerance, *tolerances)) and
                 linear_tolerance >= 1e-12 and isinstance(max_iterations, (int, np.integer)) and
                 0 <= max_iterations < _lib.NEWTON_TRACE and self.profile is None and
                 own.get('call_profile') is None and self.n_sites > 0 and
@@ -1283,7 +1285,7 @@ class NewtonBonds(FiniteBonds):
         if not np.isfinite(dt) or dt <= 0:
             raise ValueError('Positive finite dt required')
         dt = float(dt)
-        if self._native64_ready(backend, preconditioning, max_iterations, linear_tolerance):
+        if self._native64_ready(backend, preconditioning, max_iterations, linear_tolerance, (tolerance, pose_tolerance)):
             return self._native64_step(dt, external, tolerance, max_iterations, pose_tolerance, linear_tolerance,
                                        preconditioning == 'elastic')
         external = self._vec(external)
