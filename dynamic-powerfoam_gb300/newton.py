@@ -829,9 +829,9 @@ def fgmres(operator, rhs, precondition, tolerance=1e-6, restart=32, max_iteratio
     shape = rhs.shape
     b = rhs.reshape(-1).to(F64).contiguous()
     length = b.numel()
-    ws = workspace
-    if ws is None or ws.length != length or ws.width < min(restart, max_iterations):
-        ws = _Krylov(length, min(restart, max_iterations), device)
+    ws, width = workspace, max(0, min(restart, max_iterations))
+    if ws is None or ws.length != length or ws.width < width:
+        ws = _Krylov(length, width, device)
     # the kernels write norms and Hessenberg columns straight to pinned memory
     partials, arnoldi, barrier, host = ws.scratch()
     results = host.numpy()
