@@ -23,6 +23,7 @@ import torch
 from . import _lib
 
 F64 = torch.float64
+_NUMBERS = (int, float, np.number, torch.Tensor)
 
 
 class SubdivideError(RuntimeError):
@@ -1180,7 +1181,7 @@ class NewtonBonds(FiniteBonds):
         # What is not a number goes there too, to be refused by its comparisons.
         cls, own = type(self), self.__dict__
         return (self.native and backend == 'fgmres' and preconditioning in ('elastic', 'block') and
-                all(isinstance(t, (int, float, np.number, torch.Tensor)) for t in (linear_tolerance, *tolerances)) and
+                isinstance(linear_tolerance, _NUMBERS) and all(isinstance(t, _NUMBERS) for t in tolerances) and
                 linear_tolerance >= 1e-12 and isinstance(max_iterations, (int, np.integer)) and
                 0 <= max_iterations < _lib.NEWTON_TRACE and self.profile is None and
                 own.get('call_profile') is None and self.n_sites > 0 and
@@ -1224,7 +1225,8 @@ class NewtonBonds(FiniteBonds):
             partials=p(self._partials), scalars=p(self._scalars), status=p(self._status), inner=p(self._inner),
             barrier=p(self._barrier), vectors=p(vectors), krylov_width=ws.width)
         # the descriptor holds only addresses: keep what they point into alive with it
-        self._native64_desc = (key, desc, _lib.NewtonStep(), _lib.NewtonInfo(), held)
+        self._native64_desc = (key, desc, _lib.NewtonStep(), _lib.NewtonInfo(), held,
+                               max(1, lib.dpf_newton64_linear_doubles(self.n_bonds)))
         return desc
 
     def _native64_step(self, dt, external, tolerance, max_iterations, pose_tolerance, linear_tolerance, elastic):
@@ -1232,7 +1234,7 @@ class NewtonBonds(FiniteBonds):
         external, v0, r0 = self._vec(external), self._vec(self.v), self._vec(self.rotation)
         history = self._history_struct()
         desc = self._native64_buffers()
-        args, info = self._native64_desc[2:4]
+        _, _, args, info, _, linear_doubles = self._native64_desc
         n, m = self.n_sites, self.n_bonds
         e = lambda *shape: torch.empty(shape, dtype=F64, device=self.device)
         stiffness = [t.contiguous() for t in (self.kn, self.ks, self.kb, self.kt)]
@@ -1241,7 +1243,7 @@ class NewtonBonds(FiniteBonds):
         # it is left out.
         for stored in ((True, False) if elastic and self._native64_linear else (False,)):
             try:
-                linear = e(max(1, self._lib.dpf_newton64_linear_doubles(m))) if stored else None
+                linear = e(linear_doubles) if stored else None
                 tangent = (e(m, 3), e(m, 3), e(m, 3))
                 state = dict(x=e(n, 3), normal=e(m, 3), fn=e(m), fs=e(m, 3), mt=e(m), mb=e(m, 3), offset=e(m, 3))
                 v, rotation = torch.empty_like(v0), torch.empty_like(r0)
